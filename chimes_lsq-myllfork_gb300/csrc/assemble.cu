@@ -23,6 +23,7 @@
 #include <cstdio>
 #include "assemble.h"
 #include "basis.cuh"
+#include "digits.cuh"
 
 namespace cgd {
 
@@ -76,7 +77,8 @@ __device__ void slot_basis(const ModelDev& M, const FramesDev& F, int NB, int f,
 // atom and the stress/energy kernel once more; with these tables the basis is
 // evaluated once per cluster.
 template <int NBODY, typename R>
-__global__ void k_cluster_basis(ModelDev M, FramesDev F, ClusterSet CS, int64_t nq, R* __restrict__ out) {
+__global__ void k_cluster_basis(ModelDev M, FramesDev F, ClusterSet CS, int64_t nq, R* __restrict__ out,
+                                int* __restrict__ lgs) {
     constexpr int NP = NBODY == 3 ? 3 : 6;
     const int ord = NBODY == 3 ? M.order3 : M.order4;
     const int stride = 2 * ord + 4;
@@ -99,6 +101,14 @@ __global__ void k_cluster_basis(ModelDev M, FramesDev F, ClusterSet CS, int64_t 
         slot_basis<R>(M, F, NBODY, f, mm, id, CS.type[q], s, ord, o, o + ord, sb);
         o[2 * ord] = R(sb.r);
         o[2 * ord + 1] = R(sb.rab[0]); o[2 * ord + 2] = R(sb.rab[1]); o[2 * ord + 3] = R(sb.rab[2]);
+        if constexpr (sizeof(R) == 8) {
+            if (lgs) {   // a zero or non-finite distance marks the slot (r_ab / r)
+                int lg = -16384, lh = -16384;
+                for (int n = 0; n < ord; ++n) { lg = max(lg, lg_up(o[n])); lh = max(lh, lg_up(o[ord + n])); }
+                if (!(sb.r > 0.0) || lg_up(sb.r) == LG_BAD) lh = LG_BAD;
+                lgs[t] = (lh << 16) | (lg & 0xffff);
+            }
+        }
     }
 }
 
@@ -917,7 +927,7 @@ __global__ void __launch_bounds__(MB_THREADS, (PPT == 1 && sizeof(R) == 4) ? 2 :
 // Sum the cluster-chunk partials of each (frame, type) in chunk order and write the
 // stress / energy rows (PERM_SCALE and 1/V applied once, at the end).
 template <int NBODY, typename R>
-__global__ void k_virial_reduce(ModelDev M, FramesDev F, Buckets bytype, const int64_t* key_frame_ofs,
+__global__ void k_virial_reduce(ModelDev M, FramesDev F, Buckets bytype, const int64_t* key_frame_ofs, int ncomp,
                                 const R* part, int ntrue_max, int nchunks_max, R* A, int64_t lda) {
     const int ntypes = NBODY == 3 ? M.ntypes3 : M.ntypes4;
     const int f = blockIdx.x / ntypes;
@@ -935,7 +945,8 @@ __global__ void k_virial_reduce(ModelDev M, FramesDev F, Buckets bytype, const i
     for (int col = threadIdx.x; col < CT.n_true; col += blockDim.x) {
         R sv[7] = {0, 0, 0, 0, 0, 0, 0};
         for (int c = 0; c < nch; ++c)
-            for (int k = 0; k < 7; ++k) sv[k] += base[((size_t)c * 7 + k) * ntrue_max + col];
+#pragma unroll
+            for (int k = 0; k < 7; ++k) if (k < ncomp) sv[k] += base[((size_t)c * 7 + k) * ntrue_max + col];
         for (int k = 0; k < 7; ++k) sv[k] = R(sv[k] * perm);
         write_virial_rows(F, f, CT.col_base + col, sv, inv_vol, A, lda);
     }
@@ -1032,14 +1043,14 @@ size_t cluster_basis_count(int nbody, int ord, int64_t nclusters) {
 }
 
 void launch_cluster_basis(int nbody, int prec, int64_t nq, const ModelDev& M, const FramesDev& F,
-                          const ClusterSet& CS, void* basis, cudaStream_t st) {
+                          const ClusterSet& CS, void* basis, int* lgs, cudaStream_t st) {
     const int64_t n = nq * (nbody == 3 ? 3 : 6);
     if (n == 0) return;
     const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, 152 * 64);
-    if (nbody == 3 && prec == 0) k_cluster_basis<3, double><<<blocks, 256, 0, st>>>(M, F, CS, nq, (double*)basis);
-    else if (nbody == 3) k_cluster_basis<3, float><<<blocks, 256, 0, st>>>(M, F, CS, nq, (float*)basis);
-    else if (prec == 0) k_cluster_basis<4, double><<<blocks, 256, 0, st>>>(M, F, CS, nq, (double*)basis);
-    else k_cluster_basis<4, float><<<blocks, 256, 0, st>>>(M, F, CS, nq, (float*)basis);
+    if (nbody == 3 && prec == 0) k_cluster_basis<3, double><<<blocks, 256, 0, st>>>(M, F, CS, nq, (double*)basis, lgs);
+    else if (nbody == 3) k_cluster_basis<3, float><<<blocks, 256, 0, st>>>(M, F, CS, nq, (float*)basis, lgs);
+    else if (prec == 0) k_cluster_basis<4, double><<<blocks, 256, 0, st>>>(M, F, CS, nq, (double*)basis, lgs);
+    else k_cluster_basis<4, float><<<blocks, 256, 0, st>>>(M, F, CS, nq, (float*)basis, lgs);
 }
 
 template <int NBD, typename R>
@@ -1111,25 +1122,39 @@ void launch_force_mb(int nbody, int prec, int ppt, int nreal, size_t smem, const
 }
 
 template <int NBD, typename R, int PPT>
-static void virial_mb_ppt(dim3 grid, unsigned rgrid, size_t smem, const ModelDev& M, const FramesDev& F,
+static void virial_mb_ppt(dim3 grid, size_t smem, const ModelDev& M, const FramesDev& F,
                           const ClusterSet& CS, const Buckets& byt, const int64_t* kfo, int ncomp, const R* pre,
-                          R* part, int ntrue_max, int nchunks_max, R* A, int64_t lda, cudaStream_t st) {
+                          R* part, int ntrue_max, int nchunks_max, cudaStream_t st) {
     set_smem(k_virial_mb<NBD, R, PPT>, smem);
     k_virial_mb<NBD, R, PPT><<<grid, MB_THREADS, smem, st>>>(M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
                                                               nchunks_max);
-    k_virial_reduce<NBD, R><<<rgrid, 256, 0, st>>>(M, F, byt, kfo, part, ntrue_max, nchunks_max, A, lda);
 }
 
 template <int NBD, typename R>
-static void virial_mb_typed(int ppt, dim3 grid, unsigned rgrid, size_t smem, const ModelDev& M, const FramesDev& F,
+static void virial_mb_typed(int ppt, dim3 grid, size_t smem, const ModelDev& M, const FramesDev& F,
                             const ClusterSet& CS, const Buckets& byt, const int64_t* kfo, int ncomp, const void* pre,
-                            void* part, int ntrue_max, int nchunks_max, void* A, int64_t lda, cudaStream_t st) {
+                            void* part, int ntrue_max, int nchunks_max, cudaStream_t st) {
     if (ppt == 1)
-        virial_mb_ppt<NBD, R, 1>(grid, rgrid, smem, M, F, CS, byt, kfo, ncomp, (const R*)pre, (R*)part, ntrue_max,
-                                 nchunks_max, (R*)A, lda, st);
+        virial_mb_ppt<NBD, R, 1>(grid, smem, M, F, CS, byt, kfo, ncomp, (const R*)pre, (R*)part, ntrue_max,
+                                 nchunks_max, st);
     else
-        virial_mb_ppt<NBD, R, VIR_PPT>(grid, rgrid, smem, M, F, CS, byt, kfo, ncomp, (const R*)pre, (R*)part,
-                                       ntrue_max, nchunks_max, (R*)A, lda, st);
+        virial_mb_ppt<NBD, R, VIR_PPT>(grid, smem, M, F, CS, byt, kfo, ncomp, (const R*)pre, (R*)part,
+                                       ntrue_max, nchunks_max, st);
+}
+
+void launch_virial_reduce(int nbody, int prec, int nframes, int ntypes, int ncomp, const ModelDev& M,
+                          const FramesDev& F, const Buckets& byt, const int64_t* kfo, const void* part, int ntrue_max,
+                          int nchunks_max, void* A, int64_t lda, cudaStream_t st) {
+    const unsigned grid = (unsigned)(nframes * ntypes);
+    if (grid == 0) return;
+    if (nbody == 3 && prec == 0)
+        k_virial_reduce<3, double><<<grid, 256, 0, st>>>(M, F, byt, kfo, ncomp, (const double*)part, ntrue_max, nchunks_max, (double*)A, lda);
+    else if (nbody == 3)
+        k_virial_reduce<3, float><<<grid, 256, 0, st>>>(M, F, byt, kfo, ncomp, (const float*)part, ntrue_max, nchunks_max, (float*)A, lda);
+    else if (prec == 0)
+        k_virial_reduce<4, double><<<grid, 256, 0, st>>>(M, F, byt, kfo, ncomp, (const double*)part, ntrue_max, nchunks_max, (double*)A, lda);
+    else
+        k_virial_reduce<4, float><<<grid, 256, 0, st>>>(M, F, byt, kfo, ncomp, (const float*)part, ntrue_max, nchunks_max, (float*)A, lda);
 }
 
 void launch_virial_mb(int nbody, int prec, int ppt, int nframes, int ntypes, int nzchunk, int nchunks_max,
@@ -1137,19 +1162,19 @@ void launch_virial_mb(int nbody, int prec, int ppt, int nframes, int ntypes, int
                       const Buckets& byt, const int64_t* kfo, int ncomp, const void* pre, void* part, void* A,
                       int64_t lda, cudaStream_t st) {
     dim3 grid(nframes * ntypes, nzchunk, nchunks_max);
-    const unsigned rgrid = (unsigned)(nframes * ntypes);
     if (nbody == 3 && prec == 0)
-        virial_mb_typed<3, double>(ppt, grid, rgrid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
-                                   nchunks_max, A, lda, st);
+        virial_mb_typed<3, double>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+                                   nchunks_max, st);
     else if (nbody == 3)
-        virial_mb_typed<3, float>(ppt, grid, rgrid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
-                                  nchunks_max, A, lda, st);
+        virial_mb_typed<3, float>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+                                  nchunks_max, st);
     else if (prec == 0)
-        virial_mb_typed<4, double>(ppt, grid, rgrid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
-                                   nchunks_max, A, lda, st);
+        virial_mb_typed<4, double>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+                                   nchunks_max, st);
     else
-        virial_mb_typed<4, float>(ppt, grid, rgrid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
-                                  nchunks_max, A, lda, st);
+        virial_mb_typed<4, float>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+                                  nchunks_max, st);
+    launch_virial_reduce(nbody, prec, nframes, ntypes, ncomp, M, F, byt, kfo, part, ntrue_max, nchunks_max, A, lda, st);
 }
 
 void launch_max_bucket(const int64_t* key_ofs, const int64_t* kfo, int nframes, int ntypes, int* out,

@@ -128,8 +128,9 @@ void launch_virial2(int prec, int nframes, int nslice, const ModelDev& M, const 
 // Slot bases of every cluster, once per cluster: [cluster][slot][2 ord + 4] values in
 // the form's type (g, h, r, r_ab), read by the force and stress/energy kernels.
 size_t cluster_basis_count(int nbody, int ord, int64_t nclusters);
+// lgs (may be null): per slot lg_up of the largest |g| and |h| (digits.cuh), 16 bits each.
 void launch_cluster_basis(int nbody, int prec, int64_t nclusters, const ModelDev& M, const FramesDev& F,
-                          const ClusterSet& CS, void* basis, cudaStream_t st);
+                          const ClusterSet& CS, void* basis, int* lgs, cudaStream_t st);
 // pre: the cluster bases above, or nullptr to evaluate them in the kernel.  nt4:
 // threads per CTA of the 4-body kernel when it needs more than two powers per thread
 // (MB_THREADS or 2 * MB_THREADS).
@@ -141,6 +142,31 @@ void launch_force_mb(int nbody, int prec, int ppt, int nreal, size_t smem, const
 void launch_force_rg(int nbody, int prec, int nreal, int nt, size_t smem, const ModelDev& M, const FramesDev& F,
                      const ClusterSet& CS, const Buckets& inc, const int64_t* key_frame_ofs, const void* pre,
                      void* A, int64_t lda, cudaStream_t st);
+// Work lists of a call: the cluster bases, their magnitudes (one int per slot), the owners'
+// incidences by cluster type (one entry per incidence: cluster, slot order, exponents) and
+// the (owner, type) groups.
+struct OzWork {
+    OzTables tab;
+    const double* basis;
+    const int* lgs;
+    int* sq;
+    int* sdesc;
+    int* sexp;
+    int4* groups;
+};
+// Whether a model's order and table sizes suit those kernels (FP64 rows).
+bool oz_fits(int nbody, int ord, int max_words);
+void launch_force_oz(int nbody, int nreal, const ModelDev& M, const FramesDev& F, const ClusterSet& CS,
+                     const Buckets& inc, const int64_t* key_frame_ofs, const OzWork& W, double* A, int64_t lda,
+                     cudaStream_t st);
+// Partial sums of the stress / energy rows into part, as launch_virial_mb's.
+void launch_virial_oz(int nbody, int nframes, int ncomp, int nchunks_max, int ntrue_max, const ModelDev& M,
+                      const FramesDev& F, const ClusterSet& CS, const Buckets& byt, const int64_t* key_frame_ofs,
+                      const OzWork& W, double* part, cudaStream_t st);
+// The rows from the partial sums of either form.
+void launch_virial_reduce(int nbody, int prec, int nframes, int ntypes, int ncomp, const ModelDev& M,
+                          const FramesDev& F, const Buckets& byt, const int64_t* key_frame_ofs, const void* part,
+                          int ntrue_max, int nchunks_max, void* A, int64_t lda, cudaStream_t st);
 // Threads per CTA of k_force_rg.  FP64: the multiple of 32 in [max / 2, max] whose
 // ranges of ceil(n / threads) powers leave the fewest idle lanes (which still occupy
 // the FP64 pipe) over the cluster types' allowed-power counts; FP32: the maximum.

@@ -67,6 +67,16 @@ struct ModelDev {
     const int* tcol4;
 };
 
+// Column tables of the digit-product kernels (tensor_rows.cu), one set per cluster list:
+// per owner position, type and column, where the column's powers are staged, two 16-bit
+// places per word, (orbit + 1) / 2 words per column, word-major within a type.
+struct OzTables {
+    const uint32_t* cix = nullptr;
+    const int2* type = nullptr;   // per type: most powers of one column (orbit), first word
+    int ncix = 0;                 // words per owner position
+    int max_words = 0;            // most words of one type
+};
+
 // Canonical slots incident to the member at canonical position pi (nb - 1 of them,
 // k-th returned by role_slot_in) and the other slots (role_slot_out).  Edges of a
 // triplet: 0 = (0,1), 1 = (0,2), 2 = (1,2); of a quadruplet: 0 = (0,1), 1 = (0,2),

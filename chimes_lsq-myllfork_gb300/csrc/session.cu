@@ -46,7 +46,8 @@ static void rev_index(const ClusterType& ct, const int* types, int n, int8_t* ou
 
 static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, int col_base, int pchunk, DeviceModel& D,
                         const int** int_map, const int8_t** pidx, const int8_t** rev, const cgd::ClusterTypeDev** types,
-                        const uint8_t** pows, const int** grps, const uint4** offs, const int** tcols, int& max_allowed) {
+                        const uint8_t** pows, const int** grps, const uint4** offs, const int** tcols, int& max_allowed,
+                        cgd::OzTables& oz) {
     const int np = nb == 3 ? 3 : 6;
     const int dim = nb == 3 ? 1000 : 10000;
     std::vector<int> imap(dim, -1);
@@ -126,6 +127,39 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
             d.lambda[s] = j < m.pairs.size() ? m.pairs[j].lambda : 0.0;
         }
     }
+    // tensor_rows.cu's staged outputs: incident-slot and other-slot powers on grids padded
+    // to 8 powers (3-body, 24 values per incident tuple) or 4 (4-body, 72); absent powers
+    // point behind them
+    const int base = nb == 3 ? 8 : 4, row = nb == 3 ? 24 : 72, none = 64 * row;
+    std::vector<int2> ti;
+    for (const auto& d : tv) {
+        int orbit = 1;
+        for (int k = 0; k < d.n_true; ++k) orbit = std::max(orbit, gp[d.grp_offset + k + 1] - gp[d.grp_offset + k]);
+        ti.push_back(make_int2(orbit, oz.ncix));
+        const int w = (orbit + 1) / 2 * d.n_true;
+        oz.max_words = std::max(oz.max_words, w);
+        oz.ncix += w;
+    }
+    std::vector<uint32_t> cx((size_t)nb * oz.ncix, (uint32_t)none | (uint32_t)none << 16);
+    if (ord <= base)
+        for (int pi = 0; pi < nb; ++pi)
+            for (size_t t = 0; t < tv.size(); ++t) {
+                const cgd::ClusterTypeDev& d = tv[t];
+                for (int c = 0; c < d.n_true; ++c) {
+                    const int p0 = gp[d.grp_offset + c], p1 = gp[d.grp_offset + c + 1];
+                    for (int p = p0; p < p1; ++p) {
+                        const uint8_t* pp = &pw[d.pow_offset + (size_t)p * np];
+                        int ii = 0, oo = 0;
+                        for (int k = nb - 2; k >= 0; --k) ii = ii * base + pp[cgd::role_slot_in(nb, pi, k)];
+                        for (int k = np - nb; k >= 0; --k) oo = oo * base + pp[cgd::role_slot_out(nb, pi, k)];
+                        uint32_t& w = cx[(size_t)pi * oz.ncix + ti[t].y + (size_t)((p - p0) / 2) * d.n_true + c];
+                        const uint32_t v = (uint32_t)(ii * row + oo);
+                        w = (p - p0) % 2 ? (w & 0xffffu) | v << 16 : (w & 0xffff0000u) | v;
+                    }
+                }
+            }
+    oz.cix = dev_upload(D.allocs, cx.data(), cx.size());
+    oz.type = dev_upload(D.allocs, ti.data(), ti.size());
     *int_map = dev_upload(D.allocs, imap.data(), imap.size());
     *pidx = dev_upload(D.allocs, pi.data(), pi.size());
     *rev = dev_upload(D.allocs, rv.data(), rv.size());
@@ -166,10 +200,10 @@ DeviceModel::DeviceModel(const Model& m, int vir_pchunk) {
     d.pairs = dev_upload(allocs, pv.data(), pv.size());
     if (c.use3)
         upload_list(m, m.trips, 3, c.cheby3, d.col3, vir_pchunk, *this, &d.int_map3, &d.pidx3, &d.rev3, &d.types3,
-                    &d.pow3, &d.grp3, &d.offs3, &d.tcol3, max_allowed3);
+                    &d.pow3, &d.grp3, &d.offs3, &d.tcol3, max_allowed3, oz3);
     if (c.use4)
         upload_list(m, m.quads, 4, c.cheby4, d.col4, vir_pchunk, *this, &d.int_map4, &d.pidx4, &d.rev4, &d.types4,
-                    &d.pow4, &d.grp4, &d.offs4, &d.tcol4, max_allowed4);
+                    &d.pow4, &d.grp4, &d.offs4, &d.tcol4, max_allowed4, oz4);
 }
 
 DeviceModel::~DeviceModel() {
@@ -832,6 +866,30 @@ void Session::run(const DeviceFrames& df, int precision, void* A, int64_t lda, A
         cgd::BucketSpec spec2{2, 1, cfo, kfo_types, nullptr, nullptr, nullptr, CS.type};
         cgd::launch_bucket(nf, F, spec2, byt, st); L();
         mark(ST_BUCKET, false);
+        mark(nbody == 3 ? ST_FORCE3 : ST_FORCE4, true);
+        // slot bases once per cluster (the force kernel meets each cluster once per
+        // member, the stress kernel once more); evaluated in place when the fixed
+        // no-allocation scratch is in use or the table would pass kClusterBasisMax
+        void* pre = nullptr;
+        const size_t nbasis = cgd::cluster_basis_count(nbody, ord, nq);
+        const cgd::OzTables& ozt = nbody == 3 ? dm_->oz3 : dm_->oz4;
+        // FP64 rows as digit products on the tensor cores where the order fills their grids and
+        // the slot bases are tabulated, unless a force_range setting names another form.  Of 16
+        // frames of 256 C/H/N/O atoms, range form -> digit products: 4-body force rows 12.6 ->
+        // 7.0 ms, stress and energy 13.3 -> 3.2 ms; 3-body 2.8 -> 2.0 and 3.7 -> 1.4 ms
+        bool tensor = false;
+        cgd::OzWork oz{};
+        if (!S.base && nbasis * rsize <= kClusterBasisMax) {
+            pre = prec == 0 ? (void*)S.get<double>(nbasis) : (void*)S.get<float>(nbasis);
+            tensor = prec == 0 && force_range_ == 1 && cgd::oz_fits(nbody, ord, ozt.max_words);
+            int* lgs = nullptr;
+            if (tensor) {
+                lgs = S.get<int>((size_t)nq * (nbody == 3 ? 3 : 6));
+                oz = cgd::OzWork{ozt, (const double*)pre, lgs, S.get<int>((size_t)nbody * nq), S.get<int>((size_t)nbody * nq),
+                                 S.get<int>((size_t)nbody * nq), S.get<int4>((size_t)nreal * ntypes)};
+            }
+            cgd::launch_cluster_basis(nbody, prec, nq, M, F, CS, pre, lgs, st); L();
+        }
         const int ppt = (max_allowed + cgd::MB_THREADS - 1) / cgd::MB_THREADS;
         const int pp = ppt <= 1 ? 1 : (ppt <= 2 ? 2 : 8);
         // range form in FP64, and in FP32 where a type has more powers than the per-power
@@ -845,29 +903,21 @@ void Session::run(const DeviceFrames& df, int precision, void* A, int64_t lda, A
         }
         const size_t force_smem = range ? cgd::mb_range_smem(nbody, ord, ntypes * 4, rg_nt, rsize).total
                                         : cgd::mb_force_smem(nbody, ord, ntypes * 4, max_allowed, rsize).total;
-        if (!range && ppt > 8) throw Error(2, "too many allowed powers for the device force kernel");
-        if (force_smem > 227 * 1024) throw Error(2, "cluster order too large for the device force kernel");
-        mark(nbody == 3 ? ST_FORCE3 : ST_FORCE4, true);
-        // slot bases once per cluster (the force kernel meets each cluster once per
-        // member, the stress kernel once more); evaluated in place when the fixed
-        // no-allocation scratch is in use or the table would pass kClusterBasisMax
-        void* pre = nullptr;
-        const size_t nbasis = cgd::cluster_basis_count(nbody, ord, nq);
-        if (!S.base && nbasis * rsize <= kClusterBasisMax) {
-            pre = prec == 0 ? (void*)S.get<double>(nbasis) : (void*)S.get<float>(nbasis);
-            cgd::launch_cluster_basis(nbody, prec, nq, M, F, CS, pre, st); L();
-        }
-        if (range)
+        if (!tensor && !range && ppt > 8) throw Error(2, "too many allowed powers for the device force kernel");
+        if (!tensor && force_smem > 227 * 1024) throw Error(2, "cluster order too large for the device force kernel");
+        if (tensor)
+            cgd::launch_force_oz(nbody, nreal, M, F, CS, inc, kfo_atoms, oz, (double*)A, lda, st);
+        else if (range)
             cgd::launch_force_rg(nbody, prec, nreal, rg_nt, force_smem, M, F, CS, inc, kfo_atoms, pre, A, lda, st);
         else
             cgd::launch_force_mb(nbody, prec, pp, nreal, force_smem, M, F, CS, inc, kfo_atoms, pre, A, lda, st,
                                  force4_threads_);
-        L();
+        L(tensor ? 2 : 1);
         mark(nbody == 3 ? ST_FORCE3 : ST_FORCE4, false);
         CK(cudaGetLastError());
         if (virial) {
             cgd::MbVirSmem V = cgd::mb_vir_smem(nbody, ord, cgd::VIR_PPT * cgd::MB_THREADS, rsize);
-            if (V.total > 227 * 1024) throw Error(2, "cluster order too large for the device stress/energy kernel");
+            if (!tensor && V.total > 227 * 1024) throw Error(2, "cluster order too large for the device stress/energy kernel");
             const int maxz = (max_allowed + cgd::VIR_PPT * cgd::MB_THREADS - 1) / (cgd::VIR_PPT * cgd::MB_THREADS) + 1;
             int* d_max = S.get<int>(1);
             CK(cudaMemsetAsync(d_max, 0, sizeof(int), st));
@@ -887,8 +937,15 @@ void Session::run(const DeviceFrames& df, int precision, void* A, int64_t lda, A
                                    : (void*)S.get<float>((size_t)nf * ntypes * nch * 7 * ntrue_max);
             mark(nbody == 3 ? ST_VIRIAL3 : ST_VIRIAL4, true);
             const int vppt = max_allowed <= cgd::MB_THREADS ? 1 : cgd::VIR_PPT;
-            cgd::launch_virial_mb(nbody, prec, vppt, nf, ntypes, std::min(maxz, cgd::MAXCHUNK), nch, ntrue_max, V.total, M, F,
-                                  CS, byt, kfo_types, ncomp, pre, part, A, lda, st); L(2);
+            if (tensor) {
+                cgd::launch_virial_oz(nbody, nf, ncomp, nch, ntrue_max, M, F, CS, byt, kfo_types, oz, (double*)part, st);
+                cgd::launch_virial_reduce(nbody, prec, nf, ntypes, ncomp, M, F, byt, kfo_types, part, ntrue_max, nch, A,
+                                          lda, st);
+            } else {
+                cgd::launch_virial_mb(nbody, prec, vppt, nf, ntypes, std::min(maxz, cgd::MAXCHUNK), nch, ntrue_max, V.total,
+                                      M, F, CS, byt, kfo_types, ncomp, pre, part, A, lda, st);
+            }
+            L(2);
             mark(nbody == 3 ? ST_VIRIAL3 : ST_VIRIAL4, false);
             CK(cudaGetLastError());
         }

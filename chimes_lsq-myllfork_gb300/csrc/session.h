@@ -24,7 +24,8 @@ void cuda_check(cudaError_t e, const char* what);
 struct DeviceModel {
     cgd::ModelDev dev{};
     std::vector<void*> allocs;
-    int max_allowed3 = 0, max_allowed4 = 0;
+    int max_allowed3 = 0, max_allowed4 = 0;   // most allowed powers of a cluster type
+    cgd::OzTables oz3, oz4;
     explicit DeviceModel(const Model& m, int vir_pchunk);
     ~DeviceModel();
     DeviceModel(const DeviceModel&) = delete;
@@ -283,9 +284,10 @@ class Session {
     void set_refine_cache_bytes(int64_t v) { refine_cache_bytes_ = v; }
     // Threads per CTA of the 4-body force kernel (512 or 1024).
     void set_force4_threads(int v) { force4_threads_ = v == 1024 ? 1024 : 512; }
-    // many-body force rows: the range form (k_force_rg) never (0); in FP64, and in FP32
-    // where a cluster type has more allowed powers than MB_THREADS (1, the default);
-    // or always (2); else the per-power form k_force_mb
+    // many-body rows: FP64 digit products (tensor_rows.cu) where oz_fits, else the force rows
+    // by the range form (k_force_rg) in FP64, and in FP32 where a cluster type has more
+    // allowed powers than MB_THREADS (1, the default); always the range form (2); never (0):
+    // the per-power form k_force_mb
     void set_force_range(int v) { force_range_ = v < 0 ? 0 : (v > 2 ? 2 : v); }
     // Cholesky trailing updates by exact BF16 digit products on the tensor cores
     // (FP64-accurate) or by the FP64 SYRK.

@@ -14,7 +14,7 @@
 Each case runs its launch twice after the set-up, so `ncu -k regex:<kernel> -c 1`
 captures a warm launch; the synthetic inputs are seeded.  form=N sets the session's
 force_range tunable (0: the per-power force kernel k_force_mb, 2: the range form
-k_force_rg everywhere; default 1).
+k_force_rg everywhere; default 1: FP64 digit products where they apply).
 """
 import importlib
 import os
