@@ -79,138 +79,202 @@ __global__ void k_frame_setup(FramesDev F, int64_t total_ghosts) {
 }
 
 // ---------------------------------------------------------------- neighbour lists
-// One block of nw warps per real atom (nw = blockDim.x / 32, at most NEIGH_WARPS);
-// warp w scans the w-th contiguous slice of the ghost indices, so the concatenated
-// lists come out in ghost-index order and the fill pass is deterministic.  With
-// several warps the fill pass recounts each slice to place it after the slices
-// before it; batches with many atoms use one warp per atom and skip that.
-constexpr int NEIGH_WARPS = 8;
-
-__global__ void __launch_bounds__(32 * NEIGH_WARPS) k_neigh(ModelDev M, FramesDev F, NeighDev NB, int fill, int nw) {
-    __shared__ int sc[3][NEIGH_WARPS];
-    // nw > 1: one atom per block, nw warps on it; nw == 1: one atom per warp
-    const int atom = nw > 1 ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int w = nw > 1 ? threadIdx.x >> 5 : 0;
-    const int lane = threadIdx.x & 31;
-    if (atom >= NB.n_real) return;
+__device__ __forceinline__ int frame_of_real(const FramesDev& F, int64_t atom) {
     int lo = 0, hi = F.nframes - 1;
     while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
+        const int mid = (lo + hi + 1) >> 1;
         if (F.atom_ofs[mid] <= atom) lo = mid; else hi = mid - 1;
     }
-    const int f = lo;
+    return lo;
+}
+
+// Warps scan the ghosts of the images near a real atom in ghost-index order, 32 at a
+// time, nw warps sharing one atom as contiguous slices of that order, so the lists come
+// out in ghost-index order and the fill pass is deterministic.
+//  * An image of the cell that lies beyond the search radius holds no neighbour: the
+//    cell's bounding box, shifted, is tested once per image.  Ordered lists (i <= parent)
+//    start each image at the atom's own index.
+//  * FP32 distances decide except within MARGIN of a cut-off; the exact FP64 distance,
+//    whose pipe has 1/64 of the rate, is formed there and, in the fill pass, once per
+//    listed ghost with 32 of them side by side.
+// Forming it for every chunk with a candidate in every pass, dividing by the atom count per
+// ghost and scanning all atoms of a near image took 1.37 of the 1.96 ms of an MD force
+// call on frames of 64, 301, 1111 and 2600 atoms (now 0.96 ms in all), and 1.38 of 11.3 ms
+// of the FP64 rows of 32 frames of 384 (now 10.2 ms).
+constexpr int NEIGH_WARPS = 8;
+constexpr int NEIGH_IMG = 1024;   // images tested for reach (four layers); every image is scanned above
+
+template <bool FILL>
+__global__ void __launch_bounds__(32 * NEIGH_WARPS) k_neigh(ModelDev M, FramesDev F, NeighDev NB, int nw) {
+    __shared__ int sc[3][NEIGH_WARPS];
+    __shared__ int sHit[NEIGH_WARPS][64];
+    __shared__ unsigned sNear[NEIGH_WARPS][NEIGH_IMG / 32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int atom = blockIdx.x * (NEIGH_WARPS / nw) + warp / nw;   // nw divides NEIGH_WARPS
+    const int w = warp % nw;
+    const bool on = atom < NB.n_real;
+    int c2 = 0, c3 = 0, c4 = 0;
+    const unsigned lt = (1u << lane) - 1u;
+    // ---- the atom, the near images and the warp's slice of their chunks
+    const int f = on ? frame_of_real(F, atom) : 0;
     const int N = F.natoms[f];
-    const int i = atom - (int)F.atom_ofs[f];
-    const int G = N * F.nimg;
+    const int i = on ? atom - (int)F.atom_ofs[f] : 0;
     const int64_t gbase = F.ghost_ofs[f];
     const BoxDev& B = F.box[f];
     const int* typ = F.type + F.atom_ofs[f];
     const int ti = typ[i];
-    const float4 ci = reinterpret_cast<const float4*>(F.cart32)[gbase + i];
+    const float4* c32 = reinterpret_cast<const float4*>(F.cart32) + gbase;
+    const float4 ci = c32[i];
     const double* si = F.scaled + 3 * (gbase + i);
+    const bool small = B.small != 0;
     const float maxall = (float)fmax(fmax(M.maxcut2, M.order3 > 0 ? M.maxcut3 : 0.0), M.order4 > 0 ? M.maxcut4 : 0.0);
     const float pre = maxall + MARGIN + (float)NB.skin;
-    const int per = ((G + nw - 1) / nw + 31) & ~31;
-    const int g0 = w * per, g1 = min(G, g0 + per);
-    const unsigned lt = (1u << lane) - 1u;
-    // bounding box of the frame's real atoms (the first N ghosts); image k of the
-    // layers is that box shifted by one lattice translation, so an image whose box lies
-    // beyond the search radius of atom i holds none of its neighbours and is skipped
-    // (the lists keep their ghost order: only chunks without neighbours are passed over)
-    const float4* c32 = reinterpret_cast<const float4*>(F.cart32) + gbase;
-    float bmin[3] = {3.0e38f, 3.0e38f, 3.0e38f}, bmax[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-    for (int a = lane; a < N; a += 32) {
-        const float4 c = c32[a];
-        bmin[0] = fminf(bmin[0], c.x); bmin[1] = fminf(bmin[1], c.y); bmin[2] = fminf(bmin[2], c.z);
-        bmax[0] = fmaxf(bmax[0], c.x); bmax[1] = fmaxf(bmax[1], c.y); bmax[2] = fmaxf(bmax[2], c.z);
-    }
-    for (int o = 16; o > 0; o >>= 1)
-        for (int d = 0; d < 3; ++d) {
-            bmin[d] = fminf(bmin[d], __shfl_xor_sync(0xffffffffu, bmin[d], o));
-            bmax[d] = fmaxf(bmax[d], __shfl_xor_sync(0xffffffffu, bmax[d], o));
-        }
+    const float cut3 = M.order3 > 0 ? (float)(M.maxcut3 + NB.skin) : -1.0f;
+    const float cut4 = M.order4 > 0 ? (float)(M.maxcut4 + NB.skin) : -1.0f;
+    const int a0 = small ? 0 : i & ~31;               // ordered lists hold atoms a >= i
+    const int per_image = (N - a0 + 31) >> 5;
+    // images of the cell's bounding box (wrapped atoms lie in the cell) within reach of atom i
     const float reach = pre + 0.05f;   // float rounding of the images' positions stays far below 0.05 A
+    float bmin[3], bmax[3];
+    for (int d = 0; d < 3; ++d) {
+        bmin[d] = bmax[d] = 0.0f;
+        for (int q = 0; q < 3; ++q) {
+            const float h = (float)B.h[3 * d + q];
+            bmin[d] += fminf(h, 0.0f);
+            bmax[d] += fmaxf(h, 0.0f);
+        }
+    }
     const float4 c0 = c32[0];
-    auto image_far = [&](int k) {
-        const float4 ck = c32[(int64_t)k * N];
-        const float s[3] = {ck.x - c0.x, ck.y - c0.y, ck.z - c0.z};
-        const float p[3] = {ci.x, ci.y, ci.z};
-        float d2 = 0.0f;
-        for (int d = 0; d < 3; ++d) {
-            const float lo = bmin[d] + s[d], hi = bmax[d] + s[d];
-            const float e = p[d] < lo ? lo - p[d] : (p[d] > hi ? p[d] - hi : 0.0f);
-            d2 += e * e;
+    unsigned* near = sNear[warp];
+    const bool masked = F.nimg <= NEIGH_IMG;
+    int nnear = masked ? 0 : F.nimg;
+    for (int kb = 0; masked && kb < F.nimg; kb += 32) {
+        const int k = kb + lane;
+        bool in = false;
+        if (k < F.nimg) {
+            const float4 ck = c32[(int64_t)k * N];
+            const float sh[3] = {ck.x - c0.x, ck.y - c0.y, ck.z - c0.z};
+            const float p[3] = {ci.x, ci.y, ci.z};
+            float d2 = 0.0f;
+            for (int d = 0; d < 3; ++d) {
+                const float lo = bmin[d] + sh[d], hi = bmax[d] + sh[d];
+                const float e = p[d] < lo ? lo - p[d] : (p[d] > hi ? p[d] - hi : 0.0f);
+                d2 += e * e;
+            }
+            in = d2 <= reach * reach;
         }
-        return d2 > reach * reach;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (lane == 0) near[kb >> 5] = m;
+        nnear += __popc(m);
+    }
+    __syncwarp();
+    const int total = on ? nnear * per_image : 0;
+    const int t0 = (int)((int64_t)total * w / nw), t1 = (int)((int64_t)total * (w + 1) / nw);
+    auto next_near = [&](int k) {   // the first near image from k on (one exists)
+        if (!masked) return k;
+        int wd = k >> 5;
+        unsigned m = near[wd] & (0xffffffffu << (k & 31));
+        while (m == 0) m = near[++wd];
+        return wd * 32 + __ffs(m) - 1;
     };
-    auto sweep = [&](bool write, int64_t o2, int64_t o3, int64_t o4, int& c2, int& c3, int& c4) {
-        int kseen = -1;
-        bool kfar = false;
-        for (int base = g0; base < g1;) {
-            const int k = base / N;
-            if (k != kseen) { kseen = k; kfar = image_far(k); }
-            if (kfar) {   // warp-uniform: the rest of image k has no neighbour of atom i
-                base = min(g1, (k + 1) * N);
-                continue;
-            }
-            const int g = base + lane;
-            base += 32;
-            bool in2 = false, in3 = false, in4 = false;
-            double r = 0, rab[3] = {0, 0, 0};
-            int pt = 0;
-            if (g < g1 && g != i && (B.small || i <= g % N)) {
-                float4 cg = reinterpret_cast<const float4*>(F.cart32)[gbase + g];
-                float dx = cg.x - ci.x, dy = cg.y - ci.y, dz = cg.z - ci.z;
-                float r32 = sqrtf(dx * dx + dy * dy + dz * dz);
-                if (r32 < pre) {
-                    r = dist_exact(B.h, si, F.scaled + 3 * (gbase + g), rab);
-                    pt = M.int_pair_map[ti * M.natmtyp + typ[g % N]];
-                    const PairDev P = M.pairs[pt];
-                    in2 = M.order2 > 0 && r < P.smax + NB.skin && (NB.md || r > P.smin);
-                    in3 = M.order3 > 0 && r < M.maxcut3 + NB.skin;
-                    in4 = M.order4 > 0 && r < M.maxcut4 + NB.skin;
-                }
-            }
-            const unsigned b2 = __ballot_sync(0xffffffffu, in2);
-            const unsigned b3 = __ballot_sync(0xffffffffu, in3);
-            const unsigned b4 = __ballot_sync(0xffffffffu, in4);
-            if (write) {
-                if (in2) {
-                    const int64_t p = o2 + c2 + __popc(b2 & lt);
-                    NB.i2[p] = i; NB.g2[p] = g; NB.pt2[p] = pt; NB.r2[p] = r;
-                    NB.rab2[3 * p] = rab[0]; NB.rab2[3 * p + 1] = rab[1]; NB.rab2[3 * p + 2] = rab[2];
-                }
-                if (in3) { const int64_t p = o3 + c3 + __popc(b3 & lt); NB.g3[p] = g; NB.r3[p] = r; }
-                if (in4) { const int64_t p = o4 + c4 + __popc(b4 & lt); NB.g4[p] = g; NB.r4[p] = r; }
-            }
-            c2 += __popc(b2); c3 += __popc(b3); c4 += __popc(b4);
-        }
+    auto exact = [&](int g) {
+        double rab[3];
+        return dist_exact(B.h, si, F.scaled + 3 * (gbase + g), rab);
     };
-    int c2 = 0, c3 = 0, c4 = 0;
-    if (nw == 1) {   // single slice per atom: no block-level bookkeeping
-        if (fill) {
-            sweep(true, NB.ofs2[atom], NB.ofs3[atom], NB.ofs4[atom], c2, c3, c4);
+    // lists of ghost g = k N + a of atom i: bits 0..2
+    auto member_of = [&](int g, int a) -> int {
+        const float4 cg = c32[g];
+        const float dx = cg.x - ci.x, dy = cg.y - ci.y, dz = cg.z - ci.z;
+        const float r32 = sqrtf(dx * dx + dy * dy + dz * dz);
+        if (!(r32 < pre)) return 0;
+        const PairDev& P = M.pairs[M.int_pair_map[ti * M.natmtyp + typ[a]]];
+        const float smax = (float)(P.smax + NB.skin), smin = (float)P.smin;
+        const bool edge = fabsf(r32 - smax) <= MARGIN || (!NB.md && fabsf(r32 - smin) <= MARGIN) ||
+                          fabsf(r32 - cut3) <= MARGIN || fabsf(r32 - cut4) <= MARGIN;
+        int fl;
+        if (edge) {
+            const double r = exact(g);
+            fl = (M.order2 > 0 && r < P.smax + NB.skin && (NB.md || r > P.smin) ? 1 : 0) |
+                 (M.order3 > 0 && r < M.maxcut3 + NB.skin ? 2 : 0) | (M.order4 > 0 && r < M.maxcut4 + NB.skin ? 4 : 0);
         } else {
-            sweep(false, 0, 0, 0, c2, c3, c4);
-            if (lane == 0) { NB.cnt2[atom] = c2; NB.cnt3[atom] = c3; NB.cnt4[atom] = c4; }
+            fl = (M.order2 > 0 && r32 < smax && (NB.md || r32 > smin) ? 1 : 0) | (r32 < cut3 ? 2 : 0) |
+                 (r32 < cut4 ? 4 : 0);
         }
-        return;
-    }
-    sweep(false, 0, 0, 0, c2, c3, c4);
-    if (lane == 0) { sc[0][w] = c2; sc[1][w] = c3; sc[2][w] = c4; }
-    __syncthreads();
-    if (!fill) {
-        if (threadIdx.x == 0) {
-            int t2 = 0, t3 = 0, t4 = 0;
-            for (int k = 0; k < nw; ++k) { t2 += sc[0][k]; t3 += sc[1][k]; t4 += sc[2][k]; }
-            NB.cnt2[atom] = t2; NB.cnt3[atom] = t3; NB.cnt4[atom] = t4;
+        return fl;
+    };
+    int64_t o2 = 0, o3 = 0, o4 = 0;
+    int* hit = sHit[warp];
+    auto write = [&](int n) {   // the first n (<= 32) hits: exact distances side by side
+        const int v = lane < n ? hit[lane] : 0;
+        const int fl = lane < n ? (int)((unsigned)v >> 29) : 0, a = v & 8191, g = ((v >> 13) & 65535) * N + a;
+        const unsigned b2 = __ballot_sync(0xffffffffu, fl & 1);
+        const unsigned b3 = __ballot_sync(0xffffffffu, fl & 2);
+        const unsigned b4 = __ballot_sync(0xffffffffu, fl & 4);
+        if (fl) {
+            double rab[3];
+            const double r = dist_exact(B.h, si, F.scaled + 3 * (gbase + g), rab);
+            if (fl & 1) {
+                const int64_t p = o2 + __popc(b2 & lt);
+                NB.i2[p] = i; NB.g2[p] = g; NB.pt2[p] = M.int_pair_map[ti * M.natmtyp + typ[a]]; NB.r2[p] = r;
+                NB.rab2[3 * p] = rab[0]; NB.rab2[3 * p + 1] = rab[1]; NB.rab2[3 * p + 2] = rab[2];
+            }
+            if (fl & 2) { const int64_t p = o3 + __popc(b3 & lt); NB.g3[p] = g; NB.r3[p] = r; }
+            if (fl & 4) { const int64_t p = o4 + __popc(b4 & lt); NB.g4[p] = g; NB.r4[p] = r; }
         }
-        return;
+        o2 += __popc(b2); o3 += __popc(b3); o4 += __popc(b4);
+    };
+    auto sweep = [&](auto&& each) {   // each(lists, a, k) for every chunk of the slice, all lanes
+        if (t0 >= t1) return;
+        const int img = t0 / per_image;
+        int a = a0 + 32 * (t0 - img * per_image);
+        int k = next_near(0);
+        for (int n = 0; n < img; ++n) k = next_near(k + 1);
+        for (int t = t0; t < t1; ++t) {
+            const int al = a + lane, g = k * N + al;
+            const bool cand = al < N && (small || al >= i) && g != i;
+            each(cand ? member_of(g, al) : 0, al, k);
+            a += 32;
+            if (a >= N && t + 1 < t1) { a = a0; k = next_near(k + 1); }
+        }
+    };
+    // ---- count (the fill pass of several warps per atom: to place the slices)
+    if (!FILL || nw > 1) {
+        sweep([&](int fl, int, int) {
+            c2 += __popc(__ballot_sync(0xffffffffu, fl & 1));
+            c3 += __popc(__ballot_sync(0xffffffffu, fl & 2));
+            c4 += __popc(__ballot_sync(0xffffffffu, fl & 4));
+        });
+        if (lane == 0) { sc[0][warp] = c2; sc[1][warp] = c3; sc[2][warp] = c4; }
+        __syncthreads();
+        if (!FILL) {
+            if (on && w == 0 && lane == 0) {
+                int t2 = 0, t3 = 0, t4 = 0;
+                for (int k = warp; k < warp + nw; ++k) { t2 += sc[0][k]; t3 += sc[1][k]; t4 += sc[2][k]; }
+                NB.cnt2[atom] = t2; NB.cnt3[atom] = t3; NB.cnt4[atom] = t4;
+            }
+            return;
+        }
     }
-    int64_t o2 = NB.ofs2[atom], o3 = NB.ofs3[atom], o4 = NB.ofs4[atom];
-    for (int k = 0; k < w; ++k) { o2 += sc[0][k]; o3 += sc[1][k]; o4 += sc[2][k]; }
-    int d2 = 0, d3 = 0, d4 = 0;
-    sweep(true, o2, o3, o4, d2, d3, d4);
+    if (!on) return;
+    o2 = NB.ofs2[atom]; o3 = NB.ofs3[atom]; o4 = NB.ofs4[atom];
+    for (int k = warp - w; k < warp; ++k) { o2 += sc[0][k]; o3 += sc[1][k]; o4 += sc[2][k]; }
+    int pend = 0;
+    sweep([&](int fl, int a, int k) {
+        const unsigned b = __ballot_sync(0xffffffffu, fl != 0);
+        if (fl) hit[pend + __popc(b & lt)] = a | (k << 13) | (fl << 29);
+        pend += __popc(b);
+        __syncwarp();
+        if (pend >= 32) {
+            write(32);
+            __syncwarp();
+            const int rest = lane < pend - 32 ? hit[32 + lane] : 0;
+            __syncwarp();
+            if (lane < pend - 32) hit[lane] = rest;
+            pend -= 32;
+            __syncwarp();
+        }
+    });
+    write(pend);
 }
 
 // ---------------------------------------------------------------- binned neighbour lists
@@ -641,12 +705,14 @@ void launch_frame_setup(const FramesDev& F, int64_t n, cudaStream_t st) {
     if (n > 0) k_frame_setup<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(F, n);
 }
 void launch_neigh(const ModelDev& M, const FramesDev& F, const NeighDev& NB, int fill, cudaStream_t st) {
-    // enough atoms to fill the GPU with one warp each: one warp per atom
     if (NB.n_real <= 0) return;
-    if (NB.n_real >= 32768)
-        k_neigh<<<(unsigned)((NB.n_real + NEIGH_WARPS - 1) / NEIGH_WARPS), 32 * NEIGH_WARPS, 0, st>>>(M, F, NB, fill, 1);
-    else
-        k_neigh<<<(unsigned)NB.n_real, 32 * NEIGH_WARPS, 0, st>>>(M, F, NB, fill, NEIGH_WARPS);
+    // about 16 warps per SM: eight warps on an atom of a small batch, one where the atoms
+    // alone fill the GPU
+    int nw = NEIGH_WARPS;
+    while (nw > 1 && (int64_t)NB.n_real * nw > 2 * 2432) nw >>= 1;
+    const unsigned blocks = (unsigned)((NB.n_real + NEIGH_WARPS / nw - 1) / (NEIGH_WARPS / nw));
+    if (fill) k_neigh<true><<<blocks, 32 * NEIGH_WARPS, 0, st>>>(M, F, NB, nw);
+    else k_neigh<false><<<blocks, 32 * NEIGH_WARPS, 0, st>>>(M, F, NB, nw);
 }
 void launch_bins(const FramesDev& F, int64_t n, const Bins& B, cudaStream_t st) {
     if (n <= 0) return;
