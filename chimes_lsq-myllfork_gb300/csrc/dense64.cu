@@ -13,6 +13,7 @@
 #include <string>
 
 #include "dense64.h"
+#include "digits.cuh"
 #include "gram.h"
 
 namespace cgd {
@@ -91,6 +92,146 @@ __global__ void __launch_bounds__(SY_THREADS) k_syrk_tn(const double* __restrict
             }
         }
     }
+}
+
+// ---------------------------------------------------------------- X^T X as digit products
+// The same triangle with FP64 accuracy from the tensor cores (digits.cuh): column i is
+// scaled by a power of two, its entries split into eight base-256 digits, and a 64 x 64
+// tile's 36 digit products per term are summed exactly and packed every 32 rows into
+// 64-bit integers; one conversion and one addition to C per output and K slice.  In units
+// of the two columns' largest entries a term loses at most 2^-62 to rounding and 2^-59 to
+// the dropped diagonals and every 32 rows 16 * 2^-(57 + up) (up = 9 - log2 of the slice's
+// rows); an FP64 sum loses up to 2^-53 of the partial sum with every row.
+// Sixteen warps of 16 rows x 16 columns; the next 16 rows' digits are built while warps that
+// have finished theirs run the current products.  The tensor pipe is the bound (36
+// products per multiply-add on mma.sync, 606 TFLOP/s measured, or 13.9 TFLOP/s of FP64
+// arithmetic).  30,001 x 820 (with h and the
+// mirror): 19.5 -> 3.7 ms; 2,000 x 6,007: 60.2 -> 11.6 ms; against a double-double
+// reference the norm of the error is 1.0e-16 of G's (FP64 sums: 4.4e-16).
+constexpr int GD_T = 64, GD_THREADS = 512, GD_ROWS = 16;
+constexpr uint32_t GD_CHUNK = 2 * GD_T * DIG_STRIDE;   // 8 rows of K
+constexpr uint32_t GD_BUF = 2 * GD_CHUNK;
+
+// ex[i] <- the least e with |X[k][i]| <= 0.996 2^e for all k, so that the leading digit is
+// at most 127 (ex preset to a very small value; COL_BAD for infinities and NaN).
+constexpr int COL_BAD = 4096;
+__device__ __forceinline__ int col_exponent(double x) {
+    const int h = __double2hiint(x) & 0x7fffffff;
+    return h >= 0x7ff00000 ? COL_BAD : (h >> 20) - 1022 + ((h & 0xfffff) >= 0xfe000 ? 1 : 0);
+}
+__global__ void __launch_bounds__(256) k_col_exponents(const double* __restrict__ X, int64_t ldx, int64_t K, int m,
+                                                int* __restrict__ ex) {
+    const int c = blockIdx.x * 32 + (threadIdx.x & 31);
+    if (c >= m) return;
+    const int64_t step = (int64_t)gridDim.y * 8;
+    int lg = -1022;
+    int64_t k = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
+    for (; k + 3 * step < K; k += 4 * step) {   // four loads in flight
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = X[(k + u * step) * ldx + c];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) lg = max(lg, col_exponent(v[u]));
+    }
+    for (; k < K; k += step) lg = max(lg, col_exponent(X[k * ldx + c]));
+    atomicMax(ex + c, lg);
+}
+
+template <bool ATOMIC>
+__global__ void __launch_bounds__(GD_THREADS, 1) k_syrk_digits(const double* __restrict__ X, int64_t ldx, int64_t K,
+                                                               int m, double* __restrict__ C, int64_t ldc, int ntile,
+                                                               int64_t kslice, const int* __restrict__ ex) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    int ti, tj;
+    upper_pair(blockIdx.x, ntile, ti, tj);
+    const bool diag = ti == tj;
+    const int64_t kb = (int64_t)blockIdx.y * kslice, ke = min(K, kb + kslice);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // digits: a warp has 8 columns (of tile ti, then tj), a lane one column and the row pairs
+    // p and p + 4 of the 16, so that the 32 stores of a digit fall into different banks
+    const int dc = warp * 8 + (lane >> 2), p = lane & 3;
+    const int col = (dc < GD_T ? ti * GD_T + dc : tj * GD_T + dc - GD_T);
+    const bool builds = !(diag && dc >= GD_T);
+    const bool in = builds && col < m;
+    const int sh = in ? DIG_FIX - ex[col] : 0;
+    double v[4];
+    auto fetch = [&](int64_t k0) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t k = k0 + 2 * p + (u & 1) + 8 * (u >> 1);
+            v[u] = in && k < ke ? X[k * ldx + col] : 0.0;
+        }
+    };
+    auto build = [&](int buf) {
+        if (!builds) return;
+        unsigned char* row = smem + buf * GD_BUF + dc * DIG_STRIDE + 4 * p;
+        put_digits(row, to_fixed(v[0], sh), to_fixed(v[1], sh));
+        put_digits(row + GD_CHUNK, to_fixed(v[2], sh), to_fixed(v[3], sh));
+    };
+    const int mt = warp >> 2, nt = (warp & 3) * 2;
+    float acc[2][DIG_ND][4];
+    long long val[2][4];
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) val[x][r] = 0;
+    const int up = up_bits(65536u, (int)min(kslice, (int64_t)1 << 30));
+    const uint32_t base = smem_addr(smem);
+    auto products = [&](int buf) {
+#pragma unroll 1
+        for (int c8 = 0; c8 < 2; ++c8) {
+            const uint32_t t = base + buf * GD_BUF + c8 * GD_CHUNK;
+            uint32_t fa[DIG_ND][2], fb[DIG_ND];
+            load_a(fa, t + (uint32_t)(16 * mt) * DIG_STRIDE);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                load_b(fb, t + (uint32_t)((diag ? 0 : GD_T) + 8 * (nt + x)) * DIG_STRIDE);
+                mma_digits(acc[x], fa, fb);
+            }
+        }
+    };
+    auto flush = [&]() {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) val[x][r] += acc_value(acc[x], r, up);
+            acc_clear(acc[x]);
+        }
+    };
+    static_assert(2 * GD_ROWS <= MAGIC_TERMS, "exact accumulators");
+    acc_clear(acc[0]);
+    acc_clear(acc[1]);
+    const int nch = ke > kb ? (int)((ke - kb + GD_ROWS - 1) / GD_ROWS) : 0;
+    if (nch > 0) {
+        fetch(kb);
+        build(0);
+        if (nch > 1) fetch(kb + GD_ROWS);
+        __syncthreads();
+    }
+    for (int i = 0; i < nch; ++i) {
+        if (i + 1 < nch) build((i + 1) & 1);
+        if (i + 2 < nch) fetch(kb + (int64_t)(i + 2) * GD_ROWS);
+        products(i & 1);
+        if (i & 1) flush();
+        __syncthreads();
+    }
+    if (nch & 1) flush();
+    const int g4 = lane >> 2, t4 = lane & 3;
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int i = ti * GD_T + 16 * mt + g4 + 8 * (r >> 1), j = tj * GD_T + 8 * (nt + x) + 2 * t4 + (r & 1);
+            if (i < m && j < m && j >= i) {
+                const int li = ex[i], lj = ex[j];
+                const double g = li == COL_BAD || lj == COL_BAD   // infinities and NaN stay visible
+                                     ? nan("")
+                                     : from_fixed(val[x][r], li + lj + 2 - (56 + up));
+                double* o = C + (int64_t)i * ldc + j;
+                if (ATOMIC) atomicAdd(o, g);
+                else *o += g;
+            }
+        }
 }
 
 // ---------------------------------------------------------------- Cholesky
@@ -348,12 +489,35 @@ __global__ void __launch_bounds__(ATB_THREADS) k_atb_partial(const double* __res
             if (cc[u] < ncols) partial[(int64_t)blockIdx.y * ncols + cc[u]] = s[u];
     }
 }
-__global__ void k_atb_reduce(const double* __restrict__ partial, int nslices, int ncols, double* __restrict__ h) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncols) return;
+// h[c] += the partials of column c in slice order: eight warps each add a contiguous
+// eighth of the slices for 32 columns, then the eighths are added in order.  (One thread
+// per column walked all 1,024 slices of a tall block, 80 us of dependent loads.)
+__global__ void __launch_bounds__(256) k_atb_reduce(const double* __restrict__ partial, int nslices, int ncols,
+                                                    double* __restrict__ h) {
+    __shared__ double red[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = blockIdx.x * 32 + lane;
+    const int per = (nslices + 7) / 8, y0 = min(nslices, warp * per), y1 = min(nslices, y0 + per);
     double s = 0.0;
-    for (int y = 0; y < nslices; ++y) s += partial[(int64_t)y * ncols + c];
-    h[c] += s;
+    if (c < ncols) {
+        int y = y0;
+        for (; y + 8 <= y1; y += 8) {   // eight loads in flight
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = partial[(int64_t)(y + u) * ncols + c];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += v[u];
+        }
+        for (; y < y1; ++y) s += partial[(int64_t)y * ncols + c];
+    }
+    red[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && c < ncols) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += red[w][lane];
+        h[c] += t;
+    }
 }
 
 // ---------------------------------------------------------------- vectors
@@ -438,6 +602,47 @@ void syrk_tn(const double* X, int64_t ldx, int64_t K, int m, double alpha, doubl
     else
         cgd::k_syrk_tn<false><<<grid, cgd::SY_THREADS, 0, st>>>(X, ldx, K, m, alpha, C, ldc, ntile, kslice);
     ckd(cudaGetLastError(), "k_syrk_tn");
+}
+
+void gram64(const double* X, int64_t ldx, int64_t K, int m, double* C, int64_t ldc, cudaStream_t st) {
+    if (K <= 0 || m <= 0) return;
+    // Below, the exponent pass and the 512-thread CTAs' start cost what the FP64 products do
+    // (whole calls, FP64 -> digits: 300 x 400 330 -> 291 us, 1,000 x 200 398 -> 293 us; at
+    // 1,000 x 100 the FP64 products are 30 us of the call)
+    if ((double)K * m * m < 4.0e7) {
+        syrk_tn(X, ldx, K, m, 1.0, C, ldc, st);
+        return;
+    }
+    const int ntile = (m + cgd::GD_T - 1) / cgd::GD_T;
+    const int64_t npairs = (int64_t)ntile * (ntile + 1) / 2;
+    if (npairs > 0x7fffffffLL) throw std::runtime_error("gram64: matrix too large");
+    // K slices (FP64 atomics) where the triangle alone leaves SMs idle: the fewest 16-row
+    // steps on the longest CTA's path, four more per slice for its start and end
+    const int64_t sms = sm_count(), steps = (K + cgd::GD_ROWS - 1) / cgd::GD_ROWS;
+    int64_t nslice = 1, best = -1;
+    for (int64_t sl = 1; sl <= std::min<int64_t>(steps, std::max<int64_t>(1, 8 * sms / npairs)); ++sl) {
+        const int64_t cost = (npairs * sl + sms - 1) / sms * ((steps + sl - 1) / sl + 4);
+        if (best < 0 || cost < best) { best = cost; nslice = sl; }
+    }
+    const int64_t kslice = (steps + nslice - 1) / nslice * cgd::GD_ROWS;
+    nslice = (K + kslice - 1) / kslice;
+    int* ex = nullptr;
+    ckd(cudaMallocAsync((void**)&ex, sizeof(int) * m, st), "column exponents");
+    ckd(cudaMemsetAsync(ex, 0x80, sizeof(int) * m, st), "column exponents");   // a very small value
+    const unsigned strips = (unsigned)((m + 31) / 32);
+    const unsigned gy = (unsigned)std::max<int64_t>(1, std::min<int64_t>((K + 63) / 64, 8 * sms / strips));
+    cgd::k_col_exponents<<<dim3(strips, gy), 256, 0, st>>>(X, ldx, K, m, ex);
+    const size_t smem = 2 * cgd::GD_BUF;
+    const dim3 grid((unsigned)npairs, (unsigned)nslice);
+    if (nslice > 1) {
+        ckd(cudaFuncSetAttribute(cgd::k_syrk_digits<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
+        cgd::k_syrk_digits<true><<<grid, cgd::GD_THREADS, smem, st>>>(X, ldx, K, m, C, ldc, ntile, kslice, ex);
+    } else {
+        ckd(cudaFuncSetAttribute(cgd::k_syrk_digits<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
+        cgd::k_syrk_digits<false><<<grid, cgd::GD_THREADS, smem, st>>>(X, ldx, K, m, C, ldc, ntile, kslice, ex);
+    }
+    ckd(cudaGetLastError(), "k_syrk_digits");
+    ckd(cudaFreeAsync(ex, st), "column exponents");
 }
 
 bool cholesky64(double* G, int n, int* d_info, cudaStream_t st, bool tensor_updates) {
@@ -532,7 +737,7 @@ void gemv_cols64(const double* A, int64_t lda, int64_t nrows, int ncols, const d
     if (nrows <= 0) return;
     const int ns = (int)std::min<int64_t>(nrows, cgd::ATB_SLICES);
     cgd::k_atb_partial<<<dim3(1, ns), cgd::ATB_THREADS, 0, st>>>(A, lda, nrows, ncols, t, partial);
-    cgd::k_atb_reduce<<<(ncols + 127) / 128, 128, 0, st>>>(partial, ns, ncols, g);
+    cgd::k_atb_reduce<<<(ncols + 31) / 32, 256, 0, st>>>(partial, ns, ncols, g);
     ckd(cudaGetLastError(), "k_atb");
 }
 

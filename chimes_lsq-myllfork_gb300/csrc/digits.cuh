@@ -137,13 +137,13 @@ __device__ __forceinline__ long long acc_value(const float (&acc)[8][4], int k, 
     const int fr = (int)(__float_as_uint(acc[6][k]) * 256u + __float_as_uint(acc[7][k]) - c);
     const long long v = (long long)((unsigned long long)hi << 32) + ((long long)mid << 16) + (long long)lo;
     if (up >= 0) return (long long)((unsigned long long)v << up) + (((fr >> (15 - up)) + 1) >> 1);
-    return (v + (fr >> 16)) >> -up;
+    return (v + (fr >> 16) + (1ll << (-up - 1))) >> -up;   // to nearest: sums of floors would drift
 }
 // A magnitude 2^t as a share of the largest, 2^tmax, in 2^-16: integers, so that sums
 // of shares do not depend on their order.
 __device__ __forceinline__ unsigned share16(int t, int tmax) { return (65536u >> min(tmax - t, 16)) + 1u; }
 // The finest unit with room in 63 bits for outputs of at most sum / 2^16 times the
-// largest product (0.2290), sum of up to 2^15 shares over the terms times `terms`.
+// largest product (0.2481), sum of up to 2^15 shares over the terms times `terms`.
 __device__ __forceinline__ int up_bits(unsigned sum, int terms) {
     const unsigned long long b = (unsigned long long)sum * (unsigned)terms;
     const int e = 64 - __clzll((long long)b) - 16;   // 2^(e + 16) > sum terms

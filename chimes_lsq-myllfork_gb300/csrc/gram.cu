@@ -858,7 +858,7 @@ void gram_accumulate(int prec_in, const void* A, int64_t lda, int64_t nrows, int
         mark(S_ATB, false);
         ck(cudaFreeAsync(partial, st), "atb scratch free");
         mark(S_SYRK, true);
-        syrk_tn((const double*)A, lda, nrows, ncols, 1.0, G, ncols, st);
+        gram64((const double*)A, lda, nrows, ncols, G, ncols, st);
         mark(S_SYRK, false);
         return;
     }

@@ -40,7 +40,17 @@ def packed(S, up):
     fr = S[6] * 256 + S[7]
     if up >= 0:
         return (v << up) + (((fr >> (15 - up)) + 1) >> 1)
-    return (v + (fr >> 16)) >> -up
+    return (v + (fr >> 16) + (1 << (-up - 1))) >> -up
+
+
+def test_rounding_of_coarse_units_is_unbiased():
+    """Many packed values of a unit above 2^-56 add up without drift."""
+    rng = np.random.default_rng(5)
+    S = rng.integers(-(1 << 21), 1 << 21, size=(4000, 8))
+    up = -6
+    exact = sum(sum(int(s[D]) * 256 ** (7 - D) for D in range(8)) for s in S)       # units of 2^-72
+    got = sum(packed([int(v) for v in s], up) for s in S)
+    assert abs(got - Fraction(exact, 2 ** (16 - up))) <= 4 * np.sqrt(4000 / 12)
 
 
 @pytest.mark.parametrize("n,span", [(1, 0), (3, 4), (16, 12), (32, 40)])
