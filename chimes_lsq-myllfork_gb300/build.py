@@ -18,7 +18,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libchimes_gb300.so")
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 
-CU_SOURCES = ["geom.cu", "assemble.cu", "tensor_rows.cu", "ewald.cu", "session.cu", "gram.cu", "dense64.cu", "solve.cu", "md.cu", "md_host.cu", "lars.cu"]
+CU_SOURCES = ["geom.cu", "assemble.cu", "tensor_rows.cu", "ewald.cu", "session.cu", "gram.cu", "dense64.cu", "solve.cu", "md.cu", "md_tensor.cu", "md_host.cu", "lars.cu"]
 CPP_SOURCES = ["model.cpp", "capi.cpp", "textio.cpp", "mdio.cpp"]
 
 

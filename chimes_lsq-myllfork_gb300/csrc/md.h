@@ -61,6 +61,15 @@ void launch_md2(const ModelDev& M, const MdDev& D, const FramesDev& F, const Nei
 void launch_mdc(int nbody, int prec, int order, int64_t max_tiles, const ModelDev& M, const MdDev& D,
                 const FramesDev& F, const ClusterSet& CS, const MdBuckets& B, double* Fo, double* So,
                 cudaStream_t st);
+// The FP64 contraction on the tensor cores (md_tensor.cu), for the orders of
+// md_tensor_order: tables of a coefficient set (md_tensor_bytes bytes and
+// md_tensor_exponents ints per type), then the force pass as launch_mdc.
+bool md_tensor_order(int nbody, int order);
+size_t md_tensor_bytes(int nbody, int ntypes);
+int md_tensor_exponents(int nbody);
+void launch_md_tables(int nbody, int ntypes, const double* C, unsigned char* tab, int* ex, cudaStream_t st);
+void launch_mdt(int nbody, int64_t max_tiles, const ModelDev& M, const FramesDev& F, const ClusterSet& CS,
+                const MdBuckets& B, const unsigned char* tab, const int* ex, double* Fo, double* So, cudaStream_t st);
 void launch_md_finalize(int nframes, const ModelDev& M, const MdDev& D, const FramesDev& F, double* So,
                         cudaStream_t st);
 // List reuse: per-step exact filter of skin-enumerated clusters (type_out -1 when

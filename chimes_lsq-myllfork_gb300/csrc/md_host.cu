@@ -78,6 +78,17 @@ void Session::md_setup(const double* x, int nx, int precision, bool offsets, dou
     if (o4 > 0) dense(m.quads, 6, o4, m.tot_snum + m.num3, C4);
     t->dev.C3 = (const double*)up(C3.data(), C3.size() * sizeof(double));
     t->dev.C4 = (const double*)up(C4.data(), C4.size() * sizeof(double));
+    if (precision == 0)   // FP64: the contraction's digit tables
+        for (int k = 0; k < 2; ++k) {
+            const int nt = (int)(k == 0 ? m.trips : m.quads).vec.size();
+            if ((k == 0 ? o3 : o4) == 0 || nt == 0 || !cgd::md_tensor_order(3 + k, k == 0 ? o3 : o4)) continue;
+            CK(cudaMalloc((void**)&t->digits[k], cgd::md_tensor_bytes(3 + k, nt)));
+            t->allocs.push_back(t->digits[k]);
+            CK(cudaMalloc((void**)&t->digit_ex[k], sizeof(int) * (size_t)cgd::md_tensor_exponents(3 + k) * nt));
+            t->allocs.push_back(t->digit_ex[k]);
+            cgd::launch_md_tables(3 + k, nt, k == 0 ? t->dev.C3 : t->dev.C4, t->digits[k], t->digit_ex[k], stream_);
+            CK(cudaGetLastError());
+        }
     std::vector<float> C3f(C3.begin(), C3.end()), C4f(C4.begin(), C4.end());
     t->dev.C3f = (const float*)up(C3f.data(), C3f.size() * sizeof(float));
     t->dev.C4f = (const float*)up(C4f.data(), C4f.size() * sizeof(float));
@@ -197,7 +208,10 @@ void Session::md_force(const DeviceFrames& df, double* Fo, double* So, MdCounts*
         B.val = S.get<int>(n);
         cgd::launch_md_bucket(n, nf, cfo, CS.type, B, st); L(3);
         const int64_t max_tiles = (n + cgd::MDC_TILE - 1) / cgd::MDC_TILE + B.nkeys;
-        cgd::launch_mdc(nbody, md_->precision, k == 0 ? M.order3 : M.order4, max_tiles, M, D, F, CS, B, Fo, So, st);
+        if (md_->digits[k])
+            cgd::launch_mdt(nbody, max_tiles, M, F, CS, B, md_->digits[k], md_->digit_ex[k], Fo, So, st);
+        else
+            cgd::launch_mdc(nbody, md_->precision, k == 0 ? M.order3 : M.order4, max_tiles, M, D, F, CS, B, Fo, So, st);
         L();
         CK(cudaGetLastError());
     }
@@ -395,8 +409,11 @@ void Session::md_force_lists(DeviceFrames& df, MdLists& L, double* Fo, double* S
         mark(ST_BUCKET, false);
         const int64_t max_tiles = (n + cgd::MDC_TILE - 1) / cgd::MDC_TILE + L.B[k].nkeys;
         mark(k == 0 ? ST_FORCE3 : ST_FORCE4, true);
-        cgd::launch_mdc(3 + k, md_->precision, k == 0 ? M.order3 : M.order4, max_tiles, M, D, F, CS, L.B[k], Fo, So,
-                        sk);
+        if (md_->digits[k])
+            cgd::launch_mdt(3 + k, max_tiles, M, F, CS, L.B[k], md_->digits[k], md_->digit_ex[k], Fo, So, sk);
+        else
+            cgd::launch_mdc(3 + k, md_->precision, k == 0 ? M.order3 : M.order4, max_tiles, M, D, F, CS, L.B[k], Fo, So,
+                            sk);
         mark(k == 0 ? ST_FORCE3 : ST_FORCE4, false);
         if (fork) {
             CK(cudaEventRecord(md_join_[k], sk));

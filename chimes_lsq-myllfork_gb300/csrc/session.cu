@@ -141,23 +141,28 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
         oz.ncix += w;
     }
     std::vector<uint32_t> cx((size_t)nb * oz.ncix, (uint32_t)none | (uint32_t)none << 16);
+    auto spread = [&](int x, int n) {   // n base-ord powers on the padded grid
+        int y = 0, w = 1;
+        for (int k = 0; k < n; ++k) { y += x % ord * w; x /= ord; w *= base; }
+        return y;
+    };
     if (ord <= base)
-        for (int pi = 0; pi < nb; ++pi)
-            for (size_t t = 0; t < tv.size(); ++t) {
-                const cgd::ClusterTypeDev& d = tv[t];
-                for (int c = 0; c < d.n_true; ++c) {
-                    const int p0 = gp[d.grp_offset + c], p1 = gp[d.grp_offset + c + 1];
-                    for (int p = p0; p < p1; ++p) {
-                        const uint8_t* pp = &pw[d.pow_offset + (size_t)p * np];
-                        int ii = 0, oo = 0;
-                        for (int k = nb - 2; k >= 0; --k) ii = ii * base + pp[cgd::role_slot_in(nb, pi, k)];
-                        for (int k = np - nb; k >= 0; --k) oo = oo * base + pp[cgd::role_slot_out(nb, pi, k)];
-                        uint32_t& w = cx[(size_t)pi * oz.ncix + ti[t].y + (size_t)((p - p0) / 2) * d.n_true + c];
+        for (size_t t = 0; t < tv.size(); ++t) {
+            const cgd::ClusterTypeDev& d = tv[t];
+            for (int c = 0; c < d.n_true; ++c)
+                for (int p = gp[d.grp_offset + c], p0 = p; p < gp[d.grp_offset + c + 1]; ++p) {
+                    const uint4 o4 = of[d.pow_offset / np + p];
+                    const uint32_t e[4] = {o4.x, o4.y, o4.z, o4.w};
+                    const size_t at = ti[t].y + (size_t)((p - p0) / 2) * d.n_true + c;
+                    for (int pi = 0; pi < nb; ++pi) {
+                        int ii = (int)(e[pi] & 0xffffu), oo = (int)(e[pi] >> 16) - 3 * sizeI;
+                        if (ord < base) { ii = spread(ii, nb - 1); oo = spread(oo, np - nb + 1); }
+                        uint32_t& w = cx[(size_t)pi * oz.ncix + at];
                         const uint32_t v = (uint32_t)(ii * row + oo);
                         w = (p - p0) % 2 ? (w & 0xffffu) | v << 16 : (w & 0xffff0000u) | v;
                     }
                 }
-            }
+        }
     oz.cix = dev_upload(D.allocs, cx.data(), cx.size());
     oz.type = dev_upload(D.allocs, ti.data(), ti.size());
     *int_map = dev_upload(D.allocs, imap.data(), imap.size());

@@ -81,6 +81,8 @@ struct AssembleStats {
 struct MdTables {
     cgd::MdDev dev{};
     int precision = 0;                 // 0: FP64 contraction, 1: FP32 contraction
+    unsigned char* digits[2] = {nullptr, nullptr};   // 3-, 4-body digit tables (md_tensor.cu), null: not in use
+    int* digit_ex[2] = {nullptr, nullptr};
     std::vector<void*> allocs;
     ~MdTables() { for (void* p : allocs) cudaFree(p); }
 };
