@@ -112,12 +112,12 @@ constexpr int GD_T = 64, GD_THREADS = 512, GD_ROWS = 16;
 constexpr uint32_t GD_CHUNK = 2 * GD_T * DIG_STRIDE;   // 8 rows of K
 constexpr uint32_t GD_BUF = 2 * GD_CHUNK;
 
-// ex[i] <- the least e with |X[k][i]| <= 0.996 2^e for all k, so that the leading digit is
-// at most 127 (ex preset to a very small value; COL_BAD for infinities and NaN).
+// ex[i] <- the least e with |X[k][i]| < 0.9942 2^e for all k: the digits' bias adds
+// 0x80..80 / 2^63 = 1.0039, and the sum stays below 2 (ex preset to a very small value; COL_BAD for infinities and NaN).
 constexpr int COL_BAD = 4096;
 __device__ __forceinline__ int col_exponent(double x) {
     const int h = __double2hiint(x) & 0x7fffffff;
-    return h >= 0x7ff00000 ? COL_BAD : (h >> 20) - 1022 + ((h & 0xfffff) >= 0xfe000 ? 1 : 0);
+    return h >= 0x7ff00000 ? COL_BAD : (h >> 20) - 1022 + ((h & 0xfffff) >= 0xfd000 ? 1 : 0);
 }
 __global__ void __launch_bounds__(256) k_col_exponents(const double* __restrict__ X, int64_t ldx, int64_t K, int m,
                                                 int* __restrict__ ex) {

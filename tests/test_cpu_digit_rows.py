@@ -81,3 +81,8 @@ def test_extreme_digits_fit():
     for X in (m, -m, 0, 1, -1, 2 ** 62, -(2 ** 62)):
         digits(X)
     assert 32 * 8 * 128 * 128 == 2 ** 22
+    # columns of a Gram are scaled by their own exponent: entries up to (1 + 0xfd000 / 2^20) / 2
+    top = int((1 + Fraction(0xFD000, 1 << 20)) / 2 * 2 ** 63)
+    for X in (top - 1, -(top - 1)):
+        d = digits(X)
+        assert -128 <= min(d) and max(d) <= 127

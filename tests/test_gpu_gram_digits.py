@@ -51,6 +51,22 @@ def test_matches_extended_precision(cg, tmp_path, K, m):
     assert np.all(np.abs(h - (Q.T @ b.astype(np.longdouble)).astype(np.float64)) <= K * 2.0 ** -52 * (np.abs(A).T @ np.abs(b)))
 
 
+@pytest.mark.parametrize("frac", [0.9940, 0.99415, 0.9945, 0.9961, 0.99999, 1.0])
+def test_entries_just_below_a_power_of_two(cg, tmp_path, frac):
+    """The scaled leading digit at the end of its range: every entry of a column frac times
+    a power of two, both signs."""
+    torch = pytest.importorskip("torch")
+    import importlib
+    synth = importlib.import_module("chimes_lsq-myllfork_gb300.synth")
+    sess = cg.Session(cg.Model(synth.make_workload("water-2b", str(tmp_path), nframes=1, seed=3)), 0)
+    rng = np.random.default_rng(2)
+    A = np.where(rng.random((2048, 160)) < 0.5, -1.0, 1.0) * frac * np.exp2(rng.integers(-3, 4, 160))
+    G, _ = _gram(cg, sess, torch, A, np.ones(2048))
+    R = A.T @ A
+    up = np.triu(np.ones(R.shape, bool))
+    assert np.all((np.abs(G - R) <= 1e-12 * np.sqrt(np.outer(np.diag(R), np.diag(R))))[up])
+
+
 def test_non_finite_columns(cg, tmp_path):
     torch = pytest.importorskip("torch")
     import importlib
