@@ -15,6 +15,7 @@
 #include "dense64.h"
 #include "digits.cuh"
 #include "gram.h"
+#include "scratch.h"
 
 namespace cgd {
 
@@ -237,76 +238,194 @@ __global__ void __launch_bounds__(GD_THREADS, 1) k_syrk_digits(const double* __r
 // ---------------------------------------------------------------- Cholesky
 constexpr int CH_NB = 128;
 
-// Factor the kb x kb diagonal block at (k, k) of the column-major lower matrix
-// (leading dimension n) in place; info <- first non-positive pivot + 1.
-__global__ void k_potrf_block(double* __restrict__ G, int n, int k, int kb, int* info) {
-    extern __shared__ double a[];   // kb x kb, column-major
-    for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
-        const int i = idx % kb, j = idx / kb;
-        a[idx] = G[(int64_t)(k + j) * n + (k + i)];
+// A panel of CH_NB columns is factorised as two halves of CH_H.  The FP64 pipe does 2
+// multiply-adds a clock per SM, so one SM needs 90 us for a 128 x 128 block and 130 us for 64
+// rows of the panel below; with one CTA for the block and 64 rows per CTA a panel of n =
+// 5,000 took 535 us, most of the GPU idle.  Here every CTA factorises the 64 x 64 block for
+// itself (11 us of multiply-adds) and solves its share of the rows below, one share per SM,
+// and the second half's columns are updated from the first's by a third launch.  n = 5,000:
+// the panels 21.2 -> 7.3 ms; n = 1,000: the whole factorisation 4.66 -> 1.64 ms.
+constexpr int CH_H = 64, CH_B = 16, CH_LD = CH_H + 1, CH_THREADS = 256;
+
+// 16 x 16 diagonal sub-block at b0 of D (bs valid columns), by warp 0: lane r + 16 h holds
+// row r, columns 2 i + h, so that one instruction updates two columns (a warp's FP64
+// instruction takes 64 cycles of its SM quarter whatever the lanes do).  L D L^T first, one
+// reciprocal per column in the chain, and the square roots of all pivots at the end.  A
+// pivot that is not positive becomes 1; bad receives its column + 1 (the first).
+__device__ __forceinline__ void chol16(double* D, int b0, int bs, double* rdiag, int* bad) {
+    const int lane = threadIdx.x & 31, r = lane & 15, h = lane >> 4;
+    double a[CH_B / 2], piv = 1.0;
+#pragma unroll
+    for (int i = 0; i < CH_B / 2; ++i) {
+        const int c = 2 * i + h;
+        a[i] = r < bs && c <= r ? D[(b0 + r) * CH_LD + b0 + c] : (c == r ? 1.0 : 0.0);
     }
-    __syncthreads();
-    for (int j = 0; j < kb; ++j) {
-        if (threadIdx.x == 0) {
-            const double d = a[j * kb + j];
-            if (!(d > 0.0)) atomicCAS(info, 0, k + j + 1);
-            a[j * kb + j] = d > 0.0 ? sqrt(d) : 1.0;
+#pragma unroll
+    for (int j = 0; j < CH_B; ++j) {
+        const double v = __shfl_sync(0xffffffffu, a[j >> 1], r + 16 * (j & 1));   // column j, row r
+        double d = __shfl_sync(0xffffffffu, v, j);
+        if (!(d > 0.0)) {
+            if (lane == 0 && j < bs && *bad == 0) *bad = b0 + j + 1;
+            d = 1.0;
         }
-        __syncthreads();
-        const double djj = a[j * kb + j];
-        for (int i = j + 1 + threadIdx.x; i < kb; i += blockDim.x) a[j * kb + i] /= djj;
-        __syncthreads();
-        const int m = kb - j - 1;
-        for (int idx = threadIdx.x; idx < m * m; idx += blockDim.x) {
-            const int i = j + 1 + idx % m, l = j + 1 + idx / m;
-            if (i >= l) a[l * kb + i] -= a[j * kb + i] * a[j * kb + l];
+        if (r == j) piv = d;
+        const double l = v * __drcp_rn(d);
+#pragma unroll
+        for (int i = j >> 1; i < CH_B / 2; ++i) {
+            const int c = 2 * i + h;
+            const double vc = __shfl_sync(0xffffffffu, v, c);
+            if (c > j && c <= r) a[i] = fma(-l, vc, a[i]);
         }
-        __syncthreads();
+        if (h == (j & 1)) a[j >> 1] = r == j ? 1.0 : l;
     }
-    for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
-        const int i = idx % kb, j = idx / kb;
-        G[(int64_t)(k + j) * n + (k + i)] = i >= j ? a[idx] : 0.0;
+    const double sd = sqrt(piv);
+    if (h == 0) rdiag[b0 + r] = 1.0 / sd;
+#pragma unroll
+    for (int i = 0; i < CH_B / 2; ++i) {
+        const int c = 2 * i + h;
+        const double x = a[i] * __shfl_sync(0xffffffffu, sd, c);
+        if (r < bs && c < bs) D[(b0 + r) * CH_LD + b0 + c] = c <= r ? x : 0.0;
     }
 }
 
-// Panel solve X L_kk^T = P below the diagonal block at (k, k): rows k+kb+i of the
-// columns k..k+kb-1 (column-major, leading dimension n).  A CTA owns TR_R rows;
-// four threads share a row (lanes 4r..4r+3 of one warp) and split each row's dot
-// products by l mod 4, so a row's forward substitution needs only warp shuffles.
-constexpr int TR_R = 64, TR_THREADS = 256, TR_PLD = CH_NB + 4;
-__global__ void __launch_bounds__(TR_THREADS, 1) k_trsm_panel(double* __restrict__ G, int n, int k, int kb, int m) {
+// Columns k .. k + kb of the column-major lower matrix (leading dimension n, kb <= 64):
+// the diagonal block's factor and the m rows below it, R rows per CTA.  While warp 0
+// factorises the next 16 columns' diagonal sub-block, the others finish the update of the
+// columns after them.
+__global__ void __launch_bounds__(CH_THREADS) k_chol_half(double* __restrict__ G, int n, int k, int kb, int m, int R,
+                                                          int second, int* info, int* __restrict__ arrived) {
     extern __shared__ double sm[];
-    double* Ls = sm;                    // Ls[j * kb + l] = L(j, l), l <= j
-    double* Ps = sm + kb * kb;          // Ps[r * TR_PLD + l]
-    double* rdiag = Ps + TR_R * TR_PLD; // 1 / L(j, j)
-    const int i0 = blockIdx.x * TR_R;
-    const int rows = min(TR_R, m - i0);
+    double* D = sm;                          // rows 0 .. kb: the block, then this CTA's rows
+    __shared__ double rdiag[CH_H];
+    __shared__ int bad, last;
+    const int i0 = blockIdx.x * R, rows = min(R, m - i0), tot = CH_H + max(rows, 0);
+    if (threadIdx.x == 0) bad = 0;
+    {   // every load of the block in flight at once, then the rows
+        double v[CH_H * CH_H / CH_THREADS];
+#pragma unroll
+        for (int u = 0; u < CH_H * CH_H / CH_THREADS; ++u) {
+            const int idx = threadIdx.x + u * CH_THREADS, i = idx % CH_H, j = idx / CH_H;
+            v[u] = i < kb && j <= i ? G[(int64_t)(k + j) * n + k + i] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < CH_H * CH_H / CH_THREADS; ++u) {
+            const int idx = threadIdx.x + u * CH_THREADS;
+            D[(idx % CH_H) * CH_LD + idx / CH_H] = v[u];
+        }
+        for (int r = threadIdx.x & 31; r < rows; r += 32) {
+            const int w = threadIdx.x >> 5;
+#pragma unroll
+            for (int u = 0; u < CH_H / 8; ++u) {
+                const int j = w + 8 * u;
+                v[u] = j < kb ? G[(int64_t)(k + j) * n + k + kb + i0 + r] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < CH_H / 8; ++u) D[(CH_H + r) * CH_LD + w + 8 * u] = v[u];
+        }
+    }
+    __syncthreads();
+    // columns [c0, c1) of the rows from c0 on minus the product with the sub-block's columns
+    // at b0, by threads t0, t0 + step, ...: four columns per item, rows across the lanes
+    auto update = [&](int b0, int c0, int c1, int t0, int step) {
+        const int ng = (c1 - c0 + 3) >> 2, nr = tot - c0;
+        for (int t = t0; t < nr * ng; t += step) {
+            const int g = t / nr, r = c0 + t - g * nr, c = c0 + 4 * g;
+            if (r < CH_H && (r < c || r >= kb)) continue;
+            const double* p = D + r * CH_LD + b0;
+            double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int l = 0; l < CH_B; ++l) {
+                const double v = p[l];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) s[q] = fma(v, D[min(c + q, CH_H - 1) * CH_LD + b0 + l], s[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) if (c + q < c1) D[r * CH_LD + c + q] -= s[q];
+        }
+    };
+    for (int b0 = 0; b0 < kb; b0 += CH_B) {
+        const int bs = min(CH_B, kb - b0);
+        if (threadIdx.x < 32) chol16(D, b0, bs, rdiag, &bad);
+        else if (b0 > 0 && b0 + CH_B < kb) update(b0 - CH_B, b0 + CH_B, kb, threadIdx.x - 32, CH_THREADS - 32);
+        __syncthreads();
+        // the sub-block's columns of every row below, a row per thread
+        for (int r = b0 + CH_B + threadIdx.x; r < tot; r += CH_THREADS) {
+            double* p = D + r * CH_LD + b0;
+            double x[CH_B];
+#pragma unroll
+            for (int j = 0; j < CH_B; ++j) {
+                double v = j < bs ? p[j] : 0.0;
+#pragma unroll
+                for (int l = 0; l < j; ++l) v = fma(-x[l], D[(b0 + j) * CH_LD + b0 + l], v);
+                x[j] = j < bs ? v * rdiag[b0 + j] : 0.0;
+            }
+#pragma unroll
+            for (int j = 0; j < CH_B; ++j) if (j < bs) p[j] = x[j];
+        }
+        __syncthreads();
+        // the next sub-block's columns now, those after it beside its factorisation
+        if (b0 + CH_B < kb) {
+            update(b0, b0 + CH_B, min(kb, b0 + 2 * CH_B), threadIdx.x, CH_THREADS);
+            __syncthreads();
+        }
+    }
+    for (int j = threadIdx.x >> 5; j < kb; j += CH_THREADS / 32)
+        for (int r = threadIdx.x & 31; r < rows; r += 32)
+            G[(int64_t)(k + j) * n + k + kb + i0 + r] = D[(CH_H + r) * CH_LD + j];
+    // the block's factor, by the last CTA: every other has read the block by then
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(arrived, 1) == (int)gridDim.x - 1;
+        if (last) *arrived = 0;
+    }
+    __syncthreads();
+    if (!last) return;
     for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
-        const int j = idx % kb, l = idx / kb;
-        Ls[j * kb + l] = l <= j ? G[(int64_t)(k + l) * n + (k + j)] : 0.0;
+        const int i = idx % kb, j = idx / kb;
+        G[(int64_t)(k + j) * n + k + i] = i >= j ? D[i * CH_LD + j] : 0.0;
     }
-    for (int idx = threadIdx.x; idx < TR_R * kb; idx += blockDim.x) {
-        const int r = idx % TR_R, l = idx / TR_R;
-        Ps[r * TR_PLD + l] = r < rows ? G[(int64_t)(k + l) * n + (k + kb + i0 + r)] : 0.0;
+    if (second)   // the block above it, of the 128-wide block's upper triangle
+        for (int idx = threadIdx.x; idx < CH_H * kb; idx += blockDim.x)
+            G[(int64_t)(k + idx / CH_H) * n + k - CH_H + idx % CH_H] = 0.0;
+    if (threadIdx.x == 0 && bad) atomicCAS(info, 0, k + bad);
+}
+
+// The second half's columns, rows k0 + 64 and below: minus the first half's product.
+// 16 rows x kb2 columns per CTA (32 rows, 131,000 multiply-adds: 33 us of an SM), four
+// columns per thread.
+constexpr int ST_R = 16;
+__global__ void __launch_bounds__(256) k_chol_strip(double* __restrict__ G, int n, int k0, int kb2) {
+    __shared__ double Ls[CH_H][CH_H];    // Ls[l][c] = L(k0 + 64 + c, k0 + l)
+    __shared__ double Ps[CH_H][ST_R];
+    const int r = threadIdx.x % ST_R, c0 = threadIdx.x / ST_R * 4;
+    const int row = k0 + CH_H + blockIdx.x * ST_R + r;
+    {
+        double v[CH_H * CH_H / 256], p[CH_H * ST_R / 256];
+#pragma unroll
+        for (int u = 0; u < CH_H * CH_H / 256; ++u) {
+            const int idx = threadIdx.x + 256 * u, c = idx % CH_H, l = idx / CH_H;
+            v[u] = c < kb2 ? G[(int64_t)(k0 + l) * n + k0 + CH_H + c] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < CH_H * ST_R / 256; ++u)
+            p[u] = row < n ? G[(int64_t)(k0 + threadIdx.x / ST_R + 16 * u) * n + row] : 0.0;
+#pragma unroll
+        for (int u = 0; u < CH_H * CH_H / 256; ++u) (&Ls[0][0])[threadIdx.x + 256 * u] = v[u];
+#pragma unroll
+        for (int u = 0; u < CH_H * ST_R / 256; ++u) Ps[threadIdx.x / ST_R + 16 * u][r] = p[u];
     }
     __syncthreads();
-    for (int j = threadIdx.x; j < kb; j += blockDim.x) rdiag[j] = 1.0 / Ls[j * kb + j];
-    __syncthreads();
-    const int r = threadIdx.x >> 2, q = threadIdx.x & 3;
-    double* pr = Ps + r * TR_PLD;
-    for (int j = 0; j < kb; ++j) {
-        const double* lj = Ls + j * kb;
-        double s = 0.0;
-        for (int l = q; l < j; l += 4) s = fma(pr[l], lj[l], s);
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if (q == 0) pr[j] = (pr[j] - s) * rdiag[j];
-        __syncwarp();
+    double s[4] = {0, 0, 0, 0};
+#pragma unroll 8
+    for (int l = 0; l < CH_H; ++l) {
+        const double p = Ps[l][r];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s[c] = fma(p, Ls[l][c0 + c], s[c]);
     }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < TR_R * kb; idx += blockDim.x) {
-        const int rr = idx % TR_R, l = idx / TR_R;
-        if (rr < rows) G[(int64_t)(k + l) * n + (k + kb + i0 + rr)] = Ps[rr * TR_PLD + l];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int col = c0 + c;
+        if (col < kb2 && row < n && row >= k0 + CH_H + col) G[(int64_t)(k0 + CH_H + col) * n + row] -= s[c];
     }
 }
 
@@ -314,7 +433,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) k_trsm_panel(double* __restrict
 // T(i, j) = M[i*si + j*sj].  One CTA solves the whole system when n fits its shared
 // memory: blocks of 32 in solve order, warp 0 substitutes within the block with
 // shuffles, then every warp updates the remaining right-hand sides.
-constexpr int TS_THREADS = 1024, TS_SMALL = 1024, TS_BLOCK = 128;
+constexpr int TS_THREADS = 1024, TS_CHAIN = 128;
 __device__ __forceinline__ double tget(const double* M, int64_t si, int64_t sj, int64_t i, int64_t j) {
     return M[i * si + j * sj];
 }
@@ -388,35 +507,108 @@ __global__ void __launch_bounds__(TS_THREADS) k_trsv_small(const double* __restr
     for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] = xs[i];
 }
 
-// Large systems: after the block [b0, b0+bl) is solved (k_trsv_small on the block),
-// every remaining right-hand side row is updated by a grid of CTAs.
-__global__ void __launch_bounds__(256) k_trsv_update(const double* __restrict__ M, int64_t si, int64_t sj, int b0,
-                                                     int bl, int r0, int r1, double* __restrict__ x) {
-    __shared__ double xb[TS_BLOCK];
-    for (int c = threadIdx.x; c < bl; c += blockDim.x) xb[c] = x[b0 + c];
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (sj == 1) {
-        const int gw = blockIdx.x * (blockDim.x >> 5) + warp, nw = gridDim.x * (blockDim.x >> 5);
-        for (int i = r0 + gw; i < r1; i += nw) {
-            double p = 0.0;
-            for (int c = lane; c < bl; c += 32) p = fma(M[(int64_t)i * si + b0 + c], xb[c], p);
+// Large systems: one cooperative launch, the CTAs' row blocks of 64 in solve order (block b,
+// b + grid, ...).  A CTA subtracts the blocks of x before its own as they are published
+// (flag[j] != 0 once block j of x is in place), the next 64 x 64 tile of T on its way
+// meanwhile, then solves its diagonal tile and publishes.  A wait that runs out leaves NaN in
+// x.  A launch per 128 rows and one per update took 100 us a block: a factor's two solves
+// at n = 5,000 7.6 -> 1.9 ms, at n = 24,000 40 -> 9.0 ms.  Below TS_CHAIN one CTA is as fast
+// (n = 130: two solves 98 us by the chain; n = 1,000, one CTA -> chain 1,990 -> 410 us).
+constexpr int TC_B = 64, TC_THREADS = 256;
+__global__ void __launch_bounds__(TC_THREADS) k_trsv_chain(const double* __restrict__ M, int64_t si, int64_t sj, int n,
+                                                           int lower, double* __restrict__ x, int* __restrict__ flag) {
+    __shared__ double tile[TC_B][TC_B + 1];
+    __shared__ double xs[TC_B], red[4][TC_B], rd[TC_B];
+    __shared__ int ok;
+    const int tid = threadIdx.x;
+    const int nb = (n + TC_B - 1) / TC_B;
+    const bool along_i = si == 1;   // T(i, j) contiguous along i, else along j
+    double pre[TC_B * TC_B / TC_THREADS];
+    auto fetch = [&](int bi, int bj) {   // tile of row block bi, column block bj into registers
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-            if (lane == 0) x[i] -= p;
+        for (int u = 0; u < TC_B * TC_B / TC_THREADS; ++u) {
+            const int t = tid + u * TC_THREADS, p = t % TC_B, q = t / TC_B;
+            const int i = bi * TC_B + (along_i ? p : q), j = bj * TC_B + (along_i ? q : p);
+            const bool in = i < n && j < n && (bi != bj || (lower ? j <= i : j >= i));
+            pre[u] = in ? tget(M, si, sj, i, j) : (i == j ? 1.0 : 0.0);
         }
-    } else {
-        for (int i = r0 + blockIdx.x * blockDim.x + threadIdx.x; i < r1; i += gridDim.x * blockDim.x) {
-            double p0 = 0.0, p1 = 0.0;
-            int c = 0;
-#pragma unroll 8   // sixteen independent loads in flight per thread
-            for (; c + 1 < bl; c += 2) {
-                p0 = fma(tget(M, si, sj, i, b0 + c), xb[c], p0);
-                p1 = fma(tget(M, si, sj, i, b0 + c + 1), xb[c + 1], p1);
+    };
+    auto stage = [&]() {
+#pragma unroll
+        for (int u = 0; u < TC_B * TC_B / TC_THREADS; ++u) {
+            const int t = tid + u * TC_THREADS, p = t % TC_B, q = t / TC_B;
+            if (along_i) tile[p][q] = pre[u]; else tile[q][p] = pre[u];
+        }
+    };
+    for (int o = blockIdx.x; o < nb; o += gridDim.x) {
+        const int b = lower ? o : nb - 1 - o;
+        const int row = tid % TC_B, part = tid / TC_B;
+        double s = 0.0;
+        fetch(b, o == 0 ? b : (lower ? 0 : nb - 1));
+        for (int w = 0; w < o; ++w) {
+            const int j = lower ? w : nb - 1 - w;
+            __syncthreads();
+            stage();
+            fetch(b, w + 1 < o ? (lower ? w + 1 : nb - 2 - w) : b);
+            if (tid == 0) {
+                int v = 0;
+                for (int it = 0; it < (1 << 24); ++it) {
+                    asm volatile("ld.acquire.gpu.s32 %0, [%1];" : "=r"(v) : "l"(flag + j) : "memory");
+                    if (v) break;
+                }
+                ok = v == 1;
             }
-            if (c < bl) p0 = fma(tget(M, si, sj, i, b0 + c), xb[c], p0);
-            x[i] -= p0 + p1;
+            __syncthreads();
+            if (!ok) break;
+            if (tid < TC_B) xs[tid] = j * TC_B + tid < n ? __ldcg(x + j * TC_B + tid) : 0.0;
+            __syncthreads();
+#pragma unroll
+            for (int c = 0; c < TC_B / 4; ++c) s = fma(tile[row][part * (TC_B / 4) + c], xs[part * (TC_B / 4) + c], s);
         }
+        const bool good = o == 0 || ok;
+        __syncthreads();
+        stage();
+        red[part][row] = s;
+        __syncthreads();
+        if (tid < TC_B) {
+            rd[tid] = 1.0 / tile[tid][tid];
+            xs[tid] = (b * TC_B + tid < n ? x[b * TC_B + tid] : 0.0) - ((red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]));
+        }
+        __syncthreads();
+        if (tid < 32) {   // two halves of 32, one row per lane, then the other half's rows
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                const int r0 = (lower ? h : 1 - h) * 32, r1 = 32 - r0;
+                double v = xs[r0 + tid];
+                for (int q = 0; q < 32; ++q) {
+                    const int c = lower ? q : 31 - q;
+                    if (tid == c) v *= rd[r0 + c];
+                    const double xc = __shfl_sync(0xffffffffu, v, c);
+                    if (lower ? tid > c : tid < c) v = fma(-tile[r0 + tid][r0 + c], xc, v);
+                }
+                xs[r0 + tid] = v;
+                __syncwarp();
+                if (h == 0) {
+                    double u0 = 0.0, u1 = 0.0;
+#pragma unroll
+                    for (int c = 0; c < 32; c += 2) {
+                        u0 = fma(tile[r1 + tid][r0 + c], xs[r0 + c], u0);
+                        u1 = fma(tile[r1 + tid][r0 + c + 1], xs[r0 + c + 1], u1);
+                    }
+                    xs[r1 + tid] -= u0 + u1;
+                    __syncwarp();
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = b * TC_B + 32 * h + tid;
+                if (i < n) x[i] = good ? xs[32 * h + tid] : nan("");
+            }
+            __threadfence();
+            __syncwarp();
+            if (tid == 0) asm volatile("st.release.gpu.s32 [%0], %1;" ::"l"(flag + b), "r"(good ? 1 : 2) : "memory");
+        }
+        __syncthreads();
     }
 }
 
@@ -626,8 +818,7 @@ void gram64(const double* X, int64_t ldx, int64_t K, int m, double* C, int64_t l
     }
     const int64_t kslice = (steps + nslice - 1) / nslice * cgd::GD_ROWS;
     nslice = (K + kslice - 1) / kslice;
-    int* ex = nullptr;
-    ckd(cudaMallocAsync((void**)&ex, sizeof(int) * m, st), "column exponents");
+    int* ex = scratch_alloc<int>(m, st);
     ckd(cudaMemsetAsync(ex, 0x80, sizeof(int) * m, st), "column exponents");   // a very small value
     const unsigned strips = (unsigned)((m + 31) / 32);
     const unsigned gy = (unsigned)std::max<int64_t>(1, std::min<int64_t>((K + 63) / 64, 8 * sms / strips));
@@ -652,34 +843,41 @@ bool cholesky64(double* G, int n, int* d_info, cudaStream_t st, bool tensor_upda
     void* oz = nullptr;
     const bool use_oz = tensor_updates && cgd::CH_NB == 128 && n > cgd::CH_NB;
     if (use_oz) {
-        ckd(cudaMallocAsync(&oz, ozaki_scratch_bytes(n), st), "Ozaki scratch");
+        oz = scratch_alloc<unsigned char>(ozaki_scratch_bytes(n), st);
         ckd(cudaMemsetAsync(oz, 0, sizeof(int), st), "Ozaki error word");
     }
-    const size_t smem_potrf = (size_t)cgd::CH_NB * cgd::CH_NB * sizeof(double);
-    const size_t smem_trsm = ((size_t)cgd::CH_NB * cgd::CH_NB + (size_t)cgd::TR_R * cgd::TR_PLD + cgd::CH_NB) *
-                             sizeof(double);
-    ckd(cudaFuncSetAttribute(cgd::k_potrf_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_potrf),
-        "potrf smem");
-    ckd(cudaFuncSetAttribute(cgd::k_trsm_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_trsm),
-        "trsm smem");
-    for (int k = 0; k < n; k += cgd::CH_NB) {
-        const int kb = std::min(cgd::CH_NB, n - k);
-        cgd::k_potrf_block<<<1, 512, (size_t)kb * kb * sizeof(double), st>>>(G, n, k, kb, d_info);
+    int* arrived = scratch_alloc<int>(1, st);   // counter of a panel's CTAs
+    ckd(cudaMemsetAsync(arrived, 0, sizeof(int), st), "panel counter");
+    const int sms = sm_count();
+    const size_t most = 200 * 1024;
+    ckd(cudaFuncSetAttribute(cgd::k_chol_half, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most), "panel smem");
+    const int rmax = (int)(most / (cgd::CH_LD * sizeof(double))) - cgd::CH_H;
+    auto half = [&](int k, int kb, int second) {
         const int m = n - k - kb;
-        if (m > 0) {
-            const size_t sm = ((size_t)kb * kb + (size_t)cgd::TR_R * cgd::TR_PLD + kb) * sizeof(double);
-            cgd::k_trsm_panel<<<(m + cgd::TR_R - 1) / cgd::TR_R, cgd::TR_THREADS, sm, st>>>(G, n, k, kb, m);
-            // trailing update: A22 -= P P^T (P: rows k+kb.., columns k..k+kb, column-major)
-            if (use_oz && kb == 128)
-                syrk_update_ozaki(G + (int64_t)k * n + (k + kb), n, kb, m, -1.0, G + (int64_t)(k + kb) * n + (k + kb),
-                                  n, oz, st);
-            else
-                syrk_tn(G + (int64_t)k * n + (k + kb), n, kb, m, -1.0, G + (int64_t)(k + kb) * n + (k + kb), n, st);
+        const int R = std::max(8, std::min(rmax, (m + sms - 1) / sms));   // one share of the rows per SM
+        const int grid = std::max(1, (m + R - 1) / R);
+        cgd::k_chol_half<<<grid, cgd::CH_THREADS, (size_t)(cgd::CH_H + R) * cgd::CH_LD * sizeof(double), st>>>(
+            G, n, k, kb, m, R, second, d_info, arrived);
+    };
+    for (int k = 0; k < n; k += cgd::CH_NB) {
+        const int kb = std::min(cgd::CH_NB, n - k), k1 = std::min(cgd::CH_H, kb), k2 = kb - k1;
+        half(k, k1, 0);
+        if (k2 > 0) {
+            cgd::k_chol_strip<<<(n - k - k1 + cgd::ST_R - 1) / cgd::ST_R, 256, 0, st>>>(G, n, k, k2);
+            half(k + k1, k2, 1);
+        }
+        const int m = n - k - kb;
+        if (m > 0) {   // trailing update: A22 -= P P^T (P: rows k+kb.., columns k..k+kb, column-major)
+            const double* P = G + (int64_t)k * n + (k + kb);
+            double* C = G + (int64_t)(k + kb) * n + (k + kb);
+            if (use_oz && kb == 128) syrk_update_ozaki(P, n, kb, m, -1.0, C, n, oz, st);
+            else syrk_tn(P, n, kb, m, -1.0, C, n, st);
         }
         ckd(cudaGetLastError(), "cholesky step");
     }
     int info = 0, oz_err = 0;
     ckd(cudaMemcpyAsync(&info, d_info, sizeof(int), cudaMemcpyDeviceToHost, st), "info");
+    ckd(cudaFreeAsync(arrived, st), "panel counter");
     if (use_oz) {
         ckd(cudaMemcpyAsync(&oz_err, oz, sizeof(int), cudaMemcpyDeviceToHost, st), "Ozaki error word");
         ckd(cudaFreeAsync(oz, st), "Ozaki scratch");
@@ -692,27 +890,24 @@ bool cholesky64(double* G, int n, int* d_info, cudaStream_t st, bool tensor_upda
 
 void trsv64(const double* M, int64_t si, int64_t sj, int n, bool lower, double* x, cudaStream_t st) {
     if (n <= 0) return;
-    if (n <= cgd::TS_SMALL) {
+    if (n <= cgd::TS_CHAIN) {
         const size_t smem = (size_t)n * sizeof(double);
         ckd(cudaFuncSetAttribute(cgd::k_trsv_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(cgd::TS_SMALL * sizeof(double))),
+                                 (int)(cgd::TS_CHAIN * sizeof(double))),
             "trsv smem");
         cgd::k_trsv_small<<<1, cgd::TS_THREADS, smem, st>>>(M, si, sj, n, lower ? 1 : 0, x);
         ckd(cudaGetLastError(), "k_trsv_small");
         return;
     }
-    const int nb = (n + cgd::TS_BLOCK - 1) / cgd::TS_BLOCK;
-    const int grid = sm_count() * 4;
-    for (int bb = 0; bb < nb; ++bb) {
-        const int b = lower ? bb : nb - 1 - bb;
-        const int b0 = b * cgd::TS_BLOCK, bl = std::min(cgd::TS_BLOCK, n - b0);
-        // the diagonal block as a small system on x[b0 .. b0+bl)
-        cgd::k_trsv_small<<<1, cgd::TS_THREADS, (size_t)bl * sizeof(double), st>>>(M + b0 * si + b0 * sj, si, sj, bl,
-                                                                                   lower ? 1 : 0, x + b0);
-        const int r0 = lower ? b0 + bl : 0, r1 = lower ? n : b0;
-        if (r1 > r0) cgd::k_trsv_update<<<grid, 256, 0, st>>>(M, si, sj, b0, bl, r0, r1, x);
-        ckd(cudaGetLastError(), "trsv step");
-    }
+    const int nb = (n + cgd::TC_B - 1) / cgd::TC_B;
+    int* flag = scratch_alloc<int>(nb, st);
+    ckd(cudaMemsetAsync(flag, 0, sizeof(int) * nb, st), "trsv flags");
+    int lo = lower ? 1 : 0;
+    void* args[] = {(void*)&M, (void*)&si, (void*)&sj, (void*)&n, (void*)&lo, (void*)&x, (void*)&flag};
+    ckd(cudaLaunchCooperativeKernel((const void*)cgd::k_trsv_chain, dim3((unsigned)std::min(nb, sm_count())),
+                                    dim3(cgd::TC_THREADS), args, 0, st),
+        "k_trsv_chain");
+    ckd(cudaFreeAsync(flag, st), "trsv flags");
 }
 
 void cholesky_solve64(const double* L, int n, const double* h, double* x, cudaStream_t st) {
@@ -763,7 +958,7 @@ double fp64_fma_tflops(cudaStream_t st) {
     const int threads = 256, iters = 1 << 13;
     const int sms = sm_count();
     double* out = nullptr;
-    ckd(cudaMallocAsync((void**)&out, sizeof(double) * sms * 8 * threads, st), "peak scratch");
+    out = scratch_alloc<double>((size_t)sms * 8 * threads, st);
     cudaEvent_t e0, e1;
     ckd(cudaEventCreate(&e0), "event");
     ckd(cudaEventCreate(&e1), "event");
@@ -790,8 +985,8 @@ double fp64_fma_tflops(cudaStream_t st) {
     {   // and the register-blocked SYRK of this file on a 2048 x 4096 operand (FMA bound)
         const int K = 2048, m = 4096;
         double *X = nullptr, *C = nullptr;
-        ckd(cudaMallocAsync((void**)&X, sizeof(double) * K * m, st), "peak scratch");
-        ckd(cudaMallocAsync((void**)&C, sizeof(double) * m * m, st), "peak scratch");
+        X = scratch_alloc<double>((size_t)K * m, st);
+        C = scratch_alloc<double>((size_t)m * m, st);
         ckd(cudaMemsetAsync(X, 0, sizeof(double) * K * m, st), "peak scratch");   // finite operands
         ckd(cudaMemsetAsync(C, 0, sizeof(double) * m * m, st), "peak scratch");
         syrk_tn(X, m, K, m, 1.0, C, m, st);   // warm-up

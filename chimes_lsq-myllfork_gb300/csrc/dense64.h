@@ -23,8 +23,8 @@ void gram64(const double* X, int64_t ldx, int64_t K, int m, double* C, int64_t l
 // (row-major == column-major) storage: on return its column-major lower triangle
 // holds L (G = L L^T); the strict upper triangle of each diagonal block is zeroed and
 // the rest of the upper triangle keeps G's values.  128 x 128 diagonal
-// blocks are factorised in shared memory, the panel below by substitution against
-// the block, the trailing matrix by syrk_tn.  Returns false when a pivot is not
+// blocks are factorised in 64-wide halves in shared memory, the panel below against
+// them, the trailing matrix by exact digit products or syrk_tn.  Returns false when a pivot is not
 // positive (d_info: device int, first bad column + 1).
 bool cholesky64(double* G, int n, int* d_info, cudaStream_t st, bool tensor_updates = false);
 

@@ -24,6 +24,18 @@ cudaMemPool_t scratch_pool(int device);
 // device's free memory).
 void scratch_pool_trim(int device);
 
+// One stream-ordered allocation from the current device's scratch pool (cudaFreeAsync
+// returns it).  The default pool gives freed memory back to the driver at every
+// synchronisation, and a call that synchronises pays for mapping it again each time.
+template <typename T>
+T* scratch_alloc(size_t n, cudaStream_t st) {
+    int dev = 0;
+    void* p = nullptr;
+    CK(cudaGetDevice(&dev));
+    CK(cudaMallocFromPoolAsync(&p, std::max<size_t>(n * sizeof(T), 8), scratch_pool(dev), st));
+    return static_cast<T*>(p);
+}
+
 // Per-call scratch: stream-ordered device allocations from scratch_pool() released
 // at the end of the call, or -- for the no-allocation entry point -- a bump
 // allocator over the static device array below (256-byte aligned sub-buffers,

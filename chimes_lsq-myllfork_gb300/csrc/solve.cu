@@ -17,6 +17,7 @@
 
 #include "dense64.h"
 #include "gram.h"
+#include "scratch.h"
 
 namespace cg {
 
@@ -29,7 +30,7 @@ struct DevVec {
     double* p = nullptr;
     cudaStream_t st;
     DevVec(size_t n, cudaStream_t s) : st(s) {
-        cks(cudaMallocAsync((void**)&p, sizeof(double) * std::max<size_t>(n, 1), s), "solve scratch");
+        p = scratch_alloc<double>(n, s);
     }
     ~DevVec() { cudaFreeAsync(p, st); }
 };
