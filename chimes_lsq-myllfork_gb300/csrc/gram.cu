@@ -29,7 +29,9 @@
 #include <utility>
 
 #include "dense64.h"
+#include "digits.cuh"
 #include "gram.h"
+#include "scratch.h"
 
 namespace cgd {
 
@@ -482,22 +484,23 @@ __global__ void __launch_bounds__(GB_THREADS, 1)
 // (the Ozaki scheme: Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012).  Each
 // column i of X is scaled by a power of two s_i (|X / s_i| < 1) and split into OZ_S
 // signed digits, x / s_i = sum_a d_a 128^-(a+1) + r with |d_0| <= 128, |d_a| <= 64,
-// |r| < 2^-57, each an integer that BF16 holds exactly.  A digit product summed over
+// |r| <= 2^-57, each an integer that BF16 holds exactly.  A digit product summed over
 // K = 128 stays below 2^21 and the sum over the pairs (a, b) of one diagonal a + b = D
-// below 2^23, so the FP32 tensor-core accumulator of each diagonal is exact; the pairs
+// below 2^23 (D < 6: at most 2^22), so the FP32 tensor-core accumulator of each diagonal is exact; the pairs
 // with a + b >= OZ_S are dropped (below 2^-56 of the leading term), and the
 // epilogue packs sum_D S_D 128^-(D+2) into one 53-bit integer (scaled by s_i s_j).
 constexpr int OZ_S = 8;            // digits per element (57 bits)
 constexpr int OZ_K = 128;          // panel width (K, zero padded)
 constexpr int OZ_M = 128, OZ_N = 64;
-constexpr int OZ_THREADS = 192;    // warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
-constexpr int OZ_LD = 33;          // epilogue staging row (doubles)
+constexpr int OZ_EPI = 8;          // epilogue warps: two per TMEM lane quarter
+constexpr int OZ_THREADS = 64 + 32 * OZ_EPI;   // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
+constexpr int OZ_W = 16;           // columns per epilogue step
 constexpr int OZ_NBARS = 9;        // bfull, bempty, afull[2], aempty[2], tfull, tempty, done
 struct OzSmem {
     static constexpr uint32_t b = 0;                                          // OZ_S slices x 2 K halves x 8 KB
     static constexpr uint32_t a = b + OZ_S * 2 * (OZ_N * 128);                // 2 slots x 2 K halves x 16 KB
-    static constexpr uint32_t stage = a + 2 * 2 * (OZ_M * 128);               // 4 warps x 32 x OZ_LD doubles
-    static constexpr uint32_t bars = stage + 4 * 32 * OZ_LD * 8;
+    static constexpr uint32_t stage = a + 2 * 2 * (OZ_M * 128);               // OZ_EPI warps x 32 x OZ_W doubles
+    static constexpr uint32_t bars = stage + OZ_EPI * 32 * OZ_W * 8;
     static constexpr uint32_t total = bars + OZ_NBARS * 8 + 16;
 };
 static_assert(OzSmem::bars % 8 == 0, "mbarrier alignment");
@@ -505,45 +508,52 @@ static_assert(OzSmem::total + 1024 <= 227 * 1024, "shared memory per CTA");
 
 // Digit planes P[a][i][k] (bf16, k contiguous, a < OZ_S, i < mpad, k < OZ_K) and
 // scale exponents ex[i] (column i scaled by 2^-ex[i]) of the columns of X (K x m,
-// row-major, ldx).  Block: 32 columns.
+// row-major, ldx).  Block: 32 columns.  In integers from the numbers' bits: by FP64
+// multiplication and rint the 8 digits of 4,096 elements kept the FP64 pipe (2 per clock)
+// busy for 50 us.  A column that holds a NaN or an infinity has zero digits: the update
+// leaves its row and column as they are.
 __global__ void __launch_bounds__(256) k_oz_slice(const double* __restrict__ X, int64_t ldx, int K, int m, int mpad,
                                                   __nv_bfloat16* __restrict__ P, int* __restrict__ ex) {
     __shared__ double tile[OZ_K][33];
-    __shared__ double scs[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i0 = blockIdx.x * 32;
-    for (int k = w; k < OZ_K; k += 8) {
-        const int i = i0 + lane;
-        tile[k][lane] = (k < K && i < m) ? X[(int64_t)k * ldx + i] : 0.0;
-    }
-    __syncthreads();
-    for (int c = w; c < 32; c += 8) {   // column maximum -> power-of-two scale
-        double mx = 0.0;
-        for (int k = lane; k < OZ_K; k += 32) mx = fmax(mx, fabs(tile[k][c]));
-        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) {
-            int e = 0;
-            if (mx > 0.0) frexp(mx, &e);
-            scs[c] = ldexp(1.0, e);
-            if (i0 + c < mpad) ex[i0 + c] = e;
-        }
+    {
+        double v[OZ_K / 8];
+#pragma unroll
+        for (int u = 0; u < OZ_K / 8; ++u)
+            v[u] = (w + 8 * u < K && i0 + lane < m) ? X[(int64_t)(w + 8 * u) * ldx + i0 + lane] : 0.0;
+#pragma unroll
+        for (int u = 0; u < OZ_K / 8; ++u) tile[w + 8 * u][lane] = v[u];
     }
     __syncthreads();
     for (int c = w; c < 32; c += 8) {
         const int i = i0 + c;
         if (i >= mpad) continue;
-        const double inv = 1.0 / scs[c];   // a power of two: exact
+        int mx = 0;   // the column's largest high word: its exponent
+        for (int k = lane; k < OZ_K; k += 32) mx = max(mx, __double2hiint(tile[k][c]) & 0x7fffffff);
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        const int emax = max(mx >> 20, 1);   // |x| < 2^(emax - 1022)
+        const bool zero = mx == 0 || mx >= 0x7ff00000;
+        if (lane == 0) ex[i] = zero ? 0 : emax - 1022;
+        auto fixed = [&](double x) {         // x 2^(56 - ex) to nearest, |.| <= 2^56, plus 64 in each lower digit
+            const long long bits = __double_as_longlong(x);
+            const int ef = (int)((bits >> 52) & 0x7ff), s = max(ef, 1) - emax + 3;
+            long long v = (bits & 0xfffffffffffffll) | (ef ? 1ll << 52 : 0ll);
+            v = s >= 0 ? v << s : (s < -60 ? 0ll : (v + (1ll << (-s - 1))) >> -s);
+            return (zero ? 0ll : (bits < 0 ? -v : v)) + 64ll * (((1ll << 49) - 1) / 127);
+        };
         for (int h = 0; h < OZ_K; h += 64) {
             const int k = h + 2 * lane;
-            double y0 = tile[k][c] * inv, y1 = tile[k + 1][c] * inv;
+            const long long y0 = fixed(tile[k][c]), y1 = fixed(tile[k + 1][c]);
+            __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(P + (int64_t)i * OZ_K + k);
+            out[0] = __floats2bfloat162_rn((float)(int)(y0 >> 49), (float)(int)(y1 >> 49));
 #pragma unroll
-            for (int a = 0; a < OZ_S; ++a) {
-                const double t0 = y0 * 128.0, t1 = y1 * 128.0;
-                const double d0 = rint(t0), d1 = rint(t1);
-                y0 = t0 - d0;
-                y1 = t1 - d1;
-                const __nv_bfloat162 v = __floats2bfloat162_rn((float)d0, (float)d1);
-                *reinterpret_cast<__nv_bfloat162*>(P + ((int64_t)a * mpad + i) * OZ_K + k) = v;
+            for (int a = 1; a < OZ_S; ++a) {   // 0x4300 | b is the BF16 number 128 + b, b < 128
+                const unsigned b0 = (unsigned)(y0 >> (7 * (OZ_S - 1 - a))) & 127u;
+                const unsigned b1 = (unsigned)(y1 >> (7 * (OZ_S - 1 - a))) & 127u;
+                const unsigned pk = 0x43004300u | b0 | (b1 << 16);
+                out[(int64_t)a * mpad * (OZ_K / 2)] =
+                    __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&pk), __floats2bfloat162_rn(192.0f, 192.0f));
             }
         }
     }
@@ -589,7 +599,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         mbar_init(bempty, 1);
         for (int s = 0; s < 2; ++s) { mbar_init(&afull[s], 1); mbar_init(&aempty[s], 1); }
         mbar_init(tfull, 1);
-        mbar_init(tempty, 4);
+        mbar_init(tempty, OZ_EPI);
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -674,13 +684,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             umma_commit(done);
             mbar_wait(done, 0, err, 29);
         }
-    } else {   // epilogue warps 2..5
+    } else {   // epilogue warps 2..9
         const int q = warp & 3;   // TMEM lane quarter this warp may read
-        double* stg = reinterpret_cast<double*>(smem + OzSmem::stage) + (size_t)(warp - 2) * 32 * OZ_LD;
+        const int half = (warp - 2) / 4 * 32;   // its columns of the tile
+        double* stg = reinterpret_cast<double*>(smem + OzSmem::stage) + (size_t)(warp - 2) * 32 * OZ_W;
         auto prefetch_c = [&](int u) {   // the tile's rows of C into L2: 4 lines of 128 B per row
             int ti, tj;
             oz_tile(u, ntj, ti, tj);
-            for (int t = threadIdx.x - 64; t < OZ_M * 4; t += 128) {
+            for (int t = threadIdx.x - 64; t < OZ_M * 4; t += 32 * OZ_EPI) {
                 const int row = ti * OZ_M + t / 4, col = tj * OZ_N + (t % 4) * 16;
                 if (row < m && col < m) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (int64_t)row * ldc + col));
             }
@@ -690,65 +701,66 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         for (int u = blockIdx.x; u < ntiles; u += gridDim.x, ++j) {
             int ti, tj;
             oz_tile(u, ntj, ti, tj);
+            const int row0 = ti * OZ_M + q * 32;
+            const int erow = row0 + lane < m ? ex[row0 + lane] : 0;   // row r's exponent from lane r
             const bool got = mbar_wait(tfull, (uint32_t)j & 1u, err, 28);
             if (!__all_sync(0xffffffffu, got)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (*err == 0) {
-                // The diagonal sums S_D are exact integers below 2^23 (in FP32 registers).
+                // The diagonal sums S_D are exact integers in FP32: |S_D| <= 2^22 for D < 6,
+                // read from the bits of S_D + MAGIC, and below 2^23 for the last two.
                 // The element is sum_D S_D 2^(-7D-14) = V 2^-54 with the integer
                 //   V = sum_{D<6} S_D 2^(40-7D) + round((S_6 2^7 + S_7) / 2^9),   |V| < 2^62,
-                // so one conversion (rounding to 53 bits, as FP64 arithmetic would) and one
-                // FMA per element remain in FP64; the rounded tail moves V by at most 2^-55.
-                const int row0 = ti * OZ_M + q * 32;
+                // so one rounding to 53 bits (as FP64 arithmetic would) and one FMA per
+                // element remain in FP64; the rounded tail moves V by at most 2^-55.
 #pragma unroll 1
-                for (int c0 = 0; c0 < OZ_N; c0 += 32) {
-                    long long hi[32], lo[32];
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) hi[c] = lo[c] = 0;
-#pragma unroll 1
-                    for (int D = 0; D < OZ_S; ++D) {
-                        uint32_t v[32];
-                        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(D * OZ_N + c0);
-                        asm volatile(
-                            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
-                            "%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                              "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                              "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
-                              "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
-                              "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                            : "r"(taddr));
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        const int sh = D < 6 ? 40 - 7 * D : (D == 6 ? 7 : 0);
-#pragma unroll
-                        for (int c = 0; c < 32; ++c) {
-                            const long long sd = (long long)__float2int_rz(__uint_as_float(v[c])) << sh;
-                            if (D < 6) hi[c] += sd; else lo[c] += sd;
-                        }
-                    }
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) stg[lane * OZ_LD + c] = (double)(hi[c] + ((lo[c] + 256) >> 9));
-                    __syncwarp();
-                    const int col = tj * OZ_N + c0 + lane;
+                for (int c0 = half; c0 < half + 32; c0 += OZ_W) {
+                    // lane l < 16: column l of the even rows, l >= 16: of the odd ones
+                    const int cl = lane & (OZ_W - 1), col = tj * OZ_N + c0 + cl, rh = lane / OZ_W;
                     const int ecol = col < m ? ex[col] : 0;
-                    const int erow = row0 + lane < m ? ex[row0 + lane] : 0;   // row r's exponent from lane r
-                    double cold[32];   // all 32 reads in flight before the first write
+                    double cold[OZ_W];   // all reads in flight before the sums are unpacked
 #pragma unroll
-                    for (int r = 0; r < 32; ++r) {
-                        const int row = row0 + r;
+                    for (int r = 0; r < OZ_W; ++r) {
+                        const int row = row0 + 2 * r + rh;
                         cold[r] = (row < m && col < m && col >= row) ? C[(int64_t)row * ldc + col] : 0.0;
                     }
+                    uint32_t v[OZ_S][OZ_W];
 #pragma unroll
-                    for (int r = 0; r < 32; ++r) {
-                        const int row = row0 + r;
-                        const int e = __shfl_sync(0xffffffffu, erow, r) + ecol - 54;
-                        if (row < m && col < m && col >= row) {
-                            // alpha 2^(e_row + e_col - 54): a power of two times alpha
-                            const double f = (e > -1000 && e < 1000)
-                                                 ? alpha * __longlong_as_double((long long)(1023 + e) << 52)
-                                                 : ldexp(alpha, e);
-                            C[(int64_t)row * ldc + col] = fma(f, stg[r * OZ_LD + lane], cold[r]);
-                        }
+                    for (int D = 0; D < OZ_S; ++D) {
+                        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(D * OZ_N + c0);
+                        asm volatile(
+                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
+                            "%15}, [%16];"
+                            : "=r"(v[D][0]), "=r"(v[D][1]), "=r"(v[D][2]), "=r"(v[D][3]), "=r"(v[D][4]),
+                              "=r"(v[D][5]), "=r"(v[D][6]), "=r"(v[D][7]), "=r"(v[D][8]), "=r"(v[D][9]),
+                              "=r"(v[D][10]), "=r"(v[D][11]), "=r"(v[D][12]), "=r"(v[D][13]), "=r"(v[D][14]),
+                              "=r"(v[D][15])
+                            : "r"(taddr));
+                    }
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int c = 0; c < OZ_W; ++c) {
+                        auto bits = [&](int D) { return __float_as_uint(__uint_as_float(v[D][c]) + MAGIC); };
+                        constexpr unsigned k0 = MAGIC_BITS * 129u;
+                        const int t01 = (int)(bits(0) * 128u + bits(1) - k0);
+                        const int t23 = (int)(bits(2) * 128u + bits(3) - k0);
+                        const int t45 = (int)(bits(4) * 128u + bits(5) - k0);
+                        const int t67 = __float2int_rz(__uint_as_float(v[6][c])) * 128 +
+                                        __float2int_rz(__uint_as_float(v[7][c]));
+                        const long long V = (((long long)t01 << 28) + ((long long)t23 << 14) + t45) * 32 +
+                                            ((t67 + 256) >> 9);
+                        // rows of 16, columns rotated by the row: no bank conflicts either way
+                        stg[lane * OZ_W + (c ^ (lane & (OZ_W - 1)))] = __longlong_as_double(V);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int r = 0; r < OZ_W; ++r) {
+                        const int lr = 2 * r + rh, row = row0 + lr;
+                        const int e = __shfl_sync(0xffffffffu, erow, lr) + ecol - 54;
+                        if (row < m && col < m && col >= row)
+                            C[(int64_t)row * ldc + col] =
+                                fma(alpha, from_fixed(__double_as_longlong(stg[lr * OZ_W + (cl ^ (lr & (OZ_W - 1)))]), e),
+                                    cold[r]);
                     }
                     __syncwarp();
                 }
@@ -851,8 +863,7 @@ void gram_accumulate(int prec_in, const void* A, int64_t lda, int64_t nrows, int
     enum { S_ATB = 11, S_SPLIT = 12, S_TC = 13, S_SYRK = 14 };
     if (mode == 0) {   // h += A^T b (FP64, reproducible), then the FP64 SYRK of the block
         if (prec_in != 0) throw std::runtime_error("the FP64 Gram needs an FP64 A");
-        double* partial = nullptr;
-        ck(cudaMallocAsync((void**)&partial, sizeof(double) * atb_partial_doubles(nrows, ncols), st), "atb scratch");
+        double* partial = scratch_alloc<double>(atb_partial_doubles(nrows, ncols), st);
         mark(S_ATB, true);
         gemv_cols64((const double*)A, lda, nrows, ncols, b, h, partial, st);
         mark(S_ATB, false);
@@ -891,11 +902,10 @@ void gram_accumulate(int prec_in, const void* A, int64_t lda, int64_t nrows, int
     const int64_t ktiles_max = (std::min(rblock, nrows) + cgd::SPA_K - 1) / cgd::SPA_K;
     const int resident = prec_in == 0 ? split_atb_resident<double>() : split_atb_resident<float>();
     const int gx = (int)std::max<int64_t>(1, std::min<int64_t>(ktiles_max, resident / nstrip));
-    double* partial = nullptr;
     float2* bsplit = nullptr;
-    ck(cudaMallocAsync((void**)&partial, sizeof(double) * gx * ncols, st), "atb scratch");
+    double* partial = scratch_alloc<double>((size_t)gx * ncols, st);
     const int64_t kpad_max = (std::min(rblock, nrows) + cgd::GB_K - 1) / cgd::GB_K * cgd::GB_K;
-    if (prec_in != 0) ck(cudaMallocAsync((void**)&bsplit, sizeof(float2) * kpad_max, st), "b split scratch");
+    if (prec_in != 0) bsplit = scratch_alloc<float2>(kpad_max, st);
     for (int64_t r0 = 0; r0 < nrows; r0 += rblock) {
         const int64_t nr = std::min(rblock, nrows - r0);
         const int64_t kpad = (nr + cgd::GB_K - 1) / cgd::GB_K * cgd::GB_K;
