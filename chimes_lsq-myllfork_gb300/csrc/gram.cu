@@ -168,10 +168,30 @@ __global__ void k_split_reduce(const double* __restrict__ partial, int nslices, 
     h[c] += s;
 }
 
-__global__ void k_symmetrize(double* G, int n) {
-    const int i = blockIdx.y * blockDim.y + threadIdx.y;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && j < n && j < i) G[(int64_t)i * n + j] = G[(int64_t)j * n + i];
+// The strict lower triangle from the upper one, a 64 x 64 tile of the upper triangle per
+// CTA, transposed through shared memory with 16 reads in flight per thread.  Reads and
+// writes of n^2 / 2 entries each bound it; one thread per entry read column-wise: n = 6,007
+// 108 -> 55 us (42 us at the copy rate).
+constexpr int SY_B = 64, SY_THREADS = 256;
+__global__ void __launch_bounds__(SY_THREADS) k_symmetrize(double* __restrict__ G, int n) {
+    __shared__ double t[SY_B][SY_B + 1];
+    const int bi = blockIdx.y, bj = blockIdx.x;
+    if (bj < bi) return;
+    const int c = threadIdx.x % SY_B, r = threadIdx.x / SY_B;
+    constexpr int N = SY_B * SY_B / SY_THREADS, RS = SY_THREADS / SY_B;
+    const int i0 = bi * SY_B, j0 = bj * SY_B;
+    double v[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+        v[u] = i0 + r + RS * u < n && j0 + c < n ? G[(int64_t)(i0 + r + RS * u) * n + j0 + c] : 0.0;
+#pragma unroll
+    for (int u = 0; u < N; ++u) t[r + RS * u][c] = v[u];
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        const int j = j0 + r + RS * u, i = i0 + c;
+        if (j < n && i < j) G[(int64_t)j * n + i] = t[c][r + RS * u];
+    }
 }
 
 // ---------------------------------------------------------------- PTX helpers
@@ -1002,8 +1022,9 @@ void syrk_update_ozaki(const double* X, int64_t ldx, int K, int m, double alpha,
 
 void gram_symmetrize(double* G, int n, bool from_upper, cudaStream_t st) {
     (void)from_upper;
-    dim3 grid((n + 31) / 32, (n + 31) / 32);
-    cgd::k_symmetrize<<<grid, dim3(32, 32), 0, st>>>(G, n);
+    if (n <= 0) return;
+    const unsigned nb = (unsigned)((n + cgd::SY_B - 1) / cgd::SY_B);
+    cgd::k_symmetrize<<<dim3(nb, nb), cgd::SY_THREADS, 0, st>>>(G, n);
     ck(cudaGetLastError(), "k_symmetrize");
 }
 

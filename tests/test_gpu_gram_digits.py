@@ -79,3 +79,17 @@ def test_non_finite_columns(cg, tmp_path):
     bad[[5, 100]] = True
     up = np.triu(np.ones((150, 150), bool))
     assert np.array_equal(~np.isfinite(G) & up, (bad[:, None] | bad[None, :]) & up)
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 129, 820])
+def test_gram_finish_mirrors_the_upper_triangle(cg, tmp_path, n):
+    torch = pytest.importorskip("torch")
+    import ctypes
+    import importlib
+    synth = importlib.import_module("chimes_lsq-myllfork_gb300.synth")
+    sess = cg.Session(cg.Model(synth.make_workload("water-2b", str(tmp_path), nframes=1, seed=3)), 0)
+    G = torch.randn((n, n), dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(n))
+    U = torch.triu(G)
+    assert cg.lib().cg_gram_finish(sess._h, ctypes.c_void_p(G.data_ptr()), n) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(G, U + torch.triu(U, 1).T)
