@@ -10,6 +10,8 @@
 // The reference decides membership with FP64 distances; every candidate is first
 // screened with an FP32 distance (margin 1e-2 A, far above FP32 error) and only
 // candidates near a cut-off are re-decided with the exact FP64 sequence.
+#include <cooperative_groups.h>
+
 #include "dev.cuh"
 #include "kernels.h"
 
@@ -596,39 +598,43 @@ __global__ void k_quads(ModelDev M, FramesDev F, NeighDev NB, ClusterSet CS, int
 }
 
 // ---------------------------------------------------------------- bucketing
-// Stable counting sort of one frame's items by key, one CTA per frame.  The items
-// are split into contiguous ranges, one per warp (as many warps as the per-warp key
-// counts fit in shared memory); each warp counts the keys of its range, a scan turns
-// the counts into a start for every (key, warp), and each warp then places its range
-// in order, 32 items at a time, ranking equal keys with __match_any_sync.  Within a
-// key the items keep their order, so the result does not depend on timing.
+// Stable counting sort of one frame's items by key, one cluster of up to 8 CTAs per frame.
+// The items are split into contiguous ranges, one per warp (as many warps as the per-warp
+// key counts fit in shared memory); each warp counts the keys of its range, a scan over the
+// cluster's counts (distributed shared memory) gives a start for every (key, warp), and
+// each warp then places its range in order, ranking equal keys with __match_any_sync.
+// Within a key the items keep their order, so the result depends neither on timing nor on
+// the number of CTAs.  A warp's chain of loads and ranks bounds it (32 items a step), so
+// warps are what helps: 8 frames of 33 to 1,001 atoms, five sorts, one CTA a frame -> a
+// cluster: 919 -> 141 us.
 constexpr int BUCKET_THREADS = 512;
 constexpr int BUCKET_MAX_KEYS = 8192;
-constexpr int BUCKET_SMEM_INTS = 24576;   // per-warp key counts + key starts (96 KB)
+constexpr int BUCKET_SMEM_INTS = 24576;   // per-warp key counts + key totals (96 KB)
+constexpr int BUCKET_U = 4;               // items in flight per lane
 
-__device__ __forceinline__ void bucket_item(const BucketSpec& S, int N, int64_t base, int64_t t, int& key, int& val) {
+// t < nunits * members of the frame: the values are ints, so 32 bits hold it
+__device__ __forceinline__ void bucket_item(const BucketSpec& S, int N, int64_t base, unsigned t, int& key, int& val) {
     if (S.kind == 0) {
-        int64_t p = base + (t >> 1);
-        int e = (int)(t & 1);
-        key = e == 0 ? S.i2[p] : S.g2[p] % N;
+        const int64_t p = base + (t >> 1);
+        key = (t & 1u) == 0 ? S.i2[p] : S.g2[p] % N;
         val = (int)t;
     } else if (S.kind == 1) {
-        int64_t q = base + t / S.nb;
-        int e = (int)(t % S.nb);
-        int4 mm = S.m[q];
-        int g = e == 0 ? mm.x : (e == 1 ? mm.y : (e == 2 ? mm.z : mm.w));
-        key = g % N;
-        val = (int)((t / S.nb) * 4 + e);
+        const unsigned q = S.nb == 3 ? t / 3u : t / 4u;
+        const unsigned e = t - q * (unsigned)S.nb;
+        key = reinterpret_cast<const int*>(S.m + base + q)[e] % N;
+        val = (int)(q * 4u + e);
     } else {
         key = S.type[base + t];
         val = (int)t;
     }
 }
 
-__global__ void __launch_bounds__(BUCKET_THREADS) k_bucket(FramesDev F, BucketSpec S, Buckets out) {
+__global__ void __launch_bounds__(BUCKET_THREADS, 2) k_bucket(FramesDev F, BucketSpec S, Buckets out) {
     extern __shared__ int bsm[];
-    __shared__ int part[BUCKET_THREADS];
-    const int f = blockIdx.x;
+    __shared__ int part[BUCKET_THREADS / 32];
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int f = blockIdx.x / C;
     const int N = F.natoms[f];
     // pair items live in the neighbour CSR, which is indexed by global real atom
     const int64_t base = S.item_frame_ofs[f];
@@ -641,61 +647,88 @@ __global__ void __launch_bounds__(BUCKET_THREADS) k_bucket(FramesDev F, BucketSp
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int W = max(1, min((int)(blockDim.x >> 5), (BUCKET_SMEM_INTS - K) / max(K, 1)));
     int* cntw = bsm;            // [W][K]: counts, then starts
-    int* kst = bsm + W * K;     // [K]: totals, then starts
+    int* tot = bsm + W * K;     // [K]: this CTA's totals, read by the cluster
     for (int k = threadIdx.x; k < W * K; k += blockDim.x) cntw[k] = 0;
     __syncthreads();
-    const int64_t chunk = (nitems + W - 1) / W;
-    const int64_t r0 = min(nitems, (int64_t)warp * chunk), r1 = min(nitems, r0 + chunk);
+    const int64_t chunk = (nitems + W * C - 1) / (W * C);
+    const int64_t r0 = min(nitems, (int64_t)(rank * W + warp) * chunk), r1 = min(nitems, r0 + chunk);
+    int* cnt = cntw + warp * K;
+    // the next BUCKET_U x 32 items from c0 on; items past the range get a key of their own
+    auto load = [&](int64_t c0, int (&key)[BUCKET_U], int (&val)[BUCKET_U]) {
+#pragma unroll
+        for (int u = 0; u < BUCKET_U; ++u) {
+            const int64_t t = c0 + 32 * u + lane;
+            key[u] = -1 - lane;
+            val[u] = 0;
+            if (t < r1) bucket_item(S, N, base, (unsigned)t, key[u], val[u]);
+        }
+    };
     if (warp < W) {
-        for (int64_t t = r0 + lane; t < r1; t += 32) {
-            int key, val;
-            bucket_item(S, N, base, t, key, val);
-            atomicAdd(&cntw[warp * K + key], 1);
+        for (int64_t c0 = r0; c0 < r1; c0 += 32 * BUCKET_U) {
+            int key[BUCKET_U], val[BUCKET_U];
+            load(c0, key, val);
+#pragma unroll
+            for (int u = 0; u < BUCKET_U; ++u) if (key[u] >= 0) atomicAdd(&cnt[key[u]], 1);
         }
     }
     __syncthreads();
-    // per key: starts of each warp's share relative to the key, and the key's total
+    // per key: starts of each warp's share relative to the CTA's, and the CTA's total
     for (int k = threadIdx.x; k < K; k += blockDim.x) {
         int run = 0;
         for (int w = 0; w < W; ++w) { const int v = cntw[w * K + k]; cntw[w * K + k] = run; run += v; }
-        kst[k] = run;
+        tot[k] = run;
     }
-    __syncthreads();
-    // exclusive scan of the key totals
+    cl.sync();
+    // exclusive scan of the key totals, by every CTA for itself
     const int per = (K + blockDim.x - 1) / blockDim.x;
-    const int k0 = threadIdx.x * per, k1 = min(K, k0 + per);
-    int local = 0;
-    for (int k = k0; k < k1; ++k) local += kst[k];
-    part[threadIdx.x] = local;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int w = 0; w < (int)blockDim.x; ++w) { int v = part[w]; part[w] = run; run += v; }
+    const int k0 = min(K, (int)threadIdx.x * per), k1 = min(K, k0 + per);
+    auto totals = [&](int k, int& low) {   // key k's total, and the share of the CTAs before this one
+        int t = 0;
+        low = 0;
+        for (int c = 0; c < C; ++c) {
+            const int v = *cl.map_shared_rank(tot + k, c);
+            if (c < rank) low += v;
+            t += v;
+        }
+        return t;
+    };
+    int local = 0, low;
+    for (int k = k0; k < k1; ++k) local += totals(k, low);
+    int incl = local;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
     }
+    if (lane == 31) part[warp] = incl;
     __syncthreads();
-    int run = part[threadIdx.x];
-    for (int k = k0; k < k1; ++k) { int v = kst[k]; kst[k] = run; out.key_ofs[kbase + k] = vbase + run; run += v; }
-    if (threadIdx.x == 0) out.key_ofs[kbase + K] = vbase + nitems;
-    __syncthreads();
-    for (int k = threadIdx.x; k < W * K; k += blockDim.x) cntw[k] += kst[k % K];
-    __syncthreads();
+    int run = incl - local;
+    for (int w = 0; w < warp; ++w) run += part[w];
+    for (int k = k0; k < k1; ++k) {
+        const int t = totals(k, low);
+        for (int w = 0; w < W; ++w) cntw[w * K + k] += run + low;
+        if (rank == 0) out.key_ofs[kbase + k] = vbase + run;
+        run += t;
+    }
+    if (rank == 0 && threadIdx.x == 0) out.key_ofs[kbase + K] = vbase + nitems;
+    cl.sync();   // the others have read this CTA's totals; its starts are in place
     if (warp < W) {
-        int* cnt = cntw + warp * K;
-        for (int64_t c0 = r0; c0 < r1; c0 += 32) {
-            int64_t t = c0 + lane;
-            bool act = t < r1;
-            int key = -1 - lane, val = 0;
-            if (act) bucket_item(S, N, base, t, key, val);
-            unsigned peers = __match_any_sync(0xffffffffu, key);
-            int leader = __ffs(peers) - 1;
-            int rank = __popc(peers & ((1u << lane) - 1u));
-            int start = 0;
-            if (act && lane == leader) start = cnt[key];
-            start = __shfl_sync(0xffffffffu, start, leader);
-            if (act) out.val[vbase + start + rank] = val;
-            __syncwarp();
-            if (act && lane == leader) cnt[key] = start + __popc(peers);
-            __syncwarp();
+        for (int64_t c0 = r0; c0 < r1; c0 += 32 * BUCKET_U) {
+            int key[BUCKET_U], val[BUCKET_U];
+            load(c0, key, val);
+#pragma unroll
+            for (int u = 0; u < BUCKET_U; ++u) {
+                const unsigned peers = __match_any_sync(0xffffffffu, key[u]);
+                const int leader = __ffs(peers) - 1;
+                int start = 0;
+                if (key[u] >= 0 && lane == leader) {
+                    start = cnt[key[u]];
+                    cnt[key[u]] = start + __popc(peers);
+                }
+                start = __shfl_sync(0xffffffffu, start, leader);
+                if (key[u] >= 0) out.val[vbase + start + __popc(peers & ((1u << lane) - 1u))] = val[u];
+                __syncwarp();   // the next 32 items' leaders see the new starts
+            }
         }
     }
 }
@@ -745,7 +778,25 @@ void launch_bucket(int nframes, const FramesDev& F, const BucketSpec& S, const B
     if (nframes <= 0) return;
     const int smem = BUCKET_SMEM_INTS * (int)sizeof(int);
     cudaFuncSetAttribute(k_bucket, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k_bucket<<<nframes, BUCKET_THREADS, smem, st>>>(F, S, out);
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // two CTAs fit on an SM: no more than the GPU takes at once (with 8 frames, 8 CTAs each are
+    // 6.5x as fast as one; 16 would need the non-portable cluster size)
+    unsigned c = 8;
+    while (c > 1 && (int64_t)nframes * c > 2 * sms) c >>= 1;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = c;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)nframes * c);
+    cfg.blockDim = dim3(BUCKET_THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_bucket, F, S, out);
 }
 
 }  // namespace cgd
