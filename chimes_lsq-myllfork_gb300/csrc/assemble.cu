@@ -534,14 +534,16 @@ __global__ void __launch_bounds__(NT, NBODY == 3 ? (sizeof(R) == 4 ? 3 : 2) : 1)
 // finished by the thread holding its first power, which adds its neighbours' partial
 // sums from shared memory in thread order (so the result does not depend on timing).
 // The clusters of every owner role of a type are tabulated together, CB at a time,
-// and each thread reads each power's table entries for each role from offsN.  With no
+// and each thread reads each power's table entries for each role, laid out so that a warp's
+// reads are contiguous (4-body FP32 rows of 8 uneven frames, in power order -> so: 3,130 ->
+// 2,490 us; each lane had its own cache line).  With no
 // per-power accumulator arrays two CTAs fit on an SM, and one CTA's table building
 // and barriers overlap the other's FMAs.  blockDim.x (at most rg_max_threads) is chosen
 // by the host (rg_threads).  The frame's PERM_SCALE is folded into the Q table.
 template <int NBODY, typename R>
 __global__ void __launch_bounds__(rg_max_threads((int)sizeof(R)), 2) k_force_rg(ModelDev M, FramesDev F, ClusterSet CS, Buckets inc,
-                                                    const int64_t* key_frame_ofs, const R* __restrict__ pre,
-                                                    R* A, int64_t lda) {
+                                                    const int64_t* key_frame_ofs, RgTables rg,
+                                                    const R* __restrict__ pre, R* A, int64_t lda) {
     constexpr int NP = NBODY == 3 ? 3 : 6;
     constexpr int NI = NBODY - 1;
     constexpr int NO = NP - NI;
@@ -552,8 +554,6 @@ __global__ void __launch_bounds__(rg_max_threads((int)sizeof(R)), 2) k_force_rg(
     const ClusterTypeDev* types = NBODY == 3 ? M.types3 : M.types4;
     const int* grps = NBODY == 3 ? M.grp3 : M.grp4;
     const int8_t* revs = NBODY == 3 ? M.rev3 : M.rev4;
-    const uint4* offs = NBODY == 3 ? M.offs3 : M.offs4;
-    const int* tcol = NBODY == 3 ? M.tcol3 : M.tcol4;
     int sizeI = 1, sizeO = 1;
     for (int k = 0; k < NI; ++k) sizeI *= ord;
     for (int k = 0; k < NO; ++k) sizeO *= ord;
@@ -593,17 +593,19 @@ __global__ void __launch_bounds__(rg_max_threads((int)sizeof(R)), 2) k_force_rg(
     for (int64_t c0 = e0; c0 < e1; c0 += MB_MAX_ENT) {
         const int nent = (int)min((int64_t)MB_MAX_ENT, e1 - c0);
         sort_incidences<NBODY>(CS, inc, revs, typ, N, qbase, c0, nent, nkeys, sEnt, sKey, sOrd, sCnt);
-        for (int T = 0; T < ntypes; ++T) {
+        const uint4* __restrict__ offs = rg.offs + tid;
+        const int* __restrict__ cols = rg.col + tid;
+        int S = 0;
+        for (int T = 0; T < ntypes; ++T, offs += S * NT, cols += S * NT) {
             const int gbeg = T == 0 ? 0 : sCnt[T * 4 - 1], gend = sCnt[T * 4 + 3];
             const ClusterTypeDev& CT = types[T];
             const int n = CT.n_allowed;
+            S = (n + NT - 1) / NT;                             // powers per thread
             if (gbeg == gend || n == 0) continue;
-            const int S = (n + NT - 1) / NT;                   // powers per thread
-            const int pb = min(n, tid * S), pe = min(n, pb + S);
-            const int tb = CT.pow_offset / NP;                 // the type's first power in offs / tcol
+            const int np = min(n, tid * S + S) - min(n, tid * S);
             R* const acol = arow + CT.col_base;
             // the thread's first column began in an earlier thread's range
-            const bool head = pb < pe && pb > 0 && tcol[tb + pb - 1] == tcol[tb + pb];
+            const bool head = np > 0 && (cols[0] & RG_CONT);
             for (int ch0 = gbeg; ch0 < gend; ch0 += CB) {
                 const int nb = min(CB, gend - ch0);
                 const bool add = !single_pass || ch0 > gbeg;   // later chunks add to the rows
@@ -723,16 +725,16 @@ __global__ void __launch_bounds__(rg_max_threads((int)sizeof(R)), 2) k_force_rg(
                 R ax = R(0), ay = R(0), az = R(0);
                 int pcol = -1;
                 bool first = true;   // still in the thread's first column
-                for (int p = pb; p < pe; ++p) {
-                    const int col = tcol[tb + p];
-                    if (p > pb && col != pcol) {   // column pcol ended at p - 1
+                for (int i = 0; i < np; ++i) {
+                    const int col = cols[i * NT];
+                    const uint4 o4 = offs[i * NT];
+                    if (i > 0 && !(col & RG_CONT)) {   // column pcol ended at the power before
                         if (first && head) { sPart[3 * tid] = ax; sPart[3 * tid + 1] = ay; sPart[3 * tid + 2] = az; }
-                        else put(pcol, ax, ay, az);
+                        else put(pcol & ~(RG_CONT | RG_LAST), ax, ay, az);
                         first = false;
                         ax = ay = az = R(0);
                     }
                     pcol = col;
-                    const uint4 o4 = offs[tb + p];
                     const uint32_t ow[4] = {o4.x, o4.y, o4.z, o4.w};
 #pragma unroll
                     for (int r = 0; r < NBODY; ++r) {
@@ -745,8 +747,9 @@ __global__ void __launch_bounds__(rg_max_threads((int)sizeof(R)), 2) k_force_rg(
                     }
                 }
                 bool tail = false;   // the last column continues into later ranges
-                if (pb < pe) {
-                    const bool ends = pe == n || tcol[tb + pe] != pcol;
+                const bool ends = pcol & RG_LAST;
+                pcol &= ~(RG_CONT | RG_LAST);
+                if (np > 0) {
                     if (first && head) { sPart[3 * tid] = ax; sPart[3 * tid + 1] = ay; sPart[3 * tid + 2] = az; }
                     else if (ends) put(pcol, ax, ay, az);
                     else tail = true;
@@ -1073,10 +1076,10 @@ static void force_mb_ppt(int ppt, int nreal, size_t smem, const ModelDev& M, con
 }
 
 template <int NBD, typename R>
-static void force_rg(int nreal, int nt, size_t smem, const ModelDev& M, const FramesDev& F, const ClusterSet& CS,
+static void force_rg(int nreal, const RgTables& rg, size_t smem, const ModelDev& M, const FramesDev& F, const ClusterSet& CS,
                      const Buckets& inc, const int64_t* kfo, const R* pre, R* A, int64_t lda, cudaStream_t st) {
     set_smem(k_force_rg<NBD, R>, smem);
-    k_force_rg<NBD, R><<<nreal, nt, smem, st>>>(M, F, CS, inc, kfo, pre, A, lda);
+    k_force_rg<NBD, R><<<nreal, rg.nt, smem, st>>>(M, F, CS, inc, kfo, rg, pre, A, lda);
 }
 
 int rg_threads(const int* n_allowed, int ntypes, int rsize) {
@@ -1095,17 +1098,17 @@ int rg_threads(const int* n_allowed, int ntypes, int rsize) {
     return best;
 }
 
-void launch_force_rg(int nbody, int prec, int nreal, int nt, size_t smem, const ModelDev& M, const FramesDev& F,
+void launch_force_rg(int nbody, int prec, int nreal, const RgTables& rg, size_t smem, const ModelDev& M, const FramesDev& F,
                      const ClusterSet& CS, const Buckets& inc, const int64_t* kfo, const void* pre, void* A,
                      int64_t lda, cudaStream_t st) {
     if (nbody == 3 && prec == 0)
-        force_rg<3, double>(nreal, nt, smem, M, F, CS, inc, kfo, (const double*)pre, (double*)A, lda, st);
+        force_rg<3, double>(nreal, rg, smem, M, F, CS, inc, kfo, (const double*)pre, (double*)A, lda, st);
     else if (nbody == 3)
-        force_rg<3, float>(nreal, nt, smem, M, F, CS, inc, kfo, (const float*)pre, (float*)A, lda, st);
+        force_rg<3, float>(nreal, rg, smem, M, F, CS, inc, kfo, (const float*)pre, (float*)A, lda, st);
     else if (prec == 0)
-        force_rg<4, double>(nreal, nt, smem, M, F, CS, inc, kfo, (const double*)pre, (double*)A, lda, st);
+        force_rg<4, double>(nreal, rg, smem, M, F, CS, inc, kfo, (const double*)pre, (double*)A, lda, st);
     else
-        force_rg<4, float>(nreal, nt, smem, M, F, CS, inc, kfo, (const float*)pre, (float*)A, lda, st);
+        force_rg<4, float>(nreal, rg, smem, M, F, CS, inc, kfo, (const float*)pre, (float*)A, lda, st);
 }
 
 void launch_force_mb(int nbody, int prec, int ppt, int nreal, size_t smem, const ModelDev& M, const FramesDev& F,

@@ -137,9 +137,9 @@ void launch_cluster_basis(int nbody, int prec, int64_t nclusters, const ModelDev
 void launch_force_mb(int nbody, int prec, int ppt, int nreal, size_t smem, const ModelDev& M, const FramesDev& F,
                      const ClusterSet& CS, const Buckets& inc, const int64_t* key_frame_ofs, const void* pre,
                      void* A, int64_t lda, cudaStream_t st, int nt4 = MB_THREADS);
-// The same rows by the range form (k_force_rg) on nt threads per CTA;
-// smem = mb_range_smem(..., nt, ...).total.
-void launch_force_rg(int nbody, int prec, int nreal, int nt, size_t smem, const ModelDev& M, const FramesDev& F,
+// The same rows by the range form (k_force_rg) on rg.nt threads per CTA;
+// smem = mb_range_smem(..., rg.nt, ...).total.
+void launch_force_rg(int nbody, int prec, int nreal, const RgTables& rg, size_t smem, const ModelDev& M, const FramesDev& F,
                      const ClusterSet& CS, const Buckets& inc, const int64_t* key_frame_ofs, const void* pre,
                      void* A, int64_t lda, cudaStream_t st);
 // Work lists of a call: the cluster bases, their magnitudes (one int per slot), the owners'

@@ -57,14 +57,19 @@ struct ModelDev {
     const ClusterTypeDev* types4;
     const uint8_t* pow4;
     const int* grp4;
-    // Per allowed power (indexed pow_offset / nslots + p): for each canonical role pi
-    // of the owner, the power's entries in a cluster's force table (see k_force_rg):
-    // low 16 bits the M_x index, high 16 bits the Q index.  And the column of the
-    // power within its type (PARAM_INDICES).
-    const uint4* offs3;
-    const int* tcol3;
-    const uint4* offs4;
-    const int* tcol4;
+};
+
+// Powers of the cluster types as k_force_rg's threads read them: of a type with n allowed
+// powers thread t of nt takes p = t S + i, i < S = ceil(n / nt), found at i nt + t behind
+// the earlier types' S nt.  offs: for each canonical role of the owner the power's entries
+// in a cluster's force table, low 16 bits the M_x index, high 16 bits the Q index.  col: the
+// power's column within its type (PARAM_INDICES), RG_CONT set if the power before it has the
+// same one, RG_LAST if the power behind it has not.
+constexpr int RG_CONT = 1 << 30, RG_LAST = 1 << 29;
+struct RgTables {
+    const uint4* offs = nullptr;
+    const int* col = nullptr;
+    int nt = 0;
 };
 
 // Column tables of the digit-product kernels (tensor_rows.cu), one set per cluster list:

@@ -46,8 +46,8 @@ static void rev_index(const ClusterType& ct, const int* types, int n, int8_t* ou
 
 static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, int col_base, int pchunk, DeviceModel& D,
                         const int** int_map, const int8_t** pidx, const int8_t** rev, const cgd::ClusterTypeDev** types,
-                        const uint8_t** pows, const int** grps, const uint4** offs, const int** tcols, int& max_allowed,
-                        cgd::OzTables& oz) {
+                        const uint8_t** pows, const int** grps, int& max_allowed, cgd::OzTables& oz,
+                        cgd::RgTables (&rg)[2]) {
     const int np = nb == 3 ? 3 : 6;
     const int dim = nb == 3 ? 1000 : 10000;
     std::vector<int> imap(dim, -1);
@@ -171,9 +171,29 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
     *types = dev_upload(D.allocs, tv.data(), tv.size());
     *pows = dev_upload(D.allocs, pw.data(), pw.size());
     *grps = dev_upload(D.allocs, gp.data(), gp.size());
-    if (of.empty()) { of.push_back(make_uint4(0, 0, 0, 0)); tc.push_back(0); }
-    *offs = dev_upload(D.allocs, of.data(), of.size());
-    *tcols = dev_upload(D.allocs, tc.data(), tc.size());
+    std::vector<int> na;
+    for (const auto& d : tv) na.push_back(d.n_allowed);
+    for (int prec = 0; prec < 2; ++prec) {
+        const int nt = cgd::rg_threads(na.data(), (int)na.size(), prec == 0 ? 8 : 4);
+        std::vector<uint4> ro;
+        std::vector<int> rc;
+        for (const auto& d : tv) {
+            const int n = d.n_allowed, S = (n + nt - 1) / nt, p0 = d.pow_offset / np;
+            const size_t at = ro.size();
+            ro.resize(at + (size_t)S * nt, make_uint4(0, 0, 0, 0));
+            rc.resize(at + (size_t)S * nt, 0);
+            for (int p = 0; p < n; ++p) {
+                const size_t q = at + (size_t)(p % S) * nt + p / S;
+                ro[q] = of[p0 + p];
+                rc[q] = tc[p0 + p] | (p > 0 && tc[p0 + p - 1] == tc[p0 + p] ? cgd::RG_CONT : 0) |
+                        (p == n - 1 || tc[p0 + p + 1] != tc[p0 + p] ? cgd::RG_LAST : 0);
+            }
+        }
+        if (ro.empty()) { ro.push_back(make_uint4(0, 0, 0, 0)); rc.push_back(0); }
+        rg[prec].offs = dev_upload(D.allocs, ro.data(), ro.size());
+        rg[prec].col = dev_upload(D.allocs, rc.data(), rc.size());
+        rg[prec].nt = nt;
+    }
 }
 
 DeviceModel::DeviceModel(const Model& m, int vir_pchunk) {
@@ -205,10 +225,10 @@ DeviceModel::DeviceModel(const Model& m, int vir_pchunk) {
     d.pairs = dev_upload(allocs, pv.data(), pv.size());
     if (c.use3)
         upload_list(m, m.trips, 3, c.cheby3, d.col3, vir_pchunk, *this, &d.int_map3, &d.pidx3, &d.rev3, &d.types3,
-                    &d.pow3, &d.grp3, &d.offs3, &d.tcol3, max_allowed3, oz3);
+                    &d.pow3, &d.grp3, max_allowed3, oz3, rg3);
     if (c.use4)
         upload_list(m, m.quads, 4, c.cheby4, d.col4, vir_pchunk, *this, &d.int_map4, &d.pidx4, &d.rev4, &d.types4,
-                    &d.pow4, &d.grp4, &d.offs4, &d.tcol4, max_allowed4, oz4);
+                    &d.pow4, &d.grp4, max_allowed4, oz4, rg4);
 }
 
 DeviceModel::~DeviceModel() {
@@ -900,20 +920,15 @@ void Session::run(const DeviceFrames& df, int precision, void* A, int64_t lda, A
         // range form in FP64, and in FP32 where a type has more powers than the per-power
         // form has threads (with one power per thread that form fits three CTAs per SM)
         const bool range = force_range_ == 2 || (force_range_ == 1 && (prec == 0 || ppt > 1));
-        int rg_nt = cgd::rg_max_threads(rsize);
-        if (range) {
-            std::vector<int> na;
-            for (const auto& ct : (nbody == 3 ? model.trips : model.quads).vec) na.push_back(ct.excluded ? 0 : ct.n_allowed);
-            rg_nt = cgd::rg_threads(na.data(), (int)na.size(), rsize);
-        }
-        const size_t force_smem = range ? cgd::mb_range_smem(nbody, ord, ntypes * 4, rg_nt, rsize).total
+        const cgd::RgTables& rgt = (nbody == 3 ? dm_->rg3 : dm_->rg4)[prec == 0 ? 0 : 1];
+        const size_t force_smem = range ? cgd::mb_range_smem(nbody, ord, ntypes * 4, rgt.nt, rsize).total
                                         : cgd::mb_force_smem(nbody, ord, ntypes * 4, max_allowed, rsize).total;
         if (!tensor && !range && ppt > 8) throw Error(2, "too many allowed powers for the device force kernel");
         if (!tensor && force_smem > 227 * 1024) throw Error(2, "cluster order too large for the device force kernel");
         if (tensor)
             cgd::launch_force_oz(nbody, nreal, M, F, CS, inc, kfo_atoms, oz, (double*)A, lda, st);
         else if (range)
-            cgd::launch_force_rg(nbody, prec, nreal, rg_nt, force_smem, M, F, CS, inc, kfo_atoms, pre, A, lda, st);
+            cgd::launch_force_rg(nbody, prec, nreal, rgt, force_smem, M, F, CS, inc, kfo_atoms, pre, A, lda, st);
         else
             cgd::launch_force_mb(nbody, prec, pp, nreal, force_smem, M, F, CS, inc, kfo_atoms, pre, A, lda, st,
                                  force4_threads_);

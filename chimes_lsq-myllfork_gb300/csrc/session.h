@@ -26,6 +26,7 @@ struct DeviceModel {
     std::vector<void*> allocs;
     int max_allowed3 = 0, max_allowed4 = 0;   // most allowed powers of a cluster type
     cgd::OzTables oz3, oz4;
+    cgd::RgTables rg3[2], rg4[2];   // FP64, FP32
     explicit DeviceModel(const Model& m, int vir_pchunk);
     ~DeviceModel();
     DeviceModel(const DeviceModel&) = delete;
