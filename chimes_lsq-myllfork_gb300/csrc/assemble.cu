@@ -21,6 +21,8 @@
 // g_s[n] = fcut_s T_n(x_s), h_s[n] = d g_s[n] / dr_s.
 #include <algorithm>
 #include <cstdio>
+#include <type_traits>
+
 #include "assemble.h"
 #include "basis.cuh"
 #include "digits.cuh"
@@ -279,13 +281,17 @@ __global__ void k_virial2_rows(ModelDev M, FramesDev F, int nslice, const R* __r
 // ---------------------------------------------------------------- owner incidence sort
 // The owner's incidences inc.val[c0 .. c0 + nent) (cluster << 2 | member) sorted
 // stably by key = cluster type * 4 + the owner's canonical role: sEnt[k] = entry k,
-// sKey[k] its key, sOrd the entries in key order, and sCnt[key] the end of each key's
-// run (its start is the previous key's end).  Every thread of the CTA calls it; the
-// first barrier keeps a previous pass's readers of sCnt ahead of the reset.
+// sKey[k] its key (low 16 bits; above them key_sign of each slot), sOrd the entries in key
+// order, and sCnt[key] the end of each key's run (its start is the previous key's end).
+// Every thread of the CTA calls it; the first barrier keeps a previous pass's readers of
+// sCnt ahead of the reset.
 template <int NBODY>
-__device__ void sort_incidences(const ClusterSet& CS, const Buckets& inc, const int8_t* revs, const int* typ, int N,
+__device__ void sort_incidences(const ModelDev& M, const ClusterSet& CS, const Buckets& inc, const int* typ, int N,
                                 int64_t qbase, int64_t c0, int nent, int nkeys, int* sEnt, int* sKey, int* sOrd,
                                 int* sCnt) {
+    constexpr int NP = NBODY == 3 ? 3 : 6;
+    const int8_t* revs = NBODY == 3 ? M.rev3 : M.rev4;
+    const int8_t* pidx = NBODY == 3 ? M.pidx3 : M.pidx4;
     const int lane = threadIdx.x & 31;
     __syncthreads();
     for (int k = threadIdx.x; k <= nkeys; k += blockDim.x) sCnt[k] = 0;
@@ -298,18 +304,36 @@ __device__ void sort_incidences(const ClusterSet& CS, const Buckets& inc, const 
         int id = 0, w = 1;
         for (int t = 0; t < NBODY; ++t) { id += w * (typ[member(mm, t) % N] + 1); w *= 10; }
         const int pi = revs[id * NBODY + m];
+        unsigned sg = 0;
+#pragma unroll
+        for (int e = 0; e < NP; ++e) {
+            int a, b;
+            edge_members(NBODY, e, a, b);
+            sg |= (m == a ? 1u : (m == b ? 2u : 0u)) << (2 * pidx[id * NP + e]);
+        }
         sEnt[k] = v;
-        sKey[k] = T * 4 + pi;
+        sKey[k] = (T * 4 + pi) | (int)(sg << 16);
         atomicAdd(&sCnt[T * 4 + pi + 1], 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) for (int k = 1; k <= nkeys; ++k) sCnt[k] += sCnt[k - 1];
-    __syncthreads();
-    if (threadIdx.x < 32) {   // stable placement by (type, role), 32 entries at a time
+    if (threadIdx.x < 32) {
+        int run = 0;   // inclusive scan of the counts
+        for (int k0 = 0; k0 <= nkeys; k0 += 32) {
+            int v = k0 + lane <= nkeys ? sCnt[k0 + lane] : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += u;
+            }
+            if (k0 + lane <= nkeys) sCnt[k0 + lane] = run + v;
+            run += __shfl_sync(0xffffffffu, v, 31);
+        }
+        __syncwarp();
+        // stable placement by (type, role), 32 entries at a time
         for (int b = 0; b < nent; b += 32) {
             const int k = b + lane;
             const bool act = k < nent;
-            const int key = act ? sKey[k] : -1 - lane;
+            const int key = act ? sKey[k] & 0xffff : -1 - lane;
             const unsigned peers = __match_any_sync(0xffffffffu, key);
             const int leader = __ffs(peers) - 1;
             const int rank = __popc(peers & ((1u << lane) - 1u));
@@ -323,6 +347,24 @@ __device__ void sort_incidences(const ClusterSet& CS, const Buckets& inc, const 
         }
     }
     __syncthreads();
+}
+
+// The owner's sign on slot s's edge from a sorted key: +1 its first member, -1 its second, else 0.
+__device__ __forceinline__ int key_sign(int key, int s) {
+    const int c = (key >> (16 + 2 * s)) & 3;
+    return c == 1 ? 1 : (c == 2 ? -1 : 0);
+}
+
+// The next pass over an owner's sorted incidences, from ch0 on: whole cluster types while
+// they fit in cb clusters, or cb clusters of one type (counted from the type's first, so
+// that a type is cut at the same places whatever came before it).  T: the first type with
+// incidences behind ch0 (advanced), T1: the last of the pass; returns the pass's end.
+__device__ __forceinline__ int next_pass(const int* sCnt, int ntypes, int cb, int ch0, int& T, int& T1) {
+    while (sCnt[T * 4 + 3] <= ch0) ++T;
+    T1 = T;
+    if (sCnt[T * 4 + 3] - ch0 >= cb) return ch0 + cb;
+    while (T1 + 1 < ntypes && sCnt[(T1 + 1) * 4 + 3] - ch0 <= cb) ++T1;
+    return sCnt[T1 * 4 + 3];
 }
 
 // ---------------------------------------------------------------- many-body force rows
@@ -344,7 +386,6 @@ __global__ void __launch_bounds__(NT, NBODY == 3 ? (sizeof(R) == 4 ? 3 : 2) : 1)
     const ClusterTypeDev* types = NBODY == 3 ? M.types3 : M.types4;
     const uint8_t* pows = NBODY == 3 ? M.pow3 : M.pow4;
     const int* grps = NBODY == 3 ? M.grp3 : M.grp4;
-    const int8_t* revs = NBODY == 3 ? M.rev3 : M.rev4;
     int sizeI = 1, sizeO = 1;
     for (int k = 0; k < NI; ++k) sizeI *= ord;
     for (int k = 0; k < NO; ++k) sizeO *= ord;
@@ -381,7 +422,7 @@ __global__ void __launch_bounds__(NT, NBODY == 3 ? (sizeof(R) == 4 ? 3 : 2) : 1)
 
     for (int64_t c0 = e0; c0 < e1; c0 += MB_MAX_ENT) {
         const int nent = (int)min((int64_t)MB_MAX_ENT, e1 - c0);
-        sort_incidences<NBODY>(CS, inc, revs, typ, N, qbase, c0, nent, nkeys, sEnt, sKey, sOrd, sCnt);
+        sort_incidences<NBODY>(M, CS, inc, typ, N, qbase, c0, nent, nkeys, sEnt, sKey, sOrd, sCnt);
         for (int T = 0; T < ntypes; ++T) {
             const int gbeg = T == 0 ? 0 : sCnt[T * 4 - 1], gend = sCnt[T * 4 + 3];
             if (gbeg == gend) continue;
@@ -533,14 +574,17 @@ __global__ void __launch_bounds__(NT, NBODY == 3 ? (sizeof(R) == 4 ? 3 : 2) : 1)
 // and are summed in its FMA chain; a column whose powers cross a range boundary is
 // finished by the thread holding its first power, which adds its neighbours' partial
 // sums from shared memory in thread order (so the result does not depend on timing).
-// The clusters of every owner role of a type are tabulated together, CB at a time,
+// Clusters are tabulated CB at a time, whatever their type and the owner's role (next_pass),
 // and each thread reads each power's table entries for each role, laid out so that a warp's
 // reads are contiguous (4-body FP32 rows of 8 uneven frames, in power order -> so: 3,130 ->
-// 2,490 us; each lane had its own cache line).  With no
+// 2,490 us; each lane had its own cache line).  An owner has 5 to 10 clusters of each of some
+// 20 types: a pass per type and index arithmetic in run-time orders spent more instructions
+// on the tables and on each power's loop than on the products (so: 2,490 -> 1,990 us).  With no
 // per-power accumulator arrays two CTAs fit on an SM, and one CTA's table building
 // and barriers overlap the other's FMAs.  blockDim.x (at most rg_max_threads) is chosen
 // by the host (rg_threads).  The frame's PERM_SCALE is folded into the Q table.
-template <int NBODY, typename R>
+// ORD: the order as a constant, 0 for any.
+template <int NBODY, typename R, int ORD>
 __global__ void __launch_bounds__(rg_max_threads((int)sizeof(R)), 2) k_force_rg(ModelDev M, FramesDev F, ClusterSet CS, Buckets inc,
                                                     const int64_t* key_frame_ofs, RgTables rg,
                                                     const R* __restrict__ pre, R* A, int64_t lda) {
@@ -549,11 +593,10 @@ __global__ void __launch_bounds__(rg_max_threads((int)sizeof(R)), 2) k_force_rg(
     constexpr int NO = NP - NI;
     constexpr int CB = mb_force_cb((int)sizeof(R));
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int ord = NBODY == 3 ? M.order3 : M.order4;
+    const int ord = ORD ? ORD : (NBODY == 3 ? M.order3 : M.order4);
     const int ntypes = NBODY == 3 ? M.ntypes3 : M.ntypes4;
     const ClusterTypeDev* types = NBODY == 3 ? M.types3 : M.types4;
     const int* grps = NBODY == 3 ? M.grp3 : M.grp4;
-    const int8_t* revs = NBODY == 3 ? M.rev3 : M.rev4;
     int sizeI = 1, sizeO = 1;
     for (int k = 0; k < NI; ++k) sizeI *= ord;
     for (int k = 0; k < NO; ++k) sizeO *= ord;
@@ -565,14 +608,11 @@ __global__ void __launch_bounds__(rg_max_threads((int)sizeof(R)), 2) k_force_rg(
     int* sKey = reinterpret_cast<int*>(smem_raw + L.key);
     int* sOrd = reinterpret_cast<int*>(smem_raw + L.ord);
     int* sCnt = reinterpret_cast<int*>(smem_raw + L.cnt);
-    int* sQ = reinterpret_cast<int*>(smem_raw + L.q);
-    int* sM = reinterpret_cast<int*>(smem_raw + L.m);        // owner's member index in each cluster
     int* sRole = reinterpret_cast<int*>(smem_raw + L.role);  // owner's canonical role in each cluster
-    int* sSg = reinterpret_cast<int*>(smem_raw + L.sg);      // owner's sign on each slot's edge: +1, -1, 0
     R* sGH = reinterpret_cast<R*>(smem_raw + L.gh);
     R* sW = reinterpret_cast<R*>(smem_raw + L.w);
     R* sTab = reinterpret_cast<R*>(smem_raw + L.tab);
-    R* sPart = reinterpret_cast<R*>(smem_raw + L.part);
+    R* sPart = reinterpret_cast<R*>(smem_raw + L.part);      // two buffers, for one type and the next
 
     const int gatom = blockIdx.x;
     int lo = 0, hi = F.nframes - 1;
@@ -589,49 +629,24 @@ __global__ void __launch_bounds__(rg_max_threads((int)sizeof(R)), 2) k_force_rg(
     const int* typ = F.type + F.atom_ofs[f];
     R* const arow = A + (F.row_ofs[f] + 3 * (int64_t)a) * lda;
     const int tid = threadIdx.x;
+    int buf = 0;
 
     for (int64_t c0 = e0; c0 < e1; c0 += MB_MAX_ENT) {
         const int nent = (int)min((int64_t)MB_MAX_ENT, e1 - c0);
-        sort_incidences<NBODY>(CS, inc, revs, typ, N, qbase, c0, nent, nkeys, sEnt, sKey, sOrd, sCnt);
-        const uint4* __restrict__ offs = rg.offs + tid;
-        const int* __restrict__ cols = rg.col + tid;
-        int S = 0;
-        for (int T = 0; T < ntypes; ++T, offs += S * NT, cols += S * NT) {
-            const int gbeg = T == 0 ? 0 : sCnt[T * 4 - 1], gend = sCnt[T * 4 + 3];
-            const ClusterTypeDev& CT = types[T];
-            const int n = CT.n_allowed;
-            S = (n + NT - 1) / NT;                             // powers per thread
-            if (gbeg == gend || n == 0) continue;
-            const int np = min(n, tid * S + S) - min(n, tid * S);
-            R* const acol = arow + CT.col_base;
-            // the thread's first column began in an earlier thread's range
-            const bool head = np > 0 && (cols[0] & RG_CONT);
-            for (int ch0 = gbeg; ch0 < gend; ch0 += CB) {
-                const int nb = min(CB, gend - ch0);
-                const bool add = !single_pass || ch0 > gbeg;   // later chunks add to the rows
-                if (tid < nb) {
-                    const int k = sOrd[ch0 + tid];
-                    const int v = sEnt[k];
-                    sQ[tid] = v >> 2; sM[tid] = v & 3; sRole[tid] = sKey[k] & 3;
-                    if (pre) {
-                        const int4 mm = CS.m[qbase + (v >> 2)];
-                        int id = 0, w = 1;
-                        for (int u = 0; u < NBODY; ++u) { id += w * (typ[member(mm, u) % N] + 1); w *= 10; }
-                        for (int s = 0; s < NP; ++s) {
-                            int ea, eb;
-                            slot_edge(M, NBODY, id, s, ea, eb);
-                            sSg[tid * NP + s] = ((v & 3) == ea) ? 1 : (((v & 3) == eb) ? -1 : 0);
-                        }
-                    }
-                }
-                __syncthreads();
+        sort_incidences<NBODY>(M, CS, inc, typ, N, qbase, c0, nent, nkeys, sEnt, sKey, sOrd, sCnt);
+        int T = 0, T1 = 0, U = 0, tb = 0;   // U: the type whose powers start at tb in the tables
+        for (int ch0 = 0, ch1; ch0 < nent; ch0 = ch1) {
+                ch1 = next_pass(sCnt, ntypes, CB, ch0, T, T1);
+                const int nb = ch1 - ch0;
                 // (1) per (cluster, slot): basis and the owner's weighted derivative
                 if (pre) {
                     const int stride = 2 * ord + 4;
                     for (int t = tid; t < nb * NP; t += NT) {
                         const int c = t / NP, s = t % NP;
-                        const R* src = pre + ((size_t)(qbase + sQ[c]) * NP + s) * stride;
-                        const int sg = sSg[c * NP + s];
+                        const int k = sOrd[ch0 + c], key = sKey[k];
+                        if (s == 0) sRole[c] = key & 3;
+                        const R* src = pre + ((size_t)(qbase + (sEnt[k] >> 2)) * NP + s) * stride;
+                        const int sg = key_sign(key, s);
                         const R ir = sg != 0 ? R(sg) / src[2 * ord] : R(0);   // sign / r in the form's type
                         const R wx = src[2 * ord + 1] * ir, wy = src[2 * ord + 2] * ir, wz = src[2 * ord + 3] * ir;
                         R* g = sGH + ((size_t)c * NP + s) * 2 * ord;
@@ -645,13 +660,15 @@ __global__ void __launch_bounds__(rg_max_threads((int)sizeof(R)), 2) k_force_rg(
                 } else
                 for (int t = tid; t < nb * NP; t += NT) {
                     const int c = t / NP, s = t % NP;
-                    const int4 mm = CS.m[qbase + sQ[c]];
+                    const int k = sOrd[ch0 + c], v = sEnt[k], key = sKey[k];
+                    if (s == 0) sRole[c] = key & 3;
+                    const int4 mm = CS.m[qbase + (v >> 2)];
                     int id = 0, w = 1;
                     for (int u = 0; u < NBODY; ++u) { id += w * (typ[member(mm, u) % N] + 1); w *= 10; }
                     SlotBasis sb;
                     R* g = sGH + ((size_t)c * NP + s) * 2 * ord;
-                    slot_basis<R>(M, F, NBODY, f, mm, id, T, s, ord, g, g + ord, sb);
-                    const int m = sM[c];
+                    slot_basis<R>(M, F, NBODY, f, mm, id, (key & 0xffff) >> 2, s, ord, g, g + ord, sb);
+                    const int m = v & 3;
                     const double sg = (m == sb.ma) ? 1.0 : ((m == sb.mb) ? -1.0 : 0.0);
                     const double ir = sg / sb.r;
                     const R wx = R(sb.rab[0] * ir), wy = R(sb.rab[1] * ir), wz = R(sb.rab[2] * ir);
@@ -709,70 +726,253 @@ __global__ void __launch_bounds__(rg_max_threads((int)sizeof(R)), 2) k_force_rg(
                     }
                 }
                 __syncthreads();
-                // (3) the thread's powers: 3 FMAs per (power, cluster), summed per column
-                int rs[NBODY], re[NBODY];   // each role's clusters within the chunk
+                // (3) the thread's powers of each type: 3 FMAs per (power, cluster), summed per column
+                bool synced = false;
+                for (;;) {
+                    const ClusterTypeDev& CT = types[U];
+                    const int n = CT.n_allowed;
+                    const int S = (n + NT - 1) / NT;   // powers per thread
+                    const int gbeg = U == 0 ? 0 : sCnt[U * 4 - 1], gend = sCnt[U * 4 + 3];
+                    if (max(gbeg, ch0) < min(gend, ch1) && n > 0) {
+                        const uint4* __restrict__ offs = rg.offs + tb + tid;
+                        const int* __restrict__ cols = rg.col + tb + tid;
+                        const int np = min(n, tid * S + S) - min(n, tid * S);
+                        const bool add = !single_pass || ch0 > gbeg;   // later chunks add to the rows
+                        R* const acol = arow + CT.col_base;
+                        R* const part = sPart + buf * 3 * NT;
+                        buf ^= 1;
+                        // the thread's first column began in an earlier thread's range
+                        const bool head = np > 0 && (cols[0] & RG_CONT);
+                        int rs[NBODY], rn[NBODY];   // each role's first cluster of the pass (its table) and how many
 #pragma unroll
-                for (int r = 0; r < NBODY; ++r) {
-                    const int key = T * 4 + r;
-                    rs[r] = max(key == 0 ? 0 : sCnt[key - 1], ch0) - ch0;
-                    re[r] = min(sCnt[key], ch0 + nb) - ch0;
-                }
-                auto put = [&](int col, R x, R y, R z) {
-                    R* p0 = acol + col;
-                    if (add) { p0[0] += x; p0[lda] += y; p0[2 * lda] += z; }
-                    else { p0[0] = x; p0[lda] = y; p0[2 * lda] = z; }
-                };
-                R ax = R(0), ay = R(0), az = R(0);
-                int pcol = -1;
-                bool first = true;   // still in the thread's first column
-                for (int i = 0; i < np; ++i) {
-                    const int col = cols[i * NT];
-                    const uint4 o4 = offs[i * NT];
-                    if (i > 0 && !(col & RG_CONT)) {   // column pcol ended at the power before
-                        if (first && head) { sPart[3 * tid] = ax; sPart[3 * tid + 1] = ay; sPart[3 * tid + 2] = az; }
-                        else put(pcol & ~(RG_CONT | RG_LAST), ax, ay, az);
-                        first = false;
-                        ax = ay = az = R(0);
-                    }
-                    pcol = col;
-                    const uint32_t ow[4] = {o4.x, o4.y, o4.z, o4.w};
+                        for (int r = 0; r < NBODY; ++r) {
+                            const int key = U * 4 + r;
+                            const int b = max(key == 0 ? 0 : sCnt[key - 1], ch0);
+                            rs[r] = (b - ch0) * per;
+                            rn[r] = min(sCnt[key], ch1) - b;
+                        }
+                        auto put = [&](int col, R x, R y, R z) {
+                            R* p0 = acol + col;
+                            if (add) { p0[0] += x; p0[lda] += y; p0[2 * lda] += z; }
+                            else { p0[0] = x; p0[lda] = y; p0[2 * lda] = z; }
+                        };
+                        R ax = R(0), ay = R(0), az = R(0);
+                        int pcol = -1;
+                        bool first = true;   // still in the thread's first column
+                        for (int i = 0; i < np; ++i) {
+                            const int col = cols[i * NT];
+                            const uint4 o4 = offs[i * NT];
+                            if (i > 0 && !(col & RG_CONT)) {   // column pcol ended at the power before
+                                if (first && head) { part[3 * tid] = ax; part[3 * tid + 1] = ay; part[3 * tid + 2] = az; }
+                                else put(pcol & ~(RG_CONT | RG_LAST), ax, ay, az);
+                                first = false;
+                                ax = ay = az = R(0);
+                            }
+                            pcol = col;
+                            const uint32_t ow[4] = {o4.x, o4.y, o4.z, o4.w};
 #pragma unroll
-                    for (int r = 0; r < NBODY; ++r) {
-                        const int oM = (int)(ow[r] & 0xffffu), oQ = (int)(ow[r] >> 16);
-                        for (int c = rs[r]; c < re[r]; ++c) {
-                            const R* tab = sTab + (size_t)c * per;
-                            const R qv = tab[oQ];
-                            ax += tab[oM] * qv; ay += tab[sizeI + oM] * qv; az += tab[2 * sizeI + oM] * qv;
+                            for (int r = 0; r < NBODY; ++r) {
+                                const R* tm = sTab + (rs[r] + (int)(ow[r] & 0xffffu));
+                                const R* tq = sTab + (rs[r] + (int)(ow[r] >> 16));
+                                for (int c = rn[r]; c > 0; --c, tm += per, tq += per) {
+                                    const R qv = *tq;
+                                    ax += tm[0] * qv; ay += tm[sizeI] * qv; az += tm[2 * sizeI] * qv;
+                                }
+                            }
+                        }
+                        bool tail = false;   // the last column continues into later ranges
+                        const bool ends = pcol & RG_LAST;
+                        pcol &= ~(RG_CONT | RG_LAST);
+                        if (np > 0) {
+                            if (first && head) { part[3 * tid] = ax; part[3 * tid + 1] = ay; part[3 * tid + 2] = az; }
+                            else if (ends) put(pcol, ax, ay, az);
+                            else tail = true;
+                        }
+                        __syncthreads();
+                        synced = true;
+                        if (tail) {   // add the later ranges' partials of this column in thread order
+                            const int last = (grps[CT.grp_offset + pcol + 1] - 1) / S;
+                            for (int t2 = tid + 1; t2 <= last; ++t2) {
+                                ax += part[3 * t2]; ay += part[3 * t2 + 1]; az += part[3 * t2 + 2];
+                            }
+                            put(pcol, ax, ay, az);
                         }
                     }
+                    if (gend > ch1 || U == T1) break;   // the rest of this type, or the next pass's types
+                    tb += S * NT;
+                    ++U;
                 }
-                bool tail = false;   // the last column continues into later ranges
-                const bool ends = pcol & RG_LAST;
-                pcol &= ~(RG_CONT | RG_LAST);
-                if (np > 0) {
-                    if (first && head) { sPart[3 * tid] = ax; sPart[3 * tid + 1] = ay; sPart[3 * tid + 2] = az; }
-                    else if (ends) put(pcol, ax, ay, az);
-                    else tail = true;
-                }
-                __syncthreads();
-                if (tail) {   // add the later ranges' partials of this column in thread order
-                    const int last = (grps[CT.grp_offset + pcol + 1] - 1) / S;
-                    for (int t2 = tid + 1; t2 <= last; ++t2) {
-                        ax += sPart[3 * t2]; ay += sPart[3 * t2 + 1]; az += sPart[3 * t2 + 2];
-                    }
-                    put(pcol, ax, ay, az);
-                }
-            }
+                // (1) of the next pass writes neither the tables nor what (3) still reads
+                if (!synced) __syncthreads();   // every thread is past (2)
         }
     }
 }
+
+// ---------------------------------------------------------------- many-body force rows, one power per thread
+// The sums of k_force_mb<.., PPT = 1> in their order (a power's clusters by role, then the
+// column's powers, PERM_SCALE last) from tabulated bases, with the passes of k_force_rg:
+// clusters of all types and roles are tabulated CB at a time instead of one role's few.
+// Three CTAs per SM; bound by shared-memory reads.  Triplet rows of 8 uneven C/H/N/O frames,
+// k_force_mb -> this: 650 -> 460 us.
+template <int NBODY, int ORD>
+__global__ void __launch_bounds__(MB_THREADS, 3) k_force_pt(ModelDev M, FramesDev F, ClusterSet CS, Buckets inc,
+                                                            const int64_t* key_frame_ofs, RgTables rg,
+                                                            const float* __restrict__ pre, float* A, int64_t lda) {
+    constexpr int NP = NBODY == 3 ? 3 : 6;
+    constexpr int NI = NBODY - 1;
+    constexpr int NO = NP - NI;
+    constexpr int CB = mb_force_cb(4);
+    constexpr int NT = MB_THREADS;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int ord = ORD ? ORD : (NBODY == 3 ? M.order3 : M.order4);
+    const int ntypes = NBODY == 3 ? M.ntypes3 : M.ntypes4;
+    const ClusterTypeDev* types = NBODY == 3 ? M.types3 : M.types4;
+    const int* grps = NBODY == 3 ? M.grp3 : M.grp4;
+    int sizeI = 1, sizeO = 1;
+    for (int k = 0; k < NI; ++k) sizeI *= ord;
+    for (int k = 0; k < NO; ++k) sizeO *= ord;
+    const int per = 3 * sizeI + sizeO;
+    const int nkeys = ntypes * 4;
+    const MbRangeSmem L = mb_range_smem(NBODY, ord, nkeys, NT, 4);
+    int* sEnt = reinterpret_cast<int*>(smem_raw + L.ent);
+    int* sKey = reinterpret_cast<int*>(smem_raw + L.key);
+    int* sOrd = reinterpret_cast<int*>(smem_raw + L.ord);
+    int* sCnt = reinterpret_cast<int*>(smem_raw + L.cnt);
+    int* sRole = reinterpret_cast<int*>(smem_raw + L.role);
+    float* sGH = reinterpret_cast<float*>(smem_raw + L.gh);
+    float* sW = reinterpret_cast<float*>(smem_raw + L.w);
+    float* sTab = reinterpret_cast<float*>(smem_raw + L.tab);
+    float* sPart = reinterpret_cast<float*>(smem_raw + L.part);
+
+    const int gatom = blockIdx.x;
+    int lo = 0, hi = F.nframes - 1;
+    while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (F.atom_ofs[mid] <= gatom) lo = mid; else hi = mid - 1; }
+    const int f = lo;
+    const int a = gatom - (int)F.atom_ofs[f];
+    const int N = F.natoms[f];
+    const double perm = NBODY == 3 ? F.box[f].perm3 : F.box[f].perm4;
+    const int64_t kb = key_frame_ofs[f];
+    const int64_t e0 = inc.key_ofs[kb + a], e1 = inc.key_ofs[kb + a + 1];
+    const bool single_pass = (e1 - e0) <= MB_MAX_ENT;
+    const int64_t qbase = CS.ofs[F.atom_ofs[f]];
+    const int* typ = F.type + F.atom_ofs[f];
+    float* const arow = A + (F.row_ofs[f] + 3 * (int64_t)a) * lda;
+    const int tid = threadIdx.x;
+    int buf = 0;
+
+    for (int64_t c0 = e0; c0 < e1; c0 += MB_MAX_ENT) {
+        const int nent = (int)min((int64_t)MB_MAX_ENT, e1 - c0);
+        sort_incidences<NBODY>(M, CS, inc, typ, N, qbase, c0, nent, nkeys, sEnt, sKey, sOrd, sCnt);
+        int T = 0, T1 = 0, U = 0, tb = 0;   // U: the type whose powers start at tb in the tables
+        float ax = 0.0f, ay = 0.0f, az = 0.0f;   // the thread's power of type U, over its passes
+        for (int ch0 = 0, ch1; ch0 < nent; ch0 = ch1) {
+            ch1 = next_pass(sCnt, ntypes, CB, ch0, T, T1);
+            const int nb = ch1 - ch0;
+            // (1) bases and the owner's weighted derivatives, one thread per (cluster, slot, power)
+            const int stride = 2 * ord + 4;
+            for (int t = tid; t < nb * NP * ord; t += NT) {
+                const int c = t / (NP * ord), rem = t % (NP * ord), s = rem / ord, n = rem % ord;
+                const int k = sOrd[ch0 + c], key = sKey[k];
+                if (rem == 0) sRole[c] = key & 3;
+                const float* src = pre + ((size_t)(qbase + (sEnt[k] >> 2)) * NP + s) * stride;
+                const float ir = (float)key_sign(key, s) / src[2 * ord];   // sign / r
+                const float wx = src[2 * ord + 1] * ir, wy = src[2 * ord + 2] * ir, wz = src[2 * ord + 3] * ir;
+                float* g = sGH + ((size_t)c * NP + s) * 2 * ord;
+                const float gn = src[n], hn = src[ord + n];
+                g[n] = gn; g[ord + n] = hn;
+                float* hw = sW + ((size_t)c * NP + s) * 3 * ord;
+                hw[n] = hn * wx; hw[ord + n] = hn * wy; hw[2 * ord + n] = hn * wz;
+            }
+            __syncthreads();
+            // (2) M_x,y,z over the incident-slot powers, Q over the others
+            const int nzt = sizeI + sizeO;
+            for (int t = tid; t < nb * nzt; t += NT) {
+                const int c = t / nzt, z = t % nzt;
+                const int role = sRole[c];
+                const float* GH = sGH + (size_t)c * NP * 2 * ord;
+                const float* HW = sW + (size_t)c * NP * 3 * ord;
+                float* tab = sTab + (size_t)c * per;
+                if (z < sizeI) {
+                    float gs[NI], other[NI];   // the incident slots' g, and the product of the others'
+                    int pw[NI], zz = z;
+#pragma unroll
+                    for (int u = 0; u < NI; ++u) {
+                        pw[u] = zz % ord; zz /= ord;
+                        gs[u] = GH[role_slot_in(NBODY, role, u) * 2 * ord + pw[u]];
+                    }
+                    if constexpr (NI == 2) { other[0] = gs[1]; other[1] = gs[0]; }
+                    else { other[0] = gs[1] * gs[2]; other[1] = gs[0] * gs[2]; other[2] = gs[0] * gs[1]; }
+                    float mx = 0.0f, my = 0.0f, mz = 0.0f;
+#pragma unroll
+                    for (int u = 0; u < NI; ++u) {
+                        const float* hw = HW + role_slot_in(NBODY, role, u) * 3 * ord + pw[u];
+                        mx = fmaf(hw[0], other[u], mx); my = fmaf(hw[ord], other[u], my); mz = fmaf(hw[2 * ord], other[u], mz);
+                    }
+                    tab[z] = mx; tab[sizeI + z] = my; tab[2 * sizeI + z] = mz;
+                } else {
+                    int zz = z - sizeI;
+                    float prod = 1.0f;
+#pragma unroll
+                    for (int u = 0; u < NO; ++u) { prod *= GH[role_slot_out(NBODY, role, u) * 2 * ord + zz % ord]; zz /= ord; }
+                    tab[3 * sizeI + (z - sizeI)] = prod;
+                }
+            }
+            __syncthreads();
+            // (3) 3 FMAs per (cluster, power), the columns of a type behind its last cluster
+            bool synced = false;
+            for (;;) {
+                const ClusterTypeDev& CT = types[U];
+                const int gbeg = U == 0 ? 0 : sCnt[U * 4 - 1], gend = sCnt[U * 4 + 3];
+                if (max(gbeg, ch0) < min(gend, ch1)) {
+                    if (ch0 <= gbeg) ax = ay = az = 0.0f;
+                    if (tid < CT.n_allowed) {
+                        const uint4 o4 = rg.offs[tb + tid];
+                        const uint32_t ow[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+                        for (int r = 0; r < NBODY; ++r) {
+                            const int key = U * 4 + r;
+                            const int b = max(key == 0 ? 0 : sCnt[key - 1], ch0);
+                            const float* tm = sTab + (b - ch0) * per + (int)(ow[r] & 0xffffu);
+                            const float* tq = sTab + (b - ch0) * per + (int)(ow[r] >> 16);
+                            for (int c = min(sCnt[key], ch1) - b; c > 0; --c, tm += per, tq += per) {
+                                const float qv = *tq;
+                                ax = fmaf(tm[0], qv, ax); ay = fmaf(tm[sizeI], qv, ay); az = fmaf(tm[2 * sizeI], qv, az);
+                            }
+                        }
+                    }
+                    if (gend <= ch1) {   // sum the powers that share a column, then store the owner's 3 rows
+                        float* const part = sPart + buf * 3 * NT;
+                        buf ^= 1;
+                        part[3 * tid] = ax; part[3 * tid + 1] = ay; part[3 * tid + 2] = az;
+                        __syncthreads();
+                        synced = true;
+                        const int* gp = grps + CT.grp_offset;
+                        for (int col = tid; col < CT.n_true; col += NT) {
+                            float sx = 0.0f, sy = 0.0f, sz = 0.0f;
+                            for (int p = gp[col]; p < gp[col + 1]; ++p) { sx += part[3 * p]; sy += part[3 * p + 1]; sz += part[3 * p + 2]; }
+                            float* a0 = arow + CT.col_base + col;
+                            if (single_pass) { a0[0] = float(sx * perm); a0[lda] = float(sy * perm); a0[2 * lda] = float(sz * perm); }
+                            else { a0[0] += float(sx * perm); a0[lda] += float(sy * perm); a0[2 * lda] += float(sz * perm); }
+                        }
+                    }
+                }
+                if (gend > ch1 || U == T1) break;
+                tb += CT.n_allowed > 0 ? NT : 0;
+                ++U;
+            }
+            if (!synced) __syncthreads();   // every thread is past (2)
+        }
+    }
+}
+
 
 // ---------------------------------------------------------------- many-body stress/energy rows
 // grid: (frame, cluster type, group-aligned power chunk); comps as in k_virial2.
 // grid: x = frame * ntypes + type, y = group-aligned power chunk, z = cluster chunk.
 // Each CTA sums VIR_CLUSTERS clusters and stores its column partials (7 comps);
 // k_virial_reduce adds the chunks in order and writes the rows.
-template <int NBODY, typename R, int PPT>
+// ORD: the order as a constant, 0 for any.
+template <int NBODY, typename R, int PPT, int ORD>
 __global__ void __launch_bounds__(MB_THREADS, (PPT == 1 && sizeof(R) == 4) ? 2 : 1) k_virial_mb(ModelDev M, FramesDev F, ClusterSet CS, Buckets bytype,
                                                           const int64_t* key_frame_ofs, int ncomp,
                                                           const R* __restrict__ pre, R* part,
@@ -794,7 +994,7 @@ __global__ void __launch_bounds__(MB_THREADS, (PPT == 1 && sizeof(R) == 4) ? 2 :
     const int64_t c0 = t0 + (int64_t)blockIdx.z * VIR_CLUSTERS;
     if (c0 >= t1) return;
     const int64_t c1 = min(t1, c0 + (int64_t)VIR_CLUSTERS);
-    const int ord = NBODY == 3 ? M.order3 : M.order4;
+    const int ord = ORD ? ORD : (NBODY == 3 ? M.order3 : M.order4);
     const uint8_t* pows = NBODY == 3 ? M.pow3 : M.pow4;
     const int* grps = NBODY == 3 ? M.grp3 : M.grp4;
     const int N = F.natoms[f];
@@ -806,8 +1006,6 @@ __global__ void __launch_bounds__(MB_THREADS, (PPT == 1 && sizeof(R) == 4) ? 2 :
     for (int k = 0; k < N1; ++k) size1 *= ord;
     for (int k = 0; k < N2; ++k) size2 *= ord;
     const int per = 7 * size1 + 7 * size2;   // [Q1 | A1 xx..yz | Q2 | A2 xx..yz]
-    int S1[3], S2[3];
-    role_slots(NBODY, 0, S1, S2);
     const MbVirSmem L = mb_vir_smem(NBODY, ord, PPT * MB_THREADS, (int)sizeof(R));
     int* sQ = reinterpret_cast<int*>(smem_raw + L.q);
     R* sGH = reinterpret_cast<R*>(smem_raw + L.gh);
@@ -822,8 +1020,8 @@ __global__ void __launch_bounds__(MB_THREADS, (PPT == 1 && sizeof(R) == 4) ? 2 :
         if (p < pend) {
             const uint8_t* pw = pows + CT.pow_offset + (size_t)p * NP;
             int x = 0, y = 0;
-            for (int t = N1 - 1; t >= 0; --t) x = x * ord + pw[S1[t]];
-            for (int t = N2 - 1; t >= 0; --t) y = y * ord + pw[S2[t]];
+            for (int t = N1 - 1; t >= 0; --t) x = x * ord + pw[role_slot_in(NBODY, 0, t)];
+            for (int t = N2 - 1; t >= 0; --t) y = y * ord + pw[role_slot_out(NBODY, 0, t)];
             i1[k] = x; i2[k] = y;
         }
     }
@@ -867,26 +1065,37 @@ __global__ void __launch_bounds__(MB_THREADS, (PPT == 1 && sizeof(R) == 4) ? 2 :
         __syncthreads();
         for (int t = threadIdx.x; t < nb * (size1 + size2); t += blockDim.x) {
             const int c = t / (size1 + size2);
-            int z = t % (size1 + size2);
-            const bool first = z < size1;
-            const int* S = first ? S1 : S2;
-            const int ns = first ? N1 : N2;
-            if (!first) z -= size1;
+            const int z = t % (size1 + size2);
             const R* GH = sGH + (size_t)c * NP * 2 * ord;
             const R* V = sV + (size_t)c * NP * 6;
-            int pwr[3] = {0, 0, 0}, zz = z;
-            for (int u = 0; u < ns; ++u) { pwr[u] = zz % ord; zz /= ord; }
-            R q = R(1), av[6] = {0, 0, 0, 0, 0, 0};
-            for (int u = 0; u < ns; ++u) q *= GH[(size_t)S[u] * 2 * ord + pwr[u]];
-            for (int u = 0; u < ns; ++u) {
-                R prod = GH[(size_t)S[u] * 2 * ord + ord + pwr[u]];
-                for (int v2 = 0; v2 < ns; ++v2) if (v2 != u) prod *= GH[(size_t)S[v2] * 2 * ord + pwr[v2]];
-                for (int k = 0; k < 6; ++k) av[k] += prod * V[S[u] * 6 + k];
-            }
-            R* tab = sTab + (size_t)c * per + (first ? 0 : 7 * size1);
-            const int sz = first ? size1 : size2;
-            tab[z] = q;
-            for (int k = 0; k < 6; ++k) tab[(1 + k) * sz + z] = av[k];
+            // product and stress derivative over one group of slots (incident to member 0, or not)
+            auto item = [&](auto first, int zz, R* tab, int sz) {
+                constexpr int ns = decltype(first)::value ? N1 : N2;
+                constexpr auto slot = [](int u) {
+                    return decltype(first)::value ? role_slot_in(NBODY, 0, u) : role_slot_out(NBODY, 0, u);
+                };
+                const R* gh[ns];
+                const int at = zz;
+#pragma unroll
+                for (int u = 0; u < ns; ++u) { gh[u] = GH + slot(u) * 2 * ord + zz % ord; zz /= ord; }
+                R q = R(1), av[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+                for (int u = 0; u < ns; ++u) q *= *gh[u];
+#pragma unroll
+                for (int u = 0; u < ns; ++u) {
+                    R prod = gh[u][ord];
+#pragma unroll
+                    for (int v2 = 0; v2 < ns; ++v2) if (v2 != u) prod *= *gh[v2];
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) av[k] += prod * V[slot(u) * 6 + k];
+                }
+                tab[at] = q;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) tab[(1 + k) * sz + at] = av[k];
+            };
+            R* tab = sTab + (size_t)c * per;
+            if (z < size1) item(std::true_type{}, z, tab, size1);
+            else item(std::false_type{}, z - size1, tab + 7 * size1, size2);
         }
         __syncthreads();
         for (int c = 0; c < nb; ++c) {
@@ -1078,8 +1287,31 @@ static void force_mb_ppt(int ppt, int nreal, size_t smem, const ModelDev& M, con
 template <int NBD, typename R>
 static void force_rg(int nreal, const RgTables& rg, size_t smem, const ModelDev& M, const FramesDev& F, const ClusterSet& CS,
                      const Buckets& inc, const int64_t* kfo, const R* pre, R* A, int64_t lda, cudaStream_t st) {
-    set_smem(k_force_rg<NBD, R>, smem);
-    k_force_rg<NBD, R><<<nreal, rg.nt, smem, st>>>(M, F, CS, inc, kfo, rg, pre, A, lda);
+    // FP32 4-body rows of order 4, the usual one, by constants
+    if (NBD == 4 && sizeof(R) == 4 && M.order4 == 4) {
+        constexpr int O = NBD == 4 && sizeof(R) == 4 ? 4 : 0;
+        set_smem(k_force_rg<NBD, R, O>, smem);
+        k_force_rg<NBD, R, O><<<nreal, rg.nt, smem, st>>>(M, F, CS, inc, kfo, rg, pre, A, lda);
+        return;
+    }
+    set_smem(k_force_rg<NBD, R, 0>, smem);
+    k_force_rg<NBD, R, 0><<<nreal, rg.nt, smem, st>>>(M, F, CS, inc, kfo, rg, pre, A, lda);
+}
+
+template <int NBD, int ORD>
+static void force_pt(int nreal, const RgTables& rg, size_t smem, const ModelDev& M, const FramesDev& F,
+                     const ClusterSet& CS, const Buckets& inc, const int64_t* kfo, const float* pre, float* A,
+                     int64_t lda, cudaStream_t st) {
+    set_smem(k_force_pt<NBD, ORD>, smem);
+    k_force_pt<NBD, ORD><<<nreal, MB_THREADS, smem, st>>>(M, F, CS, inc, kfo, rg, pre, A, lda);
+}
+
+void launch_force_pt(int nbody, int nreal, const RgTables& rg, size_t smem, const ModelDev& M, const FramesDev& F,
+                     const ClusterSet& CS, const Buckets& inc, const int64_t* kfo, const float* pre, float* A,
+                     int64_t lda, cudaStream_t st) {
+    if (nbody == 4) force_pt<4, 0>(nreal, rg, smem, M, F, CS, inc, kfo, pre, A, lda, st);
+    else if (M.order3 == 8) force_pt<3, 8>(nreal, rg, smem, M, F, CS, inc, kfo, pre, A, lda, st);
+    else force_pt<3, 0>(nreal, rg, smem, M, F, CS, inc, kfo, pre, A, lda, st);
 }
 
 int rg_threads(const int* n_allowed, int ntypes, int rsize) {
@@ -1128,9 +1360,17 @@ template <int NBD, typename R, int PPT>
 static void virial_mb_ppt(dim3 grid, size_t smem, const ModelDev& M, const FramesDev& F,
                           const ClusterSet& CS, const Buckets& byt, const int64_t* kfo, int ncomp, const R* pre,
                           R* part, int ntrue_max, int nchunks_max, cudaStream_t st) {
-    set_smem(k_virial_mb<NBD, R, PPT>, smem);
-    k_virial_mb<NBD, R, PPT><<<grid, MB_THREADS, smem, st>>>(M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
-                                                              nchunks_max);
+    // the usual orders (8 for triplets, 4 for quadruplets) by constants in FP32
+    constexpr int O = sizeof(R) == 8 ? 0 : (NBD == 3 && PPT == 1 ? 8 : (NBD == 4 && PPT > 1 ? 4 : 0));
+    if (O > 0 && O == (NBD == 3 ? M.order3 : M.order4)) {
+        set_smem(k_virial_mb<NBD, R, PPT, O>, smem);
+        k_virial_mb<NBD, R, PPT, O><<<grid, MB_THREADS, smem, st>>>(M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+                                                                     nchunks_max);
+        return;
+    }
+    set_smem(k_virial_mb<NBD, R, PPT, 0>, smem);
+    k_virial_mb<NBD, R, PPT, 0><<<grid, MB_THREADS, smem, st>>>(M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+                                                                 nchunks_max);
 }
 
 template <int NBD, typename R>

@@ -46,12 +46,12 @@ __host__ __device__ inline MbForceSmem mb_force_smem(int nbody, int ord, int nke
 // Range form of the force kernel (k_force_rg): at most rg_max_threads threads, two CTAs
 // per SM (384 in FP64, where 80 registers a thread keep the FMA loop out of local
 // memory; 512 in FP32, whose shorter latency-bound loop gains from the extra warps).
-// Shared memory: the incidence sort, then per chunk of mb_force_cb clusters (of every
-// owner role) the slot bases, the owner-weighted derivatives and the M / Q tables,
-// and one partial column sum (3 values) per thread.
+// Shared memory: the incidence sort, then per pass of mb_force_cb clusters (of several
+// types, every owner role) the slot bases, the owner-weighted derivatives and the M / Q
+// tables, and two buffers of 3 partial sums per thread.
 __host__ __device__ constexpr int rg_max_threads(int rsize) { return rsize == 8 ? 384 : 512; }
 struct MbRangeSmem {
-    size_t ent, key, ord, cnt, q, m, role, sg, gh, w, tab, part, total;
+    size_t ent, key, ord, cnt, role, gh, w, tab, part, total;
 };
 __host__ __device__ inline MbRangeSmem mb_range_smem(int nbody, int ord, int nkeys, int nt, int rsize) {
     const int np = nbody == 3 ? 3 : 6, ni = nbody - 1, no = np - ni;
@@ -65,15 +65,12 @@ __host__ __device__ inline MbRangeSmem mb_range_smem(int nbody, int ord, int nke
     s.key = align16(s.ent + MB_MAX_ENT * sizeof(int));
     s.ord = align16(s.key + MB_MAX_ENT * sizeof(int));
     s.cnt = align16(s.ord + MB_MAX_ENT * sizeof(int));
-    s.q = align16(s.cnt + (nkeys + 1) * sizeof(int));
-    s.m = align16(s.q + cb * sizeof(int));
-    s.role = align16(s.m + cb * sizeof(int));
-    s.sg = align16(s.role + cb * sizeof(int));
-    s.gh = align16(s.sg + cb * 6 * sizeof(int));
+    s.role = align16(s.cnt + (nkeys + 1) * sizeof(int));
+    s.gh = align16(s.role + cb * sizeof(int));
     s.w = align16(s.gh + (size_t)cb * np * 2 * ord * rsize);
     s.tab = align16(s.w + (size_t)cb * np * 3 * ord * rsize);
     s.part = align16(s.tab + (size_t)cb * per * rsize);
-    s.total = align16(s.part + (size_t)nt * 3 * rsize);
+    s.total = align16(s.part + (size_t)nt * 6 * rsize);
     return s;
 }
 
@@ -142,6 +139,11 @@ void launch_force_mb(int nbody, int prec, int ppt, int nreal, size_t smem, const
 void launch_force_rg(int nbody, int prec, int nreal, const RgTables& rg, size_t smem, const ModelDev& M, const FramesDev& F,
                      const ClusterSet& CS, const Buckets& inc, const int64_t* key_frame_ofs, const void* pre,
                      void* A, int64_t lda, cudaStream_t st);
+// The sums of launch_force_mb in the same order, FP32 with tabulated bases and at most one
+// power per thread (rg.nt); smem = mb_range_smem(..., rg.nt, 4).total.
+void launch_force_pt(int nbody, int nreal, const RgTables& rg, size_t smem, const ModelDev& M, const FramesDev& F,
+                     const ClusterSet& CS, const Buckets& inc, const int64_t* key_frame_ofs, const float* pre,
+                     float* A, int64_t lda, cudaStream_t st);
 // Work lists of a call: the cluster bases, their magnitudes (one int per slot), the owners'
 // incidences by cluster type (one entry per incidence: cluster, slot order, exponents) and
 // the (owner, type) groups.

@@ -921,14 +921,18 @@ void Session::run(const DeviceFrames& df, int precision, void* A, int64_t lda, A
         // form has threads (with one power per thread that form fits three CTAs per SM)
         const bool range = force_range_ == 2 || (force_range_ == 1 && (prec == 0 || ppt > 1));
         const cgd::RgTables& rgt = (nbody == 3 ? dm_->rg3 : dm_->rg4)[prec == 0 ? 0 : 1];
-        const size_t force_smem = range ? cgd::mb_range_smem(nbody, ord, ntypes * 4, rgt.nt, rsize).total
-                                        : cgd::mb_force_smem(nbody, ord, ntypes * 4, max_allowed, rsize).total;
+        // one power per thread and tabulated FP32 bases: k_force_mb's sums by passes over all types
+        const bool pt = !range && prec != 0 && pre && ppt <= 1 && rgt.nt == cgd::MB_THREADS;
+        const size_t force_smem = range || pt ? cgd::mb_range_smem(nbody, ord, ntypes * 4, rgt.nt, rsize).total
+                                              : cgd::mb_force_smem(nbody, ord, ntypes * 4, max_allowed, rsize).total;
         if (!tensor && !range && ppt > 8) throw Error(2, "too many allowed powers for the device force kernel");
         if (!tensor && force_smem > 227 * 1024) throw Error(2, "cluster order too large for the device force kernel");
         if (tensor)
             cgd::launch_force_oz(nbody, nreal, M, F, CS, inc, kfo_atoms, oz, (double*)A, lda, st);
         else if (range)
             cgd::launch_force_rg(nbody, prec, nreal, rgt, force_smem, M, F, CS, inc, kfo_atoms, pre, A, lda, st);
+        else if (pt)
+            cgd::launch_force_pt(nbody, nreal, rgt, force_smem, M, F, CS, inc, kfo_atoms, (const float*)pre, (float*)A, lda, st);
         else
             cgd::launch_force_mb(nbody, prec, pp, nreal, force_smem, M, F, CS, inc, kfo_atoms, pre, A, lda, st,
                                  force4_threads_);
