@@ -967,15 +967,19 @@ __global__ void __launch_bounds__(MB_THREADS, 3) k_force_pt(ModelDev M, FramesDe
 
 
 // ---------------------------------------------------------------- many-body stress/energy rows
-// grid: (frame, cluster type, group-aligned power chunk); comps as in k_virial2.
-// grid: x = frame * ntypes + type, y = group-aligned power chunk, z = cluster chunk.
+// grid: x = frame * ntypes + type, y = group-aligned power chunk, z = cluster chunk, the
+// last (of the types with most clusters) first; comps as in k_virial2.
 // Each CTA sums VIR_CLUSTERS clusters and stores its column partials (7 comps);
-// k_virial_reduce adds the chunks in order and writes the rows.
+// k_virial_reduce adds the chunks in order and writes the rows.  Bound by shared-memory
+// reads (7 of either table per power and cluster, for 13 FMAs), so a thread's powers share
+// their entry of the first table and a warp's read a run of the second (vord): quadruplet rows
+// of 8 uneven C/H/N/O frames 1,230 -> 624 us (lanes in power order, one entry of each table
+// per power: two words on a bank in most reads).
 // ORD: the order as a constant, 0 for any.
 template <int NBODY, typename R, int PPT, int ORD>
 __global__ void __launch_bounds__(MB_THREADS, (PPT == 1 && sizeof(R) == 4) ? 2 : 1) k_virial_mb(ModelDev M, FramesDev F, ClusterSet CS, Buckets bytype,
                                                           const int64_t* key_frame_ofs, int ncomp,
-                                                          const R* __restrict__ pre, R* part,
+                                                          const R* __restrict__ pre, const int* __restrict__ order, R* part,
                                                           int ntrue_max, int nchunks_max) {
     constexpr int NP = NBODY == 3 ? 3 : 6;
     constexpr int N1 = NBODY - 1;
@@ -987,11 +991,12 @@ __global__ void __launch_bounds__(MB_THREADS, (PPT == 1 && sizeof(R) == 4) ? 2 :
     const int srows = F.stress_rows[f], erows = F.energy_rows[f];
     if (srows == 0 && erows == 0) return;
     const ClusterTypeDev& CT = (NBODY == 3 ? M.types3 : M.types4)[T];
+    const int zc = (int)(gridDim.z - 1 - blockIdx.z);
     if ((int)blockIdx.y >= CT.vir_nchunk) return;
     const int pbeg = CT.vir_chunk[blockIdx.y], pend = CT.vir_chunk[blockIdx.y + 1];
     const int64_t kb = key_frame_ofs[f];
     const int64_t t0 = bytype.key_ofs[kb + T], t1 = bytype.key_ofs[kb + T + 1];
-    const int64_t c0 = t0 + (int64_t)blockIdx.z * VIR_CLUSTERS;
+    const int64_t c0 = t0 + (int64_t)zc * VIR_CLUSTERS;
     if (c0 >= t1) return;
     const int64_t c1 = min(t1, c0 + (int64_t)VIR_CLUSTERS);
     const int ord = ORD ? ORD : (NBODY == 3 ? M.order3 : M.order4);
@@ -1005,24 +1010,29 @@ __global__ void __launch_bounds__(MB_THREADS, (PPT == 1 && sizeof(R) == 4) ? 2 :
     int size1 = 1, size2 = 1;
     for (int k = 0; k < N1; ++k) size1 *= ord;
     for (int k = 0; k < N2; ++k) size2 *= ord;
-    const int per = 7 * size1 + 7 * size2;   // [Q1 | A1 xx..yz | Q2 | A2 xx..yz]
+    // [Q1 | A1 xx..yz | Q2 | A2 xx..yz], in FP32 the first group's values of an entry together
+    constexpr bool VEC = sizeof(R) == 4;
+    const int per = mb_vir_per(size1, size2, (int)sizeof(R)), ofs2 = VEC ? 8 * size1 : 7 * size1;
     const MbVirSmem L = mb_vir_smem(NBODY, ord, PPT * MB_THREADS, (int)sizeof(R));
     int* sQ = reinterpret_cast<int*>(smem_raw + L.q);
     R* sGH = reinterpret_cast<R*>(smem_raw + L.gh);
     R* sV = reinterpret_cast<R*>(smem_raw + L.v);
     R* sTab = reinterpret_cast<R*>(smem_raw + L.tab);
 
-    int i1[PPT], i2[PPT];
+    // the thread's powers: one entry of the first table (-1: none), PPT of the second (0 where
+    // there is no power, whose sums are dropped)
+    int i1 = -1, i2[PPT];
+    const int* const mine = order + ((size_t)T * gridDim.y + blockIdx.y) * PPT * MB_THREADS + threadIdx.x;
 #pragma unroll
     for (int k = 0; k < PPT; ++k) {
-        const int p = pbeg + threadIdx.x + k * blockDim.x;
-        i1[k] = -1; i2[k] = 0;
-        if (p < pend) {
+        const int p = mine[k * MB_THREADS];
+        i2[k] = 0;
+        if (p >= 0) {
             const uint8_t* pw = pows + CT.pow_offset + (size_t)p * NP;
             int x = 0, y = 0;
             for (int t = N1 - 1; t >= 0; --t) x = x * ord + pw[role_slot_in(NBODY, 0, t)];
             for (int t = N2 - 1; t >= 0; --t) y = y * ord + pw[role_slot_out(NBODY, 0, t)];
-            i1[k] = x; i2[k] = y;
+            i1 = x; i2[k] = y;
         }
     }
     R acc[PPT][7];
@@ -1089,43 +1099,58 @@ __global__ void __launch_bounds__(MB_THREADS, (PPT == 1 && sizeof(R) == 4) ? 2 :
 #pragma unroll
                     for (int k = 0; k < 6; ++k) av[k] += prod * V[slot(u) * 6 + k];
                 }
-                tab[at] = q;
+                if constexpr (VEC && decltype(first)::value) {
+                    float4* o = reinterpret_cast<float4*>(tab + 8 * at);
+                    o[0] = make_float4(q, av[0], av[1], av[2]);
+                    o[1] = make_float4(av[3], av[4], av[5], 0.0f);
+                } else {
+                    tab[at] = q;
 #pragma unroll
-                for (int k = 0; k < 6; ++k) tab[(1 + k) * sz + at] = av[k];
+                    for (int k = 0; k < 6; ++k) tab[(1 + k) * sz + at] = av[k];
+                }
             };
             R* tab = sTab + (size_t)c * per;
             if (z < size1) item(std::true_type{}, z, tab, size1);
-            else item(std::false_type{}, z - size1, tab + 7 * size1, size2);
+            else item(std::false_type{}, z - size1, tab + ofs2, size2);
         }
         __syncthreads();
-        for (int c = 0; c < nb; ++c) {
-            const R* t1 = sTab + (size_t)c * per;
-            const R* t2 = t1 + 7 * size1;
+        if (i1 >= 0)
+            for (int c = 0; c < nb; ++c) {
+                const R* t1 = sTab + (size_t)c * per;
+                const R* t2 = t1 + ofs2;
+                R a[7];
+                if constexpr (VEC) {
+                    const float4* v = reinterpret_cast<const float4*>(t1 + 8 * i1);
+                    const float4 x = v[0], y = v[1];
+                    a[0] = x.x; a[1] = x.y; a[2] = x.z; a[3] = x.w; a[4] = y.x; a[5] = y.y; a[6] = y.z;
+                } else {
 #pragma unroll
-            for (int k = 0; k < PPT; ++k) {
-                if (i1[k] < 0) continue;
-                const R q1 = t1[i1[k]], q2 = t2[i2[k]];
-                acc[k][0] = fma(q1, q2, acc[k][0]);
+                    for (int cc = 0; cc < 7; ++cc) a[cc] = t1[cc * size1 + i1];
+                }
 #pragma unroll
-                for (int cc = 1; cc < 7; ++cc) {   // fully unrolled: accumulators stay in registers
-                    if (cc < ncomp) {
-                        acc[k][cc] = fma(-t1[cc * size1 + i1[k]], q2, acc[k][cc]);
-                        acc[k][cc] = fma(-q1, t2[cc * size2 + i2[k]], acc[k][cc]);
+                for (int k = 0; k < PPT; ++k) {
+                    const R q2 = t2[i2[k]];
+                    acc[k][0] = fma(a[0], q2, acc[k][0]);
+#pragma unroll
+                    for (int cc = 1; cc < 7; ++cc) {   // fully unrolled: accumulators stay in registers
+                        if (cc < ncomp) {
+                            acc[k][cc] = fma(-a[cc], q2, acc[k][cc]);
+                            acc[k][cc] = fma(-a[0], t2[cc * size2 + i2[k]], acc[k][cc]);
+                        }
                     }
                 }
             }
-        }
         __syncthreads();
     }
 #pragma unroll
     for (int k = 0; k < PPT; ++k) {
-        const int pl = threadIdx.x + k * blockDim.x;
-        if (pbeg + pl < pend)
-            for (int c = 0; c < 7; ++c) sTab[(size_t)pl * 7 + c] = acc[k][c];
+        const int p = mine[k * MB_THREADS];
+        if (p >= 0)
+            for (int c = 0; c < 7; ++c) sTab[(size_t)(p - pbeg) * 7 + c] = acc[k][c];
     }
     __syncthreads();
     const int* gp = grps + CT.grp_offset;
-    R* out = part + ((size_t)blockIdx.x * nchunks_max + blockIdx.z) * 7 * ntrue_max;
+    R* out = part + ((size_t)blockIdx.x * nchunks_max + zc) * 7 * ntrue_max;
     for (int col = threadIdx.x; col < CT.n_true; col += blockDim.x) {
         const int pa = gp[col], pb = gp[col + 1];
         if (pa < pbeg || pa >= pend) continue;
@@ -1359,29 +1384,29 @@ void launch_force_mb(int nbody, int prec, int ppt, int nreal, size_t smem, const
 template <int NBD, typename R, int PPT>
 static void virial_mb_ppt(dim3 grid, size_t smem, const ModelDev& M, const FramesDev& F,
                           const ClusterSet& CS, const Buckets& byt, const int64_t* kfo, int ncomp, const R* pre,
-                          R* part, int ntrue_max, int nchunks_max, cudaStream_t st) {
+                          const int* order, R* part, int ntrue_max, int nchunks_max, cudaStream_t st) {
     // the usual orders (8 for triplets, 4 for quadruplets) by constants in FP32
     constexpr int O = sizeof(R) == 8 ? 0 : (NBD == 3 && PPT == 1 ? 8 : (NBD == 4 && PPT > 1 ? 4 : 0));
     if (O > 0 && O == (NBD == 3 ? M.order3 : M.order4)) {
         set_smem(k_virial_mb<NBD, R, PPT, O>, smem);
-        k_virial_mb<NBD, R, PPT, O><<<grid, MB_THREADS, smem, st>>>(M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+        k_virial_mb<NBD, R, PPT, O><<<grid, MB_THREADS, smem, st>>>(M, F, CS, byt, kfo, ncomp, pre, order, part, ntrue_max,
                                                                      nchunks_max);
         return;
     }
     set_smem(k_virial_mb<NBD, R, PPT, 0>, smem);
-    k_virial_mb<NBD, R, PPT, 0><<<grid, MB_THREADS, smem, st>>>(M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+    k_virial_mb<NBD, R, PPT, 0><<<grid, MB_THREADS, smem, st>>>(M, F, CS, byt, kfo, ncomp, pre, order, part, ntrue_max,
                                                                  nchunks_max);
 }
 
 template <int NBD, typename R>
 static void virial_mb_typed(int ppt, dim3 grid, size_t smem, const ModelDev& M, const FramesDev& F,
                             const ClusterSet& CS, const Buckets& byt, const int64_t* kfo, int ncomp, const void* pre,
-                            void* part, int ntrue_max, int nchunks_max, cudaStream_t st) {
+                            const int* order, void* part, int ntrue_max, int nchunks_max, cudaStream_t st) {
     if (ppt == 1)
-        virial_mb_ppt<NBD, R, 1>(grid, smem, M, F, CS, byt, kfo, ncomp, (const R*)pre, (R*)part, ntrue_max,
+        virial_mb_ppt<NBD, R, 1>(grid, smem, M, F, CS, byt, kfo, ncomp, (const R*)pre, order, (R*)part, ntrue_max,
                                  nchunks_max, st);
     else
-        virial_mb_ppt<NBD, R, VIR_PPT>(grid, smem, M, F, CS, byt, kfo, ncomp, (const R*)pre, (R*)part,
+        virial_mb_ppt<NBD, R, VIR_PPT>(grid, smem, M, F, CS, byt, kfo, ncomp, (const R*)pre, order, (R*)part,
                                        ntrue_max, nchunks_max, st);
 }
 
@@ -1400,22 +1425,22 @@ void launch_virial_reduce(int nbody, int prec, int nframes, int ntypes, int ncom
         k_virial_reduce<4, float><<<grid, 256, 0, st>>>(M, F, byt, kfo, ncomp, (const float*)part, ntrue_max, nchunks_max, (float*)A, lda);
 }
 
-void launch_virial_mb(int nbody, int prec, int ppt, int nframes, int ntypes, int nzchunk, int nchunks_max,
+void launch_virial_mb(int nbody, int prec, int ppt, int nframes, int ntypes, int nychunk, int nchunks_max,
                       int ntrue_max, size_t smem, const ModelDev& M, const FramesDev& F, const ClusterSet& CS,
-                      const Buckets& byt, const int64_t* kfo, int ncomp, const void* pre, void* part, void* A,
-                      int64_t lda, cudaStream_t st) {
-    dim3 grid(nframes * ntypes, nzchunk, nchunks_max);
+                      const Buckets& byt, const int64_t* kfo, int ncomp, const void* pre, const int* order, void* part,
+                      void* A, int64_t lda, cudaStream_t st) {
+    dim3 grid(nframes * ntypes, nychunk, nchunks_max);
     if (nbody == 3 && prec == 0)
-        virial_mb_typed<3, double>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+        virial_mb_typed<3, double>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, order, part, ntrue_max,
                                    nchunks_max, st);
     else if (nbody == 3)
-        virial_mb_typed<3, float>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+        virial_mb_typed<3, float>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, order, part, ntrue_max,
                                   nchunks_max, st);
     else if (prec == 0)
-        virial_mb_typed<4, double>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+        virial_mb_typed<4, double>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, order, part, ntrue_max,
                                    nchunks_max, st);
     else
-        virial_mb_typed<4, float>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, part, ntrue_max,
+        virial_mb_typed<4, float>(ppt, grid, smem, M, F, CS, byt, kfo, ncomp, pre, order, part, ntrue_max,
                                   nchunks_max, st);
     launch_virial_reduce(nbody, prec, nframes, ntypes, ncomp, M, F, byt, kfo, part, ntrue_max, nchunks_max, A, lda, st);
 }

@@ -74,6 +74,11 @@ __host__ __device__ inline MbRangeSmem mb_range_smem(int nbody, int ord, int nke
     return s;
 }
 
+// Table values of a cluster in k_virial_mb: 7 per entry of either group of slots; in FP32
+// the first group's lie together, padded to 8 for vector reads.
+__host__ __device__ constexpr int mb_vir_per(int size1, int size2, int rsize) {
+    return rsize == 4 ? (8 * size1 + 7 * size2 + 3) / 4 * 4 : 7 * (size1 + size2);
+}
 struct MbVirSmem {
     size_t q, gh, v, tab, total;
 };
@@ -82,7 +87,7 @@ __host__ __device__ inline MbVirSmem mb_vir_smem(int nbody, int ord, int pchunk,
     int s1 = 1, s2 = 1;
     for (int k = 0; k < n1; ++k) s1 *= ord;
     for (int k = 0; k < n2; ++k) s2 *= ord;
-    const size_t per = 7 * (size_t)s1 + 7 * (size_t)s2;
+    const size_t per = mb_vir_per(s1, s2, rsize);
     MbVirSmem s;
     s.q = 0;
     s.gh = align16(MB_CB * sizeof(int));
@@ -176,11 +181,12 @@ int rg_threads(const int* n_allowed, int ntypes, int rsize);
 // Stress/energy rows: nchunks_max cluster chunks of VIR_CLUSTERS per (frame, type);
 // part holds nframes*ntypes*nchunks_max*7*ntrue_max partial sums (R).
 // ppt: powers per thread, 1 when every cluster type has at most MB_THREADS allowed
-// powers (fewer registers, more CTAs per SM), else VIR_PPT.
-void launch_virial_mb(int nbody, int prec, int ppt, int nframes, int ntypes, int nzchunk, int nchunks_max,
+// powers (fewer registers, more CTAs per SM), else VIR_PPT.  nychunk: most chunks of a
+// type; order: the powers of each chunk's threads (DeviceModel::vord3/4).
+void launch_virial_mb(int nbody, int prec, int ppt, int nframes, int ntypes, int nychunk, int nchunks_max,
                       int ntrue_max, size_t smem, const ModelDev& M, const FramesDev& F, const ClusterSet& CS,
-                      const Buckets& byt, const int64_t* key_frame_ofs, int ncomp, const void* pre, void* part,
-                      void* A, int64_t lda, cudaStream_t st);
+                      const Buckets& byt, const int64_t* key_frame_ofs, int ncomp, const void* pre, const int* order,
+                      void* part, void* A, int64_t lda, cudaStream_t st);
 void launch_max_bucket(const int64_t* key_ofs, const int64_t* key_frame_ofs, int nframes, int ntypes, int* out,
                        cudaStream_t st);
 void launch_energy_cols(int prec, int nframes, const ModelDev& M, const FramesDev& F, void* A, int64_t lda,

@@ -44,10 +44,11 @@ static void rev_index(const ClusterType& ct, const int* types, int n, int8_t* ou
     }
 }
 
-static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, int col_base, int pchunk, DeviceModel& D,
+static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, int col_base, DeviceModel& D,
                         const int** int_map, const int8_t** pidx, const int8_t** rev, const cgd::ClusterTypeDev** types,
                         const uint8_t** pows, const int** grps, int& max_allowed, cgd::OzTables& oz,
-                        cgd::RgTables (&rg)[2]) {
+                        cgd::RgTables (&rg)[2],
+                        const int** vord, int& nychunk) {
     const int np = nb == 3 ? 3 : 6;
     const int dim = nb == 3 ? 1000 : 10000;
     std::vector<int> imap(dim, -1);
@@ -71,6 +72,8 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
     if (3 * sizeI + sizeO > 65536) throw Error(2, "cluster order too large for the force-table offsets");
     int col = col_base;
     max_allowed = 0;
+    for (const ClusterType& ct : cl.vec) max_allowed = std::max(max_allowed, ct.excluded ? 0 : ct.n_allowed);
+    const int vgr = max_allowed <= cgd::MB_THREADS ? 1 : cgd::VIR_PPT;   // powers per thread of k_virial_mb
     for (size_t t = 0; t < cl.vec.size(); ++t) {
         const ClusterType& ct = cl.vec[t];
         cgd::ClusterTypeDev& d = tv[t];
@@ -81,7 +84,6 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
         col += d.n_true;
         d.pow_offset = (int)pw.size();
         d.grp_offset = (int)gp.size();
-        max_allowed = std::max(max_allowed, d.n_allowed);
         for (int p = 0; p < d.n_allowed; ++p)
             for (int s = 0; s < np; ++s) pw.push_back((uint8_t)ct.allowed_powers[p][s]);
         for (int p = 0; p < d.n_allowed; ++p) {
@@ -103,22 +105,33 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
             while (c <= ct.param_indices[p]) { gp.push_back(p); ++c; }
         }
         while (c <= d.n_true) { gp.push_back(d.n_allowed); ++c; }
-        // group-aligned power chunks for the stress/energy kernel
-        int nch = 0;
+        // group-aligned power chunks for the stress/energy kernel: as many powers as its
+        // threads take, each up to vgr with the same entry of the first table
+        int nch = 0, threads = 0;
         d.vir_chunk[0] = 0;
-        int start = 0;
-        while (start < d.n_allowed) {
-            int end = std::min(d.n_allowed, start + pchunk);
-            if (end < d.n_allowed) {   // move back to a group start
-                int gstart = end;
-                while (gstart > start && ct.param_indices[gstart] == ct.param_indices[gstart - 1]) --gstart;
-                if (gstart == start) throw Error(2, "power group larger than a chunk");
-                end = gstart;
+        std::vector<int> count(sizeI, 0);
+        for (int p = 0, gend; p < d.n_allowed; p = gend) {
+            for (gend = p + 1; gend < d.n_allowed && ct.param_indices[gend] == ct.param_indices[p];) ++gend;
+            auto add = [&](int by) {
+                for (int q = p; q < gend; ++q) {
+                    const int i = (int)(of[d.pow_offset / np + q].x & 0xffffu);
+                    threads -= (count[i] + vgr - 1) / vgr;
+                    count[i] += by;
+                    threads += (count[i] + vgr - 1) / vgr;
+                }
+            };
+            add(1);
+            if (threads > cgd::MB_THREADS) {   // the group opens a new chunk
+                if (p == d.vir_chunk[nch]) throw Error(2, "power group larger than a chunk");
+                if (nch + 1 >= cgd::MAXCHUNK) throw Error(2, "too many power chunks for one cluster type");
+                d.vir_chunk[++nch] = p;
+                std::fill(count.begin(), count.end(), 0);
+                threads = 0;
+                add(1);
+                if (threads > cgd::MB_THREADS) throw Error(2, "power group larger than a chunk");
             }
-            if (nch >= cgd::MAXCHUNK) throw Error(2, "too many power chunks for one cluster type");
-            d.vir_chunk[++nch] = end;
-            start = end;
         }
+        if (d.n_allowed > 0) d.vir_chunk[++nch] = d.n_allowed;
         d.vir_nchunk = nch;
         for (int s = 0; s < np; ++s) {
             d.smax[s] = ct.smax[s]; d.smin[s] = ct.smin[s]; d.xavg[s] = ct.xavg[s]; d.xdiff[s] = ct.xdiff[s];
@@ -171,6 +184,33 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
     *types = dev_upload(D.allocs, tv.data(), tv.size());
     *pows = dev_upload(D.allocs, pw.data(), pw.size());
     *grps = dev_upload(D.allocs, gp.data(), gp.size());
+    // The powers of the stress/energy kernel's threads, up to vgr of them with the same entry
+    // of the first table; the lanes of a warp then read few entries of the first table and a
+    // run of the second
+    nychunk = 1;
+    for (const auto& d : tv) nychunk = std::max(nychunk, d.vir_nchunk);
+    const int vth = cgd::MB_THREADS, pchunk = vgr * vth;
+    std::vector<int> vo(std::max<size_t>(1, tv.size() * nychunk * pchunk), -1);
+    std::vector<uint32_t> key;
+    for (size_t t = 0; t < tv.size(); ++t)
+        for (int c = 0; c < tv[t].vir_nchunk; ++c) {
+            const int p0 = tv[t].vir_chunk[c], n = tv[t].vir_chunk[c + 1] - p0;
+            const uint4* e = of.data() + tv[t].pow_offset / np + p0;   // role 0: first table | second table << 16
+            key.resize(n);
+            std::vector<int> count(sizeI + 1, 0), second(3 * sizeI + sizeO + 1, 0);
+            for (int k = 0; k < n; ++k) ++second[(e[k].x >> 16) + 1];   // by the second entry, then stably by the first
+            for (size_t k = 1; k < second.size(); ++k) second[k] += second[k - 1];
+            for (int k = 0; k < n; ++k) key[second[e[k].x >> 16]++] = (uint32_t)k;
+            for (int k = 0; k < n; ++k) ++count[e[k].x & 0xffffu];
+            std::vector<int> first(sizeI, 0), rank(sizeI, 0);   // each entry's first thread
+            for (int i = 1; i < sizeI; ++i) first[i] = first[i - 1] + (count[i - 1] + vgr - 1) / vgr;
+            int* out = vo.data() + (t * nychunk + c) * pchunk;
+            for (uint32_t k : key) {
+                const int i = (int)(e[k].x & 0xffffu), th = (count[i] + vgr - 1) / vgr, r = rank[i]++;
+                out[(size_t)(r / th) * vth + first[i] + r % th] = p0 + (int)k;
+            }
+        }
+    *vord = dev_upload(D.allocs, vo.data(), vo.size());
     std::vector<int> na;
     for (const auto& d : tv) na.push_back(d.n_allowed);
     for (int prec = 0; prec < 2; ++prec) {
@@ -196,7 +236,7 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
     }
 }
 
-DeviceModel::DeviceModel(const Model& m, int vir_pchunk) {
+DeviceModel::DeviceModel(const Model& m) {
     const Controls& c = m.ctl;
     if (c.cheby_order > cgd::MAXORD || c.cheby3 > cgd::MAXORD || c.cheby4 > cgd::MAXORD)
         throw Error(2, "Chebyshev order above the device limit");
@@ -224,11 +264,11 @@ DeviceModel::DeviceModel(const Model& m, int vir_pchunk) {
     for (const auto& p : m.pairs) pv.push_back({p.smin, p.smax, p.lambda, p.xavg, p.xdiff, p.col});
     d.pairs = dev_upload(allocs, pv.data(), pv.size());
     if (c.use3)
-        upload_list(m, m.trips, 3, c.cheby3, d.col3, vir_pchunk, *this, &d.int_map3, &d.pidx3, &d.rev3, &d.types3,
-                    &d.pow3, &d.grp3, max_allowed3, oz3, rg3);
+        upload_list(m, m.trips, 3, c.cheby3, d.col3, *this, &d.int_map3, &d.pidx3, &d.rev3, &d.types3,
+                    &d.pow3, &d.grp3, max_allowed3, oz3, rg3, &vord3, nychunk3);
     if (c.use4)
-        upload_list(m, m.quads, 4, c.cheby4, d.col4, vir_pchunk, *this, &d.int_map4, &d.pidx4, &d.rev4, &d.types4,
-                    &d.pow4, &d.grp4, max_allowed4, oz4, rg4);
+        upload_list(m, m.quads, 4, c.cheby4, d.col4, *this, &d.int_map4, &d.pidx4, &d.rev4, &d.types4,
+                    &d.pow4, &d.grp4, max_allowed4, oz4, rg4, &vord4, nychunk4);
 }
 
 DeviceModel::~DeviceModel() {
@@ -469,7 +509,7 @@ Session::Session(const Model& m, int device) : model_(m), device_(device) {
     // launch, and the other way round.
     CK(cudaStreamCreateWithFlags(&stream_, cudaStreamDefault));
     CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device));
-    dm_.reset(new DeviceModel(model_, cgd::VIR_PPT * cgd::MB_THREADS));
+    dm_.reset(new DeviceModel(model_));
 }
 
 namespace {
@@ -940,9 +980,9 @@ void Session::run(const DeviceFrames& df, int precision, void* A, int64_t lda, A
         mark(nbody == 3 ? ST_FORCE3 : ST_FORCE4, false);
         CK(cudaGetLastError());
         if (virial) {
-            cgd::MbVirSmem V = cgd::mb_vir_smem(nbody, ord, cgd::VIR_PPT * cgd::MB_THREADS, rsize);
+            const int vppt = max_allowed <= cgd::MB_THREADS ? 1 : cgd::VIR_PPT;
+            cgd::MbVirSmem V = cgd::mb_vir_smem(nbody, ord, vppt * cgd::MB_THREADS, rsize);
             if (!tensor && V.total > 227 * 1024) throw Error(2, "cluster order too large for the device stress/energy kernel");
-            const int maxz = (max_allowed + cgd::VIR_PPT * cgd::MB_THREADS - 1) / (cgd::VIR_PPT * cgd::MB_THREADS) + 1;
             int* d_max = S.get<int>(1);
             CK(cudaMemsetAsync(d_max, 0, sizeof(int), st));
             cgd::launch_max_bucket(byt.key_ofs, kfo_types, nf, ntypes, d_max, st); L();
@@ -960,14 +1000,14 @@ void Session::run(const DeviceFrames& df, int precision, void* A, int64_t lda, A
             void* part = prec == 0 ? (void*)S.get<double>((size_t)nf * ntypes * nch * 7 * ntrue_max)
                                    : (void*)S.get<float>((size_t)nf * ntypes * nch * 7 * ntrue_max);
             mark(nbody == 3 ? ST_VIRIAL3 : ST_VIRIAL4, true);
-            const int vppt = max_allowed <= cgd::MB_THREADS ? 1 : cgd::VIR_PPT;
             if (tensor) {
                 cgd::launch_virial_oz(nbody, nf, ncomp, nch, ntrue_max, M, F, CS, byt, kfo_types, oz, (double*)part, st);
                 cgd::launch_virial_reduce(nbody, prec, nf, ntypes, ncomp, M, F, byt, kfo_types, part, ntrue_max, nch, A,
                                           lda, st);
             } else {
-                cgd::launch_virial_mb(nbody, prec, vppt, nf, ntypes, std::min(maxz, cgd::MAXCHUNK), nch, ntrue_max, V.total,
-                                      M, F, CS, byt, kfo_types, ncomp, pre, part, A, lda, st);
+                cgd::launch_virial_mb(nbody, prec, vppt, nf, ntypes, nbody == 3 ? dm_->nychunk3 : dm_->nychunk4, nch,
+                                      ntrue_max, V.total, M, F, CS, byt,
+                                      kfo_types, ncomp, pre, nbody == 3 ? dm_->vord3 : dm_->vord4, part, A, lda, st);
             }
             L(2);
             mark(nbody == 3 ? ST_VIRIAL3 : ST_VIRIAL4, false);

@@ -27,7 +27,10 @@ struct DeviceModel {
     int max_allowed3 = 0, max_allowed4 = 0;   // most allowed powers of a cluster type
     cgd::OzTables oz3, oz4;
     cgd::RgTables rg3[2], rg4[2];   // FP64, FP32
-    explicit DeviceModel(const Model& m, int vir_pchunk);
+    // the powers of k_virial_mb's threads: [type][chunk][power of the thread][thread], -1: none
+    const int *vord3 = nullptr, *vord4 = nullptr;
+    int nychunk3 = 1, nychunk4 = 1;                 // most chunks of a type
+    explicit DeviceModel(const Model& m);
     ~DeviceModel();
     DeviceModel(const DeviceModel&) = delete;
     DeviceModel& operator=(const DeviceModel&) = delete;
