@@ -72,6 +72,12 @@ struct RgTables {
     int nt = 0;
 };
 
+// A cluster slot's cut-off (with the lists' skin) and its FP32 value.
+struct CutDev {
+    double cut;
+    float cutf, pad;
+};
+
 // Column tables of the digit-product kernels (tensor_rows.cu), one set per cluster list:
 // per owner position, type and column, where the column's powers are staged, two 16-bit
 // places per word, (orbit + 1) / 2 words per column, word-major within a type.
@@ -146,6 +152,24 @@ __device__ __forceinline__ double dist_exact(const double* __restrict__ h, const
     rab[1] = dot3rn(h[3], h[4], h[5], tx, ty, tz);
     rab[2] = dot3rn(h[6], h[7], h[8], tx, ty, tz);
     return __dsqrt_rn(addrn(addrn(mulrn(rab[0], rab[0]), mulrn(rab[1], rab[1])), mulrn(rab[2], rab[2])));
+}
+
+// a < b for positive numbers, by their bits: the FP64 pipe, which conversions between FP64
+// and FP32 and comparisons take too, has 1/64 of the integer rate.
+__device__ __forceinline__ bool less_pos(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); }
+
+// Distance from a cut-off within which FP32 Cartesian copies do not decide: the rounding of
+// two positions (2^-24 of their size each, below (layers + 2) times the sum of the cell's
+// entries) and of the distance, times 4, and never above MARGIN.
+constexpr float MARGIN = 1.0e-2f;
+__device__ __forceinline__ float frame_margin(const BoxDev& B, int nlayers) {
+    float s = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {   // at least |h|, from the high word
+        const int hi = __double2hiint(B.h[q]) & 0x7fffffff;
+        s += hi < 0x38200000 ? 1.0e-30f : (hi >= 0x47e00000 ? 1.0e30f : __int_as_float(((hi - 0x38000000) << 3) + 8));
+    }
+    return fminf(MARGIN, 1.0e-5f + 1.0e-6f * (float)(nlayers + 2) * s);
 }
 
 // Layer k (0-based over the (2L+1)^3-1 non-zero layers in n1,n2,n3 order).

@@ -17,7 +17,20 @@
 
 namespace cgd {
 
-static constexpr float MARGIN = 1.0e-2f;
+// The slots' cut-offs for lists of this skin.
+__global__ void k_cuts(const ClusterTypeDev* types, int n, int np, double skin, CutDev* out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n * np) return;
+    CutDev c;
+    c.cut = types[t / np].smax[t % np] + skin;
+    c.cutf = (float)c.cut;
+    c.pad = 0.0f;
+    out[t] = c;
+}
+void launch_cuts(const ModelDev& M, int nbody, double skin, CutDev* out, cudaStream_t st) {
+    const int n = nbody == 3 ? M.ntypes3 : M.ntypes4, np = nbody == 3 ? 3 : 6;
+    if (n > 0) k_cuts<<<(n * np + 127) / 128, 128, 0, st>>>(nbody == 3 ? M.types3 : M.types4, n, np, skin, out);
+}
 
 // ---------------------------------------------------------------- ghost set-up
 __global__ void k_frame_setup(FramesDev F, int64_t total_ghosts) {
@@ -96,7 +109,7 @@ __device__ __forceinline__ int frame_of_real(const FramesDev& F, int64_t atom) {
 //  * An image of the cell that lies beyond the search radius holds no neighbour: the
 //    cell's bounding box, shifted, is tested once per image.  Ordered lists (i <= parent)
 //    start each image at the atom's own index.
-//  * FP32 distances decide except within MARGIN of a cut-off; the exact FP64 distance,
+//  * FP32 distances decide except within frame_margin of a cut-off; the exact FP64 distance,
 //    whose pipe has 1/64 of the rate, is formed there and, in the fill pass, once per
 //    listed ghost with 32 of them side by side.
 // Forming it for every chunk with a candidate in every pass, dividing by the atom count per
@@ -111,6 +124,10 @@ __global__ void __launch_bounds__(32 * NEIGH_WARPS) k_neigh(ModelDev M, FramesDe
     __shared__ int sc[3][NEIGH_WARPS];
     __shared__ int sHit[NEIGH_WARPS][64];
     __shared__ unsigned sNear[NEIGH_WARPS][NEIGH_IMG / 32];
+    __shared__ float2 sPair[55];   // s_max + skin and s_min of the pair types (at most 10 atom types)
+    for (int p = threadIdx.x; p < M.npairs; p += 32 * NEIGH_WARPS)
+        sPair[p] = make_float2((float)(M.pairs[p].smax + NB.skin), (float)M.pairs[p].smin);
+    __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int atom = blockIdx.x * (NEIGH_WARPS / nw) + warp / nw;   // nw divides NEIGH_WARPS
     const int w = warp % nw;
@@ -138,10 +155,12 @@ __global__ void __launch_bounds__(32 * NEIGH_WARPS) k_neigh(ModelDev M, FramesDe
     // images of the cell's bounding box (wrapped atoms lie in the cell) within reach of atom i
     const float reach = pre + 0.05f;   // float rounding of the images' positions stays far below 0.05 A
     float bmin[3], bmax[3];
+    const float hl = lane < 9 ? (float)B.h[lane] : 0.0f;
+    const float mg = frame_margin(B, F.nlayers);
     for (int d = 0; d < 3; ++d) {
         bmin[d] = bmax[d] = 0.0f;
         for (int q = 0; q < 3; ++q) {
-            const float h = (float)B.h[3 * d + q];
+            const float h = __shfl_sync(0xffffffffu, hl, 3 * d + q);
             bmin[d] += fminf(h, 0.0f);
             bmax[d] += fmaxf(h, 0.0f);
         }
@@ -189,12 +208,13 @@ __global__ void __launch_bounds__(32 * NEIGH_WARPS) k_neigh(ModelDev M, FramesDe
         const float dx = cg.x - ci.x, dy = cg.y - ci.y, dz = cg.z - ci.z;
         const float r32 = sqrtf(dx * dx + dy * dy + dz * dz);
         if (!(r32 < pre)) return 0;
-        const PairDev& P = M.pairs[M.int_pair_map[ti * M.natmtyp + typ[a]]];
-        const float smax = (float)(P.smax + NB.skin), smin = (float)P.smin;
-        const bool edge = fabsf(r32 - smax) <= MARGIN || (!NB.md && fabsf(r32 - smin) <= MARGIN) ||
-                          fabsf(r32 - cut3) <= MARGIN || fabsf(r32 - cut4) <= MARGIN;
+        const int pt = M.int_pair_map[ti * M.natmtyp + typ[a]];
+        const float smax = sPair[pt].x, smin = sPair[pt].y;
+        const bool edge = fabsf(r32 - smax) <= mg || (!NB.md && fabsf(r32 - smin) <= mg) ||
+                          fabsf(r32 - cut3) <= mg || fabsf(r32 - cut4) <= mg;
         int fl;
         if (edge) {
+            const PairDev& P = M.pairs[pt];
             const double r = exact(g);
             fl = (M.order2 > 0 && r < P.smax + NB.skin && (NB.md || r > P.smin) ? 1 : 0) |
                  (M.order3 > 0 && r < M.maxcut3 + NB.skin ? 2 : 0) | (M.order4 > 0 && r < M.maxcut4 + NB.skin ? 4 : 0);
@@ -320,6 +340,10 @@ __global__ void k_bin_fill(FramesDev F, int64_t n, Bins B) {
 // One warp per real atom over the ghosts of the 27 bins around it; the per-ghost
 // tests are those of k_neigh.
 __global__ void __launch_bounds__(256) k_neigh_binned(ModelDev M, FramesDev F, NeighDev NB, Bins BN, int fill) {
+    __shared__ float2 sPair[55];   // s_max + skin and s_min of the pair types
+    for (int p = threadIdx.x; p < M.npairs; p += blockDim.x)
+        sPair[p] = make_float2((float)(M.pairs[p].smax + NB.skin), (float)M.pairs[p].smin);
+    __syncthreads();
     const int atom = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (atom >= NB.n_real) return;
@@ -339,6 +363,9 @@ __global__ void __launch_bounds__(256) k_neigh_binned(ModelDev M, FramesDev F, N
     const double* si = F.scaled + 3 * (gbase + i);
     const float maxall = (float)fmax(fmax(M.maxcut2, M.order3 > 0 ? M.maxcut3 : 0.0), M.order4 > 0 ? M.maxcut4 : 0.0);
     const float pre = maxall + MARGIN + (float)NB.skin;
+    const float cut3 = M.order3 > 0 ? (float)(M.maxcut3 + NB.skin) : -1.0f;
+    const float cut4 = M.order4 > 0 ? (float)(M.maxcut4 + NB.skin) : -1.0f;
+    const float mg = frame_margin(B, F.nlayers);
     const BinGrid g = BN.grid[f];
     const int L = F.nlayers;
     const int cx = bin_coord(si[0], L, g.nb[0]), cy = bin_coord(si[1], L, g.nb[1]), cz = bin_coord(si[2], L, g.nb[2]);
@@ -369,12 +396,21 @@ __global__ void __launch_bounds__(256) k_neigh_binned(ModelDev M, FramesDev F, N
                             const float ddx = cg.x - ci.x, ddy = cg.y - ci.y, ddz = cg.z - ci.z;
                             const float r32 = sqrtf(ddx * ddx + ddy * ddy + ddz * ddz);
                             if (r32 < pre) {
-                                r = dist_exact(B.h, si, F.scaled + 3 * (gbase + gg), rab);
                                 pt = M.int_pair_map[ti * M.natmtyp + typ[gg % N]];
-                                const PairDev P = M.pairs[pt];
-                                in2 = M.order2 > 0 && r < P.smax + NB.skin && (NB.md || r > P.smin);
-                                in3 = M.order3 > 0 && r < M.maxcut3 + NB.skin;
-                                in4 = M.order4 > 0 && r < M.maxcut4 + NB.skin;
+                                const float smax = sPair[pt].x, smin = sPair[pt].y;
+                                const bool edge = fabsf(r32 - smax) <= mg || (!NB.md && fabsf(r32 - smin) <= mg) ||
+                                                  fabsf(r32 - cut3) <= mg || fabsf(r32 - cut4) <= mg;
+                                in2 = M.order2 > 0 && r32 < smax && (NB.md || r32 > smin);
+                                in3 = r32 < cut3;
+                                in4 = r32 < cut4;
+                                if (edge || (fill && (in2 || in3 || in4)))
+                                    r = dist_exact(B.h, si, F.scaled + 3 * (gbase + gg), rab);
+                                if (edge) {
+                                    const PairDev& P = M.pairs[pt];
+                                    in2 = M.order2 > 0 && r < P.smax + NB.skin && (NB.md || r > P.smin);
+                                    in3 = M.order3 > 0 && r < M.maxcut3 + NB.skin;
+                                    in4 = M.order4 > 0 && r < M.maxcut4 + NB.skin;
+                                }
                             }
                         }
                     }
@@ -405,18 +441,18 @@ __device__ __forceinline__ float dist32(const float4* c, int64_t a, int64_t b) {
     return sqrtf(dx * dx + dy * dy + dz * dz);
 }
 
-// r(a,b) < smax decided exactly; FP32 settles all but the near-boundary cases.
+// r(a,b) < the cut-off decided exactly; FP32 settles all but the near-boundary cases.
 __device__ __forceinline__ bool within(const FramesDev& F, const BoxDev& B, int64_t gbase, int a, int b,
-                                       double smax, float r32) {
-    if (r32 < (float)smax - MARGIN) return true;
-    if (r32 > (float)smax + MARGIN) return false;
+                                       const CutDev& C, float r32, float mg) {
+    if (r32 < C.cutf - mg) return true;
+    if (r32 > C.cutf + mg) return false;
     double rab[3];
     double r = dist_exact(B.h, F.scaled + 3 * (gbase + a), F.scaled + 3 * (gbase + b), rab);
-    return r < smax;
+    return r < C.cut;
 }
 
-template <int NB_>
-__global__ void k_clusters(ModelDev M, FramesDev F, NeighDev NB, ClusterSet CS, int fill, int parts) {
+// Triplets: every pair of an atom's neighbours, 32 at a time.
+__global__ void k_triplets(ModelDev M, FramesDev F, NeighDev NB, ClusterSet CS, int fill, int parts) {
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const int warp = gw / parts, part = gw - warp * parts;
@@ -433,61 +469,43 @@ __global__ void k_clusters(ModelDev M, FramesDev F, NeighDev NB, ClusterSet CS, 
     const BoxDev& B = F.box[f];
     const int* typ = F.type + F.atom_ofs[f];
     const float4* c32 = reinterpret_cast<const float4*>(F.cart32);
-    const int* lg = NB_ == 3 ? NB.g3 + NB.ofs3[warp] : NB.g4 + NB.ofs4[warp];
-    const double* lr = NB_ == 3 ? NB.r3 + NB.ofs3[warp] : NB.r4 + NB.ofs4[warp];
-    const int n = NB_ == 3 ? NB.cnt3[warp] : NB.cnt4[warp];
-    const int* imap = NB_ == 3 ? M.int_map3 : M.int_map4;
-    const int8_t* pidx = NB_ == 3 ? M.pidx3 : M.pidx4;
-    const ClusterTypeDev* types = NB_ == 3 ? M.types3 : M.types4;
+    const int* lg = NB.g3 + NB.ofs3[warp];
+    const double* lr = NB.r3 + NB.ofs3[warp];
+    const int n = NB.cnt3[warp];
+    const float mg = frame_margin(B, F.nlayers);
     const bool ordered = !B.small;
     const int ti = typ[i];
     int64_t out = fill ? CS.ofs[warp] : 0;
     if (fill)
         for (int q = 0; q < part; ++q) out += CS.pcnt[(int64_t)warp * parts + q];
     int count = 0;
-    const int64_t total = NB_ == 3 ? (int64_t)n * n : (int64_t)n * n * n;
+    const int64_t total = (int64_t)n * n;
     const int64_t nbat = (total + 31) / 32;
     const int64_t b0 = nbat * part / parts * 32, b1 = min(total, nbat * (part + 1) / parts * 32);
     for (int64_t base = b0; base < b1; base += 32) {
         const int64_t t = base + lane;
         bool ok = false;
-        int j = -1, k = -1, l = -1, T = -1;
+        int j = -1, k = -1, T = -1;
         if (t < total) {
-            int a, b, c = 0;
-            if (NB_ == 3) { a = (int)(t / n); b = (int)(t % n); }
-            else { a = (int)(t / ((int64_t)n * n)); b = (int)((t / n) % n); c = (int)(t % n); }
+            const int a = n <= 65535 ? (int)((unsigned)t / (unsigned)n) : (int)(t / n), b = (int)(t - (int64_t)a * n);
             j = lg[a]; k = lg[b];
             ok = (j != k) && !(ordered && (j % N) > (k % N));
-            if (ok && NB_ == 4) {
-                l = lg[c];
-                ok = (j != l) && (k != l) && !(ordered && (k % N) > (l % N));
-            }
             if (ok) {
-                int id = (ti + 1) + 10 * (typ[j % N] + 1) + 100 * (typ[k % N] + 1) +
-                         (NB_ == 4 ? 1000 * (typ[l % N] + 1) : 0);
-                T = imap[id];
+                const int id = (ti + 1) + 10 * (typ[j % N] + 1) + 100 * (typ[k % N] + 1);
+                T = M.int_map3[id];
                 ok = T >= 0;
                 if (ok) {
-                    const ClusterTypeDev& CT = types[T];
-                    const int8_t* pm = pidx + id * (NB_ == 3 ? 3 : 6);
-                    if (NB_ == 3) {
-                        const double sk = NB.skin;
-                        ok = lr[a] < CT.smax[pm[0]] + sk && lr[b] < CT.smax[pm[1]] + sk &&
-                             within(F, B, gbase, j, k, CT.smax[pm[2]] + sk, dist32(c32, gbase + j, gbase + k));
-                    } else {
-                        const double sk = NB.skin;
-                        ok = lr[a] < CT.smax[pm[0]] + sk && lr[b] < CT.smax[pm[1]] + sk && lr[c] < CT.smax[pm[2]] + sk &&
-                             within(F, B, gbase, j, k, CT.smax[pm[3]] + sk, dist32(c32, gbase + j, gbase + k)) &&
-                             within(F, B, gbase, j, l, CT.smax[pm[4]] + sk, dist32(c32, gbase + j, gbase + l)) &&
-                             within(F, B, gbase, k, l, CT.smax[pm[5]] + sk, dist32(c32, gbase + k, gbase + l));
-                    }
+                    const CutDev* C = NB.cut3 + T * 3;
+                    const int8_t* pm = M.pidx3 + id * 3;
+                    ok = less_pos(lr[a], C[pm[0]].cut) && less_pos(lr[b], C[pm[1]].cut) &&
+                         within(F, B, gbase, j, k, C[pm[2]], dist32(c32, gbase + j, gbase + k), mg);
                 }
             }
         }
         const unsigned bal = __ballot_sync(0xffffffffu, ok);
         if (fill && ok) {
             int64_t p = out + count + __popc(bal & ((1u << lane) - 1u));
-            CS.m[p] = make_int4(i, j, k, l);
+            CS.m[p] = make_int4(i, j, k, -1);
             CS.type[p] = T;
         }
         count += __popc(bal);
@@ -502,8 +520,8 @@ __global__ void k_clusters(ModelDev M, FramesDev F, NeighDev NB, ClusterSet CS, 
     }
 }
 
-// Quadruplets in two stages (same accepted set as k_clusters<4>, different but fixed
-// order): the lanes first test (j, k) pairs -- distinct, parent-ordered, r_jk under
+// Quadruplets in two stages (every l against every pair, in a
+// fixed order): the lanes first test (j, k) pairs -- distinct, parent-ordered, r_jk under
 // the largest 4-body cut-off -- and the surviving pairs of each chunk of 32 are then
 // crossed with every l, flattened over the lanes, with the full per-slot tests.
 __global__ void k_quads(ModelDev M, FramesDev F, NeighDev NB, ClusterSet CS, int fill, int parts) {
@@ -531,6 +549,7 @@ __global__ void k_quads(ModelDev M, FramesDev F, NeighDev NB, ClusterSet CS, int
     const bool ordered = !B.small;
     const int ti = typ[i];
     const float cut = (float)(M.maxcut4 + NB.skin) + MARGIN;
+    const float mg = frame_margin(B, F.nlayers);
     int64_t out = fill ? CS.ofs[warp] : 0;
     if (fill)
         for (int q = 0; q < part; ++q) out += CS.pcnt[(int64_t)warp * parts + q];
@@ -566,14 +585,13 @@ __global__ void k_quads(ModelDev M, FramesDev F, NeighDev NB, ClusterSet CS, int
                     T = M.int_map4[id];
                     ok = T >= 0;
                     if (ok) {
-                        const ClusterTypeDev& CT = M.types4[T];
+                        const CutDev* C = NB.cut4 + T * 6;
                         const int8_t* pm = M.pidx4 + id * 6;
-                        const double sk = NB.skin;
-                        ok = lr[ab.x] < CT.smax[pm[0]] + sk && lr[ab.y] < CT.smax[pm[1]] + sk &&
-                             lr[c] < CT.smax[pm[2]] + sk &&
-                             within(F, B, gbase, j, k, CT.smax[pm[3]] + sk, dist32(c32, gbase + j, gbase + k)) &&
-                             within(F, B, gbase, j, l, CT.smax[pm[4]] + sk, dist32(c32, gbase + j, gbase + l)) &&
-                             within(F, B, gbase, k, l, CT.smax[pm[5]] + sk, dist32(c32, gbase + k, gbase + l));
+                        ok = less_pos(lr[ab.x], C[pm[0]].cut) && less_pos(lr[ab.y], C[pm[1]].cut) &&
+                             less_pos(lr[c], C[pm[2]].cut) &&
+                             within(F, B, gbase, j, k, C[pm[3]], dist32(c32, gbase + j, gbase + k), mg) &&
+                             within(F, B, gbase, j, l, C[pm[4]], dist32(c32, gbase + j, gbase + l), mg) &&
+                             within(F, B, gbase, k, l, C[pm[5]], dist32(c32, gbase + k, gbase + l), mg);
                     }
                 }
             }
@@ -771,7 +789,7 @@ void launch_clusters(int nbody, const ModelDev& M, const FramesDev& F, const Nei
     const int parts = CS.pcnt ? cluster_parts(NB.n_real) : 1;
     if (parts > 1 && !fill) cudaMemsetAsync(CS.cnt, 0, sizeof(int) * NB.n_real, st);
     const unsigned g = (unsigned)(((int64_t)NB.n_real * parts + 7) / 8);
-    if (nbody == 3) k_clusters<3><<<g, 256, 0, st>>>(M, F, NB, CS, fill, parts);
+    if (nbody == 3) k_triplets<<<g, 256, 0, st>>>(M, F, NB, CS, fill, parts);
     else k_quads<<<g, 256, 0, st>>>(M, F, NB, CS, fill, parts);
 }
 void launch_bucket(int nframes, const FramesDev& F, const BucketSpec& S, const Buckets& out, cudaStream_t st) {

@@ -20,6 +20,8 @@ struct NeighDev {
     int md;
     // MD list reuse: every cut-off of the enumeration widened by this skin (0: exact)
     double skin;
+    // cut-offs plus skin of every cluster type's slots, [type][3 or 6] (launch_cuts)
+    const CutDev* cut3; const CutDev* cut4;
 };
 
 struct ClusterSet {                               // triplets or quadruplets of a batch
@@ -71,6 +73,7 @@ struct Bins {
 // Host launchers (kernels are defined in geom.cu).
 void launch_frame_setup(const FramesDev& F, int64_t total_ghosts, cudaStream_t st);
 void launch_neigh(const ModelDev& M, const FramesDev& F, const NeighDev& NB, int fill, cudaStream_t st);
+void launch_cuts(const ModelDev& M, int nbody, double skin, CutDev* out, cudaStream_t st);
 void launch_clusters(int nbody, const ModelDev& M, const FramesDev& F, const NeighDev& NB, const ClusterSet& CS,
                      int fill, cudaStream_t st);
 void launch_bucket(int nframes, const FramesDev& F, const BucketSpec& S, const Buckets& out, cudaStream_t st);

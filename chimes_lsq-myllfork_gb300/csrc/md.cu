@@ -91,22 +91,8 @@ __global__ void __launch_bounds__(256) k_md2(ModelDev M, MdDev D, FramesDev F, N
         v[2] -= wv * R[0] * R[0]; v[3] -= wv * R[0] * R[1]; v[4] -= wv * R[0] * R[2];
         v[5] -= wv * R[1] * R[1]; v[6] -= wv * R[1] * R[2]; v[7] -= wv * R[2] * R[2];
     }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) fi[c] = warp_sum(fi[c]);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = warp_sum(v[k]);
-    if (lane == 0) {
-        const int i = warp - (int)aofs;
-        double* fo = Fo + 3 * (aofs + i);
-        if (n > 0) {
-            for (int c = 0; c < 3; ++c) atomicAdd(fo + c, fi[c]);
-            double* so = So + (size_t)f * MD_NSCALAR;
-            atomicAdd(so + 0, v[0]); atomicAdd(so + 1, v[1]);
-            atomicAdd(so + 2, v[2]); atomicAdd(so + 3, v[3]); atomicAdd(so + 4, v[4]);
-            atomicAdd(so + 5, v[3]); atomicAdd(so + 6, v[5]); atomicAdd(so + 7, v[6]);
-            atomicAdd(so + 8, v[4]); atomicAdd(so + 9, v[6]); atomicAdd(so + 10, v[7]);
-        }
-    }
+    const double x[11] = {fi[0], fi[1], fi[2], v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]};
+    pair_sums_add(x, Fo + 3 * warp, So + (size_t)f * MD_NSCALAR, n > 0);
 }
 
 // ------------------------------------------------------------------ grouping
@@ -140,7 +126,7 @@ __global__ void k_md_bucket_count(int64_t n, int nframes, const int64_t* cfo, co
                                   int* cnt) {
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
         const int64_t q = base + threadIdx.x;
-        const bool ok = q < n && type[q] >= 0;   // -1: filtered out this step
+        const bool ok = q < n;
         const int key = ok ? frame_of_cluster(cfo, nframes, q) * ntypes + type[q] : 0;
         warp_agg_inc(cnt, key, ok);
     }
@@ -180,7 +166,7 @@ __global__ void k_md_bucket_fill(int64_t n, int nframes, const int64_t* cfo, con
                                  const int64_t* start, int* cursor, int* val) {
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
         const int64_t q = base + threadIdx.x;
-        const bool ok = q < n && type[q] >= 0;
+        const bool ok = q < n;
         const int key = ok ? frame_of_cluster(cfo, nframes, q) * ntypes + type[q] : 0;
         const int slot = warp_agg_inc(cursor, key, ok);
         if (ok) val[start[key] + slot] = (int)q;
@@ -206,8 +192,10 @@ __device__ __forceinline__ void put(R (&a)[O], int i, R v) {
     for (int k = 0; k < O; ++k) if (k == i) a[k] = v;
 }
 
-// E and G_s[k] = dE/du_s[k] for one cluster: slot 0 is walked at run time, the
-// remaining slots fully unrolled (registers only).
+// E and G_s[k] = dE/du_s[k] for one cluster: slot 0 (of quadruplets slots 0 and 1) is walked
+// at run time, the remaining slots fully unrolled (registers only).  Unrolling slot 1 too
+// made 9,000 instructions that each warp fetched four times (64, 301, 1,111 and 2,600 atoms:
+// 138 -> 124 us).
 template <int O, typename R>
 __device__ __forceinline__ R contract3(const R* __restrict__ sC, const R (&u)[3][O], R (&G)[3][O]) {
     R E = R(0);
@@ -243,9 +231,10 @@ __device__ __forceinline__ R contract4(const R* __restrict__ sC, const R (&u)[6]
         const R ua = pick<O>(u[0], a);
         const R* Ca = sC + a * IPow<5, O>::v;
         R Sa = R(0);
-#pragma unroll
+#pragma unroll 1
         for (int b = 0; b < O; ++b) {
-            const R Pb = ua * u[1][b];
+            const R ub = pick<O>(u[1], b);
+            const R Pb = ua * ub;
             R Sb = R(0);
 #pragma unroll
             for (int c = 0; c < O; ++c) {
@@ -275,8 +264,8 @@ __device__ __forceinline__ R contract4(const R* __restrict__ sC, const R (&u)[6]
                 G[2][c] = fma(Pb, Sc, G[2][c]);
                 Sb = fma(u[2][c], Sc, Sb);
             }
-            G[1][b] = fma(ua, Sb, G[1][b]);
-            Sa = fma(u[1][b], Sb, Sa);
+            put<O>(G[1], b, fma(ua, Sb, pick<O>(G[1], b)));
+            Sa = fma(ub, Sb, Sa);
         }
         put<O>(G[0], a, Sa);
         E = fma(ua, Sa, E);
@@ -290,7 +279,8 @@ __device__ __forceinline__ R contract4(const R* __restrict__ sC, const R (&u)[6]
 template <typename R>
 struct SlotGeomT {
     R r, R3[3];
-    int a, b, pt;
+    int16_t pt;      // pair type; the edge's members
+    int8_t a, b;
 };
 
 template <int NBODY, typename R>
@@ -312,7 +302,7 @@ __device__ __forceinline__ void cluster_geom(const ModelDev& M, const FramesDev&
         edge_ab(NBODY, e, a, b);
         const int ga = member(mm, a), gbm = member(mm, b);
         SlotGeomT<R> g;
-        g.a = a; g.b = b;
+        g.a = (int8_t)a; g.b = (int8_t)b;
         if constexpr (sizeof(R) == 8) {
             g.r = dist_exact(B.h, F.scaled + 3 * (gb + ga), F.scaled + 3 * (gb + gbm), g.R3);
         } else {
@@ -321,7 +311,7 @@ __device__ __forceinline__ void cluster_geom(const ModelDev& M, const FramesDev&
             g.R3[0] = y.x - x.x; g.R3[1] = y.y - x.y; g.R3[2] = y.z - x.z;
             g.r = sqrtf(g.R3[0] * g.R3[0] + g.R3[1] * g.R3[1] + g.R3[2] * g.R3[2]);
         }
-        g.pt = M.int_pair_map[typ[ga % N] * M.natmtyp + typ[gbm % N]];
+        g.pt = (int16_t)M.int_pair_map[typ[ga % N] * M.natmtyp + typ[gbm % N]];
         sg[s] = g;
     }
 }
@@ -354,7 +344,7 @@ __device__ __forceinline__ void fcut_r(const ModelDev& M, R r, R rmax, R& f, R& 
 // basis_regs in FP32 arithmetic (the FP32 form); FP64 uses basis_regs itself.
 template <int O, bool WANT_G, bool WANT_H>
 __device__ __forceinline__ void basis_regs_f(const ModelDev& M, float lambda, float xavg, float xdiff, float smin,
-                                             float r, float fc, float fd, float* g, float* h) {
+                                             float dconst, float r, float fc, float fd, float* g, float* h) {
     const bool out = r < smin;
     const float rr = out ? smin : r;
     float x, ex = 0.0f;
@@ -366,7 +356,7 @@ __device__ __forceinline__ void basis_regs_f(const ModelDev& M, float lambda, fl
     if (M.trans == 0) dxdr = -ex / lambda * ixd;
     else if (M.trans == 1) dxdr = -ixd / (rr * rr);
     else dxdr = ixd;
-    dxdr *= (float)M.deriv_const;
+    dxdr *= dconst;
     const bool zero_d = out && M.fix == 1;
     float damp = 1.0f, shift = 0.0f;
     if (out && M.fix == 0) { damp = expf((r - smin) / (float)M.smooth); shift = (float)M.smooth * (damp - 1.0f); }
@@ -394,17 +384,26 @@ __device__ __forceinline__ void basis_regs_f(const ModelDev& M, float lambda, fl
     }
 }
 
-template <int O, bool WANT_G, bool WANT_H, typename R>
-__device__ __forceinline__ void basis_r(const ModelDev& M, double lambda, double xavg, double xdiff, double smin, R r,
-                                        R fc, R fd, R* g, R* h) {
-    if constexpr (sizeof(R) == 8)
-        basis_regs<O, WANT_G, WANT_H>(M, lambda, xavg, xdiff, smin, r, fc, fd, g, h);
-    else
-        basis_regs_f<O, WANT_G, WANT_H>(M, (float)lambda, (float)xavg, (float)xdiff, (float)smin, r, fc, fd, g, h);
+// Cut-off and basis of slot s of type T (pair type pt) in the form's type; the FP32 form
+// reads FP32 constants.
+template <int NBODY, int O, bool WANT_G, bool WANT_H, typename R>
+__device__ __forceinline__ void slot_basis_r(const ModelDev& M, const MdDev& D, const ClusterTypeDev& CT, int T, int s,
+                                             int pt, float dconst, R r, R* g, R* h) {
+    R fc, fd;
+    if constexpr (sizeof(R) == 8) {
+        fcut_r<R>(M, r, CT.smax[s], fc, fd);
+        basis_regs<O, WANT_G, WANT_H>(M, M.pairs[pt].lambda, CT.xavg[s], CT.xdiff[s], CT.smin[s], r, fc, fd, g, h);
+    } else {
+        const float4 c = (NBODY == 3 ? D.slot3 : D.slot4)[T * (NBODY == 3 ? 3 : 6) + s];
+        fcut_r<R>(M, r, c.x, fc, fd);
+        basis_regs_f<O, WANT_G, WANT_H>(M, D.pairs[pt].lambda, c.y, c.z, c.w, dconst, r, fc, fd, g, h);
+    }
 }
 
 template <int NBODY, int O, typename R>
-__global__ void __launch_bounds__(MDC_THREADS) k_mdc(ModelDev M, MdDev D, FramesDev F, ClusterSet CS, MdBuckets MB,
+// FP32: nine CTAs per SM (shared memory and registers), so that a thousand atoms' tiles are
+// at most two waves.
+__global__ void __launch_bounds__(MDC_THREADS, sizeof(R) == 4 ? 9 : 1) k_mdc(ModelDev M, MdDev D, FramesDev F, ClusterSet CS, MdBuckets MB,
                                                      double* Fo, double* So) {
     constexpr int NP = NBODY == 3 ? 3 : 6;
     constexpr int SZ = IPow<NP, O>::v;
@@ -428,6 +427,7 @@ __global__ void __launch_bounds__(MDC_THREADS) k_mdc(ModelDev M, MdDev D, Frames
         const int64_t aofs = F.atom_ofs[f];
         const BoxDev& B = F.box[f];
         const R perm = (R)(NBODY == 3 ? B.perm3 : B.perm4);
+        const float dconst = (float)M.deriv_const;
         const ClusterTypeDev& CT = (NBODY == 3 ? M.types3 : M.types4)[T];
         const int4 mm = CS.m[MB.val[c]];
         SlotGeomT<R>* sg = sG + (size_t)threadIdx.x * NP;
@@ -436,10 +436,7 @@ __global__ void __launch_bounds__(MDC_THREADS) k_mdc(ModelDev M, MdDev D, Frames
 #pragma unroll
         for (int s = 0; s < NP; ++s) {
             const SlotGeomT<R>& g = sg[s];
-            R fc, fd;
-            fcut_r<R>(M, g.r, (R)CT.smax[s], fc, fd);
-            basis_r<O, true, false, R>(M, M.pairs[g.pt].lambda, CT.xavg[s], CT.xdiff[s], CT.smin[s], g.r, fc, fd, u[s],
-                                       (R*)nullptr);
+            slot_basis_r<NBODY, O, true, false, R>(M, D, CT, T, s, g.pt, dconst, g.r, u[s], (R*)nullptr);
 #pragma unroll
             for (int k = 0; k < O; ++k) G[s][k] = R(0);
         }
@@ -454,11 +451,8 @@ __global__ void __launch_bounds__(MDC_THREADS) k_mdc(ModelDev M, MdDev D, Frames
 #pragma unroll
         for (int s = 0; s < NP; ++s) {
             const SlotGeomT<R>& g = sg[s];
-            R fc, fd;
-            fcut_r<R>(M, g.r, (R)CT.smax[s], fc, fd);
             R h[O];
-            basis_r<O, false, true, R>(M, M.pairs[g.pt].lambda, CT.xavg[s], CT.xdiff[s], CT.smin[s], g.r, fc, fd,
-                                       (R*)nullptr, h);
+            slot_basis_r<NBODY, O, false, true, R>(M, D, CT, T, s, g.pt, dconst, g.r, (R*)nullptr, h);
             R gs = R(0);
 #pragma unroll
             for (int k = 0; k < O; ++k) gs = fma(G[s][k], h[k], gs);
@@ -559,15 +553,16 @@ __global__ void __launch_bounds__(MDC_THREADS) k_mdc_generic(ModelDev M, MdDev D
 // Clusters of lists enumerated with a skin: keep a cluster this step iff every edge
 // is inside its slot's s_max (the same FP32-then-exact test as the enumeration);
 // type_out[q] = its type or -1.
-__device__ __forceinline__ bool within_md(const FramesDev& F, const BoxDev& B, int64_t gb, int a, int b, double smax) {
+__device__ __forceinline__ bool within_md(const FramesDev& F, const BoxDev& B, int64_t gb, int a, int b, float cutf,
+                                          const double* cut, float mg) {
     const float4* c32 = reinterpret_cast<const float4*>(F.cart32);
     const float4 x = c32[gb + a], y = c32[gb + b];
     const float dx = y.x - x.x, dy = y.y - x.y, dz = y.z - x.z;
     const float r32 = sqrtf(dx * dx + dy * dy + dz * dz);
-    if (r32 < (float)smax - 1.0e-2f) return true;
-    if (r32 > (float)smax + 1.0e-2f) return false;
+    if (r32 < cutf - mg) return true;
+    if (r32 > cutf + mg) return false;
     double rab[3];
-    return dist_exact(B.h, F.scaled + 3 * (gb + a), F.scaled + 3 * (gb + b), rab) < smax;
+    return dist_exact(B.h, F.scaled + 3 * (gb + a), F.scaled + 3 * (gb + b), rab) < *cut;
 }
 
 // The FP32 form of k_md2: geometry from the FP32 Cartesian copy, basis, cut-off,
@@ -587,38 +582,40 @@ __global__ void __launch_bounds__(256) k_md2f(ModelDev M, MdDev D, FramesDev F, 
     const float4* c32 = reinterpret_cast<const float4*>(F.cart32);
     const int64_t gb = F.ghost_ofs[f];
     const float4 xi = c32[gb + (warp - aofs)];
+    const float perm = (float)B.perm2, dconst = (float)M.deriv_const, mg = frame_margin(B, F.nlayers);
+    const float pen_dist = (float)D.pen_dist, pen_scale = (float)D.pen_scale;
     float fi[3] = {0.f, 0.f, 0.f}, v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int t = lane; t < n; t += 32) {
         const int64_t q = o + t;
         const int g = NB.g2[q], pt = NB.pt2[q];
-        const PairDev& P = M.pairs[pt];
+        const PairF P = D.pairs[pt];
         float r, R[3];
         if (NB.md == 2) {   // lists reused over steps: this step's geometry
             const float4 xg = c32[gb + g];
             R[0] = xg.x - xi.x; R[1] = xg.y - xi.y; R[2] = xg.z - xi.z;
             r = sqrtf(R[0] * R[0] + R[1] * R[1] + R[2] * R[2]);
-            if (!within_md(F, B, gb, (int)(warp - aofs), g, P.smax)) continue;
+            if (!within_md(F, B, gb, (int)(warp - aofs), g, P.smax, &M.pairs[pt].smax, mg)) continue;
         } else {
             r = (float)NB.r2[q];
             R[0] = (float)NB.rab2[3 * q]; R[1] = (float)NB.rab2[3 * q + 1]; R[2] = (float)NB.rab2[3 * q + 2];
         }
         float fc, fd;
-        fcut_r<float>(M, r, (float)P.smax, fc, fd);
+        fcut_r<float>(M, r, P.smax, fc, fd);
         // Chebyshev basis with a run-time order (as basis_regs_f)
-        const float smin = (float)P.smin, lam = (float)P.lambda;
+        const float smin = P.smin, lam = P.lambda;
         const bool out = r < smin;
         const float rr = out ? smin : r;
-        const float ixd = 1.0f / (float)P.xdiff;
+        const float ixd = 1.0f / P.xdiff;
         float x, ex = 0.0f, dxdr;
-        if (M.trans == 0) { ex = expf(-rr / lam); x = (ex - (float)P.xavg) * ixd; dxdr = -ex / lam * ixd; }
-        else if (M.trans == 1) { x = (1.0f / rr - (float)P.xavg) * ixd; dxdr = -ixd / (rr * rr); }
-        else { x = (rr - (float)P.xavg) * ixd; dxdr = ixd; }
-        dxdr *= (float)M.deriv_const;
+        if (M.trans == 0) { ex = expf(-rr / lam); x = (ex - P.xavg) * ixd; dxdr = -ex / lam * ixd; }
+        else if (M.trans == 1) { x = (1.0f / rr - P.xavg) * ixd; dxdr = -ixd / (rr * rr); }
+        else { x = (rr - P.xavg) * ixd; dxdr = ixd; }
+        dxdr *= dconst;
         const bool zero_d = out && M.fix == 1;
         float damp = 1.0f, shift = 0.0f;
         if (out && M.fix == 0) { damp = expf((r - smin) / (float)M.smooth); shift = (float)M.smooth * (damp - 1.0f); }
         const float lin = (out && M.fix == 2) ? (r - smin) : 0.0f;
-        const double* c = D.c2 + (size_t)pt * ord;
+        const float* c = D.c2f + (size_t)pt * ord;
         float t_prev = 1.0f, t_cur = x, u_prev2 = 0.0f, u_prev = 1.0f, e = 0.0f, gsum = 0.0f;
         for (int k = 1; k <= ord; ++k) {   // 2-body columns use T_1 .. T_order
             float tn, un_1;
@@ -635,17 +632,16 @@ __global__ void __launch_bounds__(256) k_md2f(ModelDev M, MdDev D, FramesDev F, 
                 if (M.fix == 0) { tn += shift * td; td *= damp; }
                 else if (M.fix == 2) tn += td * lin;
             }
-            const float ck = (float)c[k - 1];
+            const float ck = c[k - 1];
             e = fmaf(ck, fc * tn, e);
             gsum = fmaf(ck, fc * td + fd * tn, gsum);
         }
-        const float perm = (float)B.perm2;
         float es = perm * e, gs = perm * gsum;
-        if (r - (float)D.pen_dist < smin) {   // cubic penalty below s_min + d (src/Cheby.C:1900-1968)
-            const float rp = smin + (float)D.pen_dist - r;
+        if (r - pen_dist < smin) {   // cubic penalty below s_min + d (src/Cheby.C:1900-1968)
+            const float rp = smin + pen_dist - r;
             if (rp > 0.0f) {
-                gs += -3.0f * rp * rp * (float)D.pen_scale;
-                es += rp * rp * rp * (float)D.pen_scale;
+                gs += -3.0f * rp * rp * pen_scale;
+                es += rp * rp * rp * pen_scale;
             }
         }
         const float wv = gs / r;
@@ -660,47 +656,56 @@ __global__ void __launch_bounds__(256) k_md2f(ModelDev M, MdDev D, FramesDev F, 
         v[2] -= wv * R[0] * R[0]; v[3] -= wv * R[0] * R[1]; v[4] -= wv * R[0] * R[2];
         v[5] -= wv * R[1] * R[1]; v[6] -= wv * R[1] * R[2]; v[7] -= wv * R[2] * R[2];
     }
-    double fd3[3], vd[8];
-#pragma unroll
-    for (int cc = 0; cc < 3; ++cc) fd3[cc] = warp_sum((double)fi[cc]);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) vd[k] = warp_sum((double)v[k]);
-    if (lane == 0 && n > 0) {
-        double* fo = Fo + 3 * warp;
-        for (int cc = 0; cc < 3; ++cc) atomicAdd(fo + cc, fd3[cc]);
-        double* so = So + (size_t)f * MD_NSCALAR;
-        atomicAdd(so + 0, vd[0]); atomicAdd(so + 1, vd[1]);
-        atomicAdd(so + 2, vd[2]); atomicAdd(so + 3, vd[3]); atomicAdd(so + 4, vd[4]);
-        atomicAdd(so + 5, vd[3]); atomicAdd(so + 6, vd[5]); atomicAdd(so + 7, vd[6]);
-        atomicAdd(so + 8, vd[4]); atomicAdd(so + 9, vd[6]); atomicAdd(so + 10, vd[7]);
-    }
+    const double xd[11] = {fi[0], fi[1], fi[2], v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]};
+    pair_sums_add(xd, Fo + 3 * warp, So + (size_t)f * MD_NSCALAR, n > 0);
 }
 
+// All clusters of the lists in the order of their grouping, and their keys.
+__global__ void k_md_sorted(int64_t n, int nframes, const int64_t* cfo, const int4* m, const int* type, MdBuckets B,
+                            int4* m_out, int* keys) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const int q = B.val[p];
+    m_out[p] = m[q];
+    const int key = frame_of_cluster(cfo, nframes, q) * B.ntypes + type[q];
+    keys[p] = key;
+    const int64_t at = p - B.start[key];
+    if (at % MDC_TILE == 0) B.tile_key[B.tile_ofs[key] + at / MDC_TILE] = key;
+}
+
+// The clusters inside their cut-offs at this step's positions, appended to their key's
+// place: the lists are sorted by key, so a warp makes one or two atomic additions, and
+// each key has room for all its clusters, so no count and scan come first (these, a scatter
+// and a memset, took 31 of 340 us of a step of four frames of 96 to 1,024 atoms).
 template <int NBODY>
-__global__ void k_md_filter(ModelDev M, FramesDev F, ClusterSet CS, const int64_t* cfo, int64_t n, int* type_out) {
+__global__ void k_md_filter(ModelDev M, FramesDev F, const int4* m, const int* keys, const CutDev* cuts, int64_t n,
+                            MdBuckets MB) {
     constexpr int NP = NBODY == 3 ? 3 : 6;
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n) return;
-    const int f = frame_of_cluster(cfo, F.nframes, q);
-    const int4 mm = CS.m[q];
-    const int T = CS.type[q];
-    const int N = F.natoms[f];
-    const int64_t gb = F.ghost_ofs[f];
-    const int* typ = F.type + F.atom_ofs[f];
-    int id = 0, w = 1;
+    bool ok = q < n;
+    const int key = ok ? keys[q] : 0;
+    if (ok) {
+        const int f = key / MB.ntypes, T = key - f * MB.ntypes;
+        const int4 mm = m[q];
+        const int N = F.natoms[f];
+        const int64_t gb = F.ghost_ofs[f];
+        const int* typ = F.type + F.atom_ofs[f];
+        int id = 0, w = 1;
 #pragma unroll
-    for (int u = 0; u < NBODY; ++u) { id += w * (typ[member(mm, u) % N] + 1); w *= 10; }
-    const int8_t* pm = (NBODY == 3 ? M.pidx3 : M.pidx4) + id * NP;
-    const ClusterTypeDev& CT = (NBODY == 3 ? M.types3 : M.types4)[T];
-    const BoxDev& B = F.box[f];
-    bool ok = true;
+        for (int u = 0; u < NBODY; ++u) { id += w * (typ[member(mm, u) % N] + 1); w *= 10; }
+        const int8_t* pm = (NBODY == 3 ? M.pidx3 : M.pidx4) + id * NP;
+        const CutDev* C = cuts + T * NP;
+        const BoxDev& B = F.box[f];
+        const float mg = frame_margin(B, F.nlayers);
 #pragma unroll
-    for (int e = 0; e < NP; ++e) {
-        int a, b;
-        edge_ab(NBODY, e, a, b);
-        ok = ok && within_md(F, B, gb, member(mm, a), member(mm, b), CT.smax[pm[e]]);
+        for (int e = 0; e < NP; ++e) {
+            int a, b;
+            edge_ab(NBODY, e, a, b);
+            ok = ok && within_md(F, B, gb, member(mm, a), member(mm, b), C[pm[e]].cutf, &C[pm[e]].cut, mg);
+        }
     }
-    type_out[q] = ok ? T : -1;
+    const int slot = warp_agg_inc(MB.cursor, key, ok);
+    if (ok) MB.val[MB.start[key] + slot] = (int)q;
 }
 
 // Largest squared displacement since the lists were built (as ordered bits of a
@@ -751,6 +756,8 @@ __global__ void k_md_drift(FramesDev F, const unsigned char* first, int64_t n3, 
     v[i] = v[i] + 0.5 * a[i] * dt;
 }
 
+// One CTA per frame where its kinetic energy is wanted, 16 where not (four frames of up to
+// 1,024 atoms, one CTA each -> 16: 17.5 -> 4.7 us).
 __global__ void k_md_kick(FramesDev F, const double* Fo, const double* inv_mass_type, const double* mass_type,
                           double* acc, double* v, double dt, int half, const unsigned char* first, double* ke) {
     const int f = blockIdx.x;
@@ -758,13 +765,13 @@ __global__ void k_md_kick(FramesDev F, const double* Fo, const double* inv_mass_
     const int N = F.natoms[f];
     const int64_t aofs = F.atom_ofs[f];
     double k = 0.0;
-    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
         const int64_t g = 3 * aofs + i;
         const int t = F.type[aofs + i / 3];
         const double a = Fo[g] * inv_mass_type[t];
         acc[g] = a;
         if (half) v[g] = v[g] + 0.5 * a * dt;
-        k += 0.5 * mass_type[t] * v[g] * v[g];
+        if (ke) k += 0.5 * mass_type[t] * v[g] * v[g];
     }
     if (!ke) return;
     __shared__ double red[32];
@@ -803,7 +810,7 @@ __global__ void k_md_mtk_half1(FramesDev F, const double* mass_type, double* x, 
     const int64_t aofs = F.atom_ofs[f];
     double* t = th + (size_t)f * MD_TH_STRIDE;
     double k = 0.0;
-    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
         const int64_t g = 3 * aofs + i;
         k += 0.5 * mass_type[F.type[aofs + i / 3]] * v[g] * v[g];
     }
@@ -858,7 +865,7 @@ __global__ void k_md_mtk_half2(FramesDev F, const double* Fo, const double* inv_
         fT = (2.0 * (k0 / (s * s)) - nkt) / Q;
     }
     double k = 0.0;
-    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
         const int64_t g = 3 * aofs + i;
         const double vn = (v[g] + 0.5 * acc[g] * dt) / s;
         v[g] = vn;
@@ -882,7 +889,7 @@ __global__ void k_md_berend(FramesDev F, const double* mass_type, double* v, dou
     const int N = F.natoms[f];
     const int64_t aofs = F.atom_ofs[f];
     double k = 0.0;
-    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
         const int64_t g = 3 * aofs + i;
         k += 0.5 * mass_type[F.type[aofs + i / 3]] * v[g] * v[g];
     }
@@ -979,12 +986,19 @@ void launch_mdc(int nbody, int prec, int order, int64_t max_tiles, const ModelDe
     else k_mdc_generic<4><<<grid, MDC_THREADS, 0, st>>>(M, D, F, CS, B, order, Fo, So);
 }
 
-void launch_md_filter(int nbody, const ModelDev& M, const FramesDev& F, const ClusterSet& CS, const int64_t* cfo,
-                      int64_t n, int* type_out, cudaStream_t st) {
+void launch_md_sorted(int64_t n, int nframes, const int64_t* cfo, const ClusterSet& CS, const MdBuckets& B, int4* m,
+                      int* key, cudaStream_t st) {
     if (n <= 0) return;
+    k_md_sorted<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, nframes, cfo, CS.m, CS.type, B, m, key);
+}
+
+void launch_md_filter(int nbody, const ModelDev& M, const FramesDev& F, const int4* m, const int* key,
+                      const CutDev* cuts, int64_t n, const MdBuckets& B, cudaStream_t st) {
+    if (n <= 0) return;
+    cudaMemsetAsync(B.cursor, 0, sizeof(int) * B.nkeys, st);
     const unsigned g = (unsigned)((n + 255) / 256);
-    if (nbody == 3) k_md_filter<3><<<g, 256, 0, st>>>(M, F, CS, cfo, n, type_out);
-    else k_md_filter<4><<<g, 256, 0, st>>>(M, F, CS, cfo, n, type_out);
+    if (nbody == 3) k_md_filter<3><<<g, 256, 0, st>>>(M, F, m, key, cuts, n, B);
+    else k_md_filter<4><<<g, 256, 0, st>>>(M, F, m, key, cuts, n, B);
 }
 
 void launch_md_maxdisp(const double* x, const double* xref, int64_t n, unsigned long long* out, cudaStream_t st) {
@@ -1006,7 +1020,7 @@ void launch_md_kick(int nframes, const FramesDev& F, const double* Fo, const dou
                     const double* mass_type, double* acc, double* v, double dt, int half, const unsigned char* first,
                     double* ke, cudaStream_t st) {
     if (nframes > 0)
-        k_md_kick<<<nframes, 256, 0, st>>>(F, Fo, inv_mass_type, mass_type, acc, v, dt, half, first, ke);
+        k_md_kick<<<dim3(nframes, ke ? 1 : 16), ke ? 1024 : 256, 0, st>>>(F, Fo, inv_mass_type, mass_type, acc, v, dt, half, first, ke);
 }
 
 void launch_md_mtk_half1(int nframes, const FramesDev& F, const double* mass_type, double* x, double* v,
@@ -1070,7 +1084,7 @@ __global__ void k_md_npt_berend(FramesDev F, BoxDev* box, const double* mass_typ
     const int N = F.natoms[f];
     const int64_t aofs = F.atom_ofs[f];
     double k = 0.0;
-    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
         const int64_t g = 3 * aofs + i;
         k += 0.5 * mass_type[F.type[aofs + i / 3]] * v[g] * v[g];
     }
@@ -1222,7 +1236,7 @@ __global__ void k_md_nptmtk_half2(FramesDev F, const double* Fo, const double* i
         s = 1.0 + 0.5 * dt * (zT + cdof * bvT);
     }
     double k = 0.0;
-    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
         const int64_t g = 3 * aofs + i;
         const double vn = v[g] / s_used;
         v[g] = vn;
@@ -1247,7 +1261,7 @@ __global__ void k_md_vscale(FramesDev F, const double* mass_type, double* v, dou
     const int64_t aofs = F.atom_ofs[f];
     double* t = th + (size_t)f * MD_TH_STRIDE;
     double k = 0.0;
-    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
         const int64_t g = 3 * aofs + i;
         k += 0.5 * mass_type[F.type[aofs + i / 3]] * v[g] * v[g];
     }

@@ -18,12 +18,22 @@ namespace cgd {
 //   [2..10] virial tensor / V, row-major xx xy xz yx yy yz zx zy zz.
 constexpr int MD_NSCALAR = 11;
 
+// FP32 copies of a pair type's constants for the FP32 form: a conversion takes the FP64 pipe,
+// and a dozen per slot and pair outweighed the FP32 arithmetic.
+struct PairF {
+    float smin, smax, lambda, xavg, xdiff, pad[3];
+};
+
 struct MdDev {
     const double* c2;       // [npairs * order2]  coefficient of T_{n+1} of pair type
     const double* C3;       // [ntypes3 * O3^3]   dense, canonical slots, slot 0 most significant
     const double* C4;       // [ntypes4 * O4^6]
     const float* C3f;       // FP32 copies (contraction precision 1)
     const float* C4f;
+    const float* c2f;
+    const PairF* pairs;     // of the pair types' constants
+    const float4* slot3;    // [ntypes][3 or 6] s_max, x_avg, x_diff, s_min of the slots
+    const float4* slot4;
     const double* eoff;     // [natmtyp] per-atom energy offsets, or null
     double pen_dist, pen_scale;   // 2-body penalty (src/chimes_md.C:1747-1748 defaults)
     int coulomb;            // Ewald sums with the charges qtype (electron units)
@@ -40,10 +50,11 @@ void launch_md_ewald(int nframes, int nreal, int kmax_max, const ModelDev& M, co
 // order inside a group is not fixed (the forces are accumulated with atomics).
 struct MdBuckets {
     int nkeys, ntypes;
-    int64_t* start;       // [nkeys + 1] first grouped cluster of each key
+    int64_t* start;       // [nkeys + 1] where each key's clusters begin
     int* tile_ofs;        // [nkeys + 1] first MDC tile (block) of each key
-    int* cursor;          // [nkeys] fill cursors
+    int* cursor;          // [nkeys] clusters of each key (fill cursors)
     int* val;             // [n] global cluster indices, grouped
+    int* tile_key = nullptr;   // [tiles] each tile's key, where the grouping is kept (else searched)
 };
 constexpr int MDC_TILE = 64;    // clusters per contraction block
 
@@ -72,10 +83,13 @@ void launch_mdt(int nbody, int64_t max_tiles, const ModelDev& M, const FramesDev
                 const MdBuckets& B, const unsigned char* tab, const int* ex, double* Fo, double* So, cudaStream_t st);
 void launch_md_finalize(int nframes, const ModelDev& M, const MdDev& D, const FramesDev& F, double* So,
                         cudaStream_t st);
-// List reuse: per-step exact filter of skin-enumerated clusters (type_out -1 when
-// out of range), and the largest squared displacement since the lists were built.
-void launch_md_filter(int nbody, const ModelDev& M, const FramesDev& F, const ClusterSet& CS, const int64_t* cfo,
-                      int64_t n, int* type_out, cudaStream_t st);
+// Lists reused over steps: the clusters m and their keys in the order of B.val (a grouping
+// of all of them), then each step the clusters inside their cut-offs at this step's
+// positions into B.val / B.cursor, each key's from its start on.
+void launch_md_sorted(int64_t n, int nframes, const int64_t* cfo, const ClusterSet& CS, const MdBuckets& B, int4* m,
+                      int* key, cudaStream_t st);
+void launch_md_filter(int nbody, const ModelDev& M, const FramesDev& F, const int4* m, const int* key,
+                      const CutDev* cuts, int64_t n, const MdBuckets& B, cudaStream_t st);
 void launch_md_maxdisp(const double* x, const double* xref, int64_t n, unsigned long long* out, cudaStream_t st);
 
 // Velocity Verlet (CONSTRAINT::UPDATE_COORDS / UPDATE_VELOCS_HALF_1 / _2,

@@ -90,6 +90,21 @@ void Session::md_setup(const double* x, int nx, int precision, bool offsets, dou
             CK(cudaGetLastError());
         }
     std::vector<float> C3f(C3.begin(), C3.end()), C4f(C4.begin(), C4.end());
+    std::vector<float> c2f(c2.begin(), c2.end());
+    t->dev.c2f = (const float*)up(c2f.data(), c2f.size() * sizeof(float));
+    std::vector<cgd::PairF> pf;
+    for (const auto& p : m.pairs)
+        pf.push_back({(float)p.smin, (float)p.smax, (float)p.lambda, (float)p.xavg, (float)p.xdiff, {}});
+    t->dev.pairs = (const cgd::PairF*)up(pf.data(), pf.size() * sizeof(cgd::PairF));
+    auto slots = [&](const ClusterList& cl, int np) {
+        std::vector<float4> v;
+        for (const auto& ct : cl.vec)
+            for (int s = 0; s < np; ++s)
+                v.push_back(make_float4((float)ct.smax[s], (float)ct.xavg[s], (float)ct.xdiff[s], (float)ct.smin[s]));
+        return (const float4*)up(v.data(), v.size() * sizeof(float4));
+    };
+    t->dev.slot3 = o3 > 0 ? slots(m.trips, 3) : nullptr;
+    t->dev.slot4 = o4 > 0 ? slots(m.quads, 6) : nullptr;
     t->dev.C3f = (const float*)up(C3f.data(), C3f.size() * sizeof(float));
     t->dev.C4f = (const float*)up(C4f.data(), C4f.size() * sizeof(float));
     t->dev.eoff = nullptr;
@@ -150,6 +165,7 @@ void Session::md_force(const DeviceFrames& df, double* Fo, double* So, MdCounts*
     cgd::NeighDev NB{};
     NB.n_real = nreal;
     NB.md = 1;
+    NB.cut3 = dm_->cut3; NB.cut4 = dm_->cut4;
     NB.cnt2 = S.get<int>(nreal); NB.cnt3 = S.get<int>(nreal); NB.cnt4 = S.get<int>(nreal);
     NB.ofs2 = S.get<int64_t>(nreal + 1); NB.ofs3 = S.get<int64_t>(nreal + 1); NB.ofs4 = S.get<int64_t>(nreal + 1);
     cgd::launch_neigh(M, F, NB, 0, st); L();
@@ -272,6 +288,12 @@ void Session::md_lists_build(DeviceFrames& df, double skin, MdLists& L, cudaStre
     NB.n_real = nreal;
     NB.md = 2;
     NB.skin = skin;
+    for (int nb = 3; nb <= 4; ++nb) {
+        const int n = nb == 3 ? M.ntypes3 * 3 : M.ntypes4 * 6;
+        cgd::CutDev* c = (cgd::CutDev*)get(sizeof(cgd::CutDev) * n);
+        cgd::launch_cuts(M, nb, skin, c, st);
+        (nb == 3 ? NB.cut3 : NB.cut4) = c;
+    }
     NB.cnt2 = (int*)get(sizeof(int) * nreal); NB.cnt3 = (int*)get(sizeof(int) * nreal);
     NB.cnt4 = (int*)get(sizeof(int) * nreal);
     NB.ofs2 = (int64_t*)get(sizeof(int64_t) * (nreal + 1)); NB.ofs3 = (int64_t*)get(sizeof(int64_t) * (nreal + 1));
@@ -341,12 +363,14 @@ void Session::md_lists_build(DeviceFrames& df, double skin, MdLists& L, cudaStre
         if (!use[k] || L.ncl[k] == 0) continue;
         const int64_t n = L.ncl[k];
         const int ntypes = k == 0 ? M.ntypes3 : M.ntypes4;
-        L.CS[k].m = (int4*)get(sizeof(int4) * n);
-        L.CS[k].type = (int*)get(sizeof(int) * n);
+        Scratch tmp(st);   // the clusters as enumerated; the lists keep them grouped
+        L.CS[k].m = tmp.get<int4>(n);
+        L.CS[k].type = tmp.get<int>(n);
         cgd::launch_clusters(3 + k, M, F, NB, L.CS[k], 1, st);
-        L.cfo[k] = (int64_t*)get(sizeof(int64_t) * (nf + 1));
-        cgd::launch_gather_frame_ofs(L.CS[k].ofs, F.atom_ofs, nf, L.cfo[k], st);
-        L.tstep[k] = (int*)get(sizeof(int) * n);
+        int64_t* cfo = (int64_t*)get(sizeof(int64_t) * (nf + 1));
+        cgd::launch_gather_frame_ofs(L.CS[k].ofs, F.atom_ofs, nf, cfo, st);
+        L.sorted[k] = (int4*)get(sizeof(int4) * n);
+        L.key[k] = (int*)get(sizeof(int) * n);
         cgd::MdBuckets& B = L.B[k];
         B.ntypes = ntypes;
         B.nkeys = nf * ntypes;
@@ -354,6 +378,11 @@ void Session::md_lists_build(DeviceFrames& df, double skin, MdLists& L, cudaStre
         B.tile_ofs = (int*)get(sizeof(int) * (B.nkeys + 1));
         B.cursor = (int*)get(sizeof(int) * B.nkeys);
         B.val = (int*)get(sizeof(int) * n);
+        B.tile_key = (int*)get(sizeof(int) * ((n + cgd::MDC_TILE - 1) / cgd::MDC_TILE + B.nkeys));
+        cgd::launch_md_bucket(n, nf, cfo, L.CS[k].type, B, st);
+        cgd::launch_md_sorted(n, nf, cfo, L.CS[k], B, L.sorted[k], L.key[k], st);
+        L.CS[k].m = L.sorted[k];
+        L.CS[k].type = nullptr;
     }
     mark(ST_CLUSTERS, false);
     CK(cudaGetLastError());
@@ -398,14 +427,12 @@ void Session::md_force_lists(DeviceFrames& df, MdLists& L, double* Fo, double* S
     bool joined[2] = {false, false};
     for (int k = 0; k < 2; ++k) {
         const int64_t n = L.ncl[k];
-        if (n == 0 || !L.tstep[k]) continue;
+        if (n == 0) continue;
         cudaStream_t sk = fork ? md_side_[k] : st;
         if (fork) CK(cudaStreamWaitEvent(sk, md_fork_, 0));
         cgd::ClusterSet CS = L.CS[k];
         mark(ST_BUCKET, true);
-        cgd::launch_md_filter(3 + k, M, F, CS, L.cfo[k], n, L.tstep[k], sk);
-        CS.type = L.tstep[k];
-        cgd::launch_md_bucket(n, nf, L.cfo[k], L.tstep[k], L.B[k], sk);
+        cgd::launch_md_filter(3 + k, M, F, CS.m, L.key[k], k == 0 ? dm_->cut3 : dm_->cut4, n, L.B[k], sk);
         mark(ST_BUCKET, false);
         const int64_t max_tiles = (n + cgd::MDC_TILE - 1) / cgd::MDC_TILE + L.B[k].nkeys;
         mark(k == 0 ? ST_FORCE3 : ST_FORCE4, true);

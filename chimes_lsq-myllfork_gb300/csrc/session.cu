@@ -48,7 +48,7 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
                         const int** int_map, const int8_t** pidx, const int8_t** rev, const cgd::ClusterTypeDev** types,
                         const uint8_t** pows, const int** grps, int& max_allowed, cgd::OzTables& oz,
                         cgd::RgTables (&rg)[2],
-                        const int** vord, int& nychunk) {
+                        const int** vord, int& nychunk, const cgd::CutDev** cuts) {
     const int np = nb == 3 ? 3 : 6;
     const int dim = nb == 3 ? 1000 : 10000;
     std::vector<int> imap(dim, -1);
@@ -66,6 +66,9 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
     std::vector<int> gp;
     std::vector<uint4> of;      // force-table entries of each power for each owner role
     std::vector<int> tc;        // column of each power within its type
+    size_t npow = 0;
+    for (const ClusterType& ct : cl.vec) npow += ct.excluded ? 0 : ct.n_allowed;
+    pw.reserve(npow * np); of.reserve(npow); tc.reserve(npow);
     int sizeI = 1, sizeO = 1;
     for (int k = 0; k < nb - 1; ++k) sizeI *= ord;
     for (int k = 0; k < np - nb + 1; ++k) sizeO *= ord;
@@ -110,24 +113,21 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
         int nch = 0, threads = 0;
         d.vir_chunk[0] = 0;
         std::vector<int> count(sizeI, 0);
+        static_assert((cgd::VIR_PPT & (cgd::VIR_PPT - 1)) == 0, "powers per thread");
         for (int p = 0, gend; p < d.n_allowed; p = gend) {
             for (gend = p + 1; gend < d.n_allowed && ct.param_indices[gend] == ct.param_indices[p];) ++gend;
-            auto add = [&](int by) {
-                for (int q = p; q < gend; ++q) {
-                    const int i = (int)(of[d.pow_offset / np + q].x & 0xffffu);
-                    threads -= (count[i] + vgr - 1) / vgr;
-                    count[i] += by;
-                    threads += (count[i] + vgr - 1) / vgr;
-                }
+            auto add = [&]() {   // vgr is a power of two
+                for (int q = p; q < gend; ++q)
+                    threads += (count[of[d.pow_offset / np + q].x & 0xffffu]++ & (vgr - 1)) == 0;
             };
-            add(1);
+            add();
             if (threads > cgd::MB_THREADS) {   // the group opens a new chunk
                 if (p == d.vir_chunk[nch]) throw Error(2, "power group larger than a chunk");
                 if (nch + 1 >= cgd::MAXCHUNK) throw Error(2, "too many power chunks for one cluster type");
                 d.vir_chunk[++nch] = p;
                 std::fill(count.begin(), count.end(), 0);
                 threads = 0;
-                add(1);
+                add();
                 if (threads > cgd::MB_THREADS) throw Error(2, "power group larger than a chunk");
             }
         }
@@ -176,6 +176,11 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
                     }
                 }
         }
+    std::vector<cgd::CutDev> cu;
+    for (const auto& d : tv)
+        for (int s = 0; s < np; ++s) cu.push_back({d.smax[s], (float)d.smax[s], 0.0f});
+    if (cu.empty()) cu.push_back({0.0, 0.0f, 0.0f});
+    *cuts = dev_upload(D.allocs, cu.data(), cu.size());
     oz.cix = dev_upload(D.allocs, cx.data(), cx.size());
     oz.type = dev_upload(D.allocs, ti.data(), ti.size());
     *int_map = dev_upload(D.allocs, imap.data(), imap.size());
@@ -215,19 +220,23 @@ static void upload_list(const Model& m, const ClusterList& cl, int nb, int ord, 
     for (const auto& d : tv) na.push_back(d.n_allowed);
     for (int prec = 0; prec < 2; ++prec) {
         const int nt = cgd::rg_threads(na.data(), (int)na.size(), prec == 0 ? 8 : 4);
-        std::vector<uint4> ro;
-        std::vector<int> rc;
+        size_t total = 0;
+        for (const auto& d : tv) total += (size_t)((d.n_allowed + nt - 1) / nt) * nt;
+        std::vector<uint4> ro(total, make_uint4(0, 0, 0, 0));
+        std::vector<int> rc(total, 0);
+        size_t at = 0;
         for (const auto& d : tv) {
             const int n = d.n_allowed, S = (n + nt - 1) / nt, p0 = d.pow_offset / np;
-            const size_t at = ro.size();
-            ro.resize(at + (size_t)S * nt, make_uint4(0, 0, 0, 0));
-            rc.resize(at + (size_t)S * nt, 0);
-            for (int p = 0; p < n; ++p) {
-                const size_t q = at + (size_t)(p % S) * nt + p / S;
-                ro[q] = of[p0 + p];
-                rc[q] = tc[p0 + p] | (p > 0 && tc[p0 + p - 1] == tc[p0 + p] ? cgd::RG_CONT : 0) |
-                        (p == n - 1 || tc[p0 + p + 1] != tc[p0 + p] ? cgd::RG_LAST : 0);
-            }
+            const uint4* o = of.data() + p0;
+            const int* c = tc.data() + p0;
+            for (int t = 0, p = 0; p < n; ++t)
+                for (int i = 0; i < S && p < n; ++i, ++p) {
+                    const size_t q = at + (size_t)i * nt + t;
+                    ro[q] = o[p];
+                    rc[q] = c[p] | (p > 0 && c[p - 1] == c[p] ? cgd::RG_CONT : 0) |
+                            (p == n - 1 || c[p + 1] != c[p] ? cgd::RG_LAST : 0);
+                }
+            at += (size_t)S * nt;
         }
         if (ro.empty()) { ro.push_back(make_uint4(0, 0, 0, 0)); rc.push_back(0); }
         rg[prec].offs = dev_upload(D.allocs, ro.data(), ro.size());
@@ -265,10 +274,10 @@ DeviceModel::DeviceModel(const Model& m) {
     d.pairs = dev_upload(allocs, pv.data(), pv.size());
     if (c.use3)
         upload_list(m, m.trips, 3, c.cheby3, d.col3, *this, &d.int_map3, &d.pidx3, &d.rev3, &d.types3,
-                    &d.pow3, &d.grp3, max_allowed3, oz3, rg3, &vord3, nychunk3);
+                    &d.pow3, &d.grp3, max_allowed3, oz3, rg3, &vord3, nychunk3, &cut3);
     if (c.use4)
         upload_list(m, m.quads, 4, c.cheby4, d.col4, *this, &d.int_map4, &d.pidx4, &d.rev4, &d.types4,
-                    &d.pow4, &d.grp4, max_allowed4, oz4, rg4, &vord4, nychunk4);
+                    &d.pow4, &d.grp4, max_allowed4, oz4, rg4, &vord4, nychunk4, &cut4);
 }
 
 DeviceModel::~DeviceModel() {
@@ -832,6 +841,7 @@ void Session::run(const DeviceFrames& df, int precision, void* A, int64_t lda, A
     mark(ST_NEIGH, true);
     cgd::NeighDev NB{};
     NB.n_real = nreal;
+    NB.cut3 = dm_->cut3; NB.cut4 = dm_->cut4;
     NB.cnt2 = S.get<int>(nreal); NB.cnt3 = S.get<int>(nreal); NB.cnt4 = S.get<int>(nreal);
     NB.ofs2 = S.get<int64_t>(nreal + 1); NB.ofs3 = S.get<int64_t>(nreal + 1); NB.ofs4 = S.get<int64_t>(nreal + 1);
     cgd::launch_neigh(M, F, NB, 0, st); L();

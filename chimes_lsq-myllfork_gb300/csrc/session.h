@@ -26,6 +26,7 @@ struct DeviceModel {
     std::vector<void*> allocs;
     int max_allowed3 = 0, max_allowed4 = 0;   // most allowed powers of a cluster type
     cgd::OzTables oz3, oz4;
+    const cgd::CutDev *cut3 = nullptr, *cut4 = nullptr;   // cut-offs of the slots (no skin)
     cgd::RgTables rg3[2], rg4[2];   // FP64, FP32
     // the powers of k_virial_mb's threads: [type][chunk][power of the thread][thread], -1: none
     const int *vord3 = nullptr, *vord4 = nullptr;
@@ -104,8 +105,8 @@ struct MdLists {
     cgd::NeighDev NB{};
     cgd::ClusterSet CS[2]{};
     int64_t ncl[2] = {0, 0};
-    int* tstep[2] = {nullptr, nullptr};   // per-step type (-1: out of range)
-    int64_t* cfo[2] = {nullptr, nullptr};
+    int4* sorted[2] = {nullptr, nullptr};   // clusters by (frame, type), and those keys
+    int* key[2] = {nullptr, nullptr};
     cgd::MdBuckets B[2]{};
     double* xref = nullptr;               // positions at the build
     int* shift = nullptr;                 // wrap shifts at the build
