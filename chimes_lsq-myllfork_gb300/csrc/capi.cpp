@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "model.h"
+#include "scratch.h"
 #include "session.h"
 #include "md_server.h"
 #include "textio.h"
@@ -589,9 +590,7 @@ int cg_md_force(cg_session* s, const cg_frames* fr, double* forces, double* scal
         cudaStream_t st = s->s->stream();
         std::unique_ptr<cg::DeviceFrames> d = s->s->upload(fr->fb);
         const size_t nf = (size_t)fr->fb.natoms_total * 3, ns = (size_t)fr->fb.nframes * cgd::MD_NSCALAR;
-        double* dF = nullptr;
-        cg::cuda_check(cudaMallocAsync((void**)&dF, std::max<size_t>(1, nf + ns) * sizeof(double), st),
-                       "cudaMallocAsync(forces)");
+        double* dF = cg::scratch_alloc<double>(nf + ns, st);
         try {
             s->s->md_force(*d, dF, dF + nf, &s->md_last);
             cg::cuda_check(cudaMemcpyAsync(forces, dF, nf * sizeof(double), cudaMemcpyDeviceToHost, st),

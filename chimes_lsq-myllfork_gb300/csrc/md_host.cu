@@ -241,22 +241,21 @@ void Session::md_force(const DeviceFrames& df, double* Fo, double* So, MdCounts*
     if (counts) *counts = c;
 }
 
-void* MdLists::buffer(int slot, size_t bytes) {
+void* MdLists::buffer(int slot, size_t bytes, cudaStream_t st) {
     bytes = std::max<size_t>(bytes, 8);
     if ((int)allocs.size() <= slot) { allocs.resize(slot + 1, nullptr); caps.resize(slot + 1, 0); }
     if (caps[slot] < bytes) {
-        if (allocs[slot]) CK(cudaFree(allocs[slot]));
+        std::vector<void*> old(1, allocs[slot]);
+        if (old[0]) pool_free(old);
         allocs[slot] = nullptr;
         const size_t grown = bytes + bytes / 4;   // room for the next build
-        CK(cudaMalloc(&allocs[slot], grown));
+        allocs[slot] = pool_alloc(grown, st);
         caps[slot] = grown;
     }
     return allocs[slot];
 }
 
-MdLists::~MdLists() {
-    for (void* p : allocs) if (p) cudaFree(p);
-}
+MdLists::~MdLists() { pool_free(allocs); }
 
 void Session::md_lists_build(DeviceFrames& df, double skin, MdLists& L, cudaStream_t st) {
     CK(cudaSetDevice(device_));
@@ -269,7 +268,7 @@ void Session::md_lists_build(DeviceFrames& df, double skin, MdLists& L, cudaStre
     L.skin = skin;
     L.natoms = nreal;
     int slot = 0;
-    auto get = [&](size_t bytes) { return L.buffer(slot++, bytes); };
+    auto get = [&](size_t bytes) { return L.buffer(slot++, bytes, st); };
     L.shift = (int*)get(sizeof(int) * 3 * std::max(nreal, 1));
     L.xref = (double*)get(sizeof(double) * 3 * std::max(nreal, 1));
     L.dmax = (unsigned long long*)get(sizeof(unsigned long long));
@@ -820,6 +819,7 @@ size_t arena_bytes(int64_t atoms, int frames, int nimg) {
 // Device arrays of one batch composition, sized for the largest batch.
 struct ServeArena {
     std::vector<void*> allocs;
+    Layout lay;
     int* natoms = nullptr;
     int64_t *atom_ofs = nullptr, *ghost_ofs = nullptr, *row_ofs = nullptr;
     int *stress_rows = nullptr, *energy_rows = nullptr, *type = nullptr;
@@ -827,46 +827,59 @@ struct ServeArena {
     double *xyz = nullptr, *v = nullptr, *acc = nullptr, *scaled = nullptr, *Fo = nullptr, *So = nullptr;
     float* cart32 = nullptr;
     unsigned char* first = nullptr;
-    template <typename T>
-    T* get(size_t n) {
-        void* p = nullptr;
-        CK(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)));
-        allocs.push_back(p);
-        CK(cudaMemset(p, 0, std::max<size_t>(n, 1) * sizeof(T)));
-        return reinterpret_cast<T*>(p);
+    void arrays(int64_t atoms, int frames, int nimg) {
+        natoms = lay.take<int>(frames);
+        atom_ofs = lay.take<int64_t>(frames + 1);
+        ghost_ofs = lay.take<int64_t>(frames + 1);
+        row_ofs = lay.take<int64_t>(frames + 1);
+        stress_rows = lay.take<int>(frames);
+        energy_rows = lay.take<int>(frames);
+        box = lay.take<cgd::BoxDev>(frames);
+        type = lay.take<int>(atoms);
+        xyz = lay.take<double>(3 * atoms);
+        v = lay.take<double>(3 * atoms);
+        acc = lay.take<double>(3 * atoms);
+        Fo = lay.take<double>(3 * atoms);
+        So = lay.take<double>((size_t)frames * cgd::MD_NSCALAR);
+        scaled = lay.take<double>(3 * atoms * nimg);
+        cart32 = lay.take<float>(4 * atoms * nimg);
+        first = lay.take<unsigned char>(frames);
     }
-    void init(int64_t atoms, int frames, int nimg) {
-        natoms = get<int>(frames);
-        atom_ofs = get<int64_t>(frames + 1);
-        ghost_ofs = get<int64_t>(frames + 1);
-        row_ofs = get<int64_t>(frames + 1);
-        stress_rows = get<int>(frames);
-        energy_rows = get<int>(frames);
-        box = get<cgd::BoxDev>(frames);
-        type = get<int>(atoms);
-        xyz = get<double>(3 * atoms);
-        v = get<double>(3 * atoms);
-        acc = get<double>(3 * atoms);
-        Fo = get<double>(3 * atoms);
-        So = get<double>((size_t)frames * cgd::MD_NSCALAR);
-        scaled = get<double>(3 * atoms * nimg);
-        cart32 = get<float>(4 * atoms * nimg);
-        first = get<unsigned char>(frames);
+    void init(int64_t atoms, int frames, int nimg, cudaStream_t st) {
+        arrays(atoms, frames, nimg);
+        lay.base = static_cast<unsigned char*>(pool_alloc(lay.used, st));
+        allocs.push_back(lay.base);
+        CK(cudaMemsetAsync(lay.base, 0, lay.used, st));
+        lay.used = 0;
+        arrays(atoms, frames, nimg);
     }
-    ~ServeArena() { for (void* p : allocs) cudaFree(p); }
+    ~ServeArena() { pool_free(allocs); }
 };
 
-template <typename T>
-struct Pinned {
-    T* p = nullptr;
-    size_t n = 0;
-    void reserve(size_t m) {
-        if (m <= n) return;
-        if (p) cudaFreeHost(p);
-        CK(cudaMallocHost((void**)&p, std::max<size_t>(m, 1) * sizeof(T)));
-        n = m;
+// The pinned host arrays of a batch composition, one allocation.
+struct ServeHost {
+    Layout lay;
+    int *nat = nullptr, *type = nullptr;
+    int64_t *aofs = nullptr, *gofs = nullptr;
+    cgd::BoxDev* box = nullptr;
+    unsigned char* first = nullptr;
+    double* mass = nullptr;   // masses, then their inverses
+    void arrays(int64_t atoms, int frames, int ntypes) {
+        nat = lay.take<int>(frames);
+        aofs = lay.take<int64_t>(frames + 1);
+        gofs = lay.take<int64_t>(frames + 1);
+        box = lay.take<cgd::BoxDev>(frames);
+        first = lay.take<unsigned char>(frames);
+        type = lay.take<int>(atoms);
+        mass = lay.take<double>(2 * ntypes);
     }
-    ~Pinned() { if (p) cudaFreeHost(p); }
+    void init(int64_t atoms, int frames, int ntypes) {
+        arrays(atoms, frames, ntypes);
+        CK(cudaMallocHost((void**)&lay.base, lay.used));
+        lay.used = 0;
+        arrays(atoms, frames, ntypes);
+    }
+    ~ServeHost() { if (lay.base) cudaFreeHost(lay.base); }
 };
 
 double now_s(std::chrono::steady_clock::time_point t0) {
@@ -991,21 +1004,15 @@ int64_t Session::serve_loop(ServeSource& src, const double* mass_type, const MdS
         throw Error(1, "hbm_budget of " + std::to_string((long long)opt.hbm_budget) + " bytes is below the " +
                            std::to_string((long long)fixed) + " bytes of the serving arenas for max_batch_atoms");
     ServeArena arena[2];
-    arena[0].init(cap_atoms, cap_frames, nimg);
-    arena[1].init(cap_atoms, cap_frames, nimg);
-    double *dm = nullptr, *dim = nullptr;
-    CK(cudaMalloc((void**)&dm, nt * sizeof(double)));
-    CK(cudaMalloc((void**)&dim, nt * sizeof(double)));
-    std::unique_ptr<double, void (*)(double*)> g1(dm, [](double* p) { cudaFree(p); });
-    std::unique_ptr<double, void (*)(double*)> g2(dim, [](double* p) { cudaFree(p); });
-    CK(cudaMemcpy(dm, mv.data(), nt * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(dim, im.data(), nt * sizeof(double), cudaMemcpyHostToDevice));
-    Pinned<int> h_nat, h_type;
-    Pinned<int64_t> h_aofs, h_gofs;
-    Pinned<cgd::BoxDev> h_box;
-    Pinned<unsigned char> h_first;
-    h_nat.reserve(cap_frames); h_aofs.reserve(cap_frames + 1); h_gofs.reserve(cap_frames + 1);
-    h_box.reserve(cap_frames); h_first.reserve(cap_frames); h_type.reserve(cap_atoms);
+    for (ServeArena& a : arena) a.init(cap_atoms, cap_frames, nimg, st);
+    ServeHost H;
+    H.init(cap_atoms, cap_frames, nt);
+    for (int i = 0; i < nt; ++i) { H.mass[i] = mv[i]; H.mass[nt + i] = im[i]; }
+    std::vector<void*> masses(1, pool_alloc(2 * nt * sizeof(double), st));
+    std::unique_ptr<std::vector<void*>, void (*)(std::vector<void*>*)> masses_guard(
+        &masses, [](std::vector<void*>* p) { pool_free(*p); });
+    double *dm = static_cast<double*>(masses[0]), *dim = dm + nt;
+    CK(cudaMemcpyAsync(dm, H.mass, 2 * nt * sizeof(double), cudaMemcpyHostToDevice, st));
 
     // per-request state, by id
     std::vector<int> steps_done;
@@ -1058,14 +1065,14 @@ int64_t Session::serve_loop(ServeSource& src, const double* mass_type, const MdS
         if (changed) {
             // new composition in the other arena: carried-over state copied on the device
             int64_t ofs = 0;
-            h_aofs.p[0] = 0; h_gofs.p[0] = 0;
+            H.aofs[0] = 0; H.gofs[0] = 0;
             for (int k = 0; k < nf; ++k) {
                 const int r = active[k];
                 const MdRequest& q = src.request(r);
                 const int n = q.natoms;
-                h_nat.p[k] = n;
-                h_box.p[k] = boxes[r];
-                std::memcpy(h_type.p + ofs, q.types, n * sizeof(int));
+                H.nat[k] = n;
+                H.box[k] = boxes[r];
+                std::memcpy(H.type + ofs, q.types, n * sizeof(int));
                 if (first[r]) {
                     CK(cudaMemcpyAsync(B.xyz + 3 * ofs, q.xyz, 3 * n * sizeof(double), cudaMemcpyHostToDevice, st));
                     CK(cudaMemcpyAsync(B.v + 3 * ofs, q.v, 3 * n * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -1077,25 +1084,25 @@ int64_t Session::serve_loop(ServeSource& src, const double* mass_type, const MdS
                     CK(cudaMemcpyAsync(B.acc + 3 * ofs, A.acc + 3 * pos[r], bytes, cudaMemcpyDeviceToDevice, st));
                 }
                 ofs += n;
-                h_aofs.p[k + 1] = ofs;
-                h_gofs.p[k + 1] = ofs * nimg;
+                H.aofs[k + 1] = ofs;
+                H.gofs[k + 1] = ofs * nimg;
             }
-            for (int k = 0; k < nf; ++k) pos[active[k]] = h_aofs.p[k];
-            CK(cudaMemcpyAsync(B.natoms, h_nat.p, nf * sizeof(int), cudaMemcpyHostToDevice, st));
-            CK(cudaMemcpyAsync(B.atom_ofs, h_aofs.p, (nf + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-            CK(cudaMemcpyAsync(B.ghost_ofs, h_gofs.p, (nf + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-            CK(cudaMemcpyAsync(B.box, h_box.p, nf * sizeof(cgd::BoxDev), cudaMemcpyHostToDevice, st));
-            CK(cudaMemcpyAsync(B.type, h_type.p, ofs * sizeof(int), cudaMemcpyHostToDevice, st));
+            for (int k = 0; k < nf; ++k) pos[active[k]] = H.aofs[k];
+            CK(cudaMemcpyAsync(B.natoms, H.nat, nf * sizeof(int), cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(B.atom_ofs, H.aofs, (nf + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(B.ghost_ofs, H.gofs, (nf + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(B.box, H.box, nf * sizeof(cgd::BoxDev), cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(B.type, H.type, ofs * sizeof(int), cudaMemcpyHostToDevice, st));
             cur ^= 1;
             changed = false;
             lists.release();
         }
         ServeArena& C = arena[cur];
-        for (int k = 0; k < nf; ++k) h_first.p[k] = first[active[k]] ? 1 : 0;
-        CK(cudaMemcpyAsync(C.first, h_first.p, nf, cudaMemcpyHostToDevice, st));
+        for (int k = 0; k < nf; ++k) H.first[k] = first[active[k]] ? 1 : 0;
+        CK(cudaMemcpyAsync(C.first, H.first, nf, cudaMemcpyHostToDevice, st));
         DeviceFrames df;
         df.nframes = nf;
-        df.box_host.assign(h_box.p, h_box.p + nf);
+        df.box_host.assign(H.box, H.box + nf);
         df.natoms_total = active_atoms;
         df.nghosts = active_atoms * nimg;
         df.xyz = C.xyz;

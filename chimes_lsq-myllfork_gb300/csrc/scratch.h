@@ -36,6 +36,26 @@ T* scratch_alloc(size_t n, cudaStream_t st) {
     return static_cast<T*>(p);
 }
 
+// Device memory of an object that outlives a call or is shared by streams, from the scratch
+// pool: its owner may use it on any stream once the allocating stream has been synchronised,
+// and it goes back when nothing on the device can use it any more.  cudaMalloc and cudaFree
+// of a dozen arrays took half of a call on a small system.
+void* pool_alloc(size_t bytes, cudaStream_t st);
+void pool_free(std::vector<void*>& ptrs);   // synchronises the device first
+
+// Arrays laid out one behind the other, 256-byte aligned: take() adds up the sizes while
+// there is no base, and hands out the places once there is.
+struct Layout {
+    unsigned char* base = nullptr;
+    size_t used = 0;
+    template <typename T>
+    T* take(size_t n) {
+        const size_t off = (used + 255) / 256 * 256;
+        used = off + std::max<size_t>(n, 1) * sizeof(T);
+        return base ? reinterpret_cast<T*>(base + off) : nullptr;
+    }
+};
+
 // Per-call scratch: stream-ordered device allocations from scratch_pool() released
 // at the end of the call, or -- for the no-allocation entry point -- a bump
 // allocator over the static device array below (256-byte aligned sub-buffers,

@@ -388,8 +388,22 @@ FrameBatch make_batch(const Model& m, const std::vector<Frame>& frames, int firs
     return fb;
 }
 
-DeviceFrames::~DeviceFrames() {
-    for (void* p : allocs) cudaFree(p);
+DeviceFrames::~DeviceFrames() { pool_free(allocs); }
+
+void* pool_alloc(size_t bytes, cudaStream_t st) { return scratch_alloc<unsigned char>(bytes, st); }
+
+void pool_free(std::vector<void*>& ptrs) {
+    if (ptrs.empty()) return;
+    cudaPointerAttributes at{};   // the device that holds them need not be current
+    int cur = -1, dev = -1;
+    cudaGetDevice(&cur);
+    for (void* p : ptrs)
+        if (p && cudaPointerGetAttributes(&at, p) == cudaSuccess && (dev = at.device) >= 0) break;
+    if (dev >= 0 && dev != cur) cudaSetDevice(dev);
+    cudaDeviceSynchronize();
+    for (void* p : ptrs) if (p) cudaFree(p);   // pool memory: returned without a further wait
+    if (dev >= 0 && dev != cur) cudaSetDevice(cur);
+    ptrs.clear();
 }
 
 }  // namespace cg
@@ -593,24 +607,41 @@ std::unique_ptr<DeviceFrames> Session::upload(const FrameBatch& fb) {
     d.nframes = fb.nframes;
     d.nlayers = L;
     d.nimg = (2 * L + 1) * (2 * L + 1) * (2 * L + 1);
-    d.natoms = dev_upload(df->allocs, fb.natoms.data(), fb.natoms.size());
-    d.atom_ofs = dev_upload(df->allocs, fb.atom_ofs.data(), fb.atom_ofs.size());
-    d.ghost_ofs = dev_upload(df->allocs, fb.ghost_ofs.data(), fb.ghost_ofs.size());
-    d.row_ofs = dev_upload(df->allocs, fb.row_ofs.data(), fb.row_ofs.size());
-    d.stress_rows = dev_upload(df->allocs, fb.stress_rows.data(), fb.stress_rows.size());
-    d.energy_rows = dev_upload(df->allocs, fb.energy_rows.data(), fb.energy_rows.size());
-    d.box = dev_upload(df->allocs, fb.box.data(), fb.box.size());
-    d.type = dev_upload(df->allocs, fb.type.data(), fb.type.size());
-    df->xyz = dev_upload(df->allocs, fb.xyz.data(), fb.xyz.size());
-    d.xyz = df->xyz;
-    double* scaled = nullptr;
-    float* c32 = nullptr;
-    CK(cudaMalloc((void**)&scaled, std::max<int64_t>(1, fb.nghosts) * 3 * sizeof(double)));
-    df->allocs.push_back(scaled);
-    CK(cudaMalloc((void**)&c32, std::max<int64_t>(1, fb.nghosts) * 4 * sizeof(float)));
-    df->allocs.push_back(c32);
-    d.scaled = scaled;
-    d.cart32 = c32;
+    // one allocation; the host arrays packed and copied together
+    std::vector<unsigned char> host;
+    Layout lay;
+    auto put = [&](const auto& v) {
+        using T = typename std::decay<decltype(v[0])>::type;
+        T* p = lay.take<T>(v.size());
+        if (!lay.base) return p;
+        const size_t at = (size_t)(reinterpret_cast<unsigned char*>(p) - lay.base);
+        if (!v.empty()) std::memcpy(host.data() + at, v.data(), v.size() * sizeof(T));
+        return p;
+    };
+    auto arrays = [&]() {
+        d.natoms = put(fb.natoms);
+        d.atom_ofs = put(fb.atom_ofs);
+        d.ghost_ofs = put(fb.ghost_ofs);
+        d.row_ofs = put(fb.row_ofs);
+        d.stress_rows = put(fb.stress_rows);
+        d.energy_rows = put(fb.energy_rows);
+        d.box = put(fb.box);
+        d.type = put(fb.type);
+        df->xyz = put(fb.xyz);
+        d.xyz = df->xyz;
+        const size_t copied = lay.used;
+        d.scaled = lay.take<double>(std::max<int64_t>(1, fb.nghosts) * 3);
+        d.cart32 = lay.take<float>(std::max<int64_t>(1, fb.nghosts) * 4);
+        return copied;
+    };
+    const size_t copied = arrays();
+    lay.base = static_cast<unsigned char*>(pool_alloc(lay.used, stream_));
+    df->allocs.push_back(lay.base);
+    lay.used = 0;
+    host.resize(copied);
+    arrays();
+    CK(cudaMemcpyAsync(lay.base, host.data(), copied, cudaMemcpyHostToDevice, stream_));
+    CK(cudaStreamSynchronize(stream_));   // the frames may be used on any stream
     return df;
 }
 
@@ -745,16 +776,21 @@ int64_t Session::assemble_to_host(const FrameBatch& fb, int precision, int block
         cudaEvent_t copy_t0[2] = {nullptr, nullptr}, copy_t1[2] = {nullptr, nullptr};   // profiling only
         ~Res() {
             for (int i = 0; i < 2; ++i) {
-                if (dA[i]) cudaFree(dA[i]);
                 if (asm_done[i]) cudaEventDestroy(asm_done[i]);
                 if (copy_done[i]) cudaEventDestroy(copy_done[i]);
                 if (copy_t0[i]) cudaEventDestroy(copy_t0[i]);
                 if (copy_t1[i]) cudaEventDestroy(copy_t1[i]);
             }
+            std::vector<void*> own(dA, dA + 2);
+            if (dA[0]) pool_free(own);
         }
     } R;
     const int64_t lda = model_.tot_all;
-    for (int i = 0; i < 2 && i < nblk; ++i) CK(cudaMalloc(&R.dA[i], (size_t)maxrows * lda * rsz));
+    const size_t block = (size_t)maxrows * lda * rsz;
+    for (int i = 0; i < 2 && i < nblk; ++i) {   // small blocks from the pool: cudaMalloc would be most of the call
+        if (block <= size_t(256) << 20) R.dA[i] = pool_alloc(block, stream_);
+        else CK(cudaMalloc(&R.dA[i], block));
+    }
     for (int i = 0; i < 2; ++i) {
         CK(cudaEventCreateWithFlags(&R.asm_done[i], cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&R.copy_done[i], cudaEventDisableTiming));

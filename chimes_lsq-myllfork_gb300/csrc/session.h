@@ -118,7 +118,7 @@ struct MdLists {
     bool valid = false;
     int64_t builds = 0;
     void release() { valid = false; }     // the buffers stay for the next build
-    void* buffer(int slot, size_t bytes);
+    void* buffer(int slot, size_t bytes, cudaStream_t st);
     ~MdLists();
 };
 
