@@ -259,23 +259,40 @@ __global__ void k_virial2(ModelDev M, FramesDev F, NeighDev NB, int nslice, R* _
     }
 }
 
+// Grid: (frame, 32 columns); a thread per (column, component), 8 slices in flight (a thread
+// per column with one chain of reads: 155 us for 8 frames, bound by their latency; so: 9 us).
 template <typename R>
-__global__ void k_virial2_rows(ModelDev M, FramesDev F, int nslice, const R* __restrict__ part, R* A, int64_t lda) {
+__global__ void __launch_bounds__(224) k_virial2_rows(ModelDev M, FramesDev F, int nslice, const R* __restrict__ part,
+                                                      R* A, int64_t lda) {
+    __shared__ R sum[7][32];
     const int ord = M.order2;
     const int ncol = M.npairs * ord;
     const int f = blockIdx.x;
     if (F.stress_rows[f] == 0 && F.energy_rows[f] == 0) return;
-    const double inv_vol = 1.0 / F.box[f].vol;
-    const R* o = part + (int64_t)f * nslice * 7 * ncol;
-    for (int col = threadIdx.x; col < ncol; col += blockDim.x) {
-        const int base = M.pairs[col / ord].col;   // HIERARC: excluded pairs have no columns
-        if (base < 0) continue;
-        R s[7];
-        for (int k = 0; k < 7; ++k) s[k] = R(0);
-        for (int sl = 0; sl < nslice; ++sl)
-            for (int k = 0; k < 7; ++k) s[k] += o[((int64_t)sl * 7 + k) * ncol + col];
-        write_virial_rows(F, f, base + col % ord, s, inv_vol, A, lda);
+    const int c = threadIdx.x & 31, k = threadIdx.x >> 5, col = blockIdx.y * 32 + c;
+    if (col < ncol) {
+        const R* o = part + ((int64_t)f * nslice * 7 + k) * ncol + col;
+        const int64_t step = (int64_t)7 * ncol;
+        R s = R(0);
+        int sl = 0;
+        for (; sl + 8 <= nslice; sl += 8, o += 8 * step) {
+            R v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = o[u * step];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += v[u];
+        }
+        for (; sl < nslice; ++sl, o += step) s += *o;
+        sum[k][c] = s;
     }
+    __syncthreads();
+    if (k > 0 || col >= ncol) return;
+    const int base = M.pairs[col / ord].col;   // HIERARC: excluded pairs have no columns
+    if (base < 0) return;
+    R s[7];
+#pragma unroll
+    for (int q = 0; q < 7; ++q) s[q] = sum[q][c];
+    write_virial_rows(F, f, base + col % ord, s, 1.0 / F.box[f].vol, A, lda);
 }
 
 // ---------------------------------------------------------------- owner incidence sort
@@ -1179,8 +1196,9 @@ __global__ void k_virial_reduce(ModelDev M, FramesDev F, Buckets bytype, const i
     const double perm = NBODY == 3 ? B.perm3 : B.perm4;
     const double inv_vol = 1.0 / B.vol;
     const R* base = part + (size_t)blockIdx.x * nchunks_max * 7 * ntrue_max;
-    for (int col = threadIdx.x; col < CT.n_true; col += blockDim.x) {
+    for (int col = blockIdx.y * blockDim.x + threadIdx.x; col < CT.n_true; col += gridDim.y * blockDim.x) {
         R sv[7] = {0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 2
         for (int c = 0; c < nch; ++c)
 #pragma unroll
             for (int k = 0; k < 7; ++k) if (k < ncomp) sv[k] += base[((size_t)c * 7 + k) * ntrue_max + col];
@@ -1253,7 +1271,8 @@ static void virial2_launch(int nframes, int nslice, size_t sm, const ModelDev& M
                            const NeighDev& NB, void* part, void* A, int64_t lda, cudaStream_t st) {
     set_smem(k_virial2<R, MAXC>, sm);
     k_virial2<R, MAXC><<<dim3((unsigned)nframes, (unsigned)nslice), F2_THREADS, sm, st>>>(M, F, NB, nslice, (R*)part);
-    k_virial2_rows<R><<<nframes, F2_THREADS, 0, st>>>(M, F, nslice, (const R*)part, (R*)A, lda);
+    k_virial2_rows<R><<<dim3((unsigned)nframes, (unsigned)((M.npairs * M.order2 + 31) / 32)), 224, 0, st>>>(
+        M, F, nslice, (const R*)part, (R*)A, lda);
 }
 
 template <typename R>
@@ -1413,8 +1432,9 @@ static void virial_mb_typed(int ppt, dim3 grid, size_t smem, const ModelDev& M, 
 void launch_virial_reduce(int nbody, int prec, int nframes, int ntypes, int ncomp, const ModelDev& M,
                           const FramesDev& F, const Buckets& byt, const int64_t* kfo, const void* part, int ntrue_max,
                           int nchunks_max, void* A, int64_t lda, cudaStream_t st) {
-    const unsigned grid = (unsigned)(nframes * ntypes);
-    if (grid == 0) return;
+    if (nframes * ntypes <= 0) return;
+    // columns over CTAs too: with one CTA per (frame, type) 8 frames took 104 us, so 46
+    const dim3 grid((unsigned)(nframes * ntypes), (unsigned)std::max(1, (ntrue_max + 255) / 256));
     if (nbody == 3 && prec == 0)
         k_virial_reduce<3, double><<<grid, 256, 0, st>>>(M, F, byt, kfo, ncomp, (const double*)part, ntrue_max, nchunks_max, (double*)A, lda);
     else if (nbody == 3)

@@ -114,9 +114,8 @@ __device__ __forceinline__ int frame_of_real(const FramesDev& F, int64_t atom) {
 //    listed ghost with 32 of them side by side.
 // Forming it for every chunk with a candidate in every pass, dividing by the atom count per
 // ghost and scanning all atoms of a near image took 1.37 of the 1.96 ms of an MD force
-// call on frames of 64, 301, 1111 and 2600 atoms (now 0.96 ms in all), and 1.38 of 11.3 ms
-// of the FP64 rows of 32 frames of 384 (now 10.2 ms).
-constexpr int NEIGH_WARPS = 8;
+// call on frames of 64, 301, 1111 and 2600 atoms (now 0.16 of 0.66 ms), and 1.38 of 11.3 ms
+// of the FP64 rows of 32 frames of 384 (now 9.9 ms in all).
 constexpr int NEIGH_IMG = 1024;   // images tested for reach (four layers); every image is scanned above
 
 template <bool FILL>
@@ -259,14 +258,16 @@ __global__ void __launch_bounds__(32 * NEIGH_WARPS) k_neigh(ModelDev M, FramesDe
             if (a >= N && t + 1 < t1) { a = a0; k = next_near(k + 1); }
         }
     };
-    // ---- count (the fill pass of several warps per atom: to place the slices)
-    if (!FILL || nw > 1) {
+    // ---- count (without kept slice counts the fill pass of several warps per atom counts again)
+    if (!FILL || (nw > 1 && !NB.slice)) {
         sweep([&](int fl, int, int) {
             c2 += __popc(__ballot_sync(0xffffffffu, fl & 1));
             c3 += __popc(__ballot_sync(0xffffffffu, fl & 2));
             c4 += __popc(__ballot_sync(0xffffffffu, fl & 4));
         });
         if (lane == 0) { sc[0][warp] = c2; sc[1][warp] = c3; sc[2][warp] = c4; }
+        if (!FILL && on && NB.slice && lane < 3)
+            NB.slice[((int64_t)atom * NEIGH_WARPS + w) * 3 + lane] = lane == 0 ? c2 : (lane == 1 ? c3 : c4);
         __syncthreads();
         if (!FILL) {
             if (on && w == 0 && lane == 0) {
@@ -279,7 +280,12 @@ __global__ void __launch_bounds__(32 * NEIGH_WARPS) k_neigh(ModelDev M, FramesDe
     }
     if (!on) return;
     o2 = NB.ofs2[atom]; o3 = NB.ofs3[atom]; o4 = NB.ofs4[atom];
-    for (int k = warp - w; k < warp; ++k) { o2 += sc[0][k]; o3 += sc[1][k]; o4 += sc[2][k]; }
+    if (NB.slice) {
+        const int* c = NB.slice + (int64_t)atom * NEIGH_WARPS * 3;
+        for (int k = 0; k < w; ++k) { o2 += c[3 * k]; o3 += c[3 * k + 1]; o4 += c[3 * k + 2]; }
+    } else {
+        for (int k = warp - w; k < warp; ++k) { o2 += sc[0][k]; o3 += sc[1][k]; o4 += sc[2][k]; }
+    }
     int pend = 0;
     sweep([&](int fl, int a, int k) {
         const unsigned b = __ballot_sync(0xffffffffu, fl != 0);
@@ -757,10 +763,13 @@ void launch_frame_setup(const FramesDev& F, int64_t n, cudaStream_t st) {
 }
 void launch_neigh(const ModelDev& M, const FramesDev& F, const NeighDev& NB, int fill, cudaStream_t st) {
     if (NB.n_real <= 0) return;
-    // about 16 warps per SM: eight warps on an atom of a small batch, one where the atoms
-    // alone fill the GPU
+    // eight warps on an atom of a small batch, one where the atoms alone fill the GPU several
+    // times over (frames differ in size: a warp per atom of 2,600 runs 40 times as long as one
+    // of 64): 4,076 atoms in frames of 64 to 2,600, count and fill 423 -> 164 us.  Where the
+    // fill pass has to count again, no more warps than fill the GPU once.
     int nw = NEIGH_WARPS;
-    while (nw > 1 && (int64_t)NB.n_real * nw > 2 * 2432) nw >>= 1;
+    const int64_t most = NB.slice ? 16 * 2432 : 2 * 2432;
+    while (nw > 1 && (int64_t)NB.n_real * nw > most) nw >>= 1;
     const unsigned blocks = (unsigned)((NB.n_real + NEIGH_WARPS / nw - 1) / (NEIGH_WARPS / nw));
     if (fill) k_neigh<true><<<blocks, 32 * NEIGH_WARPS, 0, st>>>(M, F, NB, nw);
     else k_neigh<false><<<blocks, 32 * NEIGH_WARPS, 0, st>>>(M, F, NB, nw);

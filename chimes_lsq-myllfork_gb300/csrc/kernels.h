@@ -22,7 +22,9 @@ struct NeighDev {
     double skin;
     // cut-offs plus skin of every cluster type's slots, [type][3 or 6] (launch_cuts)
     const CutDev* cut3; const CutDev* cut4;
+    int* slice;   // [n_real * NEIGH_WARPS * 3] the count pass's lists by slice of an atom, or null
 };
+constexpr int NEIGH_WARPS = 8;   // warps per CTA of k_neigh, at most on one atom
 
 struct ClusterSet {                               // triplets or quadruplets of a batch
     int* cnt;                                     // [n_real] clusters centred on each real atom

@@ -166,6 +166,7 @@ void Session::md_force(const DeviceFrames& df, double* Fo, double* So, MdCounts*
     NB.n_real = nreal;
     NB.md = 1;
     NB.cut3 = dm_->cut3; NB.cut4 = dm_->cut4;
+    NB.slice = S.get<int>((size_t)nreal * cgd::NEIGH_WARPS * 3);
     NB.cnt2 = S.get<int>(nreal); NB.cnt3 = S.get<int>(nreal); NB.cnt4 = S.get<int>(nreal);
     NB.ofs2 = S.get<int64_t>(nreal + 1); NB.ofs3 = S.get<int64_t>(nreal + 1); NB.ofs4 = S.get<int64_t>(nreal + 1);
     cgd::launch_neigh(M, F, NB, 0, st); L();
