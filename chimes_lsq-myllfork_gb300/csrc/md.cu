@@ -957,9 +957,13 @@ template <int NBODY, typename R>
 static bool dispatch_mdc(int order, unsigned grid, const ModelDev& M, const MdDev& D, const FramesDev& F,
                          const ClusterSet& CS, const MdBuckets& B, double* Fo, double* So, cudaStream_t st) {
 #define MDC_CASE(O)                                          \
-    case O:                                                  \
-        run_mdc<NBODY, O, R>(grid, M, D, F, CS, B, Fo, So, st); \
-        return true;
+    case O:   /* the tensor-core form takes FP64 of its order */ \
+        if constexpr (sizeof(R) == 8 && O == mdt_order(NBODY)) { \
+            return false;                                     \
+        } else {                                              \
+            run_mdc<NBODY, O, R>(grid, M, D, F, CS, B, Fo, So, st); \
+            return true;                                      \
+        }
     if constexpr (NBODY == 3) {
         switch (order) { MDC_CASE(2) MDC_CASE(3) MDC_CASE(4) MDC_CASE(5) MDC_CASE(6) MDC_CASE(7) MDC_CASE(8) }
     } else {

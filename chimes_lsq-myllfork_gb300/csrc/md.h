@@ -75,7 +75,8 @@ void launch_mdc(int nbody, int prec, int order, int64_t max_tiles, const ModelDe
 // The FP64 contraction on the tensor cores (md_tensor.cu), for the orders of
 // md_tensor_order: tables of a coefficient set (md_tensor_bytes bytes and
 // md_tensor_exponents ints per type), then the force pass as launch_mdc.
-bool md_tensor_order(int nbody, int order);
+constexpr int mdt_order(int nbody) { return nbody == 3 ? 8 : 4; }
+inline bool md_tensor_order(int nbody, int order) { return order == mdt_order(nbody); }
 size_t md_tensor_bytes(int nbody, int ntypes);
 int md_tensor_exponents(int nbody);
 void launch_md_tables(int nbody, int ntypes, const double* C, unsigned char* tab, int* ex, cudaStream_t st);

@@ -391,6 +391,21 @@ void Session::md_lists_build(DeviceFrames& df, double skin, MdLists& L, cudaStre
     ++L.builds;
 }
 
+// Zeroed outputs and this step's ghost positions, by the images of the lists.
+void Session::md_step_setup(DeviceFrames& df, MdLists& L, double* Fo, double* So) {
+    cudaStream_t st = stream_;
+    const size_t nreal = (size_t)df.natoms_total;
+    CK(cudaMemsetAsync(Fo, 0, std::max<size_t>(1, nreal * 3) * sizeof(double), st));
+    CK(cudaMemsetAsync(So, 0, std::max<size_t>(1, (size_t)df.nframes * cgd::MD_NSCALAR) * sizeof(double), st));
+    cgd::FramesDev F = df.dev;
+    F.shift = L.shift;
+    F.shift_mode = 2;   // the build's images
+    mark(ST_SETUP, true);
+    cgd::launch_frame_setup(F, df.nghosts, st);
+    mark(ST_SETUP, false);
+}
+
+// The forces behind md_step_setup.
 void Session::md_force_lists(DeviceFrames& df, MdLists& L, double* Fo, double* So) {
     CK(cudaSetDevice(device_));
     if (!md_) throw Error(1, "MD coefficients are not set (cg_md_setup)");
@@ -400,14 +415,9 @@ void Session::md_force_lists(DeviceFrames& df, MdLists& L, double* Fo, double* S
     cudaStream_t st = stream_;
     const int nf = df.nframes;
     const int nreal = (int)df.natoms_total;
-    CK(cudaMemsetAsync(Fo, 0, std::max<size_t>(1, (size_t)nreal * 3) * sizeof(double), st));
-    CK(cudaMemsetAsync(So, 0, std::max<size_t>(1, (size_t)nf * cgd::MD_NSCALAR) * sizeof(double), st));
     cgd::FramesDev F = df.dev;
     F.shift = L.shift;
-    F.shift_mode = 2;   // the build's images
-    mark(ST_SETUP, true);
-    cgd::launch_frame_setup(F, df.nghosts, st);
-    mark(ST_SETUP, false);
+    F.shift_mode = 2;
     // The 2-body, 3-body and 4-body parts add into Fo / So with atomics and are
     // otherwise independent: the many-body parts run on two side streams beside the
     // 2-body kernel (a frame of ~1000 atoms gives each contraction only a few warps
@@ -460,29 +470,34 @@ void Session::md_force_lists(DeviceFrames& df, MdLists& L, double* Fo, double* S
     CK(cudaGetLastError());
 }
 
-double Session::md_lists_disp2(const DeviceFrames& df, MdLists& L) {
-    if (!L.valid || L.natoms != df.natoms_total) return HUGE_VAL;
-    cudaStream_t st = stream_;
-    CK(cudaMemsetAsync(L.dmax, 0, sizeof(unsigned long long), st));
-    cgd::launch_md_maxdisp(df.xyz, L.xref, L.natoms, L.dmax, st);
-    unsigned long long bits = 0;
-    CK(cudaMemcpyAsync(&bits, L.dmax, sizeof(bits), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    double d2;
-    std::memcpy(&d2, &bits, sizeof(d2));
-    return d2;
-}
-
 void Session::md_force_step(DeviceFrames& df, MdListSet& LS, double* Fo, double* So) {
     if (LS.next_ready) {   // built ahead during the previous step (that build has completed)
         LS.cur ^= 1;
         LS.next_ready = false;
     }
     MdLists& L = LS.current();
+    cudaStream_t st = stream_;
     const double half2 = 0.25 * md_skin_ * md_skin_;
-    double d2 = md_lists_disp2(df, L);
-    if (!(d2 <= half2) || L.skin != md_skin_) {
-        md_lists_build(df, md_skin_, L, stream_);
+    // The largest squared displacement since the build; the step is set up for these lists
+    // while the host waits for it (and again in the rare case that they have to be rebuilt).
+    double d2 = HUGE_VAL;
+    const bool usable = L.valid && L.natoms == df.natoms_total && L.skin == md_skin_;
+    if (usable) {
+        if (!md_disp_) {
+            CK(cudaMallocHost((void**)&md_disp_host_, sizeof(double)));
+            CK(cudaEventCreateWithFlags(&md_disp_, cudaEventDisableTiming));
+        }
+        CK(cudaMemsetAsync(L.dmax, 0, sizeof(unsigned long long), st));
+        cgd::launch_md_maxdisp(df.xyz, L.xref, L.natoms, L.dmax, st);
+        CK(cudaMemcpyAsync(md_disp_host_, L.dmax, sizeof(double), cudaMemcpyDeviceToHost, st));
+        CK(cudaEventRecord(md_disp_, st));
+        md_step_setup(df, L, Fo, So);
+        CK(cudaEventSynchronize(md_disp_));
+        d2 = *md_disp_host_;
+    }
+    if (!(d2 <= half2)) {
+        md_lists_build(df, md_skin_, L, st);
+        md_step_setup(df, L, Fo, So);
         d2 = 0.0;
     }
     const bool ahead = d2 > (0.75 * 0.75) * half2;   // 3/8 of the skin

@@ -364,7 +364,7 @@ k_mdt(ModelDev M, FramesDev F, ClusterSet CS, MdBuckets MB, const unsigned char*
 
 }  // namespace
 
-bool md_tensor_order(int nbody, int order) { return order == (nbody == 3 ? Mt<3>::O : Mt<4>::O); }
+static_assert(Mt<3>::O == mdt_order(3) && Mt<4>::O == mdt_order(4), "orders of the tensor-core form");
 
 size_t md_tensor_bytes(int nbody, int ntypes) {
     return (size_t)ntypes * (nbody == 3 ? mt_table(64, 8) + mt_table(8, 64) : 2 * mt_table(64, 64));

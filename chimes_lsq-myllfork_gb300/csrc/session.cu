@@ -584,6 +584,8 @@ Session::~Session() {
         if (md_join_[k]) cudaEventDestroy(md_join_[k]);
     }
     if (md_fork_) cudaEventDestroy(md_fork_);
+    if (md_disp_) cudaEventDestroy(md_disp_);
+    if (md_disp_host_) cudaFreeHost(md_disp_host_);
     if (side_stream_) cudaStreamDestroy(side_stream_);
     if (copy_stream_) cudaStreamDestroy(copy_stream_);
     for (int i = 0; i < 2; ++i) staging_free(pinned_[i], pinned_reg_[i]);
@@ -787,8 +789,9 @@ int64_t Session::assemble_to_host(const FrameBatch& fb, int precision, int block
     } R;
     const int64_t lda = model_.tot_all;
     const size_t block = (size_t)maxrows * lda * rsz;
-    for (int i = 0; i < 2 && i < nblk; ++i) {   // small blocks from the pool: cudaMalloc would be most of the call
-        if (block <= size_t(256) << 20) R.dA[i] = pool_alloc(block, stream_);
+    for (int i = 0; i < 2 && i < nblk; ++i) {   // small blocks from the pool (cudaMalloc would be most of the call; copies of
+                                                     // gigabytes out of pool memory ran at half the rate)
+        if (block <= size_t(32) << 20) R.dA[i] = pool_alloc(block, stream_);
         else CK(cudaMalloc(&R.dA[i], block));
     }
     for (int i = 0; i < 2; ++i) {

@@ -324,7 +324,7 @@ class Session {
     // rebuild test (reads the largest displacement since the build).
     void md_lists_build(DeviceFrames& df, double skin, MdLists& L, cudaStream_t st);
     void md_force_lists(DeviceFrames& df, MdLists& L, double* Fo, double* So);
-    double md_lists_disp2(const DeviceFrames& df, MdLists& L);   // largest squared displacement
+    void md_step_setup(DeviceFrames& df, MdLists& L, double* Fo, double* So);
     // One step's forces through a list set (rebuilds, look-ahead builds, switch).
     void md_force_step(DeviceFrames& df, MdListSet& LS, double* Fo, double* So);
     // Thermostat / barostat state of frame `frame` after the last md_run as CONSTRAINT's
@@ -419,6 +419,8 @@ class Session {
     unsigned char* mailbox_dev_ = nullptr;
     cudaEvent_t side_event_ = nullptr;
     cudaStream_t md_side_[2] = {nullptr, nullptr};   // many-body MD force parts beside the 2-body kernel
+    cudaEvent_t md_disp_ = nullptr;        // the displacement check's copy to md_disp_host_ (pinned)
+    double* md_disp_host_ = nullptr;
     cudaEvent_t md_fork_ = nullptr, md_join_[2] = {nullptr, nullptr};
     std::unique_ptr<DeviceModel> dm_;
     std::unique_ptr<MdTables> md_;
