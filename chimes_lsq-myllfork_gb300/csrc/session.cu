@@ -991,7 +991,7 @@ void Session::run(const DeviceFrames& df, int precision, void* A, int64_t lda, A
         // FP64 rows as digit products on the tensor cores where the order fills their grids and
         // the slot bases are tabulated, unless a force_range setting names another form.  Of 16
         // frames of 256 C/H/N/O atoms, range form -> digit products: 4-body force rows 12.6 ->
-        // 7.0 ms, stress and energy 13.3 -> 3.2 ms; 3-body 2.8 -> 2.0 and 3.7 -> 1.4 ms
+        // 7.0 ms, stress and energy 13.3 -> 3.1 ms; 3-body 2.8 -> 1.8 and 3.7 -> 1.0 ms
         bool tensor = false;
         cgd::OzWork oz{};
         if (!S.base && nbasis * rsize <= kClusterBasisMax) {

@@ -202,7 +202,8 @@ template <> struct Oz<4> {
 template <int NBODY>
 struct OzSmem {
     using O = Oz<NBODY>;
-    static constexpr size_t CHUNK = (size_t)(O::AROWS + O::BROWS) * DIG_STRIDE;   // 8 clusters
+    // 8 clusters; 64 bytes on, so that a warp's digit stores into two chunks share no bank
+    static constexpr size_t CHUNK = (size_t)(O::AROWS + O::BROWS) * DIG_STRIDE + 64;
     size_t stage, basis, idx, total;
     __host__ __device__ explicit OzSmem(int max_words) {
         stage = (OZ_CH / 8) * CHUNK;
@@ -385,10 +386,13 @@ k_force_oz(ModelDev M, FramesDev F, ClusterSet CS, Buckets inc, const int64_t* k
             // (3) products into the staged outputs (a thread meets the same ones in every chunk)
             const int nch = npair >> 2;
             const bool more = ch0 > 0;
-            auto stage2 = [&](Sum* o, const float (&acc)[ND][4], int r) {
-                Sum x = acc_value(acc, 2 * r, up), y = acc_value(acc, 2 * r + 1, up);
-                if (more) { x += o[0]; y += o[1]; }
-                o[0] = x; o[1] = y;
+            // a pair of values at a time, 16 bytes: eight lanes cover all banks (two rows of
+            // four pairs); as two 8-byte accesses they met two to a bank
+            auto stage2 = [&](Sum* at, const float (&acc)[ND][4], int r) {
+                longlong2* o = reinterpret_cast<longlong2*>(at);
+                longlong2 v = make_longlong2(acc_value(acc, 2 * r, up), acc_value(acc, 2 * r + 1, up));
+                if (more) { const longlong2 w = *o; v.x += w.x; v.y += w.y; }
+                *o = v;
             };
             if (NBODY == 4) {
                 const int mt = warp >> 1;
@@ -501,7 +505,7 @@ constexpr int VZ_THREADS = 512;
 template <int NBODY>
 struct VzSmem {
     using V = Vz<NBODY>;
-    static constexpr size_t CHUNK = (size_t)V::ROWS * DIG_STRIDE;   // 8 clusters
+    static constexpr size_t CHUNK = (size_t)V::ROWS * DIG_STRIDE + 64;   // 8 clusters, as OzSmem
     static constexpr size_t BUF = CHUNK * (V::CH / 8);
     size_t raw, basis, q, sh, total;
     size_t raw_size;
@@ -616,12 +620,26 @@ k_virial_oz(ModelDev M, FramesDev F, ClusterSet CS, Buckets bytype, const int64_
     auto slots = [&](int ch) {
         const int nb = min(CH, n - ch * CH);
         const double* raw = reinterpret_cast<const double*>(smem_raw + L.raw + (ch & 1) * L.raw_size);
-        for (int t = tid; t < nb * NP; t += VZ_THREADS) {
-            const double* src = raw + (size_t)t * stride;
-            double* o = sB + (size_t)t * SB;
-            const double r = src[2 * ord];
-            const double x[3] = {src[2 * ord + 1], src[2 * ord + 2], src[2 * ord + 3]};
-            if (NBODY == 4) {
+        if constexpr (NBODY == 3) {
+            // one division or one value per thread: six divisions of 24 (cluster, slot) pairs
+            // by one warp (an FP64 division is a dozen instructions of 64 cycles) kept the
+            // other 15 at the barrier: triplet rows of 32 frames of 384 atoms 3.71 -> 2.81 ms
+            for (int t = tid; t < nb * NP * 6; t += VZ_THREADS) {
+                const int cs = t / 6, k = t - 6 * cs;
+                const double* src = raw + (size_t)cs * stride + 2 * ord;
+                const int ka = k < 3 ? k : (k == 5 ? 1 : 0), kc = k < 3 ? k : (k == 3 ? 1 : 2);
+                sB[(size_t)cs * SB + 2 * BASE + k] = src[1 + ka] * src[1 + kc] / src[0];
+            }
+            for (int t = VZ_THREADS - 1 - tid; t < nb * NP * 2 * BASE; t += VZ_THREADS) {
+                const int cs = t / (2 * BASE), k = t % (2 * BASE), n = k % BASE;
+                sB[(size_t)cs * SB + k] = n < ord ? raw[(size_t)cs * stride + (k < BASE ? n : ord + n)] : 0.0;
+            }
+        } else {
+            for (int t = tid; t < nb * NP; t += VZ_THREADS) {
+                const double* src = raw + (size_t)t * stride;
+                double* o = sB + (size_t)t * SB;
+                const double r = src[2 * ord];
+                const double x[3] = {src[2 * ord + 1], src[2 * ord + 2], src[2 * ord + 3]};
                 const int ka = comp <= 3 ? comp - 1 : (comp == 6 ? 1 : 0), kc = comp <= 3 ? comp - 1 : (comp == 4 ? 1 : 2);
                 const double v = comp == 0 ? 0.0 : (ka == 0 ? x[0] : (ka == 1 ? x[1] : x[2])) *
                                                    (kc == 0 ? x[0] : (kc == 1 ? x[1] : x[2])) / r;
@@ -630,15 +648,6 @@ k_virial_oz(ModelDev M, FramesDev F, ClusterSet CS, Buckets bytype, const int64_
                     o[k] = k < ord ? src[k] : 0.0;
                     o[BASE + k] = k < ord ? src[ord + k] * v : 0.0;
                 }
-            } else {
-#pragma unroll
-                for (int k = 0; k < BASE; ++k) {
-                    o[k] = k < ord ? src[k] : 0.0;
-                    o[BASE + k] = k < ord ? src[ord + k] : 0.0;
-                }
-                double* v = o + 2 * BASE;
-                v[0] = x[0] * x[0] / r; v[1] = x[1] * x[1] / r; v[2] = x[2] * x[2] / r;
-                v[3] = x[0] * x[1] / r; v[4] = x[0] * x[2] / r; v[5] = x[1] * x[2] / r;
             }
         }
     };
