@@ -596,7 +596,7 @@ def main():
     roofline = {"bound": "hbm", "kernel": dom, "achieved": algo / dom_s / 1e9, "peak": hbm_peak, "unit": "GB/s",
                 "frac": algo / dom_s / 1e9 / hbm_peak, "traffic": None if tpf is None else tpf * args.frames,
                 "traffic_source": tsrc, "bytes_per_launch": algo, "peak_source": peak_kind,
-                "note": "the FP64 assembly kernels are FP64-pipe bound: see fp64"}
+                "note": "digit products on the tensor cores between integer and shared-memory work; fp64 relates the stages to the FP64 pipe"}
     # the bound that holds for the dominant kernel: its FP64 work against the FP64 rate
     # measured in this run (the better of an FMA-chain kernel and the FP64 SYRK)
     roofline_fp64 = None

@@ -10,8 +10,8 @@
 // against 11,600).  The products run on mma.sync: a contraction sums a few to a few
 // hundred clusters, far below what fills a tcgen05 pipeline, and its accumulators are
 // wanted in registers at once to be packed into integers.  16 frames of 256 C/H/N/O
-// atoms (4-body, 7,800 rows x 51,209) 36.8 -> 17.0 ms, 32 frames of 384 water atoms
-// (3-body, 820 columns) 22.5 -> 11.4 ms; the error against 64-bit references is that of
+// atoms (4-body, 7,800 rows x 51,209) 36.8 -> 14.8 ms, 32 frames of 384 water atoms
+// (3-body, 820 columns) 22.5 -> 9.0 ms; the error against 64-bit references is that of
 // the FP64 forms (2.2e-14 and 4.8e-14 of the norm, the references' own rounding among it).
 //
 // Column sums: PARAM_INDICES puts powers that permutations of equal atoms exchange
