@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(SY_THREADS) k_syrk_tn(const double* __restrict
 // have finished theirs run the current products.  The tensor pipe is the bound (36
 // products per multiply-add on mma.sync, 606 TFLOP/s measured, or 13.9 TFLOP/s of FP64
 // arithmetic).  30,001 x 820 (with h and the
-// mirror): 19.5 -> 3.7 ms; 2,000 x 6,007: 60.2 -> 11.6 ms; against a double-double
+// mirror): 19.5 -> 3.55 ms; 2,000 x 6,007: 60.2 -> 11.6 ms; against a double-double
 // reference the norm of the error is 1.0e-16 of G's (FP64 sums: 4.4e-16).
 constexpr int GD_T = 64, GD_THREADS = 512, GD_ROWS = 16;
 constexpr uint32_t GD_CHUNK = 2 * GD_T * DIG_STRIDE;   // 8 rows of K
