@@ -121,7 +121,8 @@ constexpr int NEIGH_IMG = 1024;   // images tested for reach (four layers); ever
 template <bool FILL>
 __global__ void __launch_bounds__(32 * NEIGH_WARPS) k_neigh(ModelDev M, FramesDev F, NeighDev NB, int nw) {
     __shared__ int sc[3][NEIGH_WARPS];
-    __shared__ int sHit[NEIGH_WARPS][64];
+    __shared__ int sHit[NEIGH_WARPS][64];         // ghosts: any number of image layers
+    __shared__ uint8_t sLists[NEIGH_WARPS][64];   // and their lists
     __shared__ unsigned sNear[NEIGH_WARPS][NEIGH_IMG / 32];
     __shared__ float2 sPair[55];   // s_max + skin and s_min of the pair types (at most 10 atom types)
     for (int p = threadIdx.x; p < M.npairs; p += 32 * NEIGH_WARPS)
@@ -225,9 +226,9 @@ __global__ void __launch_bounds__(32 * NEIGH_WARPS) k_neigh(ModelDev M, FramesDe
     };
     int64_t o2 = 0, o3 = 0, o4 = 0;
     int* hit = sHit[warp];
+    uint8_t* lists = sLists[warp];
     auto write = [&](int n) {   // the first n (<= 32) hits: exact distances side by side
-        const int v = lane < n ? hit[lane] : 0;
-        const int fl = lane < n ? (int)((unsigned)v >> 29) : 0, a = v & 8191, g = ((v >> 13) & 65535) * N + a;
+        const int g = lane < n ? hit[lane] : 0, fl = lane < n ? lists[lane] : 0;
         const unsigned b2 = __ballot_sync(0xffffffffu, fl & 1);
         const unsigned b3 = __ballot_sync(0xffffffffu, fl & 2);
         const unsigned b4 = __ballot_sync(0xffffffffu, fl & 4);
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(32 * NEIGH_WARPS) k_neigh(ModelDev M, FramesDe
             const double r = dist_exact(B.h, si, F.scaled + 3 * (gbase + g), rab);
             if (fl & 1) {
                 const int64_t p = o2 + __popc(b2 & lt);
-                NB.i2[p] = i; NB.g2[p] = g; NB.pt2[p] = M.int_pair_map[ti * M.natmtyp + typ[a]]; NB.r2[p] = r;
+                NB.i2[p] = i; NB.g2[p] = g; NB.pt2[p] = M.int_pair_map[ti * M.natmtyp + typ[g % N]]; NB.r2[p] = r;
                 NB.rab2[3 * p] = rab[0]; NB.rab2[3 * p + 1] = rab[1]; NB.rab2[3 * p + 2] = rab[2];
             }
             if (fl & 2) { const int64_t p = o3 + __popc(b3 & lt); NB.g3[p] = g; NB.r3[p] = r; }
@@ -289,15 +290,20 @@ __global__ void __launch_bounds__(32 * NEIGH_WARPS) k_neigh(ModelDev M, FramesDe
     int pend = 0;
     sweep([&](int fl, int a, int k) {
         const unsigned b = __ballot_sync(0xffffffffu, fl != 0);
-        if (fl) hit[pend + __popc(b & lt)] = a | (k << 13) | (fl << 29);
+        if (fl) {
+            const int at = pend + __popc(b & lt);
+            hit[at] = k * N + a;
+            lists[at] = (uint8_t)fl;
+        }
         pend += __popc(b);
         __syncwarp();
         if (pend >= 32) {
             write(32);
             __syncwarp();
-            const int rest = lane < pend - 32 ? hit[32 + lane] : 0;
+            const bool more = lane < pend - 32;
+            const int rest = more ? hit[32 + lane] : 0, rest_lists = more ? lists[32 + lane] : 0;
             __syncwarp();
-            if (lane < pend - 32) hit[lane] = rest;
+            if (more) { hit[lane] = rest; lists[lane] = (uint8_t)rest_lists; }
             pend -= 32;
             __syncwarp();
         }
