@@ -12,6 +12,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "units.h"
+
 namespace cgd {
 
 constexpr int DIG_ND = 8;          // digits, and diagonals
@@ -128,7 +130,7 @@ __device__ __forceinline__ void acc_clear(float (&acc)[DIG_ND][4]) {
 }
 
 // One output: sum_D S_D 2^(40 + up - 8 D), the digits below the unit rounded, in units of
-// 2^-(56 + up) of the product of the scaled entries (X / 2^64 each); up from up_bits().
+// 2^-(56 + up) of the product of the scaled entries (X / 2^64 each); up from up_bits() (units.h).
 __device__ __forceinline__ long long acc_value(const float (&acc)[8][4], int k, int up) {
     constexpr unsigned c = MAGIC_BITS * 257u;
     const unsigned hi = __float_as_uint(acc[0][k]) * 256u + __float_as_uint(acc[1][k]) - c;
@@ -139,17 +141,6 @@ __device__ __forceinline__ long long acc_value(const float (&acc)[8][4], int k, 
     if (up >= 0) return (long long)((unsigned long long)v << up) + (((fr >> (15 - up)) + 1) >> 1);
     return (v + (fr >> 16) + (1ll << (-up - 1))) >> -up;   // to nearest: sums of floors would drift
 }
-// A magnitude 2^t as a share of the largest, 2^tmax, in 2^-16: integers, so that sums
-// of shares do not depend on their order.
-__device__ __forceinline__ unsigned share16(int t, int tmax) { return (65536u >> min(tmax - t, 16)) + 1u; }
-// The finest unit with room in 63 bits for outputs of at most sum / 2^16 times the
-// largest product (0.2481), sum of up to 2^15 shares over the terms times `terms`.
-__device__ __forceinline__ int up_bits(unsigned sum, int terms) {
-    const unsigned long long b = (unsigned long long)sum * (unsigned)terms;
-    const int e = 64 - __clzll((long long)b) - 16;   // 2^(e + 16) > sum terms
-    return max(-40, min(8, 9 - e));
-}
-
 // v 2^e correctly rounded to FP64 in integer arithmetic (the conversion and the
 // multiplication would take the FP64 pipe, which has 1/64 of the integer rate).
 __device__ __forceinline__ double from_fixed(long long v, int e) {

@@ -175,12 +175,14 @@ __global__ void __launch_bounds__(128) k_oz_sort(ModelDev M, FramesDev F, Cluste
     for (int T = 0; T < ntypes; ++T) {
         const int g0 = T == 0 ? 0 : cnt[T - 1], g1 = cnt[T];
         const int tm = tmax[T];
-        unsigned s = 0;
+        unsigned long long s = 0;
         for (int k = g0 + lane; k < g1; k += 32) {
             const int e = sexp[e0 + k];
             s += share16((int)(short)(e & 0xffff) + (e >> 16), tm);
         }
-        s = __reduce_add_sync(0xffffffffu, s);
+        // 64-bit sum of the lanes': their low 16 bits and the rest each fit 32 bits
+        s = ((unsigned long long)__reduce_add_sync(0xffffffffu, (unsigned)(s >> 16)) << 16) +
+            __reduce_add_sync(0xffffffffu, (unsigned)(s & 0xffffu));
         if (lane == 0) {
             const int up = g1 > g0 ? up_bits(s, (NBODY == 3 ? 2 : 1) * tinfo[T].x) : 0;
             groups[(int64_t)gatom * ntypes + T] = make_int4(g0, g1 - g0, tm, up);
