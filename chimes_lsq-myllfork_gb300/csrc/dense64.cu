@@ -96,57 +96,97 @@ __global__ void __launch_bounds__(SY_THREADS) k_syrk_tn(const double* __restrict
 }
 
 // ---------------------------------------------------------------- X^T X as digit products
-// The same triangle with FP64 accuracy from the tensor cores (digits.cuh): column i is
-// scaled by a power of two, its entries split into eight base-256 digits, and a 64 x 64
-// tile's 36 digit products per term are summed exactly and packed every 32 rows into
-// 64-bit integers; one conversion and one addition to C per output and K slice.  In units
-// of the two columns' largest entries a term loses at most 2^-62 to rounding and 2^-59 to
-// the dropped diagonals and every 32 rows 16 * 2^-(57 + up) (up = 9 - log2 of the slice's
-// rows); an FP64 sum loses up to 2^-53 of the partial sum with every row.
+// The same triangle from the tensor cores (digits.cuh) with the accuracy of FP64 sums, entry
+// by entry.  Every 64 rows (a block) each column has its own power of two; its entries are
+// split into eight base-256 digits, a 64 x 64 tile's 36 digit products per term are summed
+// exactly over the block in integers, and the block's sum is rounded once to FP64 and added
+// in FP64.  In units of the two columns' powers of two a block loses about 2^-61.1 (64 terms
+// whose dropped diagonals are 2^-64.1 each, root mean square), and nothing in rows where
+// either entry is zero.
+//
+// That is less than FP64 sums lose -- at least 2^-55 of S_ij = sum |x_ki x_kj| -- unless the
+// rows of the large entries of one column meet small ones of the other.  So a ninth plane
+// holds |x| in FP16 and one more product per 16 rows estimates S: an output whose S is below
+// GD_GUARD times the root of its blocks' squared units is summed again in FP64 by the same
+// CTA (as are columns that are not finite).  Of a C/H 4-body A of 816 x 3,992 that is 5% of
+// the outputs, of a water 3-body A of 13,968 x 820 none.
+//
 // Sixteen warps of 16 rows x 16 columns; the next 16 rows' digits are built while warps that
 // have finished theirs run the current products.  The tensor pipe is the bound (36
 // products per multiply-add on mma.sync, 606 TFLOP/s measured, or 13.9 TFLOP/s of FP64
-// arithmetic).  30,001 x 820 (with h and the
-// mirror): 19.5 -> 3.55 ms; 2,000 x 6,007: 60.2 -> 11.6 ms; against a double-double
-// reference the norm of the error is 1.0e-16 of G's (FP64 sums: 4.4e-16).
-constexpr int GD_T = 64, GD_THREADS = 512, GD_ROWS = 16;
+// arithmetic).  Blocks of 32 rows leave more outputs to the digits, but FP64 has 1/64 of the
+// FP32 rate and an addition per output and 32 rows kept the tensor pipe waiting (30,001 x 820
+// 4.8 ms); blocks of 128 leave fewer (4.05 ms, but 816 x 3,992 heavy-tailed 4.1 -> 5.6 ms).
+//
+// Whole calls with h, FP64 sums -> this: 30,001 x 820 19.3 -> 4.36 ms, 2,000 x 6,007 60.0 -> 14.2,
+// 816 x 3,992 11.5 -> 2.8; entries spread by exp(2 N(0,1)): 19.3 -> 5.5, 60.0 -> 18.9, 11.5 -> 4.1.
+// Error over S against long double, root mean square: 30,001 x 820 1.9e-17 -> 4e-18, spread entries
+// 2.6e-16 -> 9e-17.  (One power of two per column over all rows and one integer over a CTA's
+// rows took 3.51 ms, but lost 7e-13 of S with spread entries.)
+constexpr int GD_T = 64, GD_THREADS = 512, GD_ROWS = 16, GD_SUM = 32, GD_BLOCK = 64;
 constexpr uint32_t GD_CHUNK = 2 * GD_T * DIG_STRIDE;   // 8 rows of K
 constexpr uint32_t GD_BUF = 2 * GD_CHUNK;
+constexpr uint32_t GD_ABS = 16 * DIG_ND;               // the FP16 plane, in a row's padding
+static_assert(GD_ABS + 16 <= DIG_STRIDE, "padding of a row");
+constexpr float GD_GUARD = 1.0f / 64.0f;               // 2^-61.1 / GD_GUARD <= 2^-55
+struct GdSmem {
+    // [8][threads]: FP64 sums; a block's integer sums, and the sums of their last 16 bits; the
+    // guard's sum of S and of the squared units
+    static constexpr size_t sum = 2 * GD_BUF;
+    static constexpr size_t whole = sum + 8 * GD_THREADS * sizeof(double);
+    static constexpr size_t part = whole + 8 * GD_THREADS * sizeof(long long);
+    static constexpr size_t size = part + 8 * GD_THREADS * sizeof(int);
+    static constexpr size_t unit = size + 8 * GD_THREADS * sizeof(float);
+    static constexpr size_t shift = unit + 8 * GD_THREADS * sizeof(float);   // [2][2 GD_T] a block's powers of two
+    static constexpr size_t total = shift + 2 * 2 * GD_T * sizeof(int);
+    // of the FP64 sums, over the digits: 64 rows of the two column groups, the outputs' list
+    static constexpr int frows = 64;
+    static constexpr size_t list = 2 * frows * GD_T * sizeof(double);
+    static_assert(list + GD_T * GD_T * sizeof(uint16_t) <= sum, "fits over the digits");
+};
 
-// ex[i] <- the least e with |X[k][i]| < 0.9942 2^e for all k: the digits' bias adds
-// 0x80..80 / 2^63 = 1.0039, and the sum stays below 2 (ex preset to a very small value; COL_BAD for infinities and NaN).
+// The least e with |x| < 0.9942 2^e: the digits' bias adds 0x80..80 / 2^63 = 1.0039, and the
+// sum stays below 2.  COL_BAD for infinities and NaN.
 constexpr int COL_BAD = 4096;
 __device__ __forceinline__ int col_exponent(double x) {
     const int h = __double2hiint(x) & 0x7fffffff;
     return h >= 0x7ff00000 ? COL_BAD : (h >> 20) - 1022 + ((h & 0xfffff) >= 0xfd000 ? 1 : 0);
 }
+// eb[block][c]: col_exponent of the block's largest entry of column c; ex[c] their largest
+// (preset to a very small value).  A warp per (block, 32 columns).
 __global__ void __launch_bounds__(256) k_col_exponents(const double* __restrict__ X, int64_t ldx, int64_t K, int m,
-                                                int* __restrict__ ex) {
+                                                int* __restrict__ ex, int16_t* __restrict__ eb) {
     const int c = blockIdx.x * 32 + (threadIdx.x & 31);
     if (c >= m) return;
-    const int64_t step = (int64_t)gridDim.y * 8;
-    int lg = -1022;
-    int64_t k = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
-    for (; k + 3 * step < K; k += 4 * step) {   // four loads in flight
-        double v[4];
+    int top = -1022;
+    for (int64_t b = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5); b * GD_BLOCK < K; b += (int64_t)gridDim.y * 8) {
+        const int64_t k0 = b * GD_BLOCK, k1 = min(K, k0 + GD_BLOCK);
+        int lg = -1022;
+        int64_t k = k0;
+        for (; k + 8 <= k1; k += 8) {   // eight loads in flight
+            double v[8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = X[(k + u * step) * ldx + c];
+            for (int u = 0; u < 8; ++u) v[u] = X[(k + u) * ldx + c];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) lg = max(lg, col_exponent(v[u]));
+            for (int u = 0; u < 8; ++u) lg = max(lg, col_exponent(v[u]));
+        }
+        for (; k < k1; ++k) lg = max(lg, col_exponent(X[k * ldx + c]));
+        eb[b * m + c] = (int16_t)lg;
+        top = max(top, lg);
     }
-    for (; k < K; k += step) lg = max(lg, col_exponent(X[k * ldx + c]));
-    atomicMax(ex + c, lg);
+    atomicMax(ex + c, top);
 }
 
 template <bool ATOMIC>
 __global__ void __launch_bounds__(GD_THREADS, 1) k_syrk_digits(const double* __restrict__ X, int64_t ldx, int64_t K,
                                                                int m, double* __restrict__ C, int64_t ldc, int ntile,
-                                                               int64_t kslice, const int* __restrict__ ex) {
+                                                               int64_t kslice, const int* __restrict__ ex,
+                                                               const int16_t* __restrict__ eb) {
     extern __shared__ __align__(16) unsigned char smem[];
     int ti, tj;
     upper_pair(blockIdx.x, ntile, ti, tj);
     const bool diag = ti == tj;
-    const int64_t kb = (int64_t)blockIdx.y * kslice, ke = min(K, kb + kslice);
+    const int64_t kb = (int64_t)blockIdx.y * kslice, ke = min(K, kb + kslice);   // kslice: a multiple of GD_SUM
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // digits: a warp has 8 columns (of tile ti, then tj), a lane one column and the row pairs
     // p and p + 4 of the 16, so that the 32 stores of a digit fall into different banks
@@ -154,54 +194,113 @@ __global__ void __launch_bounds__(GD_THREADS, 1) k_syrk_digits(const double* __r
     const int col = (dc < GD_T ? ti * GD_T + dc : tj * GD_T + dc - GD_T);
     const bool builds = !(diag && dc >= GD_T);
     const bool in = builds && col < m;
-    const int sh = in ? DIG_FIX - ex[col] : 0;
+    const int top = in ? ex[col] : 0;
     double v[4];
+    int e = 0;
+    int* const sShift = reinterpret_cast<int*>(smem + GdSmem::shift);
     auto fetch = [&](int64_t k0) {
+        e = in ? eb[k0 / GD_BLOCK * m + col] : 0;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int64_t k = k0 + 2 * p + (u & 1) + 8 * (u >> 1);
             v[u] = in && k < ke ? X[k * ldx + col] : 0.0;
         }
     };
-    auto build = [&](int buf) {
-        if (!builds) return;
-        unsigned char* row = smem + buf * GD_BUF + dc * DIG_STRIDE + 4 * p;
-        put_digits(row, to_fixed(v[0], sh), to_fixed(v[1], sh));
-        put_digits(row + GD_CHUNK, to_fixed(v[2], sh), to_fixed(v[3], sh));
+    // |x| / 2^e of two entries in FP16; what is not zero stays above zero
+    auto sizes = [&](double x0, double x1, long long X0, long long X1) {
+        auto f = [](double x, long long Xi) {
+            const unsigned hi = (unsigned)((unsigned long long)(Xi < 0 ? -Xi : Xi) >> 32);
+            const float y = __uint2float_rn(hi) * 0x1p-31f;
+            return (__double_as_longlong(x) & 0x7fffffffffffffffll) == 0 ? 0.0f : fmaxf(y, 0x1p-24f);
+        };
+        return __floats2half2_rn(f(x0, X0), f(x1, X1));
     };
-    const int mt = warp >> 2, nt = (warp & 3) * 2;
-    float acc[2][DIG_ND][4];
-    long long val[2][4];
+    auto build = [&](int i) {
+        if (!builds) return;
+        const int sh = DIG_FIX - e;
+        const int64_t k0 = kb + (int64_t)i * GD_ROWS;
+        unsigned char* row = smem + (i & 1) * GD_BUF + dc * DIG_STRIDE + 4 * p;
+        if (p == 0 && (i == 0 || k0 % GD_BLOCK == 0)) sShift[(k0 / GD_BLOCK & 1) * 2 * GD_T + dc] = e - top;
 #pragma unroll
-    for (int x = 0; x < 2; ++x)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) val[x][r] = 0;
-    const int up = up_bits(65536u, (int)min(kslice, (int64_t)1 << 30));
+        for (int c8 = 0; c8 < 2; ++c8) {
+            const long long X0 = to_fixed(v[2 * c8], sh), X1 = to_fixed(v[2 * c8 + 1], sh);
+            put_digits(row + c8 * GD_CHUNK, X0, X1);
+            *reinterpret_cast<__half2*>(row + c8 * GD_CHUNK + GD_ABS) = sizes(v[2 * c8], v[2 * c8 + 1], X0, X1);
+        }
+    };
+    const int mt = warp >> 2, nt = (warp & 3) * 2, g4 = lane >> 2, t4 = lane & 3;
+    float acc[2][DIG_ND][4], s[2][4];
     const uint32_t base = smem_addr(smem);
-    auto products = [&](int buf) {
+    const int bcol = diag ? 0 : GD_T;   // the second column group's first row of digits
+    auto products = [&](int i) {
+        const uint32_t t = base + (i & 1) * GD_BUF;
 #pragma unroll 1
         for (int c8 = 0; c8 < 2; ++c8) {
-            const uint32_t t = base + buf * GD_BUF + c8 * GD_CHUNK;
             uint32_t fa[DIG_ND][2], fb[DIG_ND];
-            load_a(fa, t + (uint32_t)(16 * mt) * DIG_STRIDE);
+            load_a(fa, t + c8 * GD_CHUNK + (uint32_t)(16 * mt) * DIG_STRIDE);
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                load_b(fb, t + (uint32_t)((diag ? 0 : GD_T) + 8 * (nt + x)) * DIG_STRIDE);
+                load_b(fb, t + c8 * GD_CHUNK + (uint32_t)(bcol + 8 * (nt + x)) * DIG_STRIDE);
                 mma_digits(acc[x], fa, fb);
             }
         }
+        uint32_t a[4], b[4];   // the FP16 plane: both groups of 8 rows in one product
+        ldsm4(a, t + (lane >> 4) * GD_CHUNK + (uint32_t)(16 * mt + (lane & 15)) * DIG_STRIDE + GD_ABS);
+        ldsm4(b, t + (lane >> 3 & 1) * GD_CHUNK + (uint32_t)(bcol + 8 * (nt + (lane >> 4)) + (lane & 7)) * DIG_STRIDE + GD_ABS);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) mma_f16(s[x], a, b[2 * x], b[2 * x + 1]);
     };
-    auto flush = [&]() {
+    double* const sSum = reinterpret_cast<double*>(smem + GdSmem::sum) + threadIdx.x;
+    long long* const sWhole = reinterpret_cast<long long*>(smem + GdSmem::whole) + threadIdx.x;
+    int* const sPart = reinterpret_cast<int*>(smem + GdSmem::part) + threadIdx.x;
+    float* const sSize = reinterpret_cast<float*>(smem + GdSmem::size) + threadIdx.x;
+    float* const sUnit = reinterpret_cast<float*>(smem + GdSmem::unit) + threadIdx.x;
+    auto collect = [&]() {   // 32 rows' sums to the block's
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
 #pragma unroll
-            for (int r = 0; r < 4; ++r) val[x][r] += acc_value(acc[x], r, up);
+            for (int r = 0; r < 4; ++r) {
+                const int o = (4 * x + r) * GD_THREADS;
+                int fr;
+                const long long w = acc_parts(acc[x], r, fr);
+                sWhole[o] += w + (fr >> 16);
+                sPart[o] += fr & 0xffff;
+            }
             acc_clear(acc[x]);
         }
     };
-    static_assert(2 * GD_ROWS <= MAGIC_TERMS, "exact accumulators");
-    acc_clear(acc[0]);
-    acc_clear(acc[1]);
+    // a block's sums in units of 2^(ex_i + ex_j), and the guard's: a unit below 2^-60 counts as
+    // that, with nothing for it in S
+    auto fold = [&](int64_t block) {
+        const int* sh = sShift + (block & 1) * 2 * GD_T;
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int o = (4 * x + r) * GD_THREADS;
+                const int d = sh[16 * mt + g4 + 8 * (r >> 1)] + sh[bcol + 8 * (nt + x) + 2 * t4 + (r & 1)];
+                sSum[o] += sum_double(sWhole[o], sPart[o], d + 2);
+                sWhole[o] = 0;
+                sPart[o] = 0;
+                if (s[x][r] > 0.0f) {
+                    const float u = __int_as_float((127 + max(min(d, 0), -60)) << 23);
+                    if (d >= -60) sSize[o] = fmaf(s[x][r], u, sSize[o]);
+                    sUnit[o] = fmaf(u, u, sUnit[o]);
+                }
+                s[x][r] = 0.0f;
+            }
+    };
+    static_assert(GD_SUM <= MAGIC_TERMS && GD_SUM == 2 * GD_ROWS, "exact accumulators");
+    static_assert(GD_BLOCK <= 128, "sum_double's range");
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        acc_clear(acc[x]);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int o = (4 * x + r) * GD_THREADS;
+            sSum[o] = 0.0; sWhole[o] = 0; sPart[o] = 0; sSize[o] = sUnit[o] = s[x][r] = 0.0f;
+        }
+    }
     const int nch = ke > kb ? (int)((ke - kb + GD_ROWS - 1) / GD_ROWS) : 0;
     if (nch > 0) {
         fetch(kb);
@@ -210,29 +309,62 @@ __global__ void __launch_bounds__(GD_THREADS, 1) k_syrk_digits(const double* __r
         __syncthreads();
     }
     for (int i = 0; i < nch; ++i) {
-        if (i + 1 < nch) build((i + 1) & 1);
+        if (i + 1 < nch) build(i + 1);
         if (i + 2 < nch) fetch(kb + (int64_t)(i + 2) * GD_ROWS);
-        products(i & 1);
-        if (i & 1) flush();
+        products(i);
+        const int64_t k1 = kb + (int64_t)(i + 1) * GD_ROWS;
+        if ((i & 1) || i + 1 == nch) collect();
+        if (k1 % GD_BLOCK == 0 || i + 1 == nch) fold((k1 - 1) / GD_BLOCK);
         __syncthreads();
     }
-    if (nch & 1) flush();
-    const int g4 = lane >> 2, t4 = lane & 3;
+    __shared__ int nlist;
+    uint16_t* const list = reinterpret_cast<uint16_t*>(smem + GdSmem::list);
+    if (threadIdx.x == 0) nlist = 0;
+    __syncthreads();   // the digits' last readers are done
+    auto add = [&](int i, int j, double g) {
+        double* o = C + (int64_t)i * ldc + j;
+        if (ATOMIC) atomicAdd(o, g);
+        else *o += g;
+    };
 #pragma unroll
     for (int x = 0; x < 2; ++x)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            const int i = ti * GD_T + 16 * mt + g4 + 8 * (r >> 1), j = tj * GD_T + 8 * (nt + x) + 2 * t4 + (r & 1);
+            const int li = 16 * mt + g4 + 8 * (r >> 1), lj = 8 * (nt + x) + 2 * t4 + (r & 1);
+            const int i = ti * GD_T + li, j = tj * GD_T + lj;
             if (i < m && j < m && j >= i) {
-                const int li = ex[i], lj = ex[j];
-                const double g = li == COL_BAD || lj == COL_BAD   // infinities and NaN stay visible
-                                     ? nan("")
-                                     : from_fixed(val[x][r], li + lj + 2 - (56 + up));
-                double* o = C + (int64_t)i * ldc + j;
-                if (ATOMIC) atomicAdd(o, g);
-                else *o += g;
+                const int ei = ex[i], ej = ex[j];
+                const int o = (4 * x + r) * GD_THREADS;
+                if (sSize[o] >= GD_GUARD * sqrtf(sUnit[o]) && ei != COL_BAD && ej != COL_BAD)
+                    add(i, j, ldexp(sSum[o], ei + ej));
+                else
+                    list[atomicAdd(&nlist, 1)] = (uint16_t)(li * GD_T + lj);
             }
         }
+    __syncthreads();
+    // the outputs that digits do not hold, by FP64 multiply-adds row after row
+    const int n = nlist;
+    constexpr int FR = GdSmem::frows;
+    double* const sA = reinterpret_cast<double*>(smem);
+    double* const sB = diag ? sA : sA + FR * GD_T;
+    for (int at = 0; at < n; at += GD_THREADS) {
+        const bool on = at + (int)threadIdx.x < n;
+        const int o = on ? list[at + threadIdx.x] : 0, li = o / GD_T, lj = o % GD_T;
+        double g = 0.0;
+        for (int64_t k0 = kb; k0 < ke; k0 += FR) {
+            __syncthreads();
+#pragma unroll 8
+            for (int t = threadIdx.x; t < (diag ? 1 : 2) * FR * GD_T; t += GD_THREADS) {
+                const int half = t / (FR * GD_T), kk = t / GD_T % FR, c = (half ? tj : ti) * GD_T + t % GD_T;
+                sA[t] = k0 + kk < ke && c < m ? X[(k0 + kk) * ldx + c] : 0.0;
+            }
+            __syncthreads();
+            if (on)
+#pragma unroll 16
+                for (int kk = 0; kk < FR; ++kk) g = fma(sA[kk * GD_T + li], sB[kk * GD_T + lj], g);
+        }
+        if (on) add(ti * GD_T + li, tj * GD_T + lj, g);
+    }
 }
 
 // ---------------------------------------------------------------- Cholesky
@@ -798,9 +930,10 @@ void syrk_tn(const double* X, int64_t ldx, int64_t K, int m, double alpha, doubl
 
 void gram64(const double* X, int64_t ldx, int64_t K, int m, double* C, int64_t ldc, cudaStream_t st) {
     if (K <= 0 || m <= 0) return;
-    // Below, the exponent pass and the 512-thread CTAs' start cost what the FP64 products do
-    // (whole calls, FP64 -> digits: 300 x 400 330 -> 291 us, 1,000 x 200 398 -> 293 us; at
-    // 1,000 x 100 the FP64 products are 30 us of the call)
+    // Below, the exponent pass and the 512-thread CTAs' start cost what the FP64 products do.
+    // Whole calls, FP64 -> digits: 300 x 400 119 -> 82 us, 1,000 x 200 141 -> 99 us; with entries over
+    // many powers of two, some outputs summed twice, 117 -> 108 and 141 -> 153 us; 1,000 x 100
+    // 90 -> 81 and 87 -> 107 us
     if ((double)K * m * m < 4.0e7) {
         syrk_tn(X, ldx, K, m, 1.0, C, ldc, st);
         return;
@@ -808,31 +941,33 @@ void gram64(const double* X, int64_t ldx, int64_t K, int m, double* C, int64_t l
     const int ntile = (m + cgd::GD_T - 1) / cgd::GD_T;
     const int64_t npairs = (int64_t)ntile * (ntile + 1) / 2;
     if (npairs > 0x7fffffffLL) throw std::runtime_error("gram64: matrix too large");
-    // K slices (FP64 atomics) where the triangle alone leaves SMs idle: the fewest 16-row
-    // steps on the longest CTA's path, four more per slice for its start and end
-    const int64_t sms = sm_count(), steps = (K + cgd::GD_ROWS - 1) / cgd::GD_ROWS;
+    // K slices (FP64 atomics) where the triangle alone leaves SMs idle: the fewest 32-row
+    // steps on the longest CTA's path, two more per slice for its start and end
+    const int64_t sms = sm_count(), steps = (K + cgd::GD_SUM - 1) / cgd::GD_SUM;
     int64_t nslice = 1, best = -1;
     for (int64_t sl = 1; sl <= std::min<int64_t>(steps, std::max<int64_t>(1, 8 * sms / npairs)); ++sl) {
-        const int64_t cost = (npairs * sl + sms - 1) / sms * ((steps + sl - 1) / sl + 4);
+        const int64_t cost = (npairs * sl + sms - 1) / sms * ((steps + sl - 1) / sl + 2);
         if (best < 0 || cost < best) { best = cost; nslice = sl; }
     }
-    const int64_t kslice = (steps + nslice - 1) / nslice * cgd::GD_ROWS;
+    const int64_t kslice = (steps + nslice - 1) / nslice * cgd::GD_SUM, blocks = (K + cgd::GD_BLOCK - 1) / cgd::GD_BLOCK;
     nslice = (K + kslice - 1) / kslice;
     int* ex = scratch_alloc<int>(m, st);
+    int16_t* eb = scratch_alloc<int16_t>((size_t)blocks * m, st);   // 1/256 of X
     ckd(cudaMemsetAsync(ex, 0x80, sizeof(int) * m, st), "column exponents");   // a very small value
     const unsigned strips = (unsigned)((m + 31) / 32);
-    const unsigned gy = (unsigned)std::max<int64_t>(1, std::min<int64_t>((K + 63) / 64, 8 * sms / strips));
-    cgd::k_col_exponents<<<dim3(strips, gy), 256, 0, st>>>(X, ldx, K, m, ex);
-    const size_t smem = 2 * cgd::GD_BUF;
+    const unsigned gy = (unsigned)std::max<int64_t>(1, std::min<int64_t>((blocks + 7) / 8, 8 * sms / strips));
+    cgd::k_col_exponents<<<dim3(strips, gy), 256, 0, st>>>(X, ldx, K, m, ex, eb);
+    const size_t smem = cgd::GdSmem::total;
     const dim3 grid((unsigned)npairs, (unsigned)nslice);
     if (nslice > 1) {
         ckd(cudaFuncSetAttribute(cgd::k_syrk_digits<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
-        cgd::k_syrk_digits<true><<<grid, cgd::GD_THREADS, smem, st>>>(X, ldx, K, m, C, ldc, ntile, kslice, ex);
+        cgd::k_syrk_digits<true><<<grid, cgd::GD_THREADS, smem, st>>>(X, ldx, K, m, C, ldc, ntile, kslice, ex, eb);
     } else {
         ckd(cudaFuncSetAttribute(cgd::k_syrk_digits<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
-        cgd::k_syrk_digits<false><<<grid, cgd::GD_THREADS, smem, st>>>(X, ldx, K, m, C, ldc, ntile, kslice, ex);
+        cgd::k_syrk_digits<false><<<grid, cgd::GD_THREADS, smem, st>>>(X, ldx, K, m, C, ldc, ntile, kslice, ex, eb);
     }
     ckd(cudaGetLastError(), "k_syrk_digits");
+    ckd(cudaFreeAsync(eb, st), "column exponents");
     ckd(cudaFreeAsync(ex, st), "column exponents");
 }
 

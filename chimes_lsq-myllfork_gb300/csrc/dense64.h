@@ -15,8 +15,8 @@ namespace cg {
 // fixed order (bit-reproducible).
 void syrk_tn(const double* X, int64_t ldx, int64_t K, int m, double alpha, double* C, int64_t ldc, cudaStream_t st);
 
-// The same with alpha = 1 for the plain form's Gram: from K m^2 = 4e7 on as exact digit
-// products on the tensor cores (k_syrk_digits), else syrk_tn.
+// The same with alpha = 1 for the plain form's Gram: from K m^2 = 4e7 on by digit products on
+// the tensor cores, each entry as accurate as by FP64 sums (k_syrk_digits), else syrk_tn.
 void gram64(const double* X, int64_t ldx, int64_t K, int m, double* C, int64_t ldc, cudaStream_t st);
 
 // In-place right-looking blocked Cholesky of a symmetric n x n matrix held in full

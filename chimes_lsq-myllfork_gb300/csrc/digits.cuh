@@ -116,6 +116,14 @@ __device__ __forceinline__ void mma_digits(float (&acc)[DIG_ND][4], const uint32
     }
 }
 
+// c += A B, one mma.sync (16 rows, 8 columns, K = 16) in FP16 with FP32 sums.
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                 "{%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
 // Accumulators start at MAGIC and hold MAGIC + S exactly while |S| <= 2^22 (32 terms of
 // 8 digit pairs); their bits minus MAGIC_BITS are S.
 constexpr float MAGIC = 12582912.0f;            // 1.5 * 2^23
@@ -129,15 +137,21 @@ __device__ __forceinline__ void acc_clear(float (&acc)[DIG_ND][4]) {
         for (int r = 0; r < 4; ++r) acc[D][r] = MAGIC;
 }
 
-// One output: sum_D S_D 2^(40 + up - 8 D), the digits below the unit rounded, in units of
-// 2^-(56 + up) of the product of the scaled entries (X / 2^64 each); up from up_bits() (units.h).
-__device__ __forceinline__ long long acc_value(const float (&acc)[8][4], int k, int up) {
+// sum_D S_D 2^(40 - 8 D) of one output: the part before the binary point, and fr / 2^16 behind it.
+__device__ __forceinline__ long long acc_parts(const float (&acc)[8][4], int k, int& fr) {
     constexpr unsigned c = MAGIC_BITS * 257u;
     const unsigned hi = __float_as_uint(acc[0][k]) * 256u + __float_as_uint(acc[1][k]) - c;
     const int mid = (int)(__float_as_uint(acc[2][k]) * 256u + __float_as_uint(acc[3][k]) - c);
     const int lo = (int)(__float_as_uint(acc[4][k]) * 256u + __float_as_uint(acc[5][k]) - c);
-    const int fr = (int)(__float_as_uint(acc[6][k]) * 256u + __float_as_uint(acc[7][k]) - c);
-    const long long v = (long long)((unsigned long long)hi << 32) + ((long long)mid << 16) + (long long)lo;
+    fr = (int)(__float_as_uint(acc[6][k]) * 256u + __float_as_uint(acc[7][k]) - c);
+    return (long long)((unsigned long long)hi << 32) + ((long long)mid << 16) + (long long)lo;
+}
+
+// One output: sum_D S_D 2^(40 + up - 8 D), the digits below the unit rounded, in units of
+// 2^-(56 + up) of the product of the scaled entries (X / 2^64 each); up from up_bits() (units.h).
+__device__ __forceinline__ long long acc_value(const float (&acc)[8][4], int k, int up) {
+    int fr;
+    const long long v = acc_parts(acc, k, fr);
     if (up >= 0) return (long long)((unsigned long long)v << up) + (((fr >> (15 - up)) + 1) >> 1);
     return (v + (fr >> 16) + (1ll << (-up - 1))) >> -up;   // to nearest: sums of floors would drift
 }
@@ -152,6 +166,15 @@ __device__ __forceinline__ double from_fixed(long long v, int e) {
     a <<= lz;
     const unsigned long long m = (a >> 11) + ((a >> 10) & 1ull);   // 2^52 <= m <= 2^53
     return __longlong_as_double((long long)(s | (((unsigned long long)(ex - 1) << 52) + m)));
+}
+
+// (whole + part / 2^16) 2^(e - 56) rounded to FP64, |whole| < 2^61.01, 0 <= part < 2^18: sums of
+// acc_parts over up to 128 terms (2^e times the product of the scaled entries).  The 78 bits are
+// cut to 60 or more of the value's own first.
+__device__ __forceinline__ double sum_double(long long whole, int part, int e) {
+    whole += part >> 16;
+    const int sh = min(16, max(__clzll(whole < 0 ? -whole : whole) - 2, 0));
+    return from_fixed((long long)((unsigned long long)whole << sh) + ((part & 0xffff) >> (16 - sh)), e - 56 - sh);
 }
 
 }  // namespace cgd
