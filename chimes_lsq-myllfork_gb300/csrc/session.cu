@@ -992,11 +992,14 @@ void Session::run(const DeviceFrames& df, int precision, void* A, int64_t lda, A
         // the slot bases are tabulated, unless a force_range setting names another form.  Of 16
         // frames of 256 C/H/N/O atoms, range form -> digit products: 4-body force rows 12.6 ->
         // 7.0 ms, stress and energy 13.3 -> 3.1 ms; 3-body 2.8 -> 1.8 and 3.7 -> 1.0 ms
+        // (The exponents of a group follow its largest cluster.  Bases that CONSTANT_DERIV continues
+        // below s_min grow without bound: one close contact, 0.9 A under an s_min of 1.3 A, left the
+        // small columns 10 to 60 times the FP64 forms' error.)
         bool tensor = false;
         cgd::OzWork oz{};
         if (!S.base && nbasis * rsize <= kClusterBasisMax) {
             pre = prec == 0 ? (void*)S.get<double>(nbasis) : (void*)S.get<float>(nbasis);
-            tensor = prec == 0 && force_range_ == 1 && cgd::oz_fits(nbody, ord, ozt.max_words);
+            tensor = prec == 0 && force_range_ == 1 && M.fix != FIX_CONSTANT_DERIV && cgd::oz_fits(nbody, ord, ozt.max_words);
             int* lgs = nullptr;
             if (tensor) {
                 lgs = S.get<int>((size_t)nq * (nbody == 3 ? 3 : 6));

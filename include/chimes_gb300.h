@@ -540,9 +540,9 @@ void cg_batch_fit_free(cg_batch_fit* b);
  * "refine_cache_mb" (device memory the streamed refinement may fill with FP64 row
  * blocks kept between passes, in MiB; -1 = what is free beyond a margin, the
  * default; 0 = assemble every block on every pass); "force_range" (the many-body
- * rows: 1, the default, FP64 rows of 3-body orders 5-8 and 4-body order 4 as exact digit
- * products on the tensor cores, the force rows of other orders and of cg_assemble_device_noalloc
- * by the range form -- each thread summing a contiguous range of a cluster type's powers
+ * rows: 1, the default, FP64 rows of 3-body orders 5-8 and 4-body order 4 as digit
+ * products on the tensor cores (not with CHEBYFIX CONSTANT_DERIV), the force rows of other
+ * orders and of cg_assemble_device_noalloc by the range form -- each thread summing a contiguous range of a cluster type's powers
  * per column -- in FP64 and, in FP32, where a type has more than 512 allowed powers; 2 the
  * range form always; 0 never -- one accumulator per power, summed per column in shared
  * memory); "host_staging" (the pinned host buffers of cg_assemble_stream: 1, the

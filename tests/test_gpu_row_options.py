@@ -32,7 +32,8 @@ OPTIONS = {
 
 
 def _patched(synth, tmp_path, name):
-    fm = synth.make_workload("chno-4b", str(tmp_path), nframes=2, seed=91, labels=False, sizes=[60, 110],
+    sizes = [24, 50] if name == "specific" else [60, 110]   # (its other types reach to 5 A: many quadruplets)
+    fm = synth.make_workload("chno-4b", str(tmp_path), nframes=2, seed=91, labels=False, sizes=sizes,
                              triclinic=False, species2=True, order=(6, 8, 4))
     text = open(fm).read()
     for old, new in OPTIONS[name]:
@@ -87,3 +88,17 @@ def test_hierarchical_exclusion(cg, oracle, tmp_path):
     O, _ = oracle.assemble(fm, nthreads=8)
     assert A.shape == O.shape
     assert np.all(np.abs(A - O) <= 1e-12 * np.abs(O) + 1e-12 * np.abs(O).max(axis=0)[None, :])
+
+
+def test_bases_continued_below_s_min_take_the_fp64_form(cg, tmp_path):
+    """CONSTANT_DERIV's bases grow without bound below s_min, and digits under a group's largest
+    magnitude would hold the other clusters' small columns less accurately: the rows are those
+    of the FP64 range form."""
+    synth = importlib.import_module("chimes_lsq-myllfork_gb300.synth")
+    fm = _patched(synth, tmp_path, "constant_deriv")
+    model = cg.Model(fm)
+    frames = cg.Frames.read(model)
+    sess = cg.Session(model, 0)
+    A = sess.assemble(frames, cg.CG_FP64)
+    sess.tune("force_range", 2)
+    assert np.array_equal(A, sess.assemble(frames, cg.CG_FP64))
