@@ -810,7 +810,7 @@ __global__ void k_md_mtk_half1(FramesDev F, const double* mass_type, double* x, 
     const int64_t aofs = F.atom_ofs[f];
     double* t = th + (size_t)f * MD_TH_STRIDE;
     double k = 0.0;
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
+    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
         const int64_t g = 3 * aofs + i;
         k += 0.5 * mass_type[F.type[aofs + i / 3]] * v[g] * v[g];
     }
@@ -865,7 +865,7 @@ __global__ void k_md_mtk_half2(FramesDev F, const double* Fo, const double* inv_
         fT = (2.0 * (k0 / (s * s)) - nkt) / Q;
     }
     double k = 0.0;
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
+    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
         const int64_t g = 3 * aofs + i;
         const double vn = (v[g] + 0.5 * acc[g] * dt) / s;
         v[g] = vn;
@@ -889,7 +889,7 @@ __global__ void k_md_berend(FramesDev F, const double* mass_type, double* v, dou
     const int N = F.natoms[f];
     const int64_t aofs = F.atom_ofs[f];
     double k = 0.0;
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
+    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
         const int64_t g = 3 * aofs + i;
         k += 0.5 * mass_type[F.type[aofs + i / 3]] * v[g] * v[g];
     }
@@ -1088,7 +1088,7 @@ __global__ void k_md_npt_berend(FramesDev F, BoxDev* box, const double* mass_typ
     const int N = F.natoms[f];
     const int64_t aofs = F.atom_ofs[f];
     double k = 0.0;
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
+    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
         const int64_t g = 3 * aofs + i;
         k += 0.5 * mass_type[F.type[aofs + i / 3]] * v[g] * v[g];
     }
@@ -1240,7 +1240,7 @@ __global__ void k_md_nptmtk_half2(FramesDev F, const double* Fo, const double* i
         s = 1.0 + 0.5 * dt * (zT + cdof * bvT);
     }
     double k = 0.0;
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
+    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
         const int64_t g = 3 * aofs + i;
         const double vn = v[g] / s_used;
         v[g] = vn;
@@ -1265,7 +1265,7 @@ __global__ void k_md_vscale(FramesDev F, const double* mass_type, double* v, dou
     const int64_t aofs = F.atom_ofs[f];
     double* t = th + (size_t)f * MD_TH_STRIDE;
     double k = 0.0;
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.y * blockDim.x) {
+    for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) {
         const int64_t g = 3 * aofs + i;
         k += 0.5 * mass_type[F.type[aofs + i / 3]] * v[g] * v[g];
     }
