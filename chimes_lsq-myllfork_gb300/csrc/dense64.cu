@@ -383,7 +383,9 @@ constexpr int CH_H = 64, CH_B = 16, CH_LD = CH_H + 1, CH_THREADS = 256;
 // row r, columns 2 i + h, so that one instruction updates two columns (a warp's FP64
 // instruction takes 64 cycles of its SM quarter whatever the lanes do).  L D L^T first, one
 // reciprocal per column in the chain, and the square roots of all pivots at the end.  A
-// pivot that is not positive becomes 1; bad receives its column + 1 (the first).
+// pivot that is not positive becomes 1; bad receives its column + 1 (the first).  TINY: pivots
+// below 2^-1000 are scaled, as the reciprocal of one below 2^-1024 is not finite.
+template <bool TINY>
 __device__ __forceinline__ void chol16(double* D, int b0, int bs, double* rdiag, int* bad) {
     const int lane = threadIdx.x & 31, r = lane & 15, h = lane >> 4;
     double a[CH_B / 2], piv = 1.0;
@@ -401,7 +403,9 @@ __device__ __forceinline__ void chol16(double* D, int b0, int bs, double* rdiag,
             d = 1.0;
         }
         if (r == j) piv = d;
-        const double l = v * __drcp_rn(d);
+        double w = v;
+        if (TINY && d < 0x1p-1000) { d *= 0x1p200; w *= 0x1p200; }
+        const double l = w * __drcp_rn(d);
 #pragma unroll
         for (int i = j >> 1; i < CH_B / 2; ++i) {
             const int c = 2 * i + h;
@@ -423,9 +427,12 @@ __device__ __forceinline__ void chol16(double* D, int b0, int bs, double* rdiag,
 // Columns k .. k + kb of the column-major lower matrix (leading dimension n, kb <= 64):
 // the diagonal block's factor and the m rows below it, R rows per CTA.  While warp 0
 // factorises the next 16 columns' diagonal sub-block, the others finish the update of the
-// columns after them.
+// columns after them.  status: a counter of the launch's CTAs, and a word that becomes 1 if a
+// pivot was below 2^-1020 (the factorisation may have failed for want of TINY, which costs 1 to 3%
+// of it, in the chain of pivots).
+template <bool TINY>
 __global__ void __launch_bounds__(CH_THREADS) k_chol_half(double* __restrict__ G, int n, int k, int kb, int m, int R,
-                                                          int second, int* info, int* __restrict__ arrived) {
+                                                          int second, int* info, int* __restrict__ status) {
     extern __shared__ double sm[];
     double* D = sm;                          // rows 0 .. kb: the block, then this CTA's rows
     __shared__ double rdiag[CH_H];
@@ -477,7 +484,7 @@ __global__ void __launch_bounds__(CH_THREADS) k_chol_half(double* __restrict__ G
     };
     for (int b0 = 0; b0 < kb; b0 += CH_B) {
         const int bs = min(CH_B, kb - b0);
-        if (threadIdx.x < 32) chol16(D, b0, bs, rdiag, &bad);
+        if (threadIdx.x < 32) chol16<TINY>(D, b0, bs, rdiag, &bad);
         else if (b0 > 0 && b0 + CH_B < kb) update(b0 - CH_B, b0 + CH_B, kb, threadIdx.x - 32, CH_THREADS - 32);
         __syncthreads();
         // the sub-block's columns of every row below, a row per thread
@@ -507,8 +514,8 @@ __global__ void __launch_bounds__(CH_THREADS) k_chol_half(double* __restrict__ G
     // the block's factor, by the last CTA: every other has read the block by then
     if (threadIdx.x == 0) {
         __threadfence();
-        last = atomicAdd(arrived, 1) == (int)gridDim.x - 1;
-        if (last) *arrived = 0;
+        last = atomicAdd(status, 1) == (int)gridDim.x - 1;
+        if (last) *status = 0;
     }
     __syncthreads();
     if (!last) return;
@@ -520,6 +527,7 @@ __global__ void __launch_bounds__(CH_THREADS) k_chol_half(double* __restrict__ G
         for (int idx = threadIdx.x; idx < CH_H * kb; idx += blockDim.x)
             G[(int64_t)(k + idx / CH_H) * n + k - CH_H + idx % CH_H] = 0.0;
     if (threadIdx.x == 0 && bad) atomicCAS(info, 0, k + bad);
+    if (!TINY && threadIdx.x < kb && rdiag[threadIdx.x] > 0x1p510) status[1] = 1;
 }
 
 // The second half's columns, rows k0 + 64 and below: minus the first half's product.
@@ -971,7 +979,7 @@ void gram64(const double* X, int64_t ldx, int64_t K, int m, double* C, int64_t l
     ckd(cudaFreeAsync(ex, st), "column exponents");
 }
 
-bool cholesky64(double* G, int n, int* d_info, cudaStream_t st, bool tensor_updates) {
+bool cholesky64(double* G, int n, int* d_info, cudaStream_t st, bool tensor_updates, bool tiny, bool* tiny_pivot) {
     ckd(cudaMemsetAsync(d_info, 0, sizeof(int), st), "info");
     // trailing updates of full 128-wide panels by exact BF16 digit products on the
     // tensor cores (syrk_update_ozaki); the FP64 SYRK otherwise
@@ -981,18 +989,19 @@ bool cholesky64(double* G, int n, int* d_info, cudaStream_t st, bool tensor_upda
         oz = scratch_alloc<unsigned char>(ozaki_scratch_bytes(n), st);
         ckd(cudaMemsetAsync(oz, 0, sizeof(int), st), "Ozaki error word");
     }
-    int* arrived = scratch_alloc<int>(1, st);   // counter of a panel's CTAs
-    ckd(cudaMemsetAsync(arrived, 0, sizeof(int), st), "panel counter");
+    int* status = scratch_alloc<int>(2, st);
+    ckd(cudaMemsetAsync(status, 0, 2 * sizeof(int), st), "panel status");
     const int sms = sm_count();
     const size_t most = 200 * 1024;
-    ckd(cudaFuncSetAttribute(cgd::k_chol_half, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most), "panel smem");
+    const auto panel = tiny ? cgd::k_chol_half<true> : cgd::k_chol_half<false>;
+    ckd(cudaFuncSetAttribute(panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most), "panel smem");
     const int rmax = (int)(most / (cgd::CH_LD * sizeof(double))) - cgd::CH_H;
     auto half = [&](int k, int kb, int second) {
         const int m = n - k - kb;
         const int R = std::max(8, std::min(rmax, (m + sms - 1) / sms));   // one share of the rows per SM
         const int grid = std::max(1, (m + R - 1) / R);
-        cgd::k_chol_half<<<grid, cgd::CH_THREADS, (size_t)(cgd::CH_H + R) * cgd::CH_LD * sizeof(double), st>>>(
-            G, n, k, kb, m, R, second, d_info, arrived);
+        panel<<<grid, cgd::CH_THREADS, (size_t)(cgd::CH_H + R) * cgd::CH_LD * sizeof(double), st>>>(G, n, k, kb, m, R, second,
+                                                                                                    d_info, status);
     };
     for (int k = 0; k < n; k += cgd::CH_NB) {
         const int kb = std::min(cgd::CH_NB, n - k), k1 = std::min(cgd::CH_H, kb), k2 = kb - k1;
@@ -1010,14 +1019,17 @@ bool cholesky64(double* G, int n, int* d_info, cudaStream_t st, bool tensor_upda
         }
         ckd(cudaGetLastError(), "cholesky step");
     }
-    int info = 0, oz_err = 0;
+    int info = 0, oz_err = 0, small = 0;
     ckd(cudaMemcpyAsync(&info, d_info, sizeof(int), cudaMemcpyDeviceToHost, st), "info");
-    ckd(cudaFreeAsync(arrived, st), "panel counter");
     if (use_oz) {
         ckd(cudaMemcpyAsync(&oz_err, oz, sizeof(int), cudaMemcpyDeviceToHost, st), "Ozaki error word");
         ckd(cudaFreeAsync(oz, st), "Ozaki scratch");
     }
     ckd(cudaStreamSynchronize(st), "cholesky");
+    if (info != 0 && tiny_pivot) ckd(cudaMemcpyAsync(&small, status + 1, sizeof(int), cudaMemcpyDeviceToHost, st), "panel status");
+    ckd(cudaFreeAsync(status, st), "panel status");
+    if (info != 0) ckd(cudaStreamSynchronize(st), "panel status");
+    if (tiny_pivot) *tiny_pivot = small != 0;
     if (oz_err) throw std::runtime_error("Cholesky trailing update timed out on its pipeline (code " +
                                          std::to_string(oz_err) + ")");
     return info == 0;

@@ -25,8 +25,10 @@ void gram64(const double* X, int64_t ldx, int64_t K, int m, double* C, int64_t l
 // the rest of the upper triangle keeps G's values.  128 x 128 diagonal
 // blocks are factorised in 64-wide halves in shared memory, the panel below against
 // them, the trailing matrix by exact digit products or syrk_tn.  Returns false when a pivot is not
-// positive (d_info: device int, first bad column + 1).
-bool cholesky64(double* G, int n, int* d_info, cudaStream_t st, bool tensor_updates = false);
+// positive (d_info: device int, first bad column + 1); *tiny_pivot tells whether a pivot was
+// below 2^-1020, with which only the form for tiny pivots is sure to go on.
+bool cholesky64(double* G, int n, int* d_info, cudaStream_t st, bool tensor_updates = false, bool tiny = false,
+                bool* tiny_pivot = nullptr);
 
 // In-place triangular solve T x = b (x holds b on entry) with T(i, j) = M[i*si + j*sj]
 // lower (forward substitution) or upper (backward substitution), n x n.

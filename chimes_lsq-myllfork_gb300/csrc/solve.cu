@@ -49,9 +49,12 @@ double factor_ridge(const double* G, int n, double ridge, double* L, int* d_info
     // mixed-precision G can be indefinite at tiny ridges.
     double used = ridge;
     for (int attempt = 0; attempt < 9; ++attempt) {
-        cks(cudaMemcpyAsync(L, G, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, st), "L = G");
-        add_diag64(L, n, used, st);
-        if (cholesky64(L, n, d_info, st, tensor_updates)) return used;
+        bool tiny = false;
+        for (int form = 0; form < (tiny ? 2 : 1); ++form) {   // again for tiny pivots, if one was met
+            cks(cudaMemcpyAsync(L, G, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, st), "L = G");
+            add_diag64(L, n, used, st);
+            if (cholesky64(L, n, d_info, st, tensor_updates, form == 1, &tiny)) return used;
+        }
         used = used > 0.0 ? used * 10.0 : 1e-12;
     }
     return -1.0;
