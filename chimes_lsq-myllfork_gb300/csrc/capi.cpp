@@ -892,6 +892,7 @@ int cg_session_tune(cg_session* s, const char* key, int value) {
         else if (k == "host_staging") s->s->set_host_staging(value);
         else if (k == "cholesky_tensor_updates") s->s->set_cholesky_tensor_updates(value != 0);
         else if (k == "refine_cache_mb") s->s->set_refine_cache_bytes(value < 0 ? -1 : (int64_t)value << 20);
+        else if (k == "release_memory") s->s->release_memory();
         else throw cg::Error(1, "unknown tuning key: " + k);
     });
 }

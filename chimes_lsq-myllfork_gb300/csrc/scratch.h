@@ -20,8 +20,9 @@ void cuda_check(cudaError_t e, const char* what);
 // work lists again, which cost tens of milliseconds per block of a streamed
 // assembly when the rest of device memory was busy.
 cudaMemPool_t scratch_pool(int device);
-// Return the pool's unused memory to the driver (before sizing a cache from the
-// device's free memory).
+// Return the pool's unused memory to the driver: before sizing a cache from the device's
+// free memory, and for callers that share the GPU with another allocator (cg_session_tune
+// "release_memory").
 void scratch_pool_trim(int device);
 
 // One stream-ordered allocation from the current device's scratch pool (cudaFreeAsync
@@ -36,10 +37,14 @@ T* scratch_alloc(size_t n, cudaStream_t st) {
     return static_cast<T*>(p);
 }
 
-// Device memory of an object that outlives a call or is shared by streams, from the scratch
-// pool: its owner may use it on any stream once the allocating stream has been synchronised,
-// and it goes back when nothing on the device can use it any more.  cudaMalloc and cudaFree
-// of a dozen arrays took half of a call on a small system.
+// Device memory of an object that outlives a call or is shared by streams: its owner may use
+// it on any stream once the allocating stream has been synchronised, and it goes back when
+// nothing on the device can use it any more.  Up to POOL_BLOCK from the scratch pool: cudaMalloc
+// and cudaFree of a dozen arrays took half of a call on a small system, and one pair takes 120
+// us (1 MiB) to 274 us (256 MiB) where the pool takes 5.  Larger blocks by cudaMalloc, so that
+// the driver has them back at once: 0.5 to 1.1 ms (512 MiB, 2 GiB) beside work on as much data.
+// Copies to the host run at the same rate out of either (193 GB/s from 64 MiB on).
+constexpr size_t POOL_BLOCK = size_t(256) << 20;
 void* pool_alloc(size_t bytes, cudaStream_t st);
 void pool_free(std::vector<void*>& ptrs);   // synchronises the device first
 

@@ -390,7 +390,12 @@ FrameBatch make_batch(const Model& m, const std::vector<Frame>& frames, int firs
 
 DeviceFrames::~DeviceFrames() { pool_free(allocs); }
 
-void* pool_alloc(size_t bytes, cudaStream_t st) { return scratch_alloc<unsigned char>(bytes, st); }
+void* pool_alloc(size_t bytes, cudaStream_t st) {
+    if (bytes <= POOL_BLOCK) return scratch_alloc<unsigned char>(bytes, st);
+    void* p = nullptr;
+    CK(cudaMalloc(&p, bytes));
+    return p;
+}
 
 void pool_free(std::vector<void*>& ptrs) {
     if (ptrs.empty()) return;
@@ -401,7 +406,7 @@ void pool_free(std::vector<void*>& ptrs) {
         if (p && cudaPointerGetAttributes(&at, p) == cudaSuccess && (dev = at.device) >= 0) break;
     if (dev >= 0 && dev != cur) cudaSetDevice(dev);
     cudaDeviceSynchronize();
-    for (void* p : ptrs) if (p) cudaFree(p);   // pool memory: returned without a further wait
+    for (void* p : ptrs) if (p) cudaFree(p);   // the pool's is returned without a further wait
     if (dev >= 0 && dev != cur) cudaSetDevice(cur);
     ptrs.clear();
 }
@@ -789,11 +794,7 @@ int64_t Session::assemble_to_host(const FrameBatch& fb, int precision, int block
     } R;
     const int64_t lda = model_.tot_all;
     const size_t block = (size_t)maxrows * lda * rsz;
-    for (int i = 0; i < 2 && i < nblk; ++i) {   // small blocks from the pool (cudaMalloc would be most of the call; copies of
-                                                     // gigabytes out of pool memory ran at half the rate)
-        if (block <= size_t(32) << 20) R.dA[i] = pool_alloc(block, stream_);
-        else CK(cudaMalloc(&R.dA[i], block));
-    }
+    for (int i = 0; i < 2 && i < nblk; ++i) R.dA[i] = pool_alloc(block, stream_);
     for (int i = 0; i < 2; ++i) {
         CK(cudaEventCreateWithFlags(&R.asm_done[i], cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&R.copy_done[i], cudaEventDisableTiming));
@@ -1302,6 +1303,12 @@ struct StreamRows {
     }
 };
 }  // namespace
+
+void Session::release_memory() {
+    CK(cudaSetDevice(device_));
+    CK(cudaStreamSynchronize(stream_));
+    scratch_pool_trim(device_);
+}
 
 void Session::refine_streamed(const double* L, int ncols, double ridge, const std::vector<const DeviceFrames*>& blocks,
                               const std::vector<const double*>& labels, const std::vector<const double*>& weights,

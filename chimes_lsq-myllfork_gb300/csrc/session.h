@@ -343,6 +343,7 @@ class Session {
     // (stress false) or nine PRESSURE_TENSORS_XYZ_ALL entries per frame (row-major).
     void md_numerical(const FrameBatch& fb, bool stress, double* out);
     double md_skin() const { return md_skin_; }
+    void release_memory();   // unused pool memory of the device back to the driver
     void set_md_skin(double s) { md_skin_ = s >= 0.0 ? s : 0.0; }
     // nsteps velocity-Verlet steps (NVE) of every frame of the batch; df's positions
     // and v [natoms_total*3] (device) are advanced in place.  mass_type: host,

@@ -551,7 +551,9 @@ void cg_batch_fit_free(cg_batch_fit* b);
  * force-row kernel when the
  * range form is not used, 512 or 1024); "cholesky_tensor_updates" (1, the
  * default: the blocked Cholesky's trailing updates from exact BF16 digit products on
- * the tensor cores, FP64-accurate; 0: the FP64 SYRK). */
+ * the tensor cores, FP64-accurate; 0: the FP64 SYRK); "release_memory" (any value: gives
+ * device memory that the library keeps for later calls -- up to 32 GiB of scratch per device,
+ * freed frames, lists and arenas of up to 256 MiB each among it -- back to the driver now). */
 int cg_session_tune(cg_session* s, const char* key, int value);
 
 const char* cg_last_error(void);
