@@ -97,48 +97,45 @@ __global__ void __launch_bounds__(SY_THREADS) k_syrk_tn(const double* __restrict
 
 // ---------------------------------------------------------------- X^T X as digit products
 // The same triangle from the tensor cores (digits.cuh) with the accuracy of FP64 sums, entry
-// by entry.  Every 64 rows (a block) each column has its own power of two; its entries are
+// by entry.  Every 32 rows (a block) each column has its own power of two; its entries are
 // split into eight base-256 digits, a 64 x 64 tile's 36 digit products per term are summed
-// exactly over the block in integers, and the block's sum is rounded once to FP64 and added
-// in FP64.  In units of the two columns' powers of two a block loses about 2^-61.1 (64 terms
-// whose dropped diagonals are 2^-64.1 each, root mean square), and nothing in rows where
-// either entry is zero.
+// exactly over the block, and the blocks' sums exactly in 128-bit integers, in units of 2^-88 of
+// the product of the columns' largest powers of two; one rounding to FP64 at the end.  In units
+// of its two powers of two a block loses about 2^-61.6 (32 terms whose dropped diagonals are
+// 2^-64.1 each, root mean square), and nothing in rows where either entry is zero.
 //
 // That is less than FP64 sums lose -- at least 2^-55 of S_ij = sum |x_ki x_kj| -- unless the
 // rows of the large entries of one column meet small ones of the other.  So a ninth plane
 // holds |x| in FP16 and one more product per 16 rows estimates S: an output whose S is below
 // GD_GUARD times the root of its blocks' squared units is summed again in FP64 by the same
-// CTA (as are columns that are not finite).  Of a C/H 4-body A of 816 x 3,992 that is 5% of
+// CTA (as are columns that are not finite).  Of a C/H 4-body A of 816 x 3,992 that is 2.5% of
 // the outputs, of a water 3-body A of 13,968 x 820 none.
 //
 // Sixteen warps of 16 rows x 16 columns; the next 16 rows' digits are built while warps that
 // have finished theirs run the current products.  The tensor pipe is the bound (36
 // products per multiply-add on mma.sync, 606 TFLOP/s measured, or 13.9 TFLOP/s of FP64
-// arithmetic).  Blocks of 32 rows leave more outputs to the digits, but FP64 has 1/64 of the
-// FP32 rate and an addition per output and 32 rows kept the tensor pipe waiting (30,001 x 820
-// 4.8 ms); blocks of 128 leave fewer (4.05 ms, but 816 x 3,992 heavy-tailed 4.1 -> 5.6 ms).
+// arithmetic).  (Blocks rounded to FP64 and added there took 4.8 ms at 30,001 x 820, at 32 rows a
+// block, 4.4 at 64: an addition at 1/64 of the FP32 rate keeps the tensor pipe waiting.)
 //
-// Whole calls with h, FP64 sums -> this: 30,001 x 820 19.3 -> 4.36 ms, 2,000 x 6,007 60.0 -> 14.2,
-// 816 x 3,992 11.5 -> 2.8; entries spread by exp(2 N(0,1)): 19.3 -> 5.5, 60.0 -> 18.9, 11.5 -> 4.1.
-// Error over S against long double, root mean square: 30,001 x 820 1.9e-17 -> 4e-18, spread entries
-// 2.6e-16 -> 9e-17.  (One power of two per column over all rows and one integer over a CTA's
-// rows took 3.51 ms, but lost 7e-13 of S with spread entries.)
-constexpr int GD_T = 64, GD_THREADS = 512, GD_ROWS = 16, GD_SUM = 32, GD_BLOCK = 64;
+// Whole calls with h, FP64 sums -> this: 30,001 x 820 19.3 -> 4.26 ms, 2,000 x 6,007 60.0 -> 14.0,
+// 816 x 3,992 11.5 -> 2.8; entries spread by exp(2 N(0,1)): 19.3 -> 5.6, 60.0 -> 18.0, 11.5 -> 3.5.
+// Error over S against long double, root mean square: 30,001 x 820 1.9e-17 -> 1.3e-18, spread
+// entries 2.6e-16 -> 2.1e-17.  (One power of two per column over all rows and one 64-bit integer
+// over a CTA's rows took 3.51 ms, but lost 7e-13 of S with spread entries.)
+constexpr int GD_T = 64, GD_THREADS = 512, GD_ROWS = 16, GD_BLOCK = 32;
 constexpr uint32_t GD_CHUNK = 2 * GD_T * DIG_STRIDE;   // 8 rows of K
 constexpr uint32_t GD_BUF = 2 * GD_CHUNK;
 constexpr uint32_t GD_ABS = 16 * DIG_ND;               // the FP16 plane, in a row's padding
 static_assert(GD_ABS + 16 <= DIG_STRIDE, "padding of a row");
-constexpr float GD_GUARD = 1.0f / 64.0f;               // 2^-61.1 / GD_GUARD <= 2^-55
+constexpr float GD_GUARD = 1.0f / 96.0f;               // 2^-61.6 / GD_GUARD <= 2^-55
+constexpr int GD_FRAC = 18;                            // a block's integer sums are kept times 2^GD_FRAC or less
 struct GdSmem {
-    // [8][threads]: FP64 sums; a block's integer sums, and the sums of their last 16 bits; the
-    // guard's sum of S and of the squared units
+    // [8][threads]: the integer sums; the guard's sum of S and of the squared units
     static constexpr size_t sum = 2 * GD_BUF;
-    static constexpr size_t whole = sum + 8 * GD_THREADS * sizeof(double);
-    static constexpr size_t part = whole + 8 * GD_THREADS * sizeof(long long);
-    static constexpr size_t size = part + 8 * GD_THREADS * sizeof(int);
-    static constexpr size_t unit = size + 8 * GD_THREADS * sizeof(float);
-    static constexpr size_t shift = unit + 8 * GD_THREADS * sizeof(float);   // [2][2 GD_T] a block's powers of two
+    static constexpr size_t guard = sum + 8 * GD_THREADS * sizeof(__int128);
+    static constexpr size_t shift = guard + 8 * GD_THREADS * sizeof(float2);   // [2][2 GD_T] a block's powers of two
     static constexpr size_t total = shift + 2 * 2 * GD_T * sizeof(int);
+    static_assert(sum % 16 == 0, "alignment");
     // of the FP64 sums, over the digits: 64 rows of the two column groups, the outputs' list
     static constexpr int frows = 64;
     static constexpr size_t list = 2 * frows * GD_T * sizeof(double);
@@ -186,7 +183,7 @@ __global__ void __launch_bounds__(GD_THREADS, 1) k_syrk_digits(const double* __r
     int ti, tj;
     upper_pair(blockIdx.x, ntile, ti, tj);
     const bool diag = ti == tj;
-    const int64_t kb = (int64_t)blockIdx.y * kslice, ke = min(K, kb + kslice);   // kslice: a multiple of GD_SUM
+    const int64_t kb = (int64_t)blockIdx.y * kslice, ke = min(K, kb + kslice);   // kslice: a multiple of GD_BLOCK
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // digits: a warp has 8 columns (of tile ti, then tj), a lane one column and the row pairs
     // p and p + 4 of the 16, so that the 32 stores of a digit fall into different banks
@@ -218,9 +215,8 @@ __global__ void __launch_bounds__(GD_THREADS, 1) k_syrk_digits(const double* __r
     auto build = [&](int i) {
         if (!builds) return;
         const int sh = DIG_FIX - e;
-        const int64_t k0 = kb + (int64_t)i * GD_ROWS;
         unsigned char* row = smem + (i & 1) * GD_BUF + dc * DIG_STRIDE + 4 * p;
-        if (p == 0 && (i == 0 || k0 % GD_BLOCK == 0)) sShift[(k0 / GD_BLOCK & 1) * 2 * GD_T + dc] = e - top;
+        if ((i & 1) == 0 && p == 0) sShift[(i >> 1 & 1) * 2 * GD_T + dc] = e - top;
 #pragma unroll
         for (int c8 = 0; c8 < 2; ++c8) {
             const long long X0 = to_fixed(v[2 * c8], sh), X1 = to_fixed(v[2 * c8 + 1], sh);
@@ -250,55 +246,45 @@ __global__ void __launch_bounds__(GD_THREADS, 1) k_syrk_digits(const double* __r
 #pragma unroll
         for (int x = 0; x < 2; ++x) mma_f16(s[x], a, b[2 * x], b[2 * x + 1]);
     };
-    double* const sSum = reinterpret_cast<double*>(smem + GdSmem::sum) + threadIdx.x;
-    long long* const sWhole = reinterpret_cast<long long*>(smem + GdSmem::whole) + threadIdx.x;
-    int* const sPart = reinterpret_cast<int*>(smem + GdSmem::part) + threadIdx.x;
-    float* const sSize = reinterpret_cast<float*>(smem + GdSmem::size) + threadIdx.x;
-    float* const sUnit = reinterpret_cast<float*>(smem + GdSmem::unit) + threadIdx.x;
-    auto collect = [&]() {   // 32 rows' sums to the block's
+    __int128* const sSum = reinterpret_cast<__int128*>(smem + GdSmem::sum) + threadIdx.x;
+    float2* const sGuard = reinterpret_cast<float2*>(smem + GdSmem::guard) + threadIdx.x;
+    // A block's sums to the outputs', in units of 2^(ex_i + ex_j - 70 - GD_FRAC): what a power of
+    // two below 2^-GD_FRAC shifts out is below the block's own loss down to 2^-29, so the guard
+    // counts a smaller unit as that.
+    auto flush = [&](int block) {
+        const int* sh = sShift + (block & 1) * 2 * GD_T;
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const int o = (4 * x + r) * GD_THREADS;
+                const int d = sh[16 * mt + g4 + 8 * (r >> 1)] + sh[bcol + 8 * (nt + x) + 2 * t4 + (r & 1)];
                 int fr;
                 const long long w = acc_parts(acc[x], r, fr);
-                sWhole[o] += w + (fr >> 16);
-                sPart[o] += fr & 0xffff;
+                const __int128 v = ((__int128)w << 16) + fr;
+                sSum[o] += d >= -GD_FRAC ? v << (d + GD_FRAC) : v >> min(-GD_FRAC - d, 127);
+                if (s[x][r] > 0.0f) {
+                    const float u = __int_as_float((127 + max(d, -29)) << 23);
+                    float2 g = sGuard[o];
+                    g.x = fmaf(s[x][r], d < -60 ? 0.0f : __int_as_float((127 + d) << 23), g.x);
+                    g.y = fmaf(u, u, g.y);
+                    sGuard[o] = g;
+                }
+                s[x][r] = 0.0f;
             }
             acc_clear(acc[x]);
         }
     };
-    // a block's sums in units of 2^(ex_i + ex_j), and the guard's: a unit below 2^-60 counts as
-    // that, with nothing for it in S
-    auto fold = [&](int64_t block) {
-        const int* sh = sShift + (block & 1) * 2 * GD_T;
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int o = (4 * x + r) * GD_THREADS;
-                const int d = sh[16 * mt + g4 + 8 * (r >> 1)] + sh[bcol + 8 * (nt + x) + 2 * t4 + (r & 1)];
-                sSum[o] += sum_double(sWhole[o], sPart[o], d + 2);
-                sWhole[o] = 0;
-                sPart[o] = 0;
-                if (s[x][r] > 0.0f) {
-                    const float u = __int_as_float((127 + max(min(d, 0), -60)) << 23);
-                    if (d >= -60) sSize[o] = fmaf(s[x][r], u, sSize[o]);
-                    sUnit[o] = fmaf(u, u, sUnit[o]);
-                }
-                s[x][r] = 0.0f;
-            }
-    };
-    static_assert(GD_SUM <= MAGIC_TERMS && GD_SUM == 2 * GD_ROWS, "exact accumulators");
-    static_assert(GD_BLOCK <= 128, "sum_double's range");
+    static_assert(GD_BLOCK <= MAGIC_TERMS && GD_BLOCK == 2 * GD_ROWS, "exact accumulators");
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
         acc_clear(acc[x]);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int o = (4 * x + r) * GD_THREADS;
-            sSum[o] = 0.0; sWhole[o] = 0; sPart[o] = 0; sSize[o] = sUnit[o] = s[x][r] = 0.0f;
+            sSum[o] = 0;
+            sGuard[o] = make_float2(0.0f, 0.0f);
+            s[x][r] = 0.0f;
         }
     }
     const int nch = ke > kb ? (int)((ke - kb + GD_ROWS - 1) / GD_ROWS) : 0;
@@ -312,9 +298,7 @@ __global__ void __launch_bounds__(GD_THREADS, 1) k_syrk_digits(const double* __r
         if (i + 1 < nch) build(i + 1);
         if (i + 2 < nch) fetch(kb + (int64_t)(i + 2) * GD_ROWS);
         products(i);
-        const int64_t k1 = kb + (int64_t)(i + 1) * GD_ROWS;
-        if ((i & 1) || i + 1 == nch) collect();
-        if (k1 % GD_BLOCK == 0 || i + 1 == nch) fold((k1 - 1) / GD_BLOCK);
+        if ((i & 1) || i + 1 == nch) flush(i >> 1);
         __syncthreads();
     }
     __shared__ int nlist;
@@ -335,8 +319,8 @@ __global__ void __launch_bounds__(GD_THREADS, 1) k_syrk_digits(const double* __r
             if (i < m && j < m && j >= i) {
                 const int ei = ex[i], ej = ex[j];
                 const int o = (4 * x + r) * GD_THREADS;
-                if (sSize[o] >= GD_GUARD * sqrtf(sUnit[o]) && ei != COL_BAD && ej != COL_BAD)
-                    add(i, j, ldexp(sSum[o], ei + ej));
+                if (sGuard[o].x >= GD_GUARD * sqrtf(sGuard[o].y) && ei != COL_BAD && ej != COL_BAD)
+                    add(i, j, int128_double(sSum[o], ei + ej - 70 - GD_FRAC));
                 else
                     list[atomicAdd(&nlist, 1)] = (uint16_t)(li * GD_T + lj);
             }
@@ -939,9 +923,9 @@ void syrk_tn(const double* X, int64_t ldx, int64_t K, int m, double alpha, doubl
 void gram64(const double* X, int64_t ldx, int64_t K, int m, double* C, int64_t ldc, cudaStream_t st) {
     if (K <= 0 || m <= 0) return;
     // Below, the exponent pass and the 512-thread CTAs' start cost what the FP64 products do.
-    // Whole calls, FP64 -> digits: 300 x 400 119 -> 82 us, 1,000 x 200 141 -> 99 us; with entries over
-    // many powers of two, some outputs summed twice, 117 -> 108 and 141 -> 153 us; 1,000 x 100
-    // 90 -> 81 and 87 -> 107 us
+    // Whole calls, FP64 -> digits: 300 x 400 119 -> 79 us, 1,000 x 200 141 -> 91 us; with entries over
+    // many powers of two, some outputs summed twice, 117 -> 91 to 121 and 141 -> 118 to 159 us;
+    // 1,000 x 100 90 -> 78 and 87 -> 89 to 108 us
     if ((double)K * m * m < 4.0e7) {
         syrk_tn(X, ldx, K, m, 1.0, C, ldc, st);
         return;
@@ -950,17 +934,17 @@ void gram64(const double* X, int64_t ldx, int64_t K, int m, double* C, int64_t l
     const int64_t npairs = (int64_t)ntile * (ntile + 1) / 2;
     if (npairs > 0x7fffffffLL) throw std::runtime_error("gram64: matrix too large");
     // K slices (FP64 atomics) where the triangle alone leaves SMs idle: the fewest 32-row
-    // steps on the longest CTA's path, two more per slice for its start and end
-    const int64_t sms = sm_count(), steps = (K + cgd::GD_SUM - 1) / cgd::GD_SUM;
+    // blocks on the longest CTA's path, two more per slice for its start and end
+    const int64_t sms = sm_count(), blocks = (K + cgd::GD_BLOCK - 1) / cgd::GD_BLOCK;
     int64_t nslice = 1, best = -1;
-    for (int64_t sl = 1; sl <= std::min<int64_t>(steps, std::max<int64_t>(1, 8 * sms / npairs)); ++sl) {
-        const int64_t cost = (npairs * sl + sms - 1) / sms * ((steps + sl - 1) / sl + 2);
+    for (int64_t sl = 1; sl <= std::min<int64_t>(blocks, std::max<int64_t>(1, 8 * sms / npairs)); ++sl) {
+        const int64_t cost = (npairs * sl + sms - 1) / sms * ((blocks + sl - 1) / sl + 2);
         if (best < 0 || cost < best) { best = cost; nslice = sl; }
     }
-    const int64_t kslice = (steps + nslice - 1) / nslice * cgd::GD_SUM, blocks = (K + cgd::GD_BLOCK - 1) / cgd::GD_BLOCK;
+    const int64_t kslice = (blocks + nslice - 1) / nslice * cgd::GD_BLOCK;
     nslice = (K + kslice - 1) / kslice;
     int* ex = scratch_alloc<int>(m, st);
-    int16_t* eb = scratch_alloc<int16_t>((size_t)blocks * m, st);   // 1/256 of X
+    int16_t* eb = scratch_alloc<int16_t>((size_t)blocks * m, st);   // 1/128 of X
     ckd(cudaMemsetAsync(ex, 0x80, sizeof(int) * m, st), "column exponents");   // a very small value
     const unsigned strips = (unsigned)((m + 31) / 32);
     const unsigned gy = (unsigned)std::max<int64_t>(1, std::min<int64_t>((blocks + 7) / 8, 8 * sms / strips));

@@ -168,13 +168,18 @@ __device__ __forceinline__ double from_fixed(long long v, int e) {
     return __longlong_as_double((long long)(s | (((unsigned long long)(ex - 1) << 52) + m)));
 }
 
-// (whole + part / 2^16) 2^(e - 56) rounded to FP64, |whole| < 2^61.01, 0 <= part < 2^18: sums of
-// acc_parts over up to 128 terms (2^e times the product of the scaled entries).  The 78 bits are
-// cut to 60 or more of the value's own first.
-__device__ __forceinline__ double sum_double(long long whole, int part, int e) {
-    whole += part >> 16;
-    const int sh = min(16, max(__clzll(whole < 0 ? -whole : whole) - 2, 0));
-    return from_fixed((long long)((unsigned long long)whole << sh) + ((part & 0xffff) >> (16 - sh)), e - 56 - sh);
+// v 2^e rounded to FP64.
+__device__ __forceinline__ double int128_double(__int128 v, int e) {
+    unsigned __int128 a = v < 0 ? -(unsigned __int128)v : (unsigned __int128)v;
+    const unsigned long long hi = (unsigned long long)(a >> 64);
+    if (hi != 0 || (long long)a < 0) {   // to 62 bits and a sticky one
+        const int s = hi != 0 ? 66 - __clzll((long long)hi) : 2;
+        const bool lost = (a & (((unsigned __int128)1 << s) - 1)) != 0;
+        a = (a >> s) | (lost ? 1 : 0);
+        e += s;
+    }
+    const long long m = (long long)a;
+    return from_fixed(v < 0 ? -m : m, e);
 }
 
 }  // namespace cgd

@@ -1,14 +1,15 @@
 """The arithmetic of the FP64 Gram's digit products (csrc/dense64.cu k_syrk_digits,
 csrc/digits.cuh) restated and checked against exact rationals: a power of two per column and
-64-row block, digits, kept diagonals, the integer sums of a block, one rounding to FP64 per
-block, and the guard that gives an output back to FP64 sums.
+32-row block, digits, kept diagonals, the blocks' sums in 128-bit integers, one rounding to
+FP64, and the guard that gives an output back to FP64 sums.
 
 Per term the digit pairs that are not formed are below 7 * 2^14 * 256^-10 * 2^2.01 of the
 product of the two powers of two and the rounding of the entries below 2^-63 of it, together
-2^-60.8; 64 terms lose at most 2^-54.8.  An output passes the guard if S = sum |x y| is at least
-1/64 of the root of the sum of its nb blocks' squared units (1% for S in FP16): the blocks'
-losses are then below sqrt(nb) 64.7 * 2^-54.8 S, and each block's rounding and addition below
-2^-52 (S + loss)."""
+2^-60.8; 32 terms lose at most 2^-55.8 of a block's unit, and shifting out what is below 2^-88
+of the largest powers of two adds 2^-59 of a unit of 2^-29 (smaller ones count as that).  An
+output passes the guard if S = sum |x y| is at least 1/96 of the root of the sum of its nb
+blocks' squared units (1% for S in FP16): the losses are then below sqrt(nb) 97 (2^-55.8 + 2^-59) S
+< sqrt(nb) 2^-49 S, and the rounding is 2^-53 of the result."""
 from fractions import Fraction
 
 import numpy as np
@@ -16,7 +17,7 @@ import pytest
 
 from test_cpu_digit_rows import digits, to_fixed
 
-BLOCK, GUARD = 64, Fraction(1, 64)
+BLOCK, GUARD, FRAC = 32, Fraction(1, 96), 18
 
 
 def exponent(col):
@@ -29,24 +30,25 @@ def exponent(col):
 
 
 def block_sum(x, y, ex, ey):
-    """sum x y of a block over the kept digit pairs, rounded to FP64 in units of 2^(ex + ey)."""
+    """sum x y of a block over the kept digit pairs, in units of 2^(ex + ey - 70)."""
     dx = [digits(to_fixed(v, 63 - ex)) for v in x]
     dy = [digits(to_fixed(v, 63 - ey)) for v in y]
     S = [sum(a[k] * b[D - k] for a, b in zip(dx, dy) for k in range(D + 1)) for D in range(8)]
-    whole, part = 0, 0
-    for lo in range(0, len(x), 32):   # collect(): 32 rows at a time, exact in the accumulators
-        s32 = [sum(a[k] * b[D - k] for a, b in zip(dx[lo:lo + 32], dy[lo:lo + 32]) for k in range(D + 1)) for D in range(8)]
-        assert max(map(abs, s32)) <= 2 ** 22
-        fr = s32[6] * 256 + s32[7]
-        whole += sum(s32[D] << (40 - 8 * D) for D in range(6)) + (fr >> 16)
-        part += fr & 0xFFFF
-    assert whole * 65536 + part == sum(S[D] << (56 - 8 * D) for D in range(8))
-    whole += part >> 16
-    assert abs(whole) < 2 ** 62
-    sh = min(16, max(64 - abs(whole).bit_length() - 2, 0))
-    v = (whole << sh) + ((part & 0xFFFF) >> (16 - sh))
-    assert abs(v) < 2 ** 63
-    return Fraction(float(v)) * Fraction(2) ** (2 - 56 - sh)
+    assert max(map(abs, S)) <= 2 ** 22          # exact in the accumulators
+    fr = S[6] * 256 + S[7]
+    whole = sum(S[D] << (40 - 8 * D) for D in range(6))
+    assert abs(whole) < 2 ** 62 and abs(fr) < 2 ** 31
+    return (whole << 16) + fr
+
+
+def int128_double(v, e):
+    """v 2^e rounded to FP64 by way of 62 bits and a sticky one."""
+    a, s = abs(v), 0
+    if a >= 1 << 63:
+        s = a.bit_length() - 62
+        a = (a >> s) | (1 if a & ((1 << s) - 1) else 0)
+    assert a < 1 << 63
+    return float((-a if v < 0 else a) * Fraction(2) ** (e + s))
 
 
 def output(x, y):
@@ -55,18 +57,20 @@ def output(x, y):
     cut = [slice(b * BLOCK, (b + 1) * BLOCK) for b in range(nb)]
     ex, ey = [exponent(x[c]) for c in cut], [exponent(y[c]) for c in cut]
     tx, ty = max(ex), max(ey)
-    total, size, unit = 0.0, Fraction(0), Fraction(0)
+    total, size, unit = 0, Fraction(0), Fraction(0)
     for c, a, b in zip(cut, ex, ey):
         d = a - tx + b - ty
-        total = total + float(block_sum(x[c], y[c], a, b) * Fraction(2) ** d)
+        v = block_sum(x[c], y[c], a, b)
+        total += v << (d + FRAC) if d >= -FRAC else v >> min(-FRAC - d, 127)
+        assert abs(total) < 2 ** 127
         s = sum(abs(Fraction(float(p)) * Fraction(float(q))) for p, q in zip(x[c], y[c])) / Fraction(2) ** (a + b)
         if s > 0:
-            u = Fraction(2) ** max(d, -60)
-            size += s * u if d >= -60 else 0
+            u = Fraction(2) ** max(d, -29)
+            size += s * Fraction(2) ** d if d >= -60 else 0
             unit += u * u
     exact = sum(Fraction(float(p)) * Fraction(float(q)) for p, q in zip(x, y))
     S = sum(abs(Fraction(float(p)) * Fraction(float(q))) for p, q in zip(x, y))
-    return Fraction(total) * Fraction(2) ** (tx + ty), size * size >= GUARD ** 2 * unit, exact, S
+    return Fraction(int128_double(total, tx + ty - 70 - FRAC)), size * size >= GUARD ** 2 * unit, exact, S
 
 
 def _inputs(kind, rng, K):
@@ -97,10 +101,16 @@ def test_accepted_outputs_are_as_good_as_fp64_sums(kind):
             continue
         accepted += 1
         nb = -(-K // BLOCK)
-        loss = Fraction(int(np.ceil(np.sqrt(nb) * 64.7 * 2 ** 8)), 2 ** 8) * Fraction(2 ** -54.8) * S
-        assert abs(v - exact) <= loss + nb * Fraction(2) ** -52 * (S + loss)
+        loss = Fraction(int(np.ceil(np.sqrt(nb) * 2 ** 8)), 2 ** 8) * Fraction(2) ** -49 * S
+        assert abs(v - exact) <= loss + Fraction(2) ** -53 * (abs(exact) + loss)
     assert accepted == 12 if kind in ("plain", "disjoint") else True
     if kind in ("spike20", "spike40"):
         assert accepted == 0       # the guard sees that S is far below the blocks' units
     if kind == "disjoint":
         assert S == 0 and v == 0
+
+
+@pytest.mark.parametrize("v", [0, 1, -1, 2 ** 62 - 1, 2 ** 62, -(2 ** 63), 2 ** 63 + 2 ** 9, 2 ** 90 + 2 ** 37, 2 ** 90 + 2 ** 37 + 1,
+                               -(2 ** 90 + 3 * 2 ** 37), 2 ** 126 - 1, -(2 ** 127 - 12345)])
+def test_rounding_of_128_bit_sums(v):
+    assert int128_double(v, -88) == float(v * Fraction(2) ** -88)

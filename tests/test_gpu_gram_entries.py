@@ -7,8 +7,8 @@ of up to 30,000 rows.
 Bound: K rounding errors of a sum are at most 2^-53 of a partial sum of |x_ki x_kj| each; taken
 as independent, 8 sqrt(K) 2^-53 S_ij holds with probability 1 - 2 exp(-32) (Higham, Mary, SIAM
 J. Sci. Comput. 41, 2019), S = |A|^T |A|.  The digit sums' own worst case is less: in units
-of a 32-row block's powers of two 32 (7 * 2^14 * 256^-10 * 2 + 2^-63) <= 2^-55.8, with units that add
-up to at most 64 S: 9.2 * 2^-53 S, and K / 32 additions."""
+of a 32-row block's powers of two 32 (7 * 2^14 * 256^-10 * 2^2.01 + 2^-63) <= 2^-55.8, with nb units whose
+root of squares is at most 97 S: below sqrt(nb) 2^-49 S <= 2.9 sqrt(K) 2^-53 S, and one rounding."""
 import importlib
 
 import numpy as np
