@@ -160,7 +160,9 @@ __device__ __forceinline__ bool less_pos(double a, double b) { return __double_a
 
 // Distance from a cut-off within which FP32 Cartesian copies do not decide: the rounding of
 // two positions (2^-24 of their size each, below (layers + 2) times the sum of the cell's
-// entries) and of the distance, times 4, and never above MARGIN.
+// entries) and of the distance, times 4, and never above MARGIN.  The cap is reached at
+// (layers + 2) * sum = 1e4 A (a cubic cell of 1,100 A with one layer) and holds, by the factor
+// of 4, up to 4e4 A; frames have at most 8,191 atoms.
 constexpr float MARGIN = 1.0e-2f;
 __device__ __forceinline__ float frame_margin(const BoxDev& B, int nlayers) {
     float s = 0.0f;

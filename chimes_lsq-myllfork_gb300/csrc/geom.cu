@@ -7,9 +7,9 @@
 //   triplet loops of Cheby::Deriv_3B     src/Cheby.C:981-1054
 //   quadruplet loops of Cheby::Deriv_4B  src/Cheby.C:1387-1500
 //   FCUT::PROCEED                        src/Fcut.C:125-140
-// The reference decides membership with FP64 distances; every candidate is first
-// screened with an FP32 distance (margin 1e-2 A, far above FP32 error) and only
-// candidates near a cut-off are re-decided with the exact FP64 sequence.
+// The reference decides membership with FP64 distances.  An FP32 distance decides where it
+// differs from the cut-off by more than frame_margin (dev.cuh), which is above the rounding of
+// the frame's FP32 positions; nearer, the exact FP64 sequence does.
 #include <cooperative_groups.h>
 
 #include "dev.cuh"
@@ -115,7 +115,7 @@ __device__ __forceinline__ int frame_of_real(const FramesDev& F, int64_t atom) {
 // Forming it for every chunk with a candidate in every pass, dividing by the atom count per
 // ghost and scanning all atoms of a near image took 1.37 of the 1.96 ms of an MD force
 // call on frames of 64, 301, 1111 and 2600 atoms (now 0.16 of 0.66 ms), and 1.38 of 11.3 ms
-// of the FP64 rows of 32 frames of 384 (now 9.9 ms in all).
+// of the FP64 rows of 32 frames of 384 (now 8.9 ms in all).
 constexpr int NEIGH_IMG = 1024;   // images tested for reach (four layers); every image is scanned above
 
 template <bool FILL>
@@ -638,7 +638,6 @@ __global__ void k_quads(ModelDev M, FramesDev F, NeighDev NB, ClusterSet CS, int
 // warps are what helps: 8 frames of 33 to 1,001 atoms, five sorts, one CTA a frame -> a
 // cluster: 919 -> 141 us.
 constexpr int BUCKET_THREADS = 512;
-constexpr int BUCKET_MAX_KEYS = 8192;
 constexpr int BUCKET_SMEM_INTS = 24576;   // per-warp key counts + key totals (96 KB)
 constexpr int BUCKET_U = 4;               // items in flight per lane
 

@@ -594,8 +594,8 @@ __device__ __forceinline__ void oz_tile(int u, int ntj, int& ti, int& tj) {
 // tile's OZ_S column-slice operands into one buffer once the previous tile's MMAs have
 // read it, and its row-slice operands through two slots; warp 1 issues the digit-pair
 // MMAs (M 128, N 64, K 16) into OZ_S TMEM accumulators (diagonal D at columns D x 64:
-// all of TMEM) once the epilogue has drained the previous tile; warps 2..5 (TMEM lane
-// quarter = warp % 4) combine the diagonals, add the tile into C and prefetch the next
+// all of TMEM) once the epilogue has drained the previous tile; warps 2..9 (TMEM lane
+// quarter = warp % 4, half of the columns each) combine the diagonals, add the tile into C and prefetch the next
 // tile's rows of C into L2.  The next tile's operands arrive while this tile's
 // epilogue runs.
 __global__ void __launch_bounds__(OZ_THREADS, 1)

@@ -550,9 +550,8 @@ __global__ void __launch_bounds__(MDC_THREADS) k_mdc_generic(ModelDev M, MdDev D
 }
 
 // ------------------------------------------------------------------ list reuse
-// Clusters of lists enumerated with a skin: keep a cluster this step iff every edge
-// is inside its slot's s_max (the same FP32-then-exact test as the enumeration);
-// type_out[q] = its type or -1.
+// r(a, b) < the cut-off at this step's positions, by the FP32-then-exact test of the
+// enumeration (cutf, cut: its FP32 and FP64 values; mg: frame_margin).
 __device__ __forceinline__ bool within_md(const FramesDev& F, const BoxDev& B, int64_t gb, int a, int b, float cutf,
                                           const double* cut, float mg) {
     const float4* c32 = reinterpret_cast<const float4*>(F.cart32);
@@ -673,8 +672,8 @@ __global__ void k_md_sorted(int64_t n, int nframes, const int64_t* cfo, const in
     if (at % MDC_TILE == 0) B.tile_key[B.tile_ofs[key] + at / MDC_TILE] = key;
 }
 
-// The clusters inside their cut-offs at this step's positions, appended to their key's
-// place: the lists are sorted by key, so a warp makes one or two atomic additions, and
+// Of lists enumerated with a skin the clusters whose every edge is inside its slot's s_max
+// at this step's positions, appended to their key's place: the lists are sorted by key, so a warp makes one or two atomic additions, and
 // each key has room for all its clusters, so no count and scan come first (these, a scatter
 // and a memset, took 31 of 340 us of a step of four frames of 96 to 1,024 atoms).
 template <int NBODY>

@@ -74,7 +74,10 @@ void launch_mdc(int nbody, int prec, int order, int64_t max_tiles, const ModelDe
                 cudaStream_t st);
 // The FP64 contraction on the tensor cores (md_tensor.cu), for the orders of
 // md_tensor_order: tables of a coefficient set (md_tensor_bytes bytes and
-// md_tensor_exponents ints per type), then the force pass as launch_mdc.
+// md_tensor_exponents ints per type), then the force pass as launch_mdc.  Its tables, staged
+// digits and unrolled sums are laid out for one order of each body (64 x 8 and 64 x 64
+// coefficients, the tensor pipe's tiles without padding): the orders of the usual bases.
+// Others keep k_mdc, one thread per cluster.
 constexpr int mdt_order(int nbody) { return nbody == 3 ? 8 : 4; }
 inline bool md_tensor_order(int nbody, int order) { return order == mdt_order(nbody); }
 size_t md_tensor_bytes(int nbody, int ntypes);

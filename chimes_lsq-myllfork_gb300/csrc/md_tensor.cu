@@ -11,8 +11,8 @@
 // coefficients are set), so the FP64 pipe is left with the bases and the halves: about
 // 1,400 of the 11,000 operations per quadruplet.  One thread per cluster walked the whole
 // tensor before: 1,000 C/H/N/O atoms, quadruplets 907 -> 222 us, triplets 285 -> 179 us;
-// 64 atoms 500 -> 59 us and 93 -> 36 us (a whole force call 1.15 -> 0.71 ms and 1.33 ->
-// 0.95 ms).  What remains is the FP64 pipe's: the bases, one exp and about 150 operations
+// 64 atoms 500 -> 59 us and 93 -> 36 us (whole force calls took 1.38 and 1.34 ms with that
+// form and take 0.66 and 0.60 now, lists and allocation included).  What remains is the FP64 pipe's: the bases, one exp and about 150 operations
 // per edge.
 #include <algorithm>
 

@@ -1,4 +1,4 @@
-// Many-body A rows as exact digit products on the tensor cores.
+// Many-body A rows as digit products on the tensor cores.
 //
 // Reference: Cheby::Deriv_3B / Deriv_4B (src/Cheby.C:880-1729).  As in assemble.cu, the
 // derivative sum of a power tuple factorises over the slots incident to the owner and
@@ -10,9 +10,14 @@
 // against 11,600).  The products run on mma.sync: a contraction sums a few to a few
 // hundred clusters, far below what fills a tcgen05 pipeline, and its accumulators are
 // wanted in registers at once to be packed into integers.  16 frames of 256 C/H/N/O
-// atoms (4-body, 7,800 rows x 51,209) 36.8 -> 14.8 ms, 32 frames of 384 water atoms
-// (3-body, 820 columns) 22.5 -> 9.0 ms; the error against 64-bit references is that of
-// the FP64 forms (2.2e-14 and 4.8e-14 of the norm, the references' own rounding among it).
+// atoms (4-body, 7,800 rows x 51,209) 36.5 -> 15.5 ms, 32 frames of 384 water atoms
+// (3-body, 820 columns) 22.4 -> 8.95 ms.
+//
+// A group (an owner's clusters of a type, or a frame's share of them) has one exponent, so the
+// digits' loss, 2^-61 of the group's largest product, is the same for all its columns.  The bases
+// have errors of 2^-53 of a cluster's largest value themselves: against long double the rows'
+// errors are those of the FP64 forms (quadruplets of 90 C/H atoms 2.5e-15 of the column's largest
+// entry, both; INVRSE_R 5.2e-16 -> 5.5e-16).  Bases without a bound (CONSTANT_DERIV) are left out.
 //
 // Column sums: PARAM_INDICES puts powers that permutations of equal atoms exchange
 // into one column, so a cluster may be taken with two of its equal atoms exchanged; the
